@@ -4,142 +4,359 @@
 // logits for that purpose (csrc/qwen3_step.cu:175 writes them, qwen3mk/kernel.py:44-50 returns them).  This is
 // that next step on the GPU, so that a sampled token can feed the following launch without a trip to the host.
 //
-// One block of 1024 threads per row; every pass streams the row (593 KB for the full vocabulary, L2 resident after
-// the first pass):
-//   1. the row maximum, together with the first histogram of
-//   2. top-k: the k-th largest logit by a radix select over the order-preserving integer image of the floats
-//      (three passes of 11, 11 and 10 bits, a histogram in shared memory each; coalesced, strided reads); every
-//      logit >= that value is kept, so ties at the threshold are all kept;
-//   3. weights w_i = exp((l_i - max) / T) of the kept logits, summed per thread over a contiguous chunk of the
-//      row (index order matters from here on), then scanned over the block;
+// A CLUSTER of blocks per row: block r of C owns a contiguous slice of the row, warp w of it a contiguous run of the
+// slice, so that sums over (block, warp, group of 32) follow the index order and every load is coalesced.  What the
+// blocks of a row have to agree on travels through distributed shared memory, one cluster barrier each:
+//   1. every block finds its maximum (lowest index on ties);
+//   2. top-k: a block whose threads have at least k elements bins its THREADS' maxima linearly between the smallest and
+//      the largest of them; the bins that hold the k largest maxima bound its own k largest elements from below, so the
+//      few elements at or above that bound (about 1.1 k of them) are the block's candidates.  The union of all blocks'
+//      candidates contains the row's k largest; every block selects the k-th largest key among them (binary search over
+//      the bits of the keys, held in registers).  A row whose candidates do not fit (large k, many equal values) goes
+//      through a radix select instead: three passes of 11, 11 and 10 bits over the order-preserving integer image of the
+//      floats, histograms summed over the cluster.  Every logit >= the k-th value is kept, so ties are all kept;
+//   3. weights w_i = exp((l_i - max) / T) of the kept logits, summed per warp, per block and over the row;
 //   4. the token is the first index whose inclusive prefix sum exceeds u * total, u in [0, 1) supplied per row
-//      by the caller (a seeded generator on the host side keeps runs reproducible); the thread whose chunk
-//      brackets the target walks its chunk in the same order it summed it.
+//      by the caller (a seeded generator on the host side keeps runs reproducible); the block whose warps' runs
+//      bracket the target walks that run, a thread an element.
 // T <= 0 or k == 1 degenerate to the arg-max (ties -> lowest index), like the decode kernels.
+//
+// A single row is bound by latency (0.6 MB, but a dozen dependent block-wide steps), a full batch by the row's bytes.  One
+// block of 1024 threads per row, as this kernel was before, left 147 SMs idle at one row and walked the 2048 bins of each
+// radix pass with one thread: 1 row, k = 50: 165 us, now 14; 64 rows, whole vocabulary: 70 us, now 25.
+#include <cooperative_groups.h>
+
 #include "q3_engine.h"
+
+namespace cg = cooperative_groups;
 
 namespace q3 {
 
 constexpr int SAMPLE_THREADS = 1024;
+constexpr int SAMPLE_WARPS = SAMPLE_THREADS / 32;
+constexpr int SAMPLE_MAX_CLUSTER = 16;
+constexpr int SAMPLE_BINS = 2048;
+constexpr int SAMPLE_CAND = 1024;     // candidates a block publishes
+constexpr int SAMPLE_KEYS = 4;        // candidates of all blocks a thread holds in the search: 4096 in all
 
 __device__ __forceinline__ unsigned ordered_key(float f) {   // monotonic in the float's value
     const unsigned b = __float_as_uint(f);
     return b ^ ((b >> 31) ? 0xffffffffu : 0x80000000u);
 }
 
-__global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const float* __restrict__ logits, int vocab, float temperature, int top_k,
-                                                               const float* __restrict__ uniform, long long* __restrict__ out) {
-    __shared__ float s_f[SAMPLE_THREADS];
-    __shared__ int s_i[SAMPLE_THREADS];
-    __shared__ unsigned s_hist[2048];
-    __shared__ unsigned s_prefix, s_need;
-    __shared__ float s_total;
-    __shared__ int s_pick;
-    const int tid = threadIdx.x, row_id = blockIdx.x;
+__device__ __forceinline__ float key_value(unsigned k) { return __uint_as_float((k >> 31) ? k ^ 0x80000000u : ~k); }   // the inverse
+
+// elements of a warp's run when a row of `vocab` words goes to `cluster` blocks
+__host__ __device__ inline int sample_run(int vocab, int cluster) {
+    return ((vocab + cluster * SAMPLE_WARPS - 1) / (cluster * SAMPLE_WARPS) + 127) / 128 * 128;
+}
+
+struct SampleShared {
+    float bmax[SAMPLE_MAX_CLUSTER];         // per block of the cluster: its maximum, ...
+    int bidx[SAMPLE_MAX_CLUSTER];           // ... where it is, ...
+    int ncand[SAMPLE_MAX_CLUSTER];          // ... how many candidates it has (-1: they did not fit), ...
+    float bsum[SAMPLE_MAX_CLUSTER];         // ... and the sum of its weights
+    float wf[SAMPLE_WARPS], wg[SAMPLE_WARPS];
+    int wi[SAMPLE_WARPS];
+    unsigned wcount[2][SAMPLE_WARPS];
+    unsigned hist[SAMPLE_BINS];
+    unsigned cand[SAMPLE_CAND];             // keys
+    unsigned sel, need, cand_n;
+};
+
+// Block-wide: the bin, counted from the largest, in which the running count of hist[] reaches `need`, and what is still
+// needed inside it (sh.sel, sh.need).  from_top: bins run from SAMPLE_BINS - 1 down, else from 0 up.
+__device__ __forceinline__ void find_bin(SampleShared& sh, unsigned c0, unsigned c1, unsigned need, bool from_top) {
+    // thread t holds the counts of the bins of rank 2 t and 2 t + 1 in walking order
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned mine = c0 + c1;
+    unsigned incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) sh.wcount[0][warp] = incl;
+    if (tid == 0) { sh.sel = from_top ? 0u : (unsigned)SAMPLE_BINS - 1u; sh.need = need; }   // (fewer than `need` keys in all: everything)
+    __syncthreads();
+    const unsigned w = sh.wcount[0][lane];
+    unsigned before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u) + incl - mine;
+    if (before < need && before + mine >= need) {
+        const bool second = before + c0 < need;
+        const int rank = 2 * tid + (second ? 1 : 0);
+        if (second) before += c0;
+        sh.sel = (unsigned)(from_top ? SAMPLE_BINS - 1 - rank : rank);
+        sh.need = need - before;
+    }
+    __syncthreads();
+}
+
+// Elements are dealt out in groups of 128 per warp, four neighbours a lane: element 4 lane + q of group j.  NQ > 0: a thread's
+// elements of the row (at most NQ groups) stay in registers; NQ == 0: every pass reads the row again (from L2).
+template <int NQ>
+__global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(const float* __restrict__ logits, int vocab, float temperature, int top_k,
+                                                                             const float* __restrict__ uniform, long long* __restrict__ out) {
+    __shared__ SampleShared sh;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row_id = blockIdx.x / C;
     const float* row = logits + (size_t)row_id * vocab;
-    const int chunk = (vocab + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
-    const int i0 = min(vocab, tid * chunk), i1 = min(vocab, i0 + chunk);
-    const bool select = top_k > 1 && top_k < vocab && temperature > 0.f;
+    // warp w of block r: elements [i0, i1), `per` of them but for the last runs of the row
+    const int per = sample_run(vocab, C);
+    const int i0 = (int)min((long long)vocab, (long long)(rank * SAMPLE_WARPS + warp) * per), i1 = min(vocab, i0 + per);
+    const bool greedy = !(temperature > 0.f) || top_k == 1;
+    const bool select = !greedy && top_k > 1 && top_k < vocab;
+    const bool vec = ((vocab & 3) | (int)(reinterpret_cast<uintptr_t>(logits) & 15)) == 0;
+    cluster.barrier_arrive();   // (a peer's shared memory may be written once the peer runs: waited for before the first exchange)
 
-    // ---- 1. maximum (and its lowest index); the histogram of the keys' top 11 bits on the side ----
-    for (int b = tid; b < 2048; b += SAMPLE_THREADS) s_hist[b] = 0u;
-    __syncthreads();
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int i = tid; i < vocab; i += SAMPLE_THREADS) {
-        const float v = row[i];
-        if (v > bv) { bv = v; bi = i; }   // a thread's indices ascend: the first maximum is the lowest
-        if (select) atomicAdd(&s_hist[ordered_key(v) >> 21], 1u);
+    auto fetch = [&](int j) -> float4 {  // group j; elements past the run are -inf, which no pass below counts
+        const int i = i0 + 128 * j + 4 * lane;
+        if (vec && i + 3 < i1) return *reinterpret_cast<const float4*>(row + i);
+        float4 v;
+        v.x = i < i1 ? row[i] : -INFINITY; v.y = i + 1 < i1 ? row[i + 1] : -INFINITY;
+        v.z = i + 2 < i1 ? row[i + 2] : -INFINITY; v.w = i + 3 < i1 ? row[i + 3] : -INFINITY;
+        return v;
+    };
+    float4 x[NQ > 0 ? NQ : 1];
+    if constexpr (NQ > 0) {
+#pragma unroll
+        for (int j = 0; j < NQ; ++j) x[j] = fetch(j);
     }
-    s_f[tid] = bv; s_i[tid] = bi;
-    __syncthreads();
-    for (int o = SAMPLE_THREADS / 2; o > 0; o >>= 1) {
-        if (tid < o) {
-            const float v = s_f[tid + o];
-            const int ix = s_i[tid + o];
-            if (v > s_f[tid] || (v == s_f[tid] && ix < s_i[tid])) { s_f[tid] = v; s_i[tid] = ix; }
+    const int groups = (i1 - i0 + 127) / 128, whole = vec ? (i1 - i0) / 128 : 0;
+    auto each = [&](auto&& f) {          // f(index, value) over this thread's elements, in ascending order
+        auto four = [&](int j, const float4& v) {
+            const int i = i0 + 128 * j + 4 * lane;
+            f(i, v.x); f(i + 1, v.y); f(i + 2, v.z); f(i + 3, v.w);
+        };
+        if constexpr (NQ > 0) {
+#pragma unroll
+            for (int j = 0; j < NQ; ++j) four(j, x[j]);
+        } else {
+            int j = 0;
+            for (; j + 4 <= whole; j += 4) {       // (no guards: the four loads leave together)
+                float4 v[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = *reinterpret_cast<const float4*>(row + i0 + 128 * (j + q) + 4 * lane);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) four(j + q, v[q]);
+            }
+            for (; j < groups; ++j) four(j, fetch(j));
         }
-        __syncthreads();
-    }
-    const float vmax = s_f[0];
-    const int imax = s_i[0];
-    __syncthreads();
-    if (!(temperature > 0.f) || top_k == 1) {
-        if (tid == 0) out[row_id] = imax;
-        return;
-    }
+    };
 
-    // ---- 2. threshold: the k-th largest key (0 keeps everything) ----
-    unsigned thresh = 0u;
+    // ---- 1. the block's maximum, and the smallest of its threads' maxima ----
+    const bool any = i0 + 4 * lane < i1;
+    float mine = -INFINITY;
+    each([&](int, float v) { mine = fmaxf(mine, v); });
+    {
+        const float bv = warp_max(mine), lo = -warp_max(any ? -mine : -INFINITY);
+        if (lane == 0) { sh.wf[warp] = bv; sh.wg[warp] = lo; }
+    }
+    if (select)
+        for (int b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) sh.hist[b] = 0u;
+    if (tid == 0) { sh.cand_n = 0u; sh.need = 0x7fffffffu; }
+    const int n_thr = __syncthreads_count(any);     // threads that have an element
+    const float bmax = warp_max(sh.wf[lane]), blo = -warp_max(-sh.wg[lane]);
+
+    // ---- 2a. the block's candidates for the k largest ----
+    int n_cand = -1;
     if (select) {
-        if (tid == 0) { s_prefix = 0u; s_need = (unsigned)top_k; }
-        __syncthreads();
-        // digit d of a key: bits [shift, shift + width)
-        for (int pass = 0; pass < 3; ++pass) {
-            const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : 0), width = pass == 2 ? 10 : 11;
-            const unsigned prefix = s_prefix;
-            if (pass > 0) {
-                for (int b = tid; b < 2048; b += SAMPLE_THREADS) s_hist[b] = 0u;
-                __syncthreads();
-                const unsigned mask = 0xffffffffu << (shift + width);
-                for (int i = tid; i < vocab; i += SAMPLE_THREADS) {
-                    const unsigned k = ordered_key(row[i]);
-                    if ((k & mask) == prefix) atomicAdd(&s_hist[(k >> shift) & ((1u << width) - 1u)], 1u);
-                }
-                __syncthreads();
-            }
-            if (tid == 0) {   // walk the bins from the top until `need` keys are covered
-                unsigned need = s_need, b = (1u << width) - 1u;
-                for (;; --b) {
-                    const unsigned n = s_hist[b];
-                    if (n >= need || b == 0u) break;
-                    need -= n;
-                }
-                s_need = need;
-                s_prefix = prefix | (b << shift);
-            }
+        const float scale = (float)(SAMPLE_BINS - 1) / (bmax - blo);
+        auto bin = [&](float v) -> int {            // non-increasing in v; anything odd (an infinite range) lands inside the bounds
+            const float d = (bmax - v) * scale;
+            return d >= 0.f ? (int)fminf(d, (float)(SAMPLE_BINS - 1)) : 0;
+        };
+        if (top_k <= n_thr) {
+            if (any) atomicAdd(&sh.hist[bin(mine)], 1u);
             __syncthreads();
+            find_bin(sh, sh.hist[2 * tid], sh.hist[2 * tid + 1], (unsigned)top_k, false);
+            const int last = (int)sh.sel;
+            if (any && bin(mine) <= last)           // (a thread whose maximum is below the bound has no candidate)
+                each([&](int i, float v) {
+                    if (bin(v) <= last && i < i1) {
+                        const unsigned n = atomicAdd(&sh.cand_n, 1u);
+                        if (n < SAMPLE_CAND) sh.cand[n] = ordered_key(v);
+                    }
+                });
+        } else {
+            // fewer threads with elements than k: every element is a candidate, if they fit
+            const int s0 = rank * SAMPLE_WARPS * per, slice = min(vocab, s0 + SAMPLE_WARPS * per) - min(vocab, s0);
+            if (slice <= SAMPLE_CAND)
+                each([&](int i, float v) { if (i < i1) sh.cand[i - s0] = ordered_key(v); });
+            if (tid == 0) sh.cand_n = (unsigned)slice;
         }
-        thresh = s_prefix;
-    }
-
-    // ---- 3. weights of the kept logits: per-thread chunk sums, then a scan over the block ----
-    const float inv_t = 1.f / temperature;
-    float mine = 0.f;
-    for (int i = i0; i < i1; ++i) {
-        const float v = row[i];
-        if (ordered_key(v) >= thresh) mine += __expf((v - vmax) * inv_t);
-    }
-    s_f[tid] = mine;
-    __syncthreads();
-    // inclusive scan (Hillis-Steele over 1024 entries)
-    for (int o = 1; o < SAMPLE_THREADS; o <<= 1) {
-        const float add = (tid >= o) ? s_f[tid - o] : 0.f;
         __syncthreads();
-        s_f[tid] += add;
-        __syncthreads();
+        n_cand = sh.cand_n <= SAMPLE_CAND ? (int)sh.cand_n : -1;
     }
-    if (tid == SAMPLE_THREADS - 1) { s_total = s_f[tid]; s_pick = -1; }
-    __syncthreads();
+    cluster.barrier_wait();
+    if (tid < C) {
+        SampleShared* peer = cluster.map_shared_rank(&sh, tid);
+        peer->bmax[rank] = bmax; peer->ncand[rank] = n_cand;
+    }
+    cluster.sync();
+    float vmax = sh.bmax[0];
+    for (int r = 1; r < C; ++r) vmax = fmaxf(vmax, sh.bmax[r]);
+    // the row's lowest index that holds the maximum (every block of the cluster takes part)
+    auto write_argmax = [&]() {
+        __syncthreads();
+        if (tid == 0) sh.need = 0x7fffffffu;
+        __syncthreads();
+        if (mine == vmax) {
+            int first = 0x7fffffff;
+            each([&](int i, float v) { if (v == vmax && i < i1) first = min(first, i); });
+            atomicMin(&sh.need, (unsigned)first);
+        }
+        __syncthreads();
+        if (tid == 0) cluster.map_shared_rank(&sh, 0)->bidx[rank] = (int)sh.need;
+        cluster.sync();
+        if (rank == 0 && tid == 0) {
+            int best = sh.bidx[0];
+            for (int r = 1; r < C; ++r) best = min(best, sh.bidx[r]);
+            out[row_id] = best < vocab ? best : 0;  // (a row of NaNs has no maximum)
+        }
+    };
+    if (greedy) { write_argmax(); return; }
 
-    // ---- 4. the first index whose inclusive prefix exceeds u * total ----
-    const float target = uniform[row_id] * s_total;
-    const float before = tid ? s_f[tid - 1] : 0.f;   // the scanned prefixes partition [0, total) exactly
-    if (mine > 0.f && before <= target && target < s_f[tid]) {
-        float run = before;
-        int pick = -1, last_kept = -1;
-        for (int i = i0; i < i1; ++i) {
-            const float v = row[i];
-            if (ordered_key(v) >= thresh) {
-                run += __expf((v - vmax) * inv_t);
-                last_kept = i;
-                if (run > target) { pick = i; break; }
+    // ---- 2b. threshold: the k-th largest key (-inf keeps everything) ----
+    float kth = -INFINITY;
+    // (`select` spelled out: nvcc 12.9 lost the branch when it reused the flag from above)
+    if (top_k > 1 && top_k < vocab) {
+        bool fits = true;
+        int total = 0;
+        for (int r = 0; r < C; ++r) { fits = fits && sh.ncand[r] >= 0; total += max(sh.ncand[r], 0); }
+        fits = fits && total <= SAMPLE_KEYS * SAMPLE_THREADS;
+        if (fits) {
+            // this thread's share of the union: the blocks' lists one after the other (0 is below every key of a number)
+            unsigned key[SAMPLE_KEYS];
+#pragma unroll
+            for (int q = 0; q < SAMPLE_KEYS; ++q) {
+                int e = q * SAMPLE_THREADS + tid, r = 0;
+                key[q] = 0u;
+                if (e < total) {
+                    while (e >= sh.ncand[r]) e -= sh.ncand[r++];
+                    key[q] = cluster.map_shared_rank(&sh, r)->cand[e];
+                }
             }
+            const bool one = total <= SAMPLE_THREADS;
+            unsigned t = 0u;
+            for (int bit = 31; bit >= 0; --bit) {   // the largest t with at least k keys >= t
+                const unsigned trial = t | (1u << bit);
+                unsigned n;
+                if (one) n = (unsigned)__syncthreads_count(key[0] >= trial);
+                else {
+                    unsigned c = 0;
+#pragma unroll
+                    for (int q = 0; q < SAMPLE_KEYS; ++q) c += key[q] >= trial ? 1u : 0u;
+                    c = __reduce_add_sync(0xffffffffu, c);
+                    if (lane == 0) sh.wcount[bit & 1][warp] = c;
+                    __syncthreads();                // (two buffers: the next round's writers cannot overtake this one's readers)
+                    n = __reduce_add_sync(0xffffffffu, sh.wcount[bit & 1][lane]);
+                }
+                if (n >= (unsigned)top_k) t = trial;
+            }
+            kth = key_value(t);
+        } else {
+            unsigned prefix = 0u, need = (unsigned)top_k;
+            for (int pass = 0; pass < 3; ++pass) {
+                const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : 0), width = pass == 2 ? 10 : 11;
+                const unsigned mask = pass == 0 ? 0u : 0xffffffffu << (shift + width);
+                for (int b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) sh.hist[b] = 0u;
+                __syncthreads();
+                each([&](int i, float v) {
+                    const unsigned k = ordered_key(v);
+                    if (i < i1 && (k & mask) == prefix) atomicAdd(&sh.hist[(k >> shift) & ((1u << width) - 1u)], 1u);
+                });
+                cluster.sync();
+                unsigned c0 = 0u, c1 = 0u;          // bins SAMPLE_BINS - 1 - 2 tid and the one below it, over the cluster
+                for (int r = 0; r < C; ++r) {
+                    const unsigned* h = cluster.map_shared_rank(&sh, r)->hist;
+                    c0 += h[SAMPLE_BINS - 1 - 2 * tid]; c1 += h[SAMPLE_BINS - 2 - 2 * tid];
+                }
+                find_bin(sh, c0, c1, need, true);
+                prefix |= sh.sel << shift;
+                need = sh.need;
+                cluster.sync();                     // every block has read this pass's histograms
+            }
+            kth = key_value(prefix);
         }
-        s_pick = pick >= 0 ? pick : last_kept;   // rounding may leave the target a hair beyond the chunk's own sum
     }
+
+    // ---- 3. weights of the kept logits: sums per warp, per block, over the row, in index order ----
+    const float inv_t = 1.f / temperature;
+    float ws = 0.f;
+    each([&](int, float v) { if (v >= kth) ws += __expf((v - vmax) * inv_t); });
+    ws = warp_sum(ws);
     __syncthreads();
-    if (tid == 0) out[row_id] = s_pick >= 0 ? s_pick : imax;   // u * total rounded up to the total: the mode is as good a token as any
+    if (lane == 0) sh.wf[warp] = ws;
+    __syncthreads();
+    float lo = 0.f, hi = 0.f, bsum = 0.f;           // this warp's bracket inside the block, and the block's sum
+    for (int w = 0; w < SAMPLE_WARPS; ++w) {        // (the same order everywhere: brackets meet without gaps)
+        if (w == warp) lo = bsum;
+        bsum += sh.wf[w];
+        if (w == warp) hi = bsum;
+    }
+    if (tid < C) cluster.map_shared_rank(&sh, tid)->bsum[rank] = bsum;
+    cluster.sync();
+    float base = 0.f, next = 0.f, total = 0.f;      // the block's bracket and the total
+    for (int r = 0; r < C; ++r) {
+        if (r == rank) base = total;
+        total += sh.bsum[r];
+        if (r == rank) next = total;
+    }
+    // ---- 4. the first index whose inclusive prefix exceeds u * total ----
+    if (!(total > 0.f && total < INFINITY)) { write_argmax(); return; }     // infinite logits: the weights are not numbers
+    float target = uniform[row_id] * total;
+    if (!(target < total)) target = __uint_as_float(__float_as_uint(total) - 1u);   // u * total rounded up to the total: the last word with a weight
+    if (!(base <= target && target < next)) return;
+    // Inside the block: base + lo of the first warp is base, base + hi of the last one is next, and both are the same sums for
+    // the neighbouring warps, so exactly one warp's run takes it.  The whole block walks that run, 1024 elements a round.
+    if (lane == 0 && base + lo <= target && target < base + hi) { sh.sel = (unsigned)warp; sh.wg[0] = base + lo; }
+    if (tid == 0) { sh.need = 0xffffffffu; sh.cand_n = 0u; }
+    __syncthreads();
+    const int r0 = (rank * SAMPLE_WARPS + (int)sh.sel) * per, r1 = min(vocab, r0 + per);
+    float run = sh.wg[0];
+    for (int first = r0; first < r1; first += SAMPLE_THREADS) {
+        const int i = first + tid;
+        const float v = i < r1 ? row[i] : -INFINITY;
+        const bool kept = i < r1 && v >= kth;
+        float incl = kept ? __expf((v - vmax) * inv_t) : 0.f;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float p = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += p;
+        }
+        if (lane == 31) sh.wf[warp] = incl;
+        __syncthreads();
+        float before = run;
+        for (int w = 0; w < SAMPLE_WARPS; ++w) {
+            if (w == warp) before = run;
+            run += sh.wf[w];
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, kept && before + incl > target), all = __ballot_sync(0xffffffffu, kept);
+        if (lane == 0 && hit) atomicMin(&sh.need, (unsigned)(first + 32 * warp + __ffs(hit) - 1));
+        if (lane == 0 && all) atomicMax(&sh.cand_n, (unsigned)(first + 32 * warp + 31 - __clz(all)));
+        __syncthreads();
+        if (sh.need != 0xffffffffu) break;
+    }
+    // rounding may leave the target a hair beyond the run's own sum: then its last kept element
+    if (tid == 0) out[row_id] = sh.need != 0xffffffffu ? (long long)sh.need : (long long)sh.cand_n;
+}
+
+template <int NQ>
+static cudaError_t launch_sample(int cluster, const float* logits, int batch, int vocab, float temperature, int top_k, const float* uniform,
+                                 long long* out, cudaStream_t st) {
+    if (cluster > 8) {   // sizes above 8 are opt-in, per device and function (setting it again changes nothing)
+        const cudaError_t e = cudaFuncSetAttribute(sample_kernel<NQ>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)batch * (unsigned)cluster); cfg.blockDim = dim3(SAMPLE_THREADS); cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, sample_kernel<NQ>, logits, vocab, temperature, top_k, uniform, out);
 }
 
 }  // namespace q3
@@ -149,9 +366,20 @@ extern "C" int q3_sample(const float* logits, int32_t batch, int32_t vocab, floa
     if (!logits || !out_tokens) return q3::engine_fail(nullptr, Q3_ERR_INVALID, "q3_sample: logits and out_tokens are required");
     if (batch < 1 || vocab < 1 || top_k < 0) return q3::engine_fail(nullptr, Q3_ERR_INVALID, "q3_sample: batch=%d vocab=%d top_k=%d out of range", batch, vocab, top_k);
     if (temperature > 0.f && top_k != 1 && !uniform) return q3::engine_fail(nullptr, Q3_ERR_INVALID, "q3_sample: sampling needs one uniform number per row");
-    q3::sample_kernel<<<batch, q3::SAMPLE_THREADS, 0, (cudaStream_t)stream>>>(logits, vocab, temperature, top_k, uniform,
-                                                                              reinterpret_cast<long long*>(out_tokens));
-    const cudaError_t err = cudaGetLastError();
+    // Blocks per row: as many as keep all rows' clusters resident at once, and at least 1024 words a block.  Measured with the
+    // full vocabulary and a cold L2, us with clusters of 1 / 2 / 4 / 8 / 16 blocks: 1 row, k = 50: 42.9 / 32.8 / 24.8 / 18.5 /
+    // 18.5; 8 rows, k = 50: 45 / 33 / 26.5 / 20.4 / 30.7; 16 rows, k = 50: 47 / 35 / 26.6 / 32.7 / 43; 33 rows, all words:
+    // 37 / 27 / 22.5 / 28.7 / 41; 64 rows, all words: 39 / 30.7 / 30.8 / 43 / 72; 64 rows, k = 50: 49 / 38.7 / 41 / 70 / 125.
+    // A thread keeps its elements in registers where it has at most three groups of four, or five.
+    int cluster = batch <= 4 ? 16 : batch <= 14 ? 8 : batch <= 48 ? 4 : batch <= 148 ? 2 : 1;
+    while (cluster > 1 && vocab < cluster * q3::SAMPLE_THREADS) cluster /= 2;
+    const int groups = q3::sample_run(vocab, cluster) / 128;
+    cudaStream_t st = (cudaStream_t)stream;
+    long long* out = reinterpret_cast<long long*>(out_tokens);
+    cudaError_t err;
+    if (groups <= 3) err = q3::launch_sample<3>(cluster, logits, batch, vocab, temperature, top_k, uniform, out, st);
+    else if (groups <= 5) err = q3::launch_sample<5>(cluster, logits, batch, vocab, temperature, top_k, uniform, out, st);
+    else err = q3::launch_sample<0>(cluster, logits, batch, vocab, temperature, top_k, uniform, out, st);
     if (err != cudaSuccess) return q3::engine_fail(nullptr, Q3_ERR_CUDA, "q3_sample: %s", cudaGetErrorString(err));
     return Q3_OK;
 }

@@ -105,3 +105,44 @@ def test_sampled_stream_feeds_the_next_launch(oracle):
         sampling.sample(out2["logits"], 0.9, 40, generator=gen, out=dev2["token"])
         toks2.append(int(dev2["token"]))
     assert toks2 == toks
+
+
+@pytest.mark.parametrize("vocab,batch", [(1, 2), (31, 1), (2047, 3), (2049, 1), (32768, 1), (32769, 9), (151936, 17), (151937, 65)])
+@pytest.mark.parametrize("top_k", [0, 2, 64, 5000])
+def test_every_split_of_a_row_over_blocks(vocab, batch, top_k):
+    """Rows on 1, 2, 4, 8 and 16 blocks, elements in registers or re-read, runs that end inside a block: fp64 rule, as above."""
+    from qwen3mk import sampling
+
+    g = torch.Generator().manual_seed(vocab * 7 + batch + top_k)
+    logits = torch.randn(batch, vocab, generator=g) * 3.0
+    logits[0, vocab // 2:] = float("-inf") if vocab > 1 else 0.0      # half the words of a row masked out
+    u = torch.rand(batch, generator=g)
+    got = sampling.sample(logits.cuda(), 0.9, top_k, u=u.cuda()).cpu()
+    keep, prob = exact(logits, 0.9, top_k)
+    cdf = prob.cumsum(dim=-1)
+    for b in range(batch):
+        j = int(got[b])
+        assert 0 <= j < vocab and bool(keep[b, j])
+        lo = float(cdf[b, j - 1]) if j else 0.0
+        assert lo - CDF_TOL <= float(u[b]) <= float(cdf[b, j]) + CDF_TOL
+    assert sampling.sample(logits.cuda(), 0.0, 0).cpu().tolist() == logits.argmax(dim=-1).tolist()
+
+
+@pytest.mark.parametrize("top_k", [3, 700, 9000])
+def test_thousands_of_equal_logits_at_the_threshold_are_all_kept(top_k):
+    """More candidates than a block publishes: the radix select decides.  Two larger words and 10000 equal ones."""
+    from qwen3mk import sampling
+
+    vocab = 40000
+    logits = torch.full((1, vocab), -4.0)
+    logits[0, 5000:15000] = 1.0
+    logits[0, [123, 39999]] = 2.0
+    keep, prob = exact(logits, 1.0, top_k)
+    assert int(keep.sum()) == 10002
+    cdf = prob.cumsum(dim=-1)[0]
+    u = torch.linspace(0.001, 0.999, 50)
+    got = sampling.sample(logits.repeat(50, 1).cuda(), 1.0, top_k, u=u.cuda()).cpu()
+    for b in range(50):
+        j = int(got[b])
+        assert bool(keep[0, j])
+        assert (float(cdf[j - 1]) if j else 0.0) - CDF_TOL <= float(u[b]) <= float(cdf[j]) + CDF_TOL
