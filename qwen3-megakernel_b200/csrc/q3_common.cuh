@@ -99,6 +99,16 @@ __device__ __forceinline__ void ld_row8(uint32_t& a, uint32_t& b, const void* pt
                  : "=&r"(a), "=&r"(b) : "l"(ptr), "r"((int)live));
 }
 
+// One lane of a converged warp.  A branch on elect.sync tells the compiler that exactly one thread follows it; behind
+// `lane == 0` it has to make every tcgen05 and TMA instruction's descriptors warp-uniform at run time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+// the warp's index as a value the compiler knows to be uniform
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // ---- programmatic dependent launch ---------------------------------------------------------------
 // The layered path is a chain of short kernels.  Each one lets its successor start launching at once
 // (`pdl_launch`) and itself waits for its predecessor's results only after its own set-up (`pdl_wait`, which
@@ -125,6 +135,20 @@ static inline cudaError_t launch_chain(void (*kernel)(KArgs...), dim3 grid, dim3
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = Q3_PDL;
     cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// the same for a grid whose x dimension is made of clusters of `cluster` blocks
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_chain_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = Q3_PDL;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

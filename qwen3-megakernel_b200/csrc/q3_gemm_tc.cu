@@ -20,6 +20,7 @@
 
 #include "q3_engine.h"
 #include "q3_gemm_tc.h"
+#include "q3_tc_ptx.cuh"
 
 namespace q3 {
 
@@ -28,56 +29,6 @@ static std::mutex& host_lock() { static std::mutex m; return m; }   // guards th
 
 constexpr int TC_THREADS = 192;    // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2..5: epilogue
 constexpr int TC_BM = 128;         // weight rows per tile (UMMA M)
-constexpr int TC_BK = 64;          // k per stage: 64 bf16 = one 128-byte swizzle row
-constexpr unsigned long long TC_WAIT_NS = 200ull * 1000 * 1000;
-
-__device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned long long tc_ns() { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
-
-// bounded mbarrier wait; on timeout sets *abort_flag and returns false
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t site) {
-    unsigned it = 0;
-    unsigned long long t0 = 0;
-    for (;;) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(tc_smem(bar)), "r"(parity) : "memory");
-        if (ok) return true;
-        if (*abort_flag) return false;
-        if ((++it & 63u) == 0) {
-            const unsigned long long t = tc_ns();
-            if (t0 == 0) t0 = t;
-            else if (t - t0 > TC_WAIT_NS) {
-                report(status, ST_MBAR_TIMEOUT, site, parity);
-                *abort_flag = 1;
-                return false;
-            }
-        }
-    }
-}
-
-// shared-memory matrix descriptor of a K-major tile with 128-byte swizzle: rows of 128 bytes, 8-row
-// groups 1024 bytes apart (stride byte offset), descriptor version 1 (Blackwell)
-__device__ __forceinline__ uint64_t tc_desc(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3ffffu) >> 4);        // start address, bits [0,14)
-    d |= (uint64_t)1 << 16;                              // leading byte offset (unused with swizzle), bits [16,30)
-    d |= (uint64_t)(1024 >> 4) << 32;                    // stride byte offset, bits [32,46)
-    d |= (uint64_t)1 << 46;                              // version
-    d |= (uint64_t)2 << 61;                              // SWIZZLE_128B
-    return d;
-}
-
-__device__ __forceinline__ void tc_ld32(uint32_t (&r)[32], uint32_t taddr) {   // 32 columns of this warp's 32 TMEM lanes; no wait
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr) : "memory");
-}
 
 template <int BN>
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w0,
@@ -89,7 +40,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     // which weight matrix this tile belongs to (grouped launches), and its first row inside that matrix
     int grp = 0, tile = blockIdx.x;
     if (p.n_groups > 1) {
@@ -143,7 +94,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             const int ahead = min(nkb, stages);   // the first ring of stages: weight tiles before the wait
             for (int kb = 0; kb < ahead; ++kb) {
                 unsigned char* st = base + (size_t)kb * stage_bytes;
@@ -152,9 +103,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
                              ::"r"(tc_smem(st)), "l"(tm_w), "r"((kb_begin + kb) * TC_BK), "r"(m0), "r"(tc_smem(&full_bar[kb])) : "memory");
             }
             pdl_wait();
-            for (int kb = 0; kb < nkb; ++kb) {
-                const int s = kb % stages;
-                if (kb >= stages && !tc_wait(&empty_bar[s], ((kb / stages) - 1) & 1, &abort_flag, p.status, 30)) break;
+            // (slot and phase are counted along: `stages` is no constant, and a division is longer than the rest of the loop)
+            for (int kb = 0, s = 0, turn = 0; kb < nkb; ++kb, ++s) {
+                if (s == stages) { s = 0; ++turn; }
+                if (turn > 0 && !tc_wait(&empty_bar[s], (turn - 1) & 1, &abort_flag, p.status, 30)) break;
                 unsigned char* st = base + (size_t)s * stage_bytes;
                 if (kb >= ahead) {
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(&full_bar[s])), "r"(stage_bytes) : "memory");
@@ -169,14 +121,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             // instruction descriptor: D fp32, A and B bf16, both K-major, N = BN (or all planes side by side), M = 128
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((wide ? nsplit * BN : BN) >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
             const int n_mma = wide ? 1 : nsplit;
             bool ok = true;
-            for (int kb = 0; kb < nkb && ok; ++kb) {
-                const int s = kb % stages;
-                ok = tc_wait(&full_bar[s], (kb / stages) & 1, &abort_flag, p.status, 31);
+            for (int kb = 0, s = 0, phase = 0; kb < nkb && ok; ++kb, ++s) {
+                if (s == stages) { s = 0; phase ^= 1; }
+                ok = tc_wait(&full_bar[s], phase, &abort_flag, p.status, 31);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t sa = tc_smem(base + (size_t)s * stage_bytes);
@@ -199,7 +151,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     } else {
         // ------------------------------------------------------------------ epilogue: TMEM -> registers -> global
         const int quad = warp & 3;                      // TMEM lanes [32 quad, 32 quad + 32) belong to this warp
-        const bool ok = tc_wait(&acc_bar, 0, &abort_flag, p.status, 32);
+        const bool ok = tc_wait_warp(&acc_bar, 0, &abort_flag, p.status, 32);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         pdl_wait();   // before the first store (the output may be something the predecessor still reads)
         if (ok) {
@@ -302,7 +254,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int nsplit = p.nsplit, stages = p.stages;
     const uint32_t a_bytes = (DUAL ? 2 : 1) * TC_BM * TC_BK * 2, b_bytes = BN * TC_BK * 2;   // DUAL: the Wg tile, then the Wu tile
     const uint32_t stage_bytes = a_bytes + nsplit * b_bytes;
@@ -351,15 +303,15 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             pdl_wait();
-            int gi = 0;
+            int s = 0, turn = 0;
             for (int it = blockIdx.x; it < w.n_items && !abort_flag; it += gridDim.x) {
                 const Item r = decode(it);
                 const CUtensorMap* tm_w = r.grp == 0 ? &tm_w0 : (r.grp == 1 ? &tm_w1 : &tm_w2);
-                for (int kb = 0; kb < r.nkb; ++kb, ++gi) {
-                    const int s = gi % stages;
-                    if (gi >= stages && !tc_wait(&empty_bar[s], ((gi / stages) - 1) & 1, &abort_flag, p.status, 36)) break;
+                for (int kb = 0; kb < r.nkb; ++kb, ++s) {
+                    if (s == stages) { s = 0; ++turn; }
+                    if (turn > 0 && !tc_wait(&empty_bar[s], (turn - 1) & 1, &abort_flag, p.status, 36)) break;
                     unsigned char* st = base + (size_t)s * stage_bytes;
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(&full_bar[s])), "r"(stage_bytes) : "memory");
                     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -376,9 +328,9 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-            int gi = 0, li = 0;
+            int s = 0, phase = 0, li = 0;
             bool ok = true;
             for (int it = blockIdx.x; it < w.n_items && ok; it += gridDim.x, ++li) {
                 const Item r = decode(it);
@@ -386,9 +338,9 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
                 // the accumulator is free once the epilogue warps have read its previous tenant out
                 if (li >= 2) ok = tc_wait(&acc_empty[acc], ((li >> 1) - 1) & 1, &abort_flag, p.status, 37);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int kb = 0; kb < r.nkb && ok; ++kb, ++gi) {
-                    const int s = gi % stages;
-                    ok = tc_wait(&full_bar[s], (gi / stages) & 1, &abort_flag, p.status, 38);
+                for (int kb = 0; kb < r.nkb && ok; ++kb, ++s) {
+                    if (s == stages) { s = 0; phase ^= 1; }
+                    ok = tc_wait(&full_bar[s], phase, &abort_flag, p.status, 38);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t sa = tc_smem(base + (size_t)s * stage_bytes);
@@ -425,7 +377,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
             const int acc = li & 1;
             float* const out = p.n_groups > 1 ? (r.grp == 0 ? p.g_out[0] : r.grp == 1 ? p.g_out[1] : p.g_out[2]) : p.out;
             const int ldo = p.n_groups > 1 ? (r.grp == 0 ? p.g_ldo[0] : r.grp == 1 ? p.g_ldo[1] : p.g_ldo[2]) : p.ldo;
-            ok = tc_wait(&acc_full[acc], (li >> 1) & 1, &abort_flag, p.status, 39);
+            ok = tc_wait_warp(&acc_full[acc], (li >> 1) & 1, &abort_flag, p.status, 39);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = r.m0 + quad * 32 + lane;    // weight row = output column (every tile is a full 128 rows)

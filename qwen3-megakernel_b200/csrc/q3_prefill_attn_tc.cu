@@ -65,6 +65,12 @@ __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile
         }
     }
 }
+// One lane of a converged warp polls for all 32: the polls of 16 softmax warps, a request a lane, delay the MMA thread's own.
+__device__ __forceinline__ bool at_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t site) {
+    int ok = 0;
+    if ((threadIdx.x & 31) == 0) ok = at_wait(bar, parity, abort_flag, status, site);
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
 
 // K-major operand, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart (as in the GEMM)
 __device__ __forceinline__ uint64_t at_desc_k(uint32_t smem_addr) {
@@ -141,7 +147,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
     __shared__ __align__(16) unsigned short pm16[2][AT_PARTS][128];
     float (*pm)[128] = reinterpret_cast<float (*)[128]>(&pm16[0][0][0]);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int g = a.heavy_first ? (int)blockIdx.x % KV_HEADS : (int)blockIdx.y;   // kv head; query heads 2g and 2g + 1
     unsigned char* sQh = at_raw;
     unsigned char* sQl = sQh + AT_Q_BYTES;
@@ -199,7 +205,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
 
         if (warp == AT_SOFT / 32) {
             // ------------------------------------------------------------------ TMA producer
-            if (lane == 0) {
+            if (elect_one()) {
                 // K and V of a tile share a stage but are released separately: the K half is free as soon as S of its tile has
                 // been computed, a whole tile before the V half (after PV), so the next K is on its way that much earlier
                 for (int t = 0; t < n_kt; ++t) {
@@ -222,7 +228,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
             }
         } else if (warp == AT_SOFT / 32 + 1) {
             // ------------------------------------------------------------------ MMA issuer
-            if (lane == 0) {
+            if (elect_one()) {
                 // D fp32, A and B bf16, M 128, N 128; bit 16: B is MN-major (V)
                 const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
                 const uint32_t idesc_o = idesc_s | (1u << 16);
@@ -282,7 +288,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
             bool ok = true;
             // O = O c + PV of tile `it` (this thread's 32 dims), once its MMAs have completed
             auto fold = [&](int it, float c) -> bool {
-                if (!at_wait(&o_full[it & 1], (it >> 1) & 1, &abort_flag, a.status, 45)) return false;
+                if (!at_wait_warp(&o_full[it & 1], (it >> 1) & 1, &abort_flag, a.status, 45)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t v0[32];
                 at_ld32(v0, trow + 256u + (uint32_t)(it & 1) * 128u);
@@ -294,7 +300,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
             };
             for (int t = 0; t < n_kt && ok; ++t) {
                 const int it = it0 + t;
-                ok = at_wait(&s_full[it & 1], (it >> 1) & 1, &abort_flag, a.status, 44);
+                ok = at_wait_warp(&s_full[it & 1], (it >> 1) & 1, &abort_flag, a.status, 44);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t r0[32];
@@ -329,7 +335,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                 }
                 lsum = lsum * c + psum;
                 // the P buffer is free once PV of the previous tile has completed (long ago in practice)
-                if (t > 0 && !at_wait(&o_full[(it - 1) & 1], ((it - 1) >> 1) & 1, &abort_flag, a.status, 46)) { ok = false; break; }
+                if (t > 0 && !at_wait_warp(&o_full[(it - 1) & 1], ((it - 1) >> 1) & 1, &abort_flag, a.status, 46)) { ok = false; break; }
                 // P[row][32 part .. 32 part + 31]: four 16-byte chunks of box part / 2, chunk slots 4 (part & 1) + ch
 #pragma unroll
                 for (int ch = 0; ch < 4; ++ch)
