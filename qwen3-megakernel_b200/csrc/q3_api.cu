@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "q3_engine.h"
+#include "q3_gemm_cl.h"
 #include "q3_gemm_tc.h"
 #include "q3_layer_tc.h"
 
@@ -105,11 +106,13 @@ extern "C" int q3_create(int device, const q3_config* cfg, q3_engine** out) {
         (rc = alloc(e, (void**)&e->status, Q3_STATUS_WORDS * 4)) ||
         (rc = alloc(e, (void**)&e->sync, Q3_SYNC_WORDS * 4)) ||
         (rc = alloc(e, (void**)&e->pf_desc, 64 + B * 32)) ||
-        (tc && ((rc = alloc(e, &e->planes, 3 * cap_pad * INTER * 2)) ||
-                (rc = alloc(e, (void**)&e->gate, B * INTER * 4)) ||
+        (rc = alloc(e, &e->planes, 3 * cap_pad * INTER * 2)) ||
+        (rc = alloc(e, &e->xplanes, 3 * cap_pad * HIDDEN * 2)) ||
+        (rc = alloc(e, (void**)&e->ssq, CL_SSQ_PARTS * cap_pad * 4)) ||
+        (rc = alloc(e, (void**)&e->logits_tc, (size_t)cfg->max_batch * cfg->vocab * 4)) ||
+        (tc && ((rc = alloc(e, (void**)&e->gate, B * INTER * 4)) ||
                 (rc = alloc(e, (void**)&e->up, B * INTER * 4)) ||
-                (rc = alloc(e, &e->lk_state, LK_STATE_BYTES)) ||
-                (cfg->max_batch >= Q3_TC_MIN_BATCH && (rc = alloc(e, (void**)&e->logits_tc, (size_t)cfg->max_batch * cfg->vocab * 4)))))) {
+                (rc = alloc(e, &e->lk_state, LK_STATE_BYTES))))) {
         strncpy(g_create_error, e->err, sizeof(g_create_error) - 1);
         q3_destroy(e);
         return rc;
@@ -140,7 +143,7 @@ extern "C" void q3_destroy(q3_engine* e) {
     delete static_cast<std::vector<GraphEntry>*>(e->graphs);
     if (e->capture_stream) cudaStreamDestroy(static_cast<cudaStream_t>(e->capture_stream));
     persist_teardown(e);
-    void* bufs[] = {e->x, e->qkv, e->attn, e->hid, e->part, e->pval, e->pidx, e->status, e->sync, e->pf_desc, e->planes, e->gate, e->up, e->logits_tc, e->lk_state};
+    void* bufs[] = {e->x, e->qkv, e->attn, e->hid, e->part, e->pval, e->pidx, e->status, e->sync, e->pf_desc, e->planes, e->xplanes, e->ssq, e->gate, e->up, e->logits_tc, e->lk_state};
     for (void* p : bufs)
         if (p) cudaFree(p);
     delete e;
@@ -240,7 +243,14 @@ extern "C" int q3_status(q3_engine* e, void* stream, uint32_t* words, int32_t n)
 // positions a split's block may take, rounded up to 32: with the split count it fixes the attention launch
 static int chunk_pad_for(int max_len, int ns) { return (((max_len + 1 + ns - 1) / ns) + 31) / 32 * 32; }
 
-static int splits_for(const q3_engine* e, int batch, int max_len) {
+// Decode steps of up to 16 sequences run as five launches per layer (q3_gemm_cl.h); larger ones, and engines without scratch
+// for the planes, keep one launch per phase.
+constexpr int CHAIN_MAX_BATCH = 16;
+static bool chain_serves(const q3_engine* e, int batch) { return e->xplanes != nullptr && batch <= CHAIN_MAX_BATCH; }
+constexpr int CHAIN_MAX_SPLITS = 8;   // the splits of a (sequence, kv head) are one cluster
+
+static int splits_for(const q3_engine* e, int batch, int max_len, bool chain) {
+    const double merge_us = chain ? 1.0 : 5.0;   // what more than one split costs beyond its blocks
     const int n = max_len + 1;
     int by_len = (n + 31) / 32;                                   // at least 32 positions per split
     // The split count with the shortest estimated launch.  A launch takes `waves` rounds of blocks; a block costs a fixed
@@ -256,9 +266,9 @@ static int splits_for(const q3_engine* e, int batch, int max_len) {
     const double per_pos = big ? 0.023 : 0.006;
     double best = 1e30;
     int s = 1;
-    for (int c = 1; c <= 16 && c <= by_len; ++c) {
+    for (int c = 1; c <= (chain ? CHAIN_MAX_SPLITS : 16) && c <= by_len; ++c) {
         const int waves = (pairs * c + slots - 1) / slots, per = (n + c - 1) / c;
-        const double t = waves * (4.0 + per_pos * per) + (c > 1 ? 5.0 : 0.0);
+        const double t = waves * (4.0 + per_pos * per) + (c > 1 ? merge_us : 0.0);
         if (t < best - 1e-9) { best = t; s = c; }
     }
     if (s < 1) s = 1;
@@ -275,7 +285,8 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
     const int B = a->batch, L = e->cfg.n_layers, V = e->cfg.vocab;
     const q3_weights& w = e->w;
     const int append = (a->flags & Q3_F_APPEND_KV) ? 1 : 0;
-    const int ns = splits_for(e, B, a->max_len);
+    const bool chain = prompt == nullptr && !layer_kernel && tc_planes == 3 && chain_serves(e, B);
+    const int ns = splits_for(e, B, a->max_len, chain);
     // From Q3_TC_MIN_BATCH tokens on, the projections are tensor-core GEMMs over bf16 planes of the
     // activations (tc_planes = 3: exact to fp32); below that, CUDA-core matrix-vector kernels.
     const bool tc = B >= Q3_TC_MIN_BATCH && e->planes != nullptr;
@@ -307,8 +318,61 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
     long long cover = (long long)ns * pad - 1;
     if (cover > e->rope_n - 1) cover = e->rope_n - 1;
     const int len_bound = (int)cover;
-    LAUNCH(launch_embed(reinterpret_cast<const long long*>(a->token), bf(w.embed), V, e->x, e->status, B, st, arg_keys, arg_tickets, a->seq_len, len_bound));
-    // Decode batches of 4..64 sequences: two launches per layer, the split attention and the persistent layer kernel
+    if (chain) {
+        // q/k/v | attention | Wo | gate/up | down: each product finishes its rows and writes the planes of the next one, so
+        // that nothing stands between them; the residual's planes and the others alternate between two buffers
+        const int rows = gemm_cluster_rows(B), ssq_ld = (e->cap + 127) / 128 * 128;
+        bf16_raw* xp = reinterpret_cast<bf16_raw*>(e->xplanes);
+        LAUNCH(launch_embed_planes(reinterpret_cast<const long long*>(a->token), bf(w.embed), V, e->x, bf(w.ln1), xp, rows, 3, e->ssq, ssq_ld, e->status, B, st,
+                                   arg_keys, arg_tickets, a->seq_len, len_bound));
+        for (int l = 0; l < L; ++l) {
+            ClusterGemmCall c{};
+            c.nsplit = 3; c.prow = rows; c.n_tok = B; c.ssq = e->ssq; c.ssq_ld = ssq_ld; c.status = e->status;
+            ClusterGemmCall q = c;
+            q.kind = CL_QKV; q.K = HIDDEN; q.in = xp; q.out = e->qkv;
+            q.w[0] = bf(w.wq) + (size_t)l * Q_DIM * HIDDEN; q.w[1] = bf(w.wk) + (size_t)l * KV_DIM * HIDDEN; q.w[2] = bf(w.wv) + (size_t)l * KV_DIM * HIDDEN;
+            LAUNCH(launch_gemm_cluster(q, st));
+
+            AttnArgs t{};
+            t.qkv = e->qkv; t.seq_k = a->seq_k; t.seq_v = a->seq_v;
+            t.seq_layer_stride = reinterpret_cast<const long long*>(a->seq_layer_stride);
+            t.seq_len = a->seq_len; t.part = e->part; t.layer = l; t.n_splits = ns; t.chunk_pad = pad; t.len_bound = len_bound;
+            t.fused_prep = 1; t.qn = bf(w.qn); t.kn = bf(w.kn); t.rope = e->rope;
+            t.k_write = reinterpret_cast<bf16_raw*>(a->k_write); t.v_write = reinterpret_cast<bf16_raw*>(a->v_write);
+            t.n_layers = L; t.append = append;
+            if (ns <= CHAIN_MAX_SPLITS) {
+                t.planes_out = planes; t.plane_rows = rows; t.cluster = ns > 1;
+                LAUNCH(launch_attn_split(t, B, st));
+            } else {   // caches longer than a cluster's splits hold: partials in memory and a merge launch
+                LAUNCH(launch_attn_planes(t, planes, rows, 3, B, st));
+                ++e->launches;
+            }
+
+            ClusterGemmCall o = c;
+            o.kind = CL_RESID; o.K = Q_DIM; o.in = planes; o.out = e->x; o.planes = xp; o.gain = bf(w.ln2) + (size_t)l * HIDDEN;
+            o.w[0] = bf(w.wo) + (size_t)l * HIDDEN * Q_DIM;
+            LAUNCH(launch_gemm_cluster(o, st));
+            ClusterGemmCall g = c;
+            g.kind = CL_SILU; g.K = HIDDEN; g.in = xp; g.planes = planes;
+            g.w[0] = bf(w.wg) + (size_t)l * INTER * HIDDEN; g.w[1] = bf(w.wu) + (size_t)l * INTER * HIDDEN;
+            LAUNCH(launch_gemm_cluster(g, st));
+            ClusterGemmCall d = c;
+            d.kind = CL_RESID; d.K = INTER; d.in = planes; d.out = e->x; d.planes = xp;
+            d.gain = l + 1 < L ? bf(w.ln1) + (size_t)(l + 1) * HIDDEN : bf(w.fnorm);
+            d.w[0] = bf(w.wd) + (size_t)l * HIDDEN * INTER;
+            LAUNCH(launch_gemm_cluster(d, st));
+        }
+        if (V % 128 == 0) {   // the LM head reads the last planes and applies the final norm's scale itself
+            float* logits = a->logits ? a->logits : e->logits_tc;
+            GemmTcCall h{bf(w.embed), xp, logits, nullptr, V, 0, V, B, HIDDEN, 3, rows, e->status, e->ssq, ssq_ld};
+            LAUNCH(launch_gemm_tc(h, st));
+            LAUNCH(launch_argmax_rows(logits, V, reinterpret_cast<long long*>(a->next_token), a->seq_len, append, B, st, arg_keys, arg_tickets));
+            return Q3_OK;
+        }
+    } else {
+        LAUNCH(launch_embed(reinterpret_cast<const long long*>(a->token), bf(w.embed), V, e->x, e->status, B, st, arg_keys, arg_tickets, a->seq_len, len_bound));
+    }
+    // The fused path, decode batches of 4..64 sequences: two launches per layer, the split attention and the persistent layer kernel
     // (everything between two attentions: merge, Wo, norm, gate/up, SiLU, down, norm, q/k/v of the next layer).
     const bool lk = layer_kernel && tc && prompt == nullptr && tc_planes == 3 && layer_tc_supports(e, B);
     if (lk) LAUNCH(launch_layer_tc(e, LK_MODE_FIRST, 0, B, st));
@@ -327,7 +391,7 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
         LAUNCH(launch_attn_split(t, B, st));
         LAUNCH(launch_layer_tc(e, l + 1 < L ? LK_MODE_MID : LK_MODE_LAST, l, B, st));
     }
-    for (int l = 0; !lk && l < L; ++l) {
+    for (int l = 0; !lk && !chain && l < L; ++l) {
         GemvArgs g{};
         // qkv = rms(x, ln1) @ [wq; wk; wv]^T
         if (tc) {
@@ -484,7 +548,11 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
     CU(e, cudaSetDevice(e->device));
     cudaStream_t st = (cudaStream_t)stream;
     uint32_t path = a->flags & Q3_F_PATH_MASK;
-    if (path == Q3_F_PATH_AUTO) path = persist_supports(e, a) ? Q3_F_PATH_PERSIST : Q3_F_PATH_LAYERED;
+    // The persistent kernel decodes one sequence per launch: from two on, one chain over all of them is as fast or faster (at
+    // 16 / 250 / 1000 positions, one after the other against the chain: two sequences 691 / 773 / 913 and 666 / 781 / 818 us,
+    // three 1032 / 1159 / 1370 and 676 / 796 / 873 us; one sequence 347 / 383 / 455 and 662 / 658 / 676 us).
+    if (path == Q3_F_PATH_AUTO)
+        path = persist_supports(e, a) && (a->batch == 1 || !chain_serves(e, a->batch)) ? Q3_F_PATH_PERSIST : Q3_F_PATH_LAYERED;
     if (path == Q3_F_PATH_PERSIST) {
         if (!persist_supports(e, a))
             return fail(e, Q3_ERR_UNSUPPORTED, "q3_decode: the persistent kernel does not serve batch %d at length %d", a->batch, a->max_len);
@@ -499,7 +567,7 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
     q3_decode_args key = *a;
     key.max_len = 0;
     key.reserved = 0;
-    const int ns = splits_for(e, a->batch, a->max_len);
+    const int ns = splits_for(e, a->batch, a->max_len, !layer_kernel && chain_serves(e, a->batch));
     const int pad = chunk_pad_for(a->max_len, ns);
     auto* cache = graph_cache(e);
     GraphEntry* hit = nullptr;

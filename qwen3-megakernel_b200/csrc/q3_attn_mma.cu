@@ -53,7 +53,21 @@ __device__ __forceinline__ uint32_t am_transpose(uint32_t w) {   // 8 x 8 matrix
     return d;
 }
 
-template <int AM_WARPS>
+__device__ __forceinline__ void am_store_planes(const AttnArgs& a, int b, int col, float v) {   // the three bf16 planes of one output element
+    const bf16_raw h = f_to_bf(v);
+    const float r1 = v - bf_to_f(h);
+    const bf16_raw m = f_to_bf(r1);
+    bf16_raw* dst = a.planes_out + (size_t)b * Q_DIM + col;
+    dst[0] = h;
+    dst[(size_t)a.plane_rows * Q_DIM] = m;
+    dst[(size_t)2 * a.plane_rows * Q_DIM] = f_to_bf(r1 - bf_to_f(m));
+}
+
+// CL: the splits of a (sequence, kv head) are the blocks of a cluster (at most AM_CLUSTER); every block sends its partial to the
+// first one through distributed shared memory and that one writes the output planes: no merge launch, no partials in global memory.
+constexpr int AM_CLUSTER = 8;
+
+template <int AM_WARPS, bool CL>
 __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma_kernel(const AttnArgs a) {
     constexpr int AM_THREADS = AM_WARPS * 32;
     pdl_launch();
@@ -63,6 +77,8 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
     __shared__ __align__(16) float s_o[AM_WARPS][2][HEAD_DIM];
     __shared__ float s_m[AM_WARPS][2], s_l[AM_WARPS][2], s_ns[2];
     __shared__ int s_last;
+    __shared__ float s_part[CL ? AM_CLUSTER : 1][2][HEAD_DIM + 2];   // CL, first block: the splits' outputs, maxima and sums
+    if (CL) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");   // (matched before the first remote store)
 
     const int sp = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -252,6 +268,7 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
         }
         if (lane == 0) { s_ns[0] = s0; s_ns[1] = s1; }
     }
+    if (CL) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     __syncthreads();
     {
         // thread d: both heads; combine the warps' partials and the new token under one maximum
@@ -273,25 +290,48 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
                 L += wgt;
                 acc = fmaf(s_new[3][d], wgt, acc);
             }
+            if (CL) {
+                const uint32_t own = am_smem(&s_part[sp][hh][0]);
+                uint32_t dst;
+                asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(dst) : "r"(own));
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + d * 4), "f"(acc) : "memory");
+                if (d == 0) {
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + HEAD_DIM * 4), "f"(M) : "memory");
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + HEAD_DIM * 4 + 4), "f"(L) : "memory");
+                }
+                continue;
+            }
             if (a.merged != nullptr && a.n_splits == 1) {       // the only split: this is the head's output (the new token is in it, so L > 0)
                 a.merged[(size_t)b * Q_DIM + (size_t)(2 * g + hh) * HEAD_DIM + d] = acc / L;
                 continue;
             }
             if (a.planes_out != nullptr && a.n_splits == 1) {   // ... or as the three bf16 planes
-                const float v = acc / L;
-                const bf16_raw h = f_to_bf(v);
-                const float r1 = v - bf_to_f(h);
-                const bf16_raw m = f_to_bf(r1);
-                bf16_raw* dst = a.planes_out + (size_t)b * Q_DIM + (size_t)(2 * g + hh) * HEAD_DIM + d;
-                dst[0] = h;
-                dst[(size_t)a.plane_rows * Q_DIM] = m;
-                dst[(size_t)2 * a.plane_rows * Q_DIM] = f_to_bf(r1 - bf_to_f(m));
+                am_store_planes(a, b, (2 * g + hh) * HEAD_DIM + d, acc / L);
                 continue;
             }
             float* out = a.part + (((size_t)b * Q_HEADS + 2 * g + hh) * a.n_splits + sp) * ATTN_PART_STRIDE;
             if (d == 0) { out[0] = M * AM_LN2; out[1] = L; }     // an empty chunk publishes (-inf, 0, 0); the maximum in natural units
             out[4 + d] = acc;
         }
+    }
+    if (CL) {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        if (sp != 0) return;
+        for (int i = tid; i < 2 * HEAD_DIM; i += AM_THREADS) {
+            const int hh = i >> 7, d = i & (HEAD_DIM - 1);
+            float M = -INFINITY;
+            for (int s = 0; s < a.n_splits; ++s) M = fmaxf(M, s_part[s][hh][HEAD_DIM]);
+            float L = 0.f, acc = 0.f;
+            for (int s = 0; s < a.n_splits; ++s) {
+                const float ms = s_part[s][hh][HEAD_DIM];
+                const float w = ms > -INFINITY ? am_ex2(ms - M) : 0.f;      // an empty chunk has (-inf, 0, 0)
+                L = fmaf(s_part[s][hh][HEAD_DIM + 1], w, L);
+                acc = fmaf(s_part[s][hh][d], w, acc);
+            }
+            am_store_planes(a, b, (2 * g + hh) * HEAD_DIM + d, acc / L);
+        }
+        return;
     }
     if (a.merged != nullptr && a.n_splits > 1) {
         // the last block of this (sequence, kv head) to get here merges all splits of its two heads: no merge launch
@@ -321,6 +361,11 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
     }
 }
 
+template <int W, bool CL>
+static cudaError_t am_prepare() {
+    return cudaFuncSetAttribute(attn_mma_kernel<W, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, W * AM_STAGES * AM_STAGE);
+}
+
 cudaError_t launch_attn_mma(const AttnArgs& a, int batch, cudaStream_t st) {
     if (a.chunk_pad < 32 || a.chunk_pad % 32 || a.n_splits < 1) return cudaErrorInvalidValue;
     static int sm_count[64] = {};
@@ -328,16 +373,24 @@ cudaError_t launch_attn_mma(const AttnArgs& a, int batch, cudaStream_t st) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!sm_count[dev]) {   // (a benign race between host threads: the same values are written)
-        constexpr size_t four = (size_t)4 * AM_STAGES * AM_STAGE;
-        if ((e = cudaFuncSetAttribute(attn_mma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)four)) != cudaSuccess) return e;
-        if ((e = cudaFuncSetAttribute(attn_mma_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * four))) != cudaSuccess) return e;
+        if ((e = am_prepare<4, false>()) != cudaSuccess || (e = am_prepare<8, false>()) != cudaSuccess || (e = am_prepare<4, true>()) != cudaSuccess ||
+            (e = am_prepare<8, true>()) != cudaSuccess)
+            return e;
         int n = 0;
         if ((e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
         sm_count[dev] = n;
     }
     const dim3 grid(a.n_splits, KV_HEADS, batch);
-    if (KV_HEADS * batch >= sm_count[dev]) return launch_chain(attn_mma_kernel<4>, grid, dim3(128), (size_t)4 * AM_STAGES * AM_STAGE, st, a);
-    return launch_chain(attn_mma_kernel<8>, grid, dim3(256), (size_t)8 * AM_STAGES * AM_STAGE, st, a);
+    const bool big = KV_HEADS * batch >= sm_count[dev];
+    const int warps = big ? 4 : 8;
+    const size_t smem = (size_t)warps * AM_STAGES * AM_STAGE;
+    if (a.cluster) {
+        if (a.n_splits > AM_CLUSTER || a.planes_out == nullptr) return cudaErrorInvalidValue;
+        if (big) return launch_chain_cluster(attn_mma_kernel<4, true>, grid, dim3(128), smem, a.n_splits, st, a);
+        return launch_chain_cluster(attn_mma_kernel<8, true>, grid, dim3(256), smem, a.n_splits, st, a);
+    }
+    if (big) return launch_chain(attn_mma_kernel<4, false>, grid, dim3(128), smem, st, a);
+    return launch_chain(attn_mma_kernel<8, false>, grid, dim3(256), smem, st, a);
 }
 
 }  // namespace q3

@@ -30,7 +30,7 @@ static std::mutex& host_lock() { static std::mutex m; return m; }   // guards th
 constexpr int TC_THREADS = 192;    // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2..5: epilogue
 constexpr int TC_BM = 128;         // weight rows per tile (UMMA M)
 
-template <int BN>
+template <int BN, bool SCALE>   // SCALE: every token's column is multiplied by its RMS norm's scale (GemmTcParams::ssq)
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w0,
                                                                 const __grid_constant__ CUtensorMap tm_w1,
                                                                 const __grid_constant__ CUtensorMap tm_w2,
@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     __shared__ __align__(8) uint64_t full_bar[8], empty_bar[8], acc_bar;
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_flag;
+    __shared__ float s_scale[SCALE ? BN : 1];
 
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     // which weight matrix this tile belongs to (grouped launches), and its first row inside that matrix
@@ -151,6 +152,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     } else {
         // ------------------------------------------------------------------ epilogue: TMEM -> registers -> global
         const int quad = warp & 3;                      // TMEM lanes [32 quad, 32 quad + 32) belong to this warp
+        if constexpr (SCALE) {                          // the planes lack their norm's scale: one per token, while the MMAs run
+            pdl_wait();
+#pragma unroll 4
+            for (int j = warp - 2; j < BN; j += 4) {
+                const float ss = warp_sum(n0 + j < p.n_tok ? p.ssq[(size_t)lane * p.ssq_ld + n0 + j] : 0.f);
+                if (lane == 0) s_scale[j] = rsqrtf(ss / (float)HIDDEN + EPS);
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
         const bool ok = tc_wait_warp(&acc_bar, 0, &abort_flag, p.status, 32);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         pdl_wait();   // before the first store (the output may be something the predecessor still reads)
@@ -197,6 +207,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
                         const int t = n0 + c * 32 + j;
                         if (t < p.n_tok) {
                             float v = __uint_as_float(r[j]);
+                            if constexpr (SCALE) v *= s_scale[c * 32 + j];
                             float* dst = out + (size_t)t * ldo + row;
                             if (p.epi == TC_EPI_ATOMIC) {
                                 atomicAdd(dst, v);   // split-K: `out` already holds zero or the residual
@@ -465,15 +476,16 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// 2-D bf16 tensor [rows, cols] row-major, box [box_rows, 64 columns], 128-byte swizzle
-static bool make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+// bf16 tensor [planes, rows, cols] row-major (two-dimensional when planes is 0), box [all planes, box_rows, 64 columns],
+// 128-byte swizzle
+static bool make_map(CUtensorMap* m, const void* ptr, uint64_t planes, uint64_t rows, uint64_t cols, uint32_t box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
-    const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {cols * 2};
-    const cuuint32_t box[2] = {TC_BK, box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint64_t dims[3] = {cols, rows, planes};
+    const cuuint64_t strides[2] = {cols * 2, rows * cols * 2};
+    const cuuint32_t box[3] = {TC_BK, box_rows, (cuuint32_t)planes};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, planes ? 3 : 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -538,7 +550,7 @@ static cudaError_t launch_persist(const CUtensorMap* tw, const CUtensorMap& tx, 
     return launch_chain(gemm_tc_persist_kernel<DUAL>, dim3(grid), dim3(TP_THREADS), smem, st, tw[0], tw[1], tw[2], tx, p, w);
 }
 
-template <int BN>
+template <int BN, bool SCALE = false>
 static cudaError_t launch_bn(const CUtensorMap* tw, const CUtensorMap& tx, GemmTcParams p, int n_rows, int n_tok, int sm_count, cudaStream_t st) {
     // n_rows: all weight rows of the launch (the sum over the groups); tw: three maps (unused ones repeat the first)
     const int nkb = p.K / TC_BK;
@@ -580,30 +592,30 @@ static cudaError_t launch_bn(const CUtensorMap* tw, const CUtensorMap& tx, GemmT
         if (e != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return cudaErrorInvalidDevice;
         std::lock_guard<std::mutex> hold(host_lock());
         if (!attr_set[dev]) {
-            e = cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+            e = cudaFuncSetAttribute(gemm_tc_kernel<BN, SCALE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
             if (e != cudaSuccess) return e;
             attr_set[dev] = true;
         }
     }
     dim3 grid((n_rows + TC_BM - 1) / TC_BM, (n_tok + BN - 1) / BN, ksplit);
-    return launch_chain(gemm_tc_kernel<BN>, grid, dim3(TC_THREADS), smem, st, tw[0], tw[1], tw[2], tx, p);
+    return launch_chain(gemm_tc_kernel<BN, SCALE>, grid, dim3(TC_THREADS), smem, st, tw[0], tw[1], tw[2], tx, p);
 }
 
 // Encoding a tensor map costs a few microseconds of host time; a step issues hundreds of GEMMs over the
 // same few hundred (pointer, shape) pairs, so the maps are cached.
-struct MapKey { const void* p; uint64_t rows, cols; uint32_t box; };
+struct MapKey { const void* p; uint64_t planes, rows, cols; uint32_t box; };
 struct MapEntry { MapKey k; CUtensorMap m; };
 static std::vector<MapEntry>& map_cache() { static std::vector<MapEntry> c; return c; }
 // (device addresses are unique across the GPUs of a process, so one cache serves them all; it is locked because
 // engines on different host threads share it)
-static bool cached_map(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out) {
+static bool cached_map(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out, uint64_t planes = 0) {
     std::lock_guard<std::mutex> hold(host_lock());
     auto& c = map_cache();
     for (auto& e : c)
-        if (e.k.p == ptr && e.k.rows == rows && e.k.cols == cols && e.k.box == box_rows) { *out = e.m; return true; }
+        if (e.k.p == ptr && e.k.planes == planes && e.k.rows == rows && e.k.cols == cols && e.k.box == box_rows) { *out = e.m; return true; }
     if (c.size() > 4096) c.clear();
-    MapEntry e{{ptr, rows, cols, box_rows}, {}};
-    if (!make_map(&e.m, ptr, rows, cols, box_rows)) return false;
+    MapEntry e{{ptr, planes, rows, cols, box_rows}, {}};
+    if (!make_map(&e.m, ptr, planes, rows, cols, box_rows)) return false;
     c.push_back(e);
     *out = e.m;
     return true;
@@ -614,8 +626,8 @@ bool gemm_tc_splits_k(int n_rows, int n_tok, int K) {
     const int bn = n_tok <= 32 ? 32 : (n_tok <= 64 ? 64 : 128);
     return k_slices(n_rows, n_tok, bn, K / TC_BK, sm_count_of_current_device()) > 1;
 }
-bool tc_cached_map(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out) {
-    return cached_map(ptr, rows, cols, box_rows, out);
+bool tc_cached_map(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out, uint64_t planes) {
+    return cached_map(ptr, rows, cols, box_rows, out, planes);
 }
 static int sm_count_of_current_device() {
     static int sms[MAX_DEVICES] = {};
@@ -637,9 +649,15 @@ cudaError_t launch_gemm_tc(const GemmTcCall& c, cudaStream_t st) {
     GemmTcParams p{};
     p.out = c.out; p.resid = c.resid; p.ldo = c.ldo; p.ldr = c.ldr; p.n_rows = c.n_rows; p.n_tok = c.n_tok; p.K = c.K;
     p.nsplit = c.nsplit; p.plane_rows = c.plane_rows; p.epi = c.resid ? TC_EPI_RESID : TC_EPI_STORE; p.status = c.status;
+    p.ssq = c.ssq; p.ssq_ld = c.ssq_ld;
     const int sm_count = sm_count_of_current_device();
     if (sm_count < 1) return cudaErrorInvalidDevice;
     const CUtensorMap maps[3] = {tw, tw, tw};
+    if (c.ssq != nullptr) {
+        if (bn == 32) return launch_bn<32, true>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
+        if (bn == 64) return launch_bn<64, true>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
+        return launch_bn<128, true>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
+    }
     if (persist_serves(c.n_rows, c.n_tok, c.nsplit, c.plane_rows, sm_count)) {
         CUtensorMap txp;
         if (!cached_map(c.x_planes, (uint64_t)c.nsplit * c.plane_rows, (uint64_t)c.K, (uint32_t)TP_BN, &txp)) return cudaErrorUnknown;

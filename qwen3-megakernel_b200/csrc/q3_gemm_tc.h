@@ -29,6 +29,8 @@ struct GemmTcParams {
     int g_tiles[3];
     float* g_out[3];
     int g_ldo[3];
+    const float* ssq;      // column t is scaled by rsqrt(sum of the 32 parts ssq[i * ssq_ld + t] / 1024 + eps) (gemm_tc_kernel<., true>)
+    int ssq_ld;
 };
 
 // host-side call
@@ -40,6 +42,8 @@ struct GemmTcCall {
     int ldo, ldr;
     int n_rows, n_tok, K, nsplit, plane_rows;
     uint32_t* status;
+    const float* ssq;      // not null: the planes lack their RMS norm's scale, the epilogue applies it (never the persistent kernel)
+    int ssq_ld;
 };
 
 cudaError_t launch_gemm_tc(const GemmTcCall& c, cudaStream_t st);
@@ -78,6 +82,6 @@ bool gemm_tc_splits_k(int n_rows, int n_tok, int K);
 
 // A cached tensor map of a row-major bf16 matrix [rows, cols]: boxes of 64 columns x box_rows rows, 128-byte swizzle,
 // out-of-range rows read as zeros.  (CUtensorMap is declared by <cuda.h>, which the caller includes.)
-bool tc_cached_map(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, ::CUtensorMap_st* out);
+bool tc_cached_map(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, ::CUtensorMap_st* out, uint64_t planes = 0);
 
 }  // namespace q3

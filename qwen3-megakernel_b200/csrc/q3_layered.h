@@ -80,6 +80,7 @@ struct AttnArgs {
     // [3][plane_rows][2048] the Wo GEMM reads
     bf16_raw* planes_out;
     int plane_rows;
+    int cluster;                      // the splits are a cluster of blocks (at most 8) that writes planes_out itself
 };
 
 cudaError_t launch_gemv(int K, int epi, const GemvArgs& a, int grid_x, cudaStream_t st);

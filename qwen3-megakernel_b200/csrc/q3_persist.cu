@@ -56,7 +56,7 @@ constexpr int WO_SLICES = 9;                  // row slices of Wo; CTA c < 144 o
 constexpr int F_CTAS = Q_HEADS * WO_SLICES;   // 144
 constexpr int GROUP_CTAS = 2 * WO_SLICES;     // CTAs sharing one kv head
 constexpr int WO_ROWS_MAX = 116;              // largest slice: 4 * ceil(256 / 9)
-constexpr int PERSIST_MAX_BATCH = 3;          // sequences served by back-to-back launches
+constexpr int PERSIST_MAX_BATCH = 3;          // sequences served by back-to-back launches when the caller asks for this kernel
 constexpr int MIN_GRID = 147;                 // row shares must fit the shared-memory slots
 constexpr int SC_HALF = 128;                  // the score buffer holds 3 * SC_HALF floats
 constexpr int SPLIT_SC = 3 * SC_HALF / 2;     // split attention: scores kept per head = the most positions a CTA takes (192)
@@ -1481,9 +1481,7 @@ void persist_teardown(q3_engine* e) {
     e->p_state = nullptr;
 }
 
-// Batches of up to PERSIST_MAX_BATCH sequences are served as one launch per sequence (measured at 1024 cached
-// positions: 2 sequences 2 x 0.47 ms against 1.60 ms on the layered path; from 4 sequences on the layered path's
-// tensor-core projections win).
+// Batches of up to PERSIST_MAX_BATCH sequences are served as one launch per sequence (q3_decode picks it for one sequence only).
 bool persist_supports(const q3_engine* e, const q3_decode_args* a) {
     const PersistState* s = static_cast<const PersistState*>(e->p_state);
     if (s == nullptr || a->batch < 1) return false;

@@ -63,4 +63,22 @@ __device__ __forceinline__ void tc_ld32(uint32_t (&r)[32], uint32_t taddr) {   /
                  : "r"(taddr) : "memory");
 }
 
+__device__ __forceinline__ void tc_ld16(uint32_t* r, uint32_t taddr) {   // 16 columns of this warp's 32 TMEM lanes; no wait
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+
+// one 2-D box [rows of the map's box] x [64 k] into shared memory, counted on an mbarrier
+__device__ __forceinline__ void tc_load_box(uint32_t dst, const void* map, int k, int row, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(k), "r"(row), "r"(tc_smem(bar)) : "memory");
+}
+// a 3-D box [all planes] x [rows of the map's box] x [64 k]
+__device__ __forceinline__ void tc_load_planes(uint32_t dst, const void* map, int k, int row, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(dst), "l"(map), "r"(k), "r"(row), "r"(0), "r"(tc_smem(bar)) : "memory");
+}
+
 }  // namespace q3

@@ -152,6 +152,35 @@ def test_ragged_batch(oracle, path, batch):
         gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{path} seq {b} len {lens[b]}")
 
 
+@pytest.mark.parametrize("batch", [1, 2, 15, 16, 17, 31, 32, 63, 64])
+def test_batches_at_the_edges_of_the_token_tiles(oracle, batch):
+    """The cluster GEMMs tile the tokens by 16, 32 and 64 and a row's owner is its index modulo the cluster size; the
+    longest sequence decides the attention split, so the empty and the one-position cache get splits with nothing in
+    them.  Sums are added in a fixed order: a second launch repeats the first one's bits."""
+    from qwen3mk.kernel import SeqTable
+
+    shp = oracle.Shape(layers=2, vocab=2048)
+    inp = oracle.synthetic(53, shp, context=8)
+    w = oracle.to_fp32(inp)
+    g = torch.Generator().manual_seed(100 + batch)
+    lens = ([1300, 0, 1, 33] + torch.randint(1, 200, (batch,), generator=g).tolist())[:batch]
+    toks = torch.randint(0, 2048, (batch,), generator=g)
+    kcs = [(torch.randn(2, max(n, 1), 8, 128, generator=g) * 0.1).to(torch.bfloat16) for n in lens]
+    vcs = [(torch.randn(2, max(n, 1), 8, 128, generator=g) * 0.1).to(torch.bfloat16) for n in lens]
+    mk = engine("layered", layers=2, vocab=2048, max_batch=batch)
+    seqs = SeqTable([k.cuda() for k in kcs], [v.cuda() for v in vcs], lens)
+    out = mk.bind_sequences(to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}), toks.cuda(), seqs)
+    mk.launch()
+    mk.status()
+    first = {k: v.clone() for k, v in out.items()}
+    refs = oracle.decode_batch(w, toks.tolist(), [k[:, :n] for k, n in zip(kcs, lens)], [v[:, :n] for v, n in zip(vcs, lens)])
+    for b, ref in enumerate(refs):
+        gate_step(oracle, {k: out[k][b] for k in out}, ref, f"seq {b} len {lens[b]}")
+    mk.launch()
+    mk.status()
+    assert all(torch.equal(first[k], out[k]) for k in first)
+
+
 @pytest.mark.parametrize("path", PATHS)
 def test_prefill_2048_then_greedy_decode(oracle, small, path):
     """The benchmark's third shape on a small model: a 2048-token prompt on the GPU, then chained greedy steps over
