@@ -1,5 +1,6 @@
 // C ABI of the engine (declared in include/q3mk.h): engine life cycle, argument checks, path
 // selection and the per-step launch sequence of the layered path.
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -243,11 +244,11 @@ extern "C" int q3_status(q3_engine* e, void* stream, uint32_t* words, int32_t n)
 // positions a split's block may take, rounded up to 32: with the split count it fixes the attention launch
 static int chunk_pad_for(int max_len, int ns) { return (((max_len + 1 + ns - 1) / ns) + 31) / 32 * 32; }
 
-// Decode steps of up to 16 sequences run as five launches per layer (q3_gemm_cl.h); larger ones, and engines without scratch
+// Decode steps of up to 64 sequences run as five launches per layer (q3_gemm_cl.h); larger ones, and engines without scratch
 // for the planes, keep one launch per phase.
-constexpr int CHAIN_MAX_BATCH = 16;
+constexpr int CHAIN_MAX_BATCH = 64;
 static bool chain_serves(const q3_engine* e, int batch) { return e->xplanes != nullptr && batch <= CHAIN_MAX_BATCH; }
-constexpr int CHAIN_MAX_SPLITS = 8;   // the splits of a (sequence, kv head) are one cluster
+constexpr int CHAIN_MAX_SPLITS = 8;   // the splits of a (sequence, kv head) are one cluster (16: one sequence at 5000 positions 897 us, 8: 793)
 
 static int splits_for(const q3_engine* e, int batch, int max_len, bool chain) {
     const double merge_us = chain ? 1.0 : 5.0;   // what more than one split costs beyond its blocks
@@ -261,14 +262,19 @@ static int splits_for(const q3_engine* e, int batch, int max_len, bool chain) {
     //   batch 24 x 1024, 1 / 3: 1336 / 1463; batch 48 x 1024, 1 / 2: 2235 / 2214; batch 20 x 4096, 2 / 3: 2814 / 2415.
     //   Smaller batches: eight-warp blocks, one per SM, 6 ns per position.  Batch 8 x 1024, 1 / 2 splits: 1000 / 1035 us;
     //   batch 4 x 512: 882 / 920; batch 16 x 2048: 1446 / 1597.
-    const bool big = KV_HEADS * batch >= e->sm_count;
+    //   The chain: four-warp blocks for every batch (two of them, or one and a block of a neighbouring product, share an SM), a cluster
+    //   costs 1 us, and blocks beyond the first round start as others end.  Batch 8 x 1024, 1 / 2 / 3 / 4 / 8 splits: 889 / 785 / 744 /
+    //   734 / 913 us; 27 ragged up to 2048: 1429 / 1381 / 1496 / 1596 / 1958; 64 x 1024: 2344 / 2631 / 2682 / 2841 / 3916; three at 900
+    //   (eight steps): 6329 / 5786 / 5473 / 5337 / 5139.
+    const bool big = chain || KV_HEADS * batch >= e->sm_count;
     const int slots = (big ? 2 : 1) * e->sm_count, pairs = KV_HEADS * batch;
     const double per_pos = big ? 0.023 : 0.006;
     double best = 1e30;
     int s = 1;
     for (int c = 1; c <= (chain ? CHAIN_MAX_SPLITS : 16) && c <= by_len; ++c) {
         const int waves = (pairs * c + slots - 1) / slots, per = (n + c - 1) / c;
-        const double t = waves * (4.0 + per_pos * per) + (c > 1 ? merge_us : 0.0);
+        const double rounds = chain ? fmax(1.0, (double)pairs * c / slots) : waves;
+        const double t = 4.0 * waves + per_pos * per * rounds + (c > 1 ? merge_us : 0.0);
         if (t < best - 1e-9) { best = t; s = c; }
     }
     if (s < 1) s = 1;
@@ -341,7 +347,7 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
             t.k_write = reinterpret_cast<bf16_raw*>(a->k_write); t.v_write = reinterpret_cast<bf16_raw*>(a->v_write);
             t.n_layers = L; t.append = append;
             if (ns <= CHAIN_MAX_SPLITS) {
-                t.planes_out = planes; t.plane_rows = rows; t.cluster = ns > 1;
+                t.planes_out = planes; t.plane_rows = rows; t.cluster = ns > 1; t.early = 1;
                 LAUNCH(launch_attn_split(t, B, st));
             } else {   // caches longer than a cluster's splits hold: partials in memory and a merge launch
                 LAUNCH(launch_attn_planes(t, planes, rows, 3, B, st));
@@ -549,8 +555,8 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     uint32_t path = a->flags & Q3_F_PATH_MASK;
     // The persistent kernel decodes one sequence per launch: from two on, one chain over all of them is as fast or faster (at
-    // 16 / 250 / 1000 positions, one after the other against the chain: two sequences 691 / 773 / 913 and 666 / 781 / 818 us,
-    // three 1032 / 1159 / 1370 and 676 / 796 / 873 us; one sequence 347 / 383 / 455 and 662 / 658 / 676 us).
+    // 16 / 250 / 1000 positions, one after the other against the chain: two sequences 691 / 773 / 913 and 574 / 605 / 618 us,
+    // three 1035 / 1160 / 1369 and 582 / 609 / 632 us; one sequence 347 / 384 / 456 and 567 / 591 / 603 us).
     if (path == Q3_F_PATH_AUTO)
         path = persist_supports(e, a) && (a->batch == 1 || !chain_serves(e, a->batch)) ? Q3_F_PATH_PERSIST : Q3_F_PATH_LAYERED;
     if (path == Q3_F_PATH_PERSIST) {

@@ -65,19 +65,22 @@ __device__ __forceinline__ void am_store_planes(const AttnArgs& a, int b, int co
 
 // CL: the splits of a (sequence, kv head) are the blocks of a cluster (at most AM_CLUSTER); every block sends its partial to the
 // first one through distributed shared memory and that one writes the output planes: no merge launch, no partials in global memory.
-constexpr int AM_CLUSTER = 8;
+constexpr int AM_CLUSTER = 16;
+constexpr int AM_PART = 2 * (HEAD_DIM + 2) * 4;     // bytes of a split's partial
 
 template <int AM_WARPS, bool CL>
 __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma_kernel(const AttnArgs a) {
     constexpr int AM_THREADS = AM_WARPS * 32;
     pdl_launch();
-    pdl_wait();
+    if (!a.early) pdl_wait();
     extern __shared__ __align__(128) unsigned char am_raw[];
     __shared__ __align__(16) float s_new[4][HEAD_DIM];           // q head 2g, q head 2g + 1, the new token's k and v rows
     __shared__ __align__(16) float s_o[AM_WARPS][2][HEAD_DIM];
     __shared__ float s_m[AM_WARPS][2], s_l[AM_WARPS][2], s_ns[2];
     __shared__ int s_last;
-    __shared__ float s_part[CL ? AM_CLUSTER : 1][2][HEAD_DIM + 2];   // CL, first block: the splits' outputs, maxima and sums
+    // CL, first block: the splits' outputs, maxima and sums, behind the stages (sized for the launch's cluster, so that two blocks
+    // of a small cluster and a block of a neighbouring launch fit on an SM)
+    float (*s_part)[2][HEAD_DIM + 2] = reinterpret_cast<float (*)[2][HEAD_DIM + 2]>(am_raw + (size_t)AM_WARPS * AM_STAGES * AM_STAGE);
     if (CL) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");   // (matched before the first remote store)
 
     const int sp = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
@@ -118,6 +121,7 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
     };
 #pragma unroll
     for (int i = 0; i < AM_STAGES - 1; ++i) issue(i);
+    if (a.early) pdl_wait();     // lengths and cached rows were complete before this launch could start: only `qkv` is the predecessor's
 
     // ---- the two q heads, the k row and the v row of the new token: as prepared by head_prep_kernel, or prepared here ----
     for (int role = warp; role < 4; role += AM_WARPS) {   // a warp per vector: q head 2g, q head 2g + 1, k, v; four dims a lane
@@ -193,7 +197,7 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
         asm volatile("cp.async.wait_group %0;" ::"n"(AM_STAGES - 1) : "memory");
         __syncwarp();
         const uint32_t kst = am_smem(stage0 + (size_t)(i % AM_STAGES) * AM_STAGE), vst = kst + AM_HALF;
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
+        float c[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};     // (two chains: the products of one wait for one another)
         {
             const int row = lrow + (lmat & 1) * 8;               // matrices: (pos 0-7 | 8-15) x (dims lo 8 | hi 8) of the k step
 #pragma unroll
@@ -202,8 +206,10 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
                 const uint32_t addr = kst + (uint32_t)(row * 256 + (((2 * ks + (lmat >> 1)) ^ (row & 7)) << 4));
                 asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(af[0]), "=r"(af[1]), "=r"(af[2]), "=r"(af[3]) : "r"(addr));
                 am_mma(c, af, qh[ks][0], qh[ks][1]);
-                am_mma(c, af, ql[ks][0], ql[ks][1]);
+                am_mma(c2, af, ql[ks][0], ql[ks][1]);
             }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) c[j] += c2[j];
         }
         // c[0], c[1]: position fg, heads 2 ft, 2 ft + 1; c[2], c[3]: position fg + 8
         const int pa = w0 + i * AM_TILE + fg;
@@ -363,7 +369,7 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
 
 template <int W, bool CL>
 static cudaError_t am_prepare() {
-    return cudaFuncSetAttribute(attn_mma_kernel<W, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, W * AM_STAGES * AM_STAGE);
+    return cudaFuncSetAttribute(attn_mma_kernel<W, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, W * AM_STAGES * AM_STAGE + (CL ? AM_CLUSTER * AM_PART : 0));
 }
 
 cudaError_t launch_attn_mma(const AttnArgs& a, int batch, cudaStream_t st) {
@@ -374,7 +380,7 @@ cudaError_t launch_attn_mma(const AttnArgs& a, int batch, cudaStream_t st) {
     if (e != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!sm_count[dev]) {   // (a benign race between host threads: the same values are written)
         if ((e = am_prepare<4, false>()) != cudaSuccess || (e = am_prepare<8, false>()) != cudaSuccess || (e = am_prepare<4, true>()) != cudaSuccess ||
-            (e = am_prepare<8, true>()) != cudaSuccess)
+            (e = cudaFuncSetAttribute(attn_mma_kernel<4, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
             return e;
         int n = 0;
         if ((e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
@@ -382,14 +388,13 @@ cudaError_t launch_attn_mma(const AttnArgs& a, int batch, cudaStream_t st) {
     }
     const dim3 grid(a.n_splits, KV_HEADS, batch);
     const bool big = KV_HEADS * batch >= sm_count[dev];
-    const int warps = big ? 4 : 8;
-    const size_t smem = (size_t)warps * AM_STAGES * AM_STAGE;
+    const int warps = big || a.early ? 4 : 8;
+    const size_t smem = (size_t)(a.cluster ? 4 : warps) * AM_STAGES * AM_STAGE;
     if (a.cluster) {
         if (a.n_splits > AM_CLUSTER || a.planes_out == nullptr) return cudaErrorInvalidValue;
-        if (big) return launch_chain_cluster(attn_mma_kernel<4, true>, grid, dim3(128), smem, a.n_splits, st, a);
-        return launch_chain_cluster(attn_mma_kernel<8, true>, grid, dim3(256), smem, a.n_splits, st, a);
+        return launch_chain_cluster(attn_mma_kernel<4, true>, grid, dim3(128), smem + (size_t)a.n_splits * AM_PART, a.n_splits, st, a);
     }
-    if (big) return launch_chain(attn_mma_kernel<4, false>, grid, dim3(128), smem, st, a);
+    if (warps == 4) return launch_chain(attn_mma_kernel<4, false>, grid, dim3(128), smem, st, a);
     return launch_chain(attn_mma_kernel<8, false>, grid, dim3(256), smem, st, a);
 }
 

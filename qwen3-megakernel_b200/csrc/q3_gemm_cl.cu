@@ -1,7 +1,7 @@
 // The dense products of a layer for decode batches and short prompts: tcgen05 GEMMs whose k slices are the blocks of a
 // cluster.
 //
-// With 1..128 tokens a layer's weights are a few megabytes per product, so what a launch costs is latency, and what a
+// With 1..64 tokens a layer's weights are a few megabytes per product, so what a launch costs is latency, and what a
 // layer costs is the number of launches that wait for one another.  A product whose tiles are cut along K to occupy
 // the GPU has to add its slices up again.  Adding them with fp32 atomics to global memory leaves the finished row to
 // the NEXT launch, so every product drags a second launch behind it that normalises or applies SiLU, writes the bf16
@@ -17,6 +17,11 @@
 //   CL_QKV    128-row tiles of [Wq; Wk; Wv]: 32 tiles        qkv = (planes . W) * r
 //   CL_RESID  64-row tiles of Wo or Wd: 16 tiles             x += planes . W; planes of x * gain; sums of squares
 //   CL_SILU   64 rows of Wg and the same 64 of Wu: 48 tiles  planes of silu(gate * r) * (up * r)
+//
+// Measured (one B200, us per step, before -> after): 8 sequences x 1024 positions 984 -> 735, 64 x 1024 2333 -> 2075, one at
+// 5000 positions 1606 -> 793.  What bounds it: a launch is about 3.4 us of latencies in series (release of the wait to the first
+// plane 0.5, products 0.7, partial tile out 0.3, to the owners 0.5, finished row 0.6, end of the grid to the next release 0.7) beside
+// 1..2 us of weight bytes that overlap them.
 //
 // Weight tiles are requested before the wait for the previous launch, so that their latency overlaps its tail.
 #include <cuda.h>
@@ -50,23 +55,22 @@ __device__ __forceinline__ uint32_t cl_map(uint32_t smem_addr, int rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
     return a;
 }
-__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+// (relaxed: no data is handed over by the cluster's barrier, only the mbarriers' initialisation, which has its own fence)
+__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
 __device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 __device__ __forceinline__ void cl_store_planes(bf16_raw* p, size_t plane, int nsplit, float v) {
     const bf16_raw h = f_to_bf(v);
+    const float r1 = v - bf_to_f(h);
+    const bf16_raw m = f_to_bf(r1), l = f_to_bf(r1 - bf_to_f(m));
     p[0] = h;
-    if (nsplit > 1) {
-        const float r1 = v - bf_to_f(h);
-        const bf16_raw m = f_to_bf(r1);
-        p[plane] = m;
-        if (nsplit > 2) p[2 * plane] = f_to_bf(r1 - bf_to_f(m));
-    }
+    if (nsplit > 1) p[plane] = m;
+    if (nsplit > 2) p[2 * plane] = l;
 }
 
 template <int KIND, int BN> struct ClShape {
     static constexpr int TM = KIND == CL_RESID ? 64 : 128;                                // rows of the weight tile
-    static constexpr int C = KIND == CL_RESID ? 8 : 4;   // k slices = blocks of the cluster
+    static constexpr int C = KIND == CL_RESID ? 8 : 4;                                      // k slices = blocks of the cluster
     static constexpr int SLOTS = (BN + C - 1) / C;                                        // tokens a block owns
     static constexpr int RED_BYTES = C * SLOTS * TM * 4;                                  // partial tiles of the owned tokens
 };
@@ -118,7 +122,9 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
-    pdl_launch();
+    // The attention launch that follows q/k/v reads lengths and cache rows before it waits: it may start only once everything
+    // before this launch has completed (below).  The others' successors read nothing but weights early.
+    if (KIND != CL_QKV) pdl_launch();
     cl_arrive();      // (matched before the first remote copy: every block of the cluster has set its barriers up by then)
 
     const int te = (int)threadIdx.x - 64;        // 0..127 in the epilogue warps
@@ -145,6 +151,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
             for (int kb = 0; kb < ahead; ++kb) weights(kb, kb);
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_x) : "memory");
             pdl_wait();
+            if (KIND == CL_QKV) pdl_launch();
             for (int kb = 0, s = 0, turn = 0; kb < nkb; ++kb, ++s) {
                 if (s == stages) { s = 0; ++turn; }
                 if (turn > 0) {
@@ -160,14 +167,16 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
         // ------------------------------------------------------------------ MMA issuer
         if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((cols >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
-            for (int kb = 0, s = 0, phase = 0; kb < nkb; ++kb, ++s) {
-                if (s == stages) { s = 0; phase ^= 1; }
+            // (descriptors count 16-byte units: a k step of 16 elements is 2 of them, a stage stage_bytes / 16)
+            const uint64_t da0 = tc_desc(tc_smem(base)), db0 = tc_desc(tc_smem(base) + A_BYTES);
+            uint64_t ds = 0;
+            for (int kb = 0, s = 0, phase = 0; kb < nkb; ++kb, ++s, ds += stage_bytes >> 4) {
+                if (s == stages) { s = 0; phase ^= 1; ds = 0; }
                 if (!tc_wait(&full_bar[s], phase, &abort_flag, p.status, 51)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t sa = tc_smem(base + (size_t)s * stage_bytes), sb = sa + A_BYTES;
 #pragma unroll
                 for (int k = 0; k < TC_BK / 16; ++k) {
-                    const uint64_t da = tc_desc(sa + k * 32), db = tc_desc(sb + k * 32);
+                    const uint64_t da = da0 + ds + 2 * k, db = db0 + ds + 2 * k;
                     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
                                  ::"r"(tmem_base), "l"(da), "l"(db), "r"(idesc), "r"((uint32_t)(kb | k)), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
@@ -189,10 +198,11 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
     }
 
     // ---------------------------------------------------------------------- epilogue
-    float gain = 0.f;
-    if (KIND == CL_RESID) gain = bf_to_f(p.gain[tile * TM + orow]);
-    pdl_wait();
+    const float gain = KIND == CL_RESID ? bf_to_f(p.gain[tile * TM + orow]) : 0.f;
+    const int quad = warp & 3;                   // TMEM lanes [32 quad, 32 quad + 32) belong to this warp
+    const size_t plane = (size_t)p.prow * p.ldp;
     float xr[KIND == CL_RESID ? PER : 1];
+    pdl_wait();
     // while the products run: the scale of the owned rows, or the residual they are added to
     if (KIND != CL_RESID) {
 #pragma unroll 4
@@ -207,7 +217,6 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
             xr[i] = s < my_slots ? p.out[(size_t)(n0 + s * C + rank) * p.ldo + tile * TM + orow] : 0.f;
         }
     }
-    const int quad = warp & 3;                   // TMEM lanes [32 quad, 32 quad + 32) belong to this warp
     tc_wait_warp(&acc_bar, 0, &abort_flag, p.status, 52);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // The partial tile goes to this block's staging area (the stages are free: every MMA has completed), token by token and
@@ -242,8 +251,8 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    asm volatile("bar.arrive 2, 160;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("bar.arrive 2, 160;" ::: "memory");
     cl_wait();                                   // every block of the cluster has set its mbarrier up
     asm volatile("bar.sync 1, 128;" ::: "memory");
     if (te < C && slots_of(te) > 0) {
@@ -256,7 +265,6 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
     cl_arrive();      // (matched before the exit: this block has received everything, so nobody's copies are still under way then)
 
     // the owned tokens: add the slices in order and finish the row
-    const size_t plane = (size_t)p.prow * p.ldp;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const int s = osub + i * OSTEP, t = n0 + s * C + rank;
@@ -321,11 +329,13 @@ cudaError_t launch_embed_planes(const long long* token, const bf16_raw* embed, i
 }
 
 // ---- host side ------------------------------------------------------------------------------------------------------
-static int cl_tile(int n_tok) { return n_tok <= 16 ? 16 : n_tok <= 32 ? 32 : n_tok <= 64 ? 64 : 128; }
+// Tokens per tile.  Wider tiles need more shared memory than the neighbouring launches leave: batch 64 x 1024 with tiles of 16 / 32 /
+// 64: 2419 / 2075 / 2349 us per step.
+static int cl_tile(int n_tok) { return n_tok <= 16 ? 16 : 32; }
 
-// (a plane's rows are a multiple of 32, so that the LM head's 32-token tile can read the planes of 16 tokens or fewer)
+// (a plane's rows are a multiple of the LM head's token tile, which reads the last planes: 32 / 64 / 128)
 int gemm_cluster_rows(int n_tok) {
-    const int bn = n_tok <= 32 ? 32 : cl_tile(n_tok);
+    const int bn = n_tok <= 32 ? 32 : n_tok <= 64 ? 64 : 128;
     return (n_tok + bn - 1) / bn * bn;
 }
 
@@ -343,8 +353,8 @@ static cudaError_t launch_cl(const CUtensorMap* tw, const CUtensorMap& tx, Clust
     }
     const int stage_bytes = S::TM * TC_BK * 2 + p.nsplit * BN * TC_BK * 2;
     // Half of an SM's shared memory, so that the next launch's blocks find room while this one's are still there: they set up
-    // and fetch their weights before they wait (batch 8 x 1024, 72 / 112 / 200 KB: 939 / 873 / 873 us per step; batch 27
-    // ragged up to 2048: 1890 / 1740 / 1951 us).
+    // and fetch their weights before they wait (batch 64 x 1024, 75 / 90 / 112 KB: 2118 / 2104 / 2075 us per step; 27 ragged
+    // up to 2048: 1460 / 1437 / 1383 us).
     int stages = (112 * 1024 - S::RED_BYTES - 1024) / stage_bytes;
     const int nkb = (p.kb_total + S::C - 1) / S::C;
     if (stages > nkb) stages = nkb;
@@ -364,12 +374,8 @@ static cudaError_t launch_cl(const CUtensorMap* tw, const CUtensorMap& tx, Clust
 
 template <int KIND>
 static cudaError_t launch_kind(const CUtensorMap* tw, const CUtensorMap& tx, const ClusterGemmParams& p, int tiles, int bn, cudaStream_t st) {
-    switch (bn) {
-        case 16: return launch_cl<KIND, 16>(tw, tx, p, tiles, st);
-        case 32: return launch_cl<KIND, 32>(tw, tx, p, tiles, st);
-        case 64: return launch_cl<KIND, 64>(tw, tx, p, tiles, st);
-        default: return launch_cl<KIND, 128>(tw, tx, p, tiles, st);
-    }
+    if (bn == 16) return launch_cl<KIND, 16>(tw, tx, p, tiles, st);
+    return launch_cl<KIND, 32>(tw, tx, p, tiles, st);
 }
 
 cudaError_t launch_gemm_cluster(const ClusterGemmCall& c, cudaStream_t st) {

@@ -80,7 +80,9 @@ struct AttnArgs {
     // [3][plane_rows][2048] the Wo GEMM reads
     bf16_raw* planes_out;
     int plane_rows;
-    int cluster;                      // the splits are a cluster of blocks (at most 8) that writes planes_out itself
+    int cluster;                      // the splits are a cluster of blocks (at most 16) that writes planes_out itself
+    int early;                        // the predecessor lets this launch start only when everything before it has completed: lengths and
+                                      // cached rows may be read before the wait (blocks of four warps, which fit beside its blocks)
 };
 
 cudaError_t launch_gemv(int K, int epi, const GemvArgs& a, int grid_x, cudaStream_t st);

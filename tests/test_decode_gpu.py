@@ -179,8 +179,7 @@ def test_batches_at_the_edges_of_the_token_tiles(oracle, batch):
     mk.launch()
     mk.status()
     # (the logits of so small a vocabulary are K-slices added with atomics; the rows have been through every cluster GEMM)
-    if batch <= 16:   # (larger batches add split products with atomics)
-        assert all(torch.equal(first[k], out[k]) for k in ("k_write", "v_write"))
+    assert all(torch.equal(first[k], out[k]) for k in ("k_write", "v_write"))
 
 
 @pytest.mark.parametrize("path", PATHS)
