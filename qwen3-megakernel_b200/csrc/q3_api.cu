@@ -33,12 +33,6 @@ int q3::engine_fail(q3_engine* e, int code, const char* fmt, ...) {
             return fail(e, Q3_ERR_CUDA, "%s failed: %s (%s:%d)", #call, cudaGetErrorString(err__), __FILE__, __LINE__); \
     } while (0)
 
-static int alloc(q3_engine* e, void** p, size_t bytes) {
-    CU(e, cudaMalloc(p, bytes));
-    CU(e, cudaMemset(*p, 0, bytes));
-    return Q3_OK;
-}
-
 // ------------------------------------------------------------------------------------------------
 // CUDA graphs for the layered step: a step is hundreds of small launches whose arguments all live in
 // device memory, so a call with the same argument block can replay a captured graph instead of
@@ -96,28 +90,31 @@ extern "C" int q3_create(int device, const q3_config* cfg, q3_engine** out) {
     e->part_slots = (int)((B < 16 ? B : 16) * Q3_MAX_SPLITS > 2 * B ? (B < 16 ? B : 16) * Q3_MAX_SPLITS : 2 * B);
     const bool tc = e->cap >= Q3_TC_MIN_BATCH;
     const size_t cap_pad = (B + 127) / 128 * 128;
-    int rc;
-    if ((rc = alloc(e, (void**)&e->x, B * HIDDEN * 4)) ||
-        (rc = alloc(e, (void**)&e->qkv, B * QKV_DIM * 4)) ||
-        (rc = alloc(e, (void**)&e->attn, B * Q_DIM * 4)) ||
-        (rc = alloc(e, (void**)&e->hid, B * INTER * 4)) ||
-        (rc = alloc(e, (void**)&e->part, (size_t)e->part_slots * Q_HEADS * ATTN_PART_STRIDE * 4)) ||
-        (rc = alloc(e, (void**)&e->pval, (size_t)cfg->max_batch * e->lm_grid * 4)) ||
-        (rc = alloc(e, (void**)&e->pidx, (size_t)cfg->max_batch * e->lm_grid * 4)) ||
-        (rc = alloc(e, (void**)&e->status, Q3_STATUS_WORDS * 4)) ||
-        (rc = alloc(e, (void**)&e->sync, Q3_SYNC_WORDS * 4)) ||
-        (rc = alloc(e, (void**)&e->pf_desc, 64 + B * 32)) ||
-        (rc = alloc(e, &e->planes, 3 * cap_pad * INTER * 2)) ||
-        (rc = alloc(e, &e->xplanes, 3 * cap_pad * HIDDEN * 2)) ||
-        (rc = alloc(e, (void**)&e->ssq, CL_SSQ_PARTS * cap_pad * 4)) ||
-        (rc = alloc(e, (void**)&e->logits_tc, (size_t)cfg->max_batch * cfg->vocab * 4)) ||
-        (tc && ((rc = alloc(e, (void**)&e->gate, B * INTER * 4)) ||
-                (rc = alloc(e, (void**)&e->up, B * INTER * 4)) ||
-                (rc = alloc(e, &e->lk_state, LK_STATE_BYTES))))) {
-        strncpy(g_create_error, e->err, sizeof(g_create_error) - 1);
+    // one allocation for all of it: every cudaMalloc and cudaFree of an engine's life costs its caller about a millisecond
+    struct Part { void** p; size_t bytes; };
+    const Part parts[] = {
+        {(void**)&e->x, B * HIDDEN * 4}, {(void**)&e->qkv, B * QKV_DIM * 4}, {(void**)&e->attn, B * Q_DIM * 4}, {(void**)&e->hid, B * INTER * 4},
+        {(void**)&e->part, (size_t)e->part_slots * Q_HEADS * ATTN_PART_STRIDE * 4},
+        {(void**)&e->pval, (size_t)cfg->max_batch * e->lm_grid * 4}, {(void**)&e->pidx, (size_t)cfg->max_batch * e->lm_grid * 4},
+        {(void**)&e->status, Q3_STATUS_WORDS * 4}, {(void**)&e->sync, Q3_SYNC_WORDS * 4}, {&e->pf_desc, 64 + B * 32},
+        {&e->planes, 3 * cap_pad * INTER * 2}, {&e->xplanes, 3 * cap_pad * HIDDEN * 2}, {(void**)&e->ssq, CL_SSQ_PARTS * cap_pad * 4},
+        {(void**)&e->logits_tc, (size_t)cfg->max_batch * cfg->vocab * 4},
+        {(void**)&e->gate, tc ? B * INTER * 4 : 0}, {(void**)&e->up, tc ? B * INTER * 4 : 0}, {&e->lk_state, tc ? (size_t)LK_STATE_BYTES : 0}};
+    auto padded = [](size_t n) { return (n + 1023) / 1024 * 1024; };
+    size_t total = 0;
+    for (const Part& p : parts) total += padded(p.bytes);
+    cudaError_t err = cudaMalloc(&e->scratch, total);
+    if (err == cudaSuccess) err = cudaMemset(e->scratch, 0, total);
+    if (err != cudaSuccess) {
         q3_destroy(e);
-        return rc;
+        return fail(nullptr, Q3_ERR_CUDA, "q3_create: scratch of %zu bytes: %s", total, cudaGetErrorString(err));
     }
+    char* at = static_cast<char*>(e->scratch);
+    for (const Part& p : parts) {
+        *p.p = p.bytes ? at : nullptr;
+        at += padded(p.bytes);
+    }
+    int rc;
     {
         cudaStream_t cs = nullptr;
         if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) {
@@ -144,9 +141,7 @@ extern "C" void q3_destroy(q3_engine* e) {
     delete static_cast<std::vector<GraphEntry>*>(e->graphs);
     if (e->capture_stream) cudaStreamDestroy(static_cast<cudaStream_t>(e->capture_stream));
     persist_teardown(e);
-    void* bufs[] = {e->x, e->qkv, e->attn, e->hid, e->part, e->pval, e->pidx, e->status, e->sync, e->pf_desc, e->planes, e->xplanes, e->ssq, e->gate, e->up, e->logits_tc, e->lk_state};
-    for (void* p : bufs)
-        if (p) cudaFree(p);
+    if (e->scratch) cudaFree(e->scratch);
     delete e;
 }
 

@@ -24,7 +24,7 @@ struct q3_engine {
     int sm_count;
     int max_splits;     // attention splits the partial buffer is sized for
     int lm_grid;        // LM-head blocks the argmax partial buffers are sized for
-    // scratch (device)
+    void* scratch;      // the device allocation all of the following lie in
     float* x;       // [max_batch, 1024]  residual stream
     float* qkv;     // [max_batch, 4096]
     float* attn;    // [max_batch, 2048]

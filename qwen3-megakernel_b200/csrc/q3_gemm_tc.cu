@@ -30,7 +30,7 @@ static std::mutex& host_lock() { static std::mutex m; return m; }   // guards th
 constexpr int TC_THREADS = 192;    // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2..5: epilogue
 constexpr int TC_BM = 128;         // weight rows per tile (UMMA M)
 
-template <int BN, bool SCALE>   // SCALE: every token's column is multiplied by its RMS norm's scale (GemmTcParams::ssq)
+template <int BN, bool SCALE>   // SCALE: every token's column is multiplied by its RMS norm's scale (sums of squares in GemmTcParams::resid)
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w0,
                                                                 const __grid_constant__ CUtensorMap tm_w1,
                                                                 const __grid_constant__ CUtensorMap tm_w2,
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
             pdl_wait();
 #pragma unroll 4
             for (int j = warp - 2; j < BN; j += 4) {
-                const float ss = warp_sum(n0 + j < p.n_tok ? p.ssq[(size_t)lane * p.ssq_ld + n0 + j] : 0.f);
+                const float ss = warp_sum(n0 + j < p.n_tok ? p.resid[(size_t)lane * p.ldr + n0 + j] : 0.f);
                 if (lane == 0) s_scale[j] = rsqrtf(ss / (float)HIDDEN + EPS);
             }
             asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -649,11 +649,12 @@ cudaError_t launch_gemm_tc(const GemmTcCall& c, cudaStream_t st) {
     GemmTcParams p{};
     p.out = c.out; p.resid = c.resid; p.ldo = c.ldo; p.ldr = c.ldr; p.n_rows = c.n_rows; p.n_tok = c.n_tok; p.K = c.K;
     p.nsplit = c.nsplit; p.plane_rows = c.plane_rows; p.epi = c.resid ? TC_EPI_RESID : TC_EPI_STORE; p.status = c.status;
-    p.ssq = c.ssq; p.ssq_ld = c.ssq_ld;
     const int sm_count = sm_count_of_current_device();
     if (sm_count < 1) return cudaErrorInvalidDevice;
     const CUtensorMap maps[3] = {tw, tw, tw};
     if (c.ssq != nullptr) {
+        if (c.resid != nullptr) return cudaErrorInvalidValue;
+        p.resid = c.ssq; p.ldr = c.ssq_ld;
         if (bn == 32) return launch_bn<32, true>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
         if (bn == 64) return launch_bn<64, true>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
         return launch_bn<128, true>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);

@@ -12,7 +12,8 @@ enum { TC_EPI_STORE = 0, TC_EPI_RESID = 1, TC_EPI_ATOMIC = 2 };
 // device-side parameters
 struct GemmTcParams {
     float* out;            // [n_tok, ldo] fp32; element (t, n) at out[t * ldo + n]
-    const float* resid;    // TC_EPI_RESID: out = resid + acc (may alias out)
+    const float* resid;    // TC_EPI_RESID: out = resid + acc (may alias out).  gemm_tc_kernel<., true>: the partial sums of squares, column t is
+                           // scaled by rsqrt(sum of the 32 parts resid[i * ldr + t] / 1024 + eps)
     int ldo, ldr;
     int n_rows;            // weight rows (multiple of 128)
     int n_tok;             // valid tokens
@@ -29,8 +30,6 @@ struct GemmTcParams {
     int g_tiles[3];
     float* g_out[3];
     int g_ldo[3];
-    const float* ssq;      // column t is scaled by rsqrt(sum of the 32 parts ssq[i * ssq_ld + t] / 1024 + eps) (gemm_tc_kernel<., true>)
-    int ssq_ld;
 };
 
 // host-side call
