@@ -26,6 +26,8 @@
 // radix pass with one thread: 1 row, k = 50: 165 us, now 14; 64 rows, whole vocabulary: 70 us, now 25.
 #include <cooperative_groups.h>
 
+#include <cfloat>
+
 #include "q3_engine.h"
 
 namespace cg = cooperative_groups;
@@ -283,9 +285,12 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     }
 
     // ---- 3. weights of the kept logits: sums per warp, per block, over the row, in index order ----
+    // (a word masked with -inf weighs nothing at any temperature, and so does what lies past the end of a run: with 1 / T = 0 the
+    // exponential of the product would be NaN, not 0)
     const float inv_t = 1.f / temperature;
+    const float least = fmaxf(kth, -FLT_MAX);
     float ws = 0.f;
-    each([&](int, float v) { if (v >= kth) ws += __expf((v - vmax) * inv_t); });
+    each([&](int, float v) { if (v >= least) ws += __expf((v - vmax) * inv_t); });
     ws = warp_sum(ws);
     __syncthreads();
     if (lane == 0) sh.wf[warp] = ws;
@@ -320,7 +325,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
         const int i = first + tid;
         const float v = i < r1 ? row[i] : -INFINITY;
         const bool kept = i < r1 && v >= kth;
-        float incl = kept ? __expf((v - vmax) * inv_t) : 0.f;
+        float incl = v >= least ? __expf((v - vmax) * inv_t) : 0.f;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const float p = __shfl_up_sync(0xffffffffu, incl, o);

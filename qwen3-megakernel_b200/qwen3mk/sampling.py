@@ -43,10 +43,10 @@ def sample_reference(logits: torch.Tensor, temperature: float, top_k: int, u: to
     rows = logits.reshape(-1, logits.shape[-1]).double()
     if temperature <= 0 or top_k == 1:
         return rows.argmax(dim=-1).reshape(logits.shape[:-1])
-    keep = torch.ones_like(rows, dtype=torch.bool)
+    keep = rows > float("-inf")         # a masked word weighs nothing, at an infinite temperature too
     if 0 < top_k < rows.shape[-1]:
         kth = rows.topk(top_k, dim=-1).values[:, -1:]
-        keep = rows >= kth
+        keep &= rows >= kth
     w = torch.where(keep, torch.exp((rows - rows.max(dim=-1, keepdim=True).values) / temperature), torch.zeros_like(rows))
     cdf = w.cumsum(dim=-1)
     target = u.reshape(-1, 1).double().to(rows.device) * cdf[:, -1:]

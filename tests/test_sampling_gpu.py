@@ -146,3 +146,30 @@ def test_thousands_of_equal_logits_at_the_threshold_are_all_kept(top_k):
         j = int(got[b])
         assert bool(keep[0, j])
         assert (float(cdf[j - 1]) if j else 0.0) - CDF_TOL <= float(u[b]) <= float(cdf[j]) + CDF_TOL
+
+
+@pytest.mark.parametrize("vocab", [31, 2049, 151936])
+@pytest.mark.parametrize("top_k", [0, 50])
+@pytest.mark.parametrize("masked", [False, True])
+def test_infinite_temperature_draws_evenly_among_the_kept_words(vocab, top_k, masked):
+    """Every weight is 1 then, and the sums are counts, exact in fp32: the token is the kept word of rank floor(u * n), but
+    for the rounding of u * n itself (half a unit in the last place, below 0.01 of a word at these sizes)."""
+    from qwen3mk import sampling
+
+    g = torch.Generator().manual_seed(vocab + top_k)
+    logits = torch.randn(40, vocab, generator=g) * 3.0
+    if masked:
+        logits[:, 1::3] = float("-inf")
+    u = torch.rand(40, generator=g)
+    got = sampling.sample(logits.cuda(), float("inf"), top_k, u=u.cuda()).cpu()
+    for b in range(40):
+        row = logits[b]
+        kept = (row > float("-inf")).nonzero().flatten()
+        if 0 < top_k < vocab:
+            kept = kept[row[kept] >= row.topk(top_k).values[-1]]
+        rank = (kept == int(got[b])).nonzero()
+        assert rank.numel() == 1, f"row {b}: token {int(got[b])} is not among the kept words"
+        want = float(u[b].double()) * len(kept)
+        assert int(rank) - 0.01 <= want <= int(rank) + 1.01
+    ref = sampling.sample_reference(logits, float("inf"), top_k, u)
+    assert int((ref != got).sum()) <= 1
