@@ -324,8 +324,11 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     for (int first = r0; first < r1; first += SAMPLE_THREADS) {
         const int i = first + tid;
         const float v = i < r1 ? row[i] : -INFINITY;
-        const bool kept = i < r1 && v >= kth;
-        float incl = v >= least ? __expf((v - vmax) * inv_t) : 0.f;
+        // (the scan adds the same weights in another order for every lane, so a word without weight may see a larger prefix than the
+        // word before it: only one with a weight is a candidate)
+        const float own = v >= least ? __expf((v - vmax) * inv_t) : 0.f;
+        const bool kept = own > 0.f;
+        float incl = own;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const float p = __shfl_up_sync(0xffffffffu, incl, o);
@@ -344,7 +347,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
         __syncthreads();
         if (sh.need != 0xffffffffu) break;
     }
-    // rounding may leave the target a hair beyond the run's own sum: then its last kept element
+    // rounding may leave the target a hair beyond the run's own sum: then its last element with a weight
     if (tid == 0) out[row_id] = sh.need != 0xffffffffu ? (long long)sh.need : (long long)sh.cand_n;
 }
 

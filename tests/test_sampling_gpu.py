@@ -173,3 +173,25 @@ def test_infinite_temperature_draws_evenly_among_the_kept_words(vocab, top_k, ma
         assert int(rank) - 0.01 <= want <= int(rank) + 1.01
     ref = sampling.sample_reference(logits, float("inf"), top_k, u)
     assert int((ref != got).sum()) <= 1
+
+
+@pytest.mark.parametrize("vocab,batch", [(256, 20000), (5000, 1000), (151936, 30)])
+def test_a_word_without_weight_is_never_drawn(vocab, batch):
+    """Half of the words are masked, and the uniform numbers lie on the first boundaries of the row's own prefix sums and a few units
+    in the last place beside them, where the order of the additions decides on which side a target falls: a masked word must
+    not get it."""
+    from qwen3mk import sampling
+
+    g = torch.Generator().manual_seed(vocab)
+    logits = torch.randn(batch, vocab, generator=g)
+    logits[torch.rand(batch, vocab, generator=g) < 0.5] = float("-inf")
+    w = torch.where(logits > float("-inf"), torch.exp((logits - logits.amax(dim=-1, keepdim=True)) / 0.9), torch.zeros(()))
+    cdf = w.double().cumsum(dim=-1)
+    cdf /= cdf[:, -1:].clone()
+    dev = logits.cuda()
+    for trial in range(3):
+        u = cdf.gather(1, torch.randint(1, 64, (batch, 1), generator=g))[:, 0].float()
+        for ulps in range(-12, 13):
+            got = sampling.sample(dev, 0.9, 0, u=(u * (1.0 + ulps * 2.0 ** -24)).cuda()).cpu()
+            bad = (logits.gather(1, got[:, None])[:, 0] == float("-inf")).nonzero().flatten().tolist()
+            assert not bad, f"trial {trial}: {len(bad)} rows drew masked words: row {bad[0]}, word {int(got[bad[0]])}"
