@@ -285,12 +285,12 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     }
 
     // ---- 3. weights of the kept logits: sums per warp, per block, over the row, in index order ----
-    // (a word masked with -inf weighs nothing at any temperature, and so does what lies past the end of a run: with 1 / T = 0 the
+    // (a logit that is no number makes the total one, too: below; a word masked with -inf weighs nothing at any temperature, and so does what lies past the end of a run: with 1 / T = 0 the
     // exponential of the product would be NaN, not 0)
     const float inv_t = 1.f / temperature;
     const float least = fmaxf(kth, -FLT_MAX);
     float ws = 0.f;
-    each([&](int, float v) { if (v >= least) ws += __expf((v - vmax) * inv_t); });
+    each([&](int, float v) { if (!(v < least)) ws += __expf((v - vmax) * inv_t); });
     ws = warp_sum(ws);
     __syncthreads();
     if (lane == 0) sh.wf[warp] = ws;
@@ -310,8 +310,10 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
         if (r == rank) next = total;
     }
     // ---- 4. the first index whose inclusive prefix exceeds u * total ----
-    if (!(total > 0.f && total < INFINITY)) { write_argmax(); return; }     // infinite logits: the weights are not numbers
-    float target = uniform[row_id] * total;
+    // Weights that are not numbers (infinite logits, or a NaN among them), or a u outside [0, 1): no draw, the arg-max.
+    const float u = uniform[row_id];
+    if (!(total > 0.f && total < INFINITY && u >= 0.f && u < 1.f)) { write_argmax(); return; }
+    float target = u * total;
     if (!(target < total)) target = __uint_as_float(__float_as_uint(total) - 1u);   // u * total rounded up to the total: the last word with a weight
     if (!(base <= target && target < next)) return;
     // Inside the block: base + lo of the first warp is base, base + hi of the last one is next, and both are the same sums for

@@ -195,3 +195,20 @@ def test_a_word_without_weight_is_never_drawn(vocab, batch):
             got = sampling.sample(dev, 0.9, 0, u=(u * (1.0 + ulps * 2.0 ** -24)).cuda()).cpu()
             bad = (logits.gather(1, got[:, None])[:, 0] == float("-inf")).nonzero().flatten().tolist()
             assert not bad, f"trial {trial}: {len(bad)} rows drew masked words: row {bad[0]}, word {int(got[bad[0]])}"
+
+
+@pytest.mark.parametrize("vocab", [31, 2049, 151936])
+@pytest.mark.parametrize("top_k", [0, 50])
+def test_numbers_that_are_no_draw_give_the_argmax(vocab, top_k):
+    """A uniform number outside [0, 1) and a row with an infinite logit or a NaN have no draw: the arg-max of the numbers."""
+    from qwen3mk import sampling
+
+    g = torch.Generator().manual_seed(vocab)
+    logits = torch.randn(6, vocab, generator=g)
+    u = torch.tensor([-0.25, 1.0, 1.5, float("nan"), 0.5, 0.5])
+    want = logits.argmax(dim=-1)
+    logits[4, [7, 20]] = float("inf")
+    want[4] = 7
+    logits[5, int(want[5]) - 1] = float("nan")
+    out = torch.full((6,), -1, dtype=torch.int64, device="cuda")
+    assert sampling.sample(logits.cuda(), 0.9, top_k, u=u.cuda(), out=out).tolist() == want.tolist()
