@@ -340,7 +340,7 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
             t.seq_len = a->seq_len; t.part = e->part; t.layer = l; t.n_splits = ns; t.chunk_pad = pad; t.len_bound = len_bound;
             t.fused_prep = 1; t.qn = bf(w.qn); t.kn = bf(w.kn); t.rope = e->rope;
             t.k_write = reinterpret_cast<bf16_raw*>(a->k_write); t.v_write = reinterpret_cast<bf16_raw*>(a->v_write);
-            t.n_layers = L; t.append = append;
+            t.n_layers = L; t.append = append; t.qp_planes = B < Q3_TC_MIN_BATCH ? 3 : 2;
             if (ns <= CHAIN_MAX_SPLITS) {
                 t.planes_out = planes; t.plane_rows = rows; t.cluster = ns > 1; t.early = 1;
                 LAUNCH(launch_attn_split(t, B, st));
@@ -363,7 +363,9 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
             d.w[0] = bf(w.wd) + (size_t)l * HIDDEN * INTER;
             LAUNCH(launch_gemm_cluster(d, st));
         }
-        if (V % 128 == 0) {   // the LM head reads the last planes and applies the final norm's scale itself
+        // The LM head reads the last planes and applies the final norm's scale itself.  Few sequences keep the matrix-vector one: a tile's
+        // 64 additions into one accumulator, each truncated, leave logits 9.8e-7 from fp64, fp32 FMAs 1.2e-7 (19 us a step more for three).
+        if (V % 128 == 0 && B >= Q3_TC_MIN_BATCH) {
             float* logits = a->logits ? a->logits : e->logits_tc;
             GemmTcCall h{bf(w.embed), xp, logits, nullptr, V, 0, V, B, HIDDEN, 3, rows, e->status, e->ssq, ssq_ld};
             LAUNCH(launch_gemm_tc(h, st));

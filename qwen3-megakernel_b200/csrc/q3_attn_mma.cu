@@ -8,9 +8,14 @@
 // Only two of the eight head columns are real (the GQA pair that shares the K/V stream); the rest is padding the tensor
 // pipe does not mind, because the kernel is bound by bytes: the point of the tensor cores here is the INSTRUCTION count.
 // The CUDA-core kernel this replaced spent about 26 instructions per 256-byte row (unpack, 32 FMAs, shuffles) and topped out near 4 TB/s
-// on issue slots; this one spends about 8.  Accuracy: Q and P enter as two bf16 planes each (hi + lo), so scores and
-// outputs carry fp32-grade inputs against the exact bf16 K and V; the softmax runs in fp32 on base-2 exponentials
-// (log2 e is folded into the scale of Q).  Each warp owns a contiguous run of the chunk's positions with its own running
+// on issue slots; this one spends about 8.  Accuracy: Q and P enter as PL bf16 planes each against the exact bf16 K and V; the
+// softmax runs in fp32 on base-2 exponentials (log2 e is folded into the scale of Q).  Two planes are 16 significant bits.  Three
+// are fp32's 24, and then a tile's value products go to fresh accumulators that are added with rounding, because the
+// tensor core truncates what it adds to an accumulator.  Fewer than Q3_TC_MIN_BATCH sequences take three planes, so that a step costs
+// no accuracy against the kernels that serve one sequence in fp32: full model, logits rel-L2 against fp64 with two / three planes
+// (everything else in the step as accurate) 1.6e-5 / 1.7e-6 for two and three sequences; three planes, four accumulators in the
+// products and the LM head in fp32 cost three sequences at 900 positions 22 us a step (655 -> 677) and two at 3400 45 (739 -> 784).
+// Each warp owns a contiguous run of the chunk's positions with its own running
 // maximum; the warps and the new token's fp32 row are combined at the end, and the partial (max, sum, o[128]) per
 // head goes out in the format of the split kernel, so the merge (fused or separate) is unchanged.
 //
@@ -68,7 +73,7 @@ __device__ __forceinline__ void am_store_planes(const AttnArgs& a, int b, int co
 constexpr int AM_CLUSTER = 16;
 constexpr int AM_PART = 2 * (HEAD_DIM + 2) * 4;     // bytes of a split's partial
 
-template <int AM_WARPS, bool CL>
+template <int AM_WARPS, bool CL, int PL>
 __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma_kernel(const AttnArgs a) {
     constexpr int AM_THREADS = AM_WARPS * 32;
     pdl_launch();
@@ -168,8 +173,8 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
     }
     __syncthreads();
 
-    // ---- Q^T as the B operand: column fg is head fg (two real heads), k = dims; hi and lo planes; scores in units of log2 ----
-    uint32_t qh[8][2], ql[8][2];
+    // ---- Q^T as the B operand: column fg is head fg (two real heads), k = dims; PL planes; scores in units of log2 ----
+    uint32_t q[PL][8][2];
     {
         constexpr float QS = ATTN_SCALE * AM_LOG2E;
 #pragma unroll
@@ -181,8 +186,11 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
                     const float2 q2 = *reinterpret_cast<const float2*>(&s_new[fg][ks * 16 + h * 8 + 2 * ft]);
                     x0 = q2.x * QS; x1 = q2.y * QS;
                 }
-                qh[ks][h] = am_pack(x0, x1);
-                ql[ks][h] = am_pack(x0 - bf_lo(qh[ks][h]), x1 - bf_hi(qh[ks][h]));
+#pragma unroll
+                for (int j = 0; j < PL; ++j) {
+                    q[j][ks][h] = am_pack(x0, x1);
+                    x0 -= bf_lo(q[j][ks][h]); x1 -= bf_hi(q[j][ks][h]);
+                }
             }
     }
 
@@ -197,7 +205,7 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
         asm volatile("cp.async.wait_group %0;" ::"n"(AM_STAGES - 1) : "memory");
         __syncwarp();
         const uint32_t kst = am_smem(stage0 + (size_t)(i % AM_STAGES) * AM_STAGE), vst = kst + AM_HALF;
-        float c[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};     // (two chains: the products of one wait for one another)
+        float c[4] = {0.f, 0.f, 0.f, 0.f}, cl[PL - 1][4] = {};   // (a chain per plane: the products of one wait for one another)
         {
             const int row = lrow + (lmat & 1) * 8;               // matrices: (pos 0-7 | 8-15) x (dims lo 8 | hi 8) of the k step
 #pragma unroll
@@ -205,11 +213,12 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
                 uint32_t af[4];
                 const uint32_t addr = kst + (uint32_t)(row * 256 + (((2 * ks + (lmat >> 1)) ^ (row & 7)) << 4));
                 asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(af[0]), "=r"(af[1]), "=r"(af[2]), "=r"(af[3]) : "r"(addr));
-                am_mma(c, af, qh[ks][0], qh[ks][1]);
-                am_mma(c2, af, ql[ks][0], ql[ks][1]);
+                am_mma(c, af, q[0][ks][0], q[0][ks][1]);
+#pragma unroll
+                for (int j = 1; j < PL; ++j) am_mma(cl[j - 1], af, q[j][ks][0], q[j][ks][1]);
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) c[j] += c2[j];
+            for (int j = 0; j < 4; ++j) c[j] += PL == 3 ? cl[0][j] + cl[PL - 2][j] : cl[0][j];
         }
         // c[0], c[1]: position fg, heads 2 ft, 2 ft + 1; c[2], c[3]: position fg + 8
         const int pa = w0 + i * AM_TILE + fg;
@@ -227,20 +236,35 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
         const float ea0 = am_ex2(sa0 - n0), ea1 = am_ex2(sa1 - n1), eb0 = am_ex2(sb0 - n0), eb1 = am_ex2(sb1 - n1);
         l0 = fmaf(l0, f0, ea0 + eb0);
         l1 = fmaf(l1, f1, ea1 + eb1);
-        // P as hi + lo planes; transposed 8 x 8 blocks make the B operand (k = positions, n = heads)
-        const uint32_t pah = am_pack(ea0, ea1), pbh = am_pack(eb0, eb1);
-        const uint32_t pal = am_pack(ea0 - bf_lo(pah), ea1 - bf_hi(pah)), pbl = am_pack(eb0 - bf_lo(pbh), eb1 - bf_hi(pbh));
-        const uint32_t bh0 = am_transpose(pah), bh1 = am_transpose(pbh), bl0 = am_transpose(pal), bl1 = am_transpose(pbl);
+        // P as planes; transposed 8 x 8 blocks make the B operand (k = positions, n = heads)
+        uint32_t b0[PL], b1[PL];
+        {
+            float xa0 = ea0, xa1 = ea1, xb0 = eb0, xb1 = eb1;
+#pragma unroll
+            for (int j = 0; j < PL; ++j) {
+                const uint32_t pa2 = am_pack(xa0, xa1), pb2 = am_pack(xb0, xb1);
+                xa0 -= bf_lo(pa2); xa1 -= bf_hi(pa2); xb0 -= bf_lo(pb2); xb1 -= bf_hi(pb2);
+                b0[j] = am_transpose(pa2); b1[j] = am_transpose(pb2);
+            }
+        }
         {
             const int row = lrow + (lmat >> 1) * 8;              // matrices: (dims lo 8 | hi 8) x (pos 0-7 | 8-15), transposed on load
 #pragma unroll
             for (int mt = 0; mt < 8; ++mt) {
-                o[mt][0] *= f0; o[mt][1] *= f1; o[mt][2] *= f0; o[mt][3] *= f1;
                 uint32_t af[4];
                 const uint32_t addr = vst + (uint32_t)(row * 256 + (((2 * mt + (lmat & 1)) ^ (row & 7)) << 4));
                 asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(af[0]), "=r"(af[1]), "=r"(af[2]), "=r"(af[3]) : "r"(addr));
-                am_mma(o[mt], af, bh0, bh1);
-                am_mma(o[mt], af, bl0, bl1);
+                if constexpr (PL == 2) {
+                    o[mt][0] *= f0; o[mt][1] *= f1; o[mt][2] *= f0; o[mt][3] *= f1;
+                    am_mma(o[mt], af, b0[0], b1[0]);
+                    am_mma(o[mt], af, b0[1], b1[1]);
+                } else {
+                    float t[PL][4] = {};
+#pragma unroll
+                    for (int j = 0; j < PL; ++j) am_mma(t[j], af, b0[j], b1[j]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) o[mt][j] = fmaf(o[mt][j], j & 1 ? f1 : f0, t[0][j] + (t[1][j] + t[PL - 1][j]));
+                }
             }
         }
         __syncwarp();                                            // the stage is refilled by the next iteration's copies
@@ -367,9 +391,19 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
     }
 }
 
-template <int W, bool CL>
+template <int W, bool CL, int PL>
 static cudaError_t am_prepare() {
-    return cudaFuncSetAttribute(attn_mma_kernel<W, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, W * AM_STAGES * AM_STAGE + (CL ? AM_CLUSTER * AM_PART : 0));
+    const cudaError_t e = cudaFuncSetAttribute(attn_mma_kernel<W, CL, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, W * AM_STAGES * AM_STAGE + (CL ? AM_CLUSTER * AM_PART : 0));
+    return e != cudaSuccess || !CL ? e : cudaFuncSetAttribute(attn_mma_kernel<W, CL, PL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+
+template <int PL>
+static cudaError_t am_launch(const AttnArgs& a, dim3 grid, int warps, cudaStream_t st) {
+    const size_t smem = (size_t)(a.cluster ? 4 : warps) * AM_STAGES * AM_STAGE;
+    if (a.cluster)
+        return launch_chain_cluster(attn_mma_kernel<4, true, PL>, grid, dim3(128), smem + (size_t)a.n_splits * AM_PART, a.n_splits, st, a);
+    if (warps == 4) return launch_chain(attn_mma_kernel<4, false, PL>, grid, dim3(128), smem, st, a);
+    return launch_chain(attn_mma_kernel<8, false, PL>, grid, dim3(256), smem, st, a);
 }
 
 cudaError_t launch_attn_mma(const AttnArgs& a, int batch, cudaStream_t st) {
@@ -379,8 +413,8 @@ cudaError_t launch_attn_mma(const AttnArgs& a, int batch, cudaStream_t st) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!sm_count[dev]) {   // (a benign race between host threads: the same values are written)
-        if ((e = am_prepare<4, false>()) != cudaSuccess || (e = am_prepare<8, false>()) != cudaSuccess || (e = am_prepare<4, true>()) != cudaSuccess ||
-            (e = cudaFuncSetAttribute(attn_mma_kernel<4, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
+        if ((e = am_prepare<4, false, 2>()) != cudaSuccess || (e = am_prepare<8, false, 2>()) != cudaSuccess || (e = am_prepare<4, true, 2>()) != cudaSuccess ||
+            (e = am_prepare<4, false, 3>()) != cudaSuccess || (e = am_prepare<8, false, 3>()) != cudaSuccess || (e = am_prepare<4, true, 3>()) != cudaSuccess)
             return e;
         int n = 0;
         if ((e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
@@ -389,13 +423,8 @@ cudaError_t launch_attn_mma(const AttnArgs& a, int batch, cudaStream_t st) {
     const dim3 grid(a.n_splits, KV_HEADS, batch);
     const bool big = KV_HEADS * batch >= sm_count[dev];
     const int warps = big || a.early ? 4 : 8;
-    const size_t smem = (size_t)(a.cluster ? 4 : warps) * AM_STAGES * AM_STAGE;
-    if (a.cluster) {
-        if (a.n_splits > AM_CLUSTER || a.planes_out == nullptr) return cudaErrorInvalidValue;
-        return launch_chain_cluster(attn_mma_kernel<4, true>, grid, dim3(128), smem + (size_t)a.n_splits * AM_PART, a.n_splits, st, a);
-    }
-    if (warps == 4) return launch_chain(attn_mma_kernel<4, false>, grid, dim3(128), smem, st, a);
-    return launch_chain(attn_mma_kernel<8, false>, grid, dim3(256), smem, st, a);
+    if (a.cluster && (a.n_splits > AM_CLUSTER || a.planes_out == nullptr)) return cudaErrorInvalidValue;
+    return a.qp_planes == 3 ? am_launch<3>(a, grid, warps, st) : am_launch<2>(a, grid, warps, st);
 }
 
 }  // namespace q3

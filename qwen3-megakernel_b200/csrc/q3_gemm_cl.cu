@@ -18,6 +18,13 @@
 //   CL_RESID  64-row tiles of Wo or Wd: 16 tiles             x += planes . W; planes of x * gain; sums of squares
 //   CL_SILU   64 rows of Wg and the same 64 of Wu: 48 tiles  planes of silu(gate * r) * (up * r)
 //
+// NACC: accumulators the k steps of a slice go to in turn.  The tensor core truncates every sum it adds to an accumulator, so the
+// result is short by about half a unit in the last place a step; the epilogue adds the accumulators with rounding.  Fewer than
+// Q3_TC_MIN_BATCH sequences take four, because the kernels that serve them otherwise add in fp32 or exactly: logits rel-L2 against
+// fp64, two sequences at 16 / 1000 positions and three at 900, with two accumulators 1.31, 1.84 and 1.79e-6, with four 1.16, 1.66 and
+// 1.66e-6 (with one, and the LM head truncating as well, 2.16, 2.70 and 2.68e-6); the persistent kernel, one sequence after the other,
+// 1.23, 1.76 and 1.83e-6.  In larger batches the two planes of the attention leave 1.7e-5 whatever the products do.
+//
 // Measured (one B200, us per step, before -> after): 8 sequences x 1024 positions 984 -> 735, 64 x 1024 2333 -> 2075, one at
 // 5000 positions 1606 -> 793.  What bounds it: a launch is about 3.4 us of latencies in series (release of the wait to the first
 // plane 0.5, products 0.7, partial tile out 0.3, to the owners 0.5, finished row 0.6, end of the grid to the next release 0.7) beside
@@ -35,6 +42,8 @@ namespace q3 {
 
 constexpr int CL_THREADS = 192;   // warp 0: TMA, warp 1: MMA and TMEM, warps 2..5: epilogue
 constexpr int CL_MAX_STAGES = 6;
+constexpr int CL_FEW = 4;          // most tokens of the kernels with several accumulators
+static_assert(Q3_TC_MIN_BATCH <= CL_FEW, "a batch below it fits");
 
 struct ClusterGemmParams {
     int kb_total;                 // k blocks of 64
@@ -75,7 +84,7 @@ template <int KIND, int BN> struct ClShape {
     static constexpr int RED_BYTES = C * SLOTS * TM * 4;                                  // partial tiles of the owned tokens
 };
 
-template <int KIND, int BN>
+template <int KIND, int BN, int NACC>
 __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
                                                                      const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_x,
                                                                      const ClusterGemmParams p) {
@@ -113,7 +122,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
         abort_flag = 0;
     }
     // the planes of a stage lie side by side: nsplit * BN columns of one B operand (192 at most)
-    const uint32_t cols = (uint32_t)(nsplit * BN), tmem_cols = cols <= 32 ? 32u : cols <= 64 ? 64u : cols <= 128 ? 128u : 256u;
+    const uint32_t cols = (uint32_t)(nsplit * BN), acc_cols = cols <= 32 ? 32u : cols <= 64 ? 64u : cols <= 128 ? 128u : 256u, tmem_cols = NACC * acc_cols;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_base_s)), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -179,7 +188,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
                     const uint64_t da = da0 + ds + 2 * k, db = db0 + ds + 2 * k;
                     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                                 ::"r"(tmem_base), "l"(da), "l"(db), "r"(idesc), "r"((uint32_t)(kb | k)), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
+                                 ::"r"(tmem_base + (uint32_t)(k % NACC) * acc_cols), "l"(da), "l"(db), "r"(idesc), "r"((uint32_t)(kb | (k / NACC))), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&empty_bar[s])) : "memory");
             }
@@ -225,6 +234,25 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
     {
         const bool live = TM == 128 || lane < 16;
         float* stage = reinterpret_cast<float*>(base) + (TM == 128 ? quad * 32 + lane : quad * 16 + (lane & 15));   // [C][SLOTS][TM]
+        if constexpr (NACC > 1) {            // at most CL_FEW tokens: their columns of every accumulator and plane under one wait
+            uint32_t r[NACC][3][CL_FEW];
+#pragma unroll
+            for (int ac = 0; ac < NACC; ++ac)
+#pragma unroll
+                for (int sp = 0; sp < 3; ++sp) tc_ld4(r[ac][sp], tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)ac * acc_cols + sp * BN);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < CL_FEW; ++j) {
+                float v[3];
+#pragma unroll
+                for (int sp = 0; sp < 3; ++sp) {
+                    v[sp] = __uint_as_float(r[0][sp][j]);
+#pragma unroll
+                    for (int ac = 1; ac < NACC; ++ac) v[sp] += __uint_as_float(r[ac][sp][j]);
+                }
+                if (live) stage[((j % C) * SLOTS + j / C) * TM] = v[0] + (v[1] + v[2]);
+            }
+        } else {
         constexpr int STEP = BN < 32 ? BN : 32;
 #pragma unroll
         for (int c0 = 0; c0 < BN; c0 += STEP) {
@@ -248,6 +276,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
                 if (nsplit > 2) v += __uint_as_float(q2[j]);
                 if (live) stage[(((c0 + j) % C) * SLOTS + (c0 + j) / C) * TM] = v;
             }
+        }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -339,7 +368,7 @@ int gemm_cluster_rows(int n_tok) {
     return (n_tok + bn - 1) / bn * bn;
 }
 
-template <int KIND, int BN>
+template <int KIND, int BN, int NACC>
 static cudaError_t launch_cl(const CUtensorMap* tw, const CUtensorMap& tx, ClusterGemmParams p, int tiles, cudaStream_t st) {
     using S = ClShape<KIND, BN>;
     constexpr int MAX_SMEM = 220 * 1024;
@@ -348,7 +377,7 @@ static cudaError_t launch_cl(const CUtensorMap* tw, const CUtensorMap& tx, Clust
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!attr_set[dev]) {
-        if ((e = cudaFuncSetAttribute(gemm_cluster_kernel<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(gemm_cluster_kernel<KIND, BN, NACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM)) != cudaSuccess) return e;
         attr_set[dev] = true;
     }
     const int stage_bytes = S::TM * TC_BK * 2 + p.nsplit * BN * TC_BK * 2;
@@ -362,20 +391,26 @@ static cudaError_t launch_cl(const CUtensorMap* tw, const CUtensorMap& tx, Clust
     const int need = (S::RED_BYTES + stage_bytes - 1) / stage_bytes;   // the stages also hold the outgoing partial tile
     if (stages < need) stages = need;
     p.stages = stages;
-    // A block holds its TMEM columns until its whole cluster has met, so the blocks of a launch that share an SM must all get
-    // theirs at once: the shared memory asked for never lets more of them in than 512 columns serve.
-    const int cols = p.nsplit * BN, tmem_cols = cols <= 32 ? 32 : cols <= 64 ? 64 : cols <= 128 ? 128 : 256;
-    const int floor_bytes = 228 * 1024 / (512 / tmem_cols + 1) + 1;
+    // A block holds its TMEM columns until its whole cluster has met, so every block on an SM has to get its columns without waiting
+    // for another's: whatever cluster products share an SM, of this launch, of its neighbours in the stream or of an engine on
+    // another stream, their columns never exceed the SM's 512.  Every block asks for so much shared memory that at most three fit, and one with
+    // 256 columns for so much that no third fits beside two of them: 3 x 128 or 256 + 2 x 128 or 2 x 256 at most.  The
+    // layer kernel (q3_layer_tc.cu), whose blocks wait for one another too, leaves room for one block of 128 columns beside its
+    // 128.  The other kernels with TMEM wait for nothing but their predecessor in the stream, which has all its columns by then.
+    constexpr int SM_SMEM = 228 * 1024, THIRD = 58 * 1024, HALF = 88 * 1024;
+    static_assert(4 * THIRD > SM_SMEM && 2 * HALF + THIRD > SM_SMEM && NACC * BN * 4 <= 256, "TMEM columns of an SM");
     int smem = stages * stage_bytes + S::RED_BYTES + 1024;
-    if (smem < floor_bytes) smem = floor_bytes;
-    return launch_chain_cluster(gemm_cluster_kernel<KIND, BN>, dim3(S::C, tiles, (p.n_tok + BN - 1) / BN), dim3(CL_THREADS), (size_t)smem, S::C, st,
+    const int least = NACC * p.nsplit * BN > 128 ? HALF : THIRD;
+    if (smem < least) smem = least;
+    return launch_chain_cluster(gemm_cluster_kernel<KIND, BN, NACC>, dim3(S::C, tiles, (p.n_tok + BN - 1) / BN), dim3(CL_THREADS), (size_t)smem, S::C, st,
                                 tw[0], tw[1], tw[2], tx, p);
 }
 
 template <int KIND>
 static cudaError_t launch_kind(const CUtensorMap* tw, const CUtensorMap& tx, const ClusterGemmParams& p, int tiles, int bn, cudaStream_t st) {
-    if (bn == 16) return launch_cl<KIND, 16>(tw, tx, p, tiles, st);
-    return launch_cl<KIND, 32>(tw, tx, p, tiles, st);
+    if (p.n_tok < Q3_TC_MIN_BATCH && p.nsplit == 3) return launch_cl<KIND, 16, 4>(tw, tx, p, tiles, st);
+    if (bn == 16) return launch_cl<KIND, 16, 1>(tw, tx, p, tiles, st);
+    return launch_cl<KIND, 32, 1>(tw, tx, p, tiles, st);
 }
 
 cudaError_t launch_gemm_cluster(const ClusterGemmCall& c, cudaStream_t st) {

@@ -81,6 +81,7 @@ struct AttnArgs {
     bf16_raw* planes_out;
     int plane_rows;
     int cluster;                      // the splits are a cluster of blocks (at most 16) that writes planes_out itself
+    int qp_planes;                    // bf16 planes q and the probabilities enter the products as: 3, or 2 (any other value)
     int early;                        // the predecessor lets this launch start only when everything before it has completed: lengths and
                                       // cached rows may be read before the wait (blocks of four warps, which fit beside its blocks)
 };

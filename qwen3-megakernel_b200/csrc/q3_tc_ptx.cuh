@@ -70,6 +70,10 @@ __device__ __forceinline__ void tc_ld16(uint32_t* r, uint32_t taddr) {   // 16 c
                  : "r"(taddr) : "memory");
 }
 
+__device__ __forceinline__ void tc_ld4(uint32_t (&r)[4], uint32_t taddr) {   // 4 columns of this warp's 32 TMEM lanes; no wait
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+
 // one 2-D box [rows of the map's box] x [64 k] into shared memory, counted on an mbarrier
 __device__ __forceinline__ void tc_load_box(uint32_t dst, const void* map, int k, int row, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"

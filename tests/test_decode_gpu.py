@@ -182,6 +182,61 @@ def test_batches_at_the_edges_of_the_token_tiles(oracle, batch):
     assert all(torch.equal(first[k], out[k]) for k in ("k_write", "v_write"))
 
 
+def decode_fp64(inp, tokens, kcs, vcs, rope):
+    """The decode step in fp64 from the bf16 weights and rows and the engine's RoPE table: logits [batch, vocab]."""
+    w = {k: v.double() for k, v in inp.items() if k not in ("token", "kcache", "vcache")}
+
+    def norm(x, gain):
+        return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-6) * gain
+
+    def turn(x, pos):
+        c, s = rope[pos].double().split(64)
+        return torch.cat([x[:, :64] * c - x[:, 64:] * s, x[:, 64:] * c + x[:, :64] * s], dim=1)
+
+    rows = []
+    for tok, kc, vc in zip(tokens, kcs, vcs):
+        n = kc.shape[1]
+        x = w["embed"][int(tok)]
+        for l in range(w["wq"].shape[0]):
+            h = norm(x, w["ln1"][l])
+            q = turn(norm((w["wq"][l] @ h).view(16, 128), w["qn"][l]), n)
+            k = turn(norm((w["wk"][l] @ h).view(8, 128), w["kn"][l]), n)
+            k_all = torch.cat([kc[l].double(), k[None]]).repeat_interleave(2, dim=1)
+            v_all = torch.cat([vc[l].double(), (w["wv"][l] @ h).view(1, 8, 128)]).repeat_interleave(2, dim=1)
+            p = torch.softmax(torch.einsum("hd,shd->hs", q, k_all) / 128 ** 0.5, dim=-1)
+            x = x + w["wo"][l] @ torch.einsum("hs,shd->hd", p, v_all).reshape(2048)
+            h = norm(x, w["ln2"][l])
+            x = x + w["wd"][l] @ (torch.nn.functional.silu(w["wg"][l] @ h) * (w["wu"][l] @ h))
+        rows.append(w["embed"] @ norm(x, w["fnorm"]))
+    return torch.stack(rows)
+
+
+def test_few_sequences_are_as_close_to_fp64_as_one(oracle):
+    """Two and three sequences run as a batch, one runs in the persistent kernel, whose products and sums are fp32 or
+    better: a batch must not be further from fp64.  Over nine batches the two differ by the luck of the roundings, a few
+    percent of 2e-6; two bf16 planes of q and the probabilities would be eight times as far."""
+    from qwen3mk.kernel import SeqTable
+
+    shp = oracle.Shape(layers=6, vocab=2048)
+    far = {"auto": 0.0, "persist": 0.0}
+    for seed, lens in enumerate([(16, 30), (250, 250), (1000, 700), (3000, 1500), (900, 600, 300), (3400, 20, 5), (60, 61), (2000, 1), (500, 400, 450)]):
+        inp = oracle.synthetic(60 + seed, shp, context=1)
+        g = torch.Generator().manual_seed(seed)
+        toks = torch.randint(0, 2048, (len(lens),), generator=g)
+        kcs = [torch.randn(6, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens]
+        vcs = [torch.randn(6, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens]
+        for path in far:
+            mk = engine(path, layers=6, vocab=2048, max_batch=len(lens))
+            out = mk.bind_sequences(to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}), toks.cuda(), SeqTable([k.cuda() for k in kcs], [v.cuda() for v in vcs]))
+            mk.launch()
+            mk.status()
+            if path == "auto":
+                ref = decode_fp64(inp, toks, kcs, vcs, mk.rope.cpu())
+            far[path] += oracle.rel_l2(out["logits"], ref) / 9
+    print(f"mean logits rel-L2 against fp64: batch {far['auto']:.2e}, one at a time {far['persist']:.2e}")
+    assert far["auto"] <= 1.15 * far["persist"]
+
+
 @pytest.mark.parametrize("path", PATHS)
 def test_prefill_2048_then_greedy_decode(oracle, small, path):
     """The benchmark's third shape on a small model: a 2048-token prompt on the GPU, then chained greedy steps over
