@@ -36,10 +36,16 @@ int q3::engine_fail(q3_engine* e, int code, const char* fmt, ...) {
 // ------------------------------------------------------------------------------------------------
 // CUDA graphs for the layered step: a step is hundreds of small launches whose arguments all live in
 // device memory, so a call with the same argument block can replay a captured graph instead of
-// re-issuing them.  A key is seen uncaptured once (which also performs one-time function attribute
-// set-up), captured on its second use, and replayed afterwards.  Weights, RoPE table or trace changes
+// re-issuing them.  A key's first uses are plain launches (which also perform one-time function attribute
+// set-up), then it is captured, and replayed afterwards.  Weights, RoPE table or trace changes
 // drop the cache.
 // ------------------------------------------------------------------------------------------------
+// The key holds the addresses of one bind, so every bind captures anew.  A capture costs the host 450 to 850 us, beside 360 for the
+// plain launches of a step; after three steps that are launched without waiting the GPU is far enough behind to hide it (8 x 1024, a fresh
+// bind of 8 steps, capture on the 2nd / 4th: 6070 / 5910 us; of 2 steps 1680 / 1540).  Two sequences pay it back more slowly,
+// for the persistent kernel serves them almost as fast: from eight steps on even a caller who waits for every step has gained it (at 16
+// positions 4 steps: persistent 2880, captured on the 4th 3110; a plain step 669 against 728).
+static int plain_uses(int batch) { return batch == 2 ? 8 : 3; }
 struct GraphEntry {
     q3_decode_args key;
     int n_splits;
@@ -551,9 +557,10 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
     CU(e, cudaSetDevice(e->device));
     cudaStream_t st = (cudaStream_t)stream;
     uint32_t path = a->flags & Q3_F_PATH_MASK;
-    // The persistent kernel decodes one sequence per launch: from two on, one chain over all of them is as fast or faster (at
-    // 16 / 250 / 1000 positions, one after the other against the chain: two sequences 691 / 773 / 913 and 574 / 605 / 618 us,
-    // three 1035 / 1160 / 1369 and 582 / 609 / 632 us; one sequence 347 / 384 / 456 and 567 / 591 / 603 us).
+    // The persistent kernel decodes one sequence per launch: from two on, one chain over all of them is faster and as close to fp64 (one
+    // after the other against the chain: two sequences at 16 / 250 / 3400 positions 702 / 755 / 1341 and 593 / 622 / 766 us, three at 900
+    // 1331 and 651 us; in plain launches, before a graph replays them, two at 16 positions 703 and 650 us; one sequence at 16 / 250 /
+    // 1000 347 / 384 / 456 us against 567 and more).
     if (path == Q3_F_PATH_AUTO)
         path = persist_supports(e, a) && (a->batch == 1 || !chain_serves(e, a->batch)) ? Q3_F_PATH_PERSIST : Q3_F_PATH_LAYERED;
     if (path == Q3_F_PATH_PERSIST) {
@@ -586,7 +593,7 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
         e->launches += hit->launches;
         return Q3_OK;
     }
-    if (hit->seen++ == 0) return decode_layered(e, a, st, 3, nullptr, layer_kernel);   // first use: plain launches
+    if (hit->seen++ < plain_uses(a->batch)) return decode_layered(e, a, st, 3, nullptr, layer_kernel);
     const int64_t before = e->launches;
     // capture on the engine's own stream (the legacy default stream cannot be captured); nothing runs during capture
     cudaStream_t cs = static_cast<cudaStream_t>(e->capture_stream);
