@@ -31,6 +31,12 @@
 // 1..2 us of weight bytes that overlap them.
 //
 // Weight tiles are requested before the wait for the previous launch, so that their latency overlaps its tail.
+//
+// A wait that gives up (status words).  A block whose accumulator is not complete sends nothing and stores nothing; one that does
+// not receive every partial stores nothing.  Whoever gave up still meets its cluster at every barrier, and a partial tile is only
+// ever sent before the last one: behind it nobody sends any more, and a block that still lacks a partial waits once more, for
+// copies that were on their way when it gave up, before it leaves.  The receivers' limit is twice the senders', so a
+// late sender has given up or delivered before a receiver gives up.  The stages and TMEM are drained the same way.
 #include <cuda.h>
 
 #include "q3_engine.h"
@@ -42,6 +48,7 @@ namespace q3 {
 
 constexpr int CL_THREADS = 192;   // warp 0: TMA, warp 1: MMA and TMEM, warps 2..5: epilogue
 constexpr int CL_MAX_STAGES = 6;
+constexpr unsigned long long CL_RED_WAIT_NS = 2 * TC_WAIT_NS;
 constexpr int CL_FEW = 4;          // most tokens of the kernels with several accumulators
 static_assert(Q3_TC_MIN_BATCH <= CL_FEW, "a batch below it fits");
 
@@ -142,7 +149,9 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
     const int orow = KIND == CL_QKV ? te : te & 63, osub = KIND == CL_QKV ? 0 : te >> 6;
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (elect_one()) {
+        int armed = 0;                           // k blocks whose loads have been requested
+        const bool one = elect_one();
+        if (one) {
             const CUtensorMap* tm_w = &tm_w0;
             int m0 = tile * TM;
             if (KIND == CL_QKV) {
@@ -155,6 +164,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
                 asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(&full_bar[s])), "r"(stage_bytes) : "memory");
                 tc_load_box(st, tm_w, (kb0 + kb) * TC_BK, m0, &full_bar[s]);
                 if (KIND == CL_SILU) tc_load_box(st + A_BYTES / 2, &tm_w1, (kb0 + kb) * TC_BK, m0, &full_bar[s]);
+                armed = kb + 1;
             };
             const int ahead = min(nkb, stages);
             for (int kb = 0; kb < ahead; ++kb) weights(kb, kb);
@@ -172,7 +182,13 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
         }
         __syncwarp();
         cl_wait();
-    } else if (warp == 1) {
+        cl_arrive();
+        cl_wait();
+        if (one && abort_flag)                   // (the last `stages` of them may still be on their way)
+            for (int kb = max(0, armed - stages); kb < armed; ++kb) tc_drain(&full_bar[kb % stages], (kb / stages) & 1);
+        return;
+    }
+    if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
         if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((cols >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
@@ -197,10 +213,10 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
         __syncwarp();
         cl_wait();
         asm volatile("bar.sync 2, 160;" ::: "memory");              // the epilogue warps have read the accumulator
+        if (abort_flag) tc_drain(&acc_bar, 0);                      // ... or gave it up: the products that were issued end first
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
-    }
-    if (warp < 2) {
         cl_arrive();
         cl_wait();
         return;
@@ -226,12 +242,13 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
             xr[i] = s < my_slots ? p.out[(size_t)(n0 + s * C + rank) * p.ldo + tile * TM + orow] : 0.f;
         }
     }
-    tc_wait_warp(&acc_bar, 0, &abort_flag, p.status, 52);
+    // (the MMA thread commits to acc_bar after a wait of its own gave up, too, so that its products can be drained: the flag tells)
+    const bool summed = __all_sync(0xffffffffu, tc_wait_warp(&acc_bar, 0, &abort_flag, p.status, 52) && !abort_flag);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // The partial tile goes to this block's staging area (the stages are free: every MMA has completed), token by token and
     // grouped by owner, and from there to the owners with one bulk copy each, counted on the owner's mbarrier.
     // (a tile of 64 rows occupies the first 16 lanes of every 32-lane quarter)
-    {
+    if (summed) {
         const bool live = TM == 128 || lane < 16;
         float* stage = reinterpret_cast<float*>(base) + (TM == 128 ? quad * 32 + lane : quad * 16 + (lane & 15));   // [C][SLOTS][TM]
         if constexpr (NACC > 1) {            // at most CL_FEW tokens: their columns of every accumulator and plane under one wait
@@ -284,20 +301,21 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
     asm volatile("bar.arrive 2, 160;" ::: "memory");
     cl_wait();                                   // every block of the cluster has set its mbarrier up
     asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (te < C && slots_of(te) > 0) {
+    const bool whole = !abort_flag;               // no warp of this block gave up on the accumulator
+    if (whole && te < C && slots_of(te) > 0) {
         const uint32_t src = tc_smem(base) + (uint32_t)(te * SLOTS * TM * 4);
         asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                      ::"r"(cl_map(tc_smem(red + (size_t)rank * SLOTS * TM), te)), "r"(src), "r"((uint32_t)(slots_of(te) * TM * 4)), "r"(cl_map(tc_smem(&red_bar), te)) : "memory");
     }
     __syncwarp();
-    if (my_slots > 0) tc_wait_warp(&red_bar, 0, &abort_flag, p.status, 53);
-    cl_arrive();      // (matched before the exit: this block has received everything, so nobody's copies are still under way then)
+    const bool received = my_slots > 0 && whole && tc_wait_warp(&red_bar, 0, &abort_flag, p.status, 53, CL_RED_WAIT_NS);
+    cl_arrive();      // (matched before the exit: this block sends nothing any more)
 
     // the owned tokens: add the slices in order and finish the row
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const int s = osub + i * OSTEP, t = n0 + s * C + rank;
-        if (s >= my_slots) break;
+        if (s >= my_slots || !received) break;
         const float* src = red + s * TM + orow;
         float v = src[0];
 #pragma unroll
@@ -321,6 +339,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
         }
     }
     cl_wait();
+    if (my_slots > 0 && !received && te == 0) tc_drain(&red_bar, 0);
 }
 
 // ---- embedding gather with the first layer's planes: one block per sequence ----------------------------------------

@@ -11,7 +11,8 @@ __device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__
 __device__ __forceinline__ unsigned long long tc_ns() { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
 
 // bounded mbarrier wait; on timeout sets *abort_flag and returns false
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t site) {
+[[nodiscard]] __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t site,
+                                                      unsigned long long limit = TC_WAIT_NS) {
     unsigned it = 0;
     unsigned long long t0 = 0;
     for (;;) {
@@ -23,7 +24,7 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile
         if ((++it & 63u) == 0) {
             const unsigned long long t = tc_ns();
             if (t0 == 0) t0 = t;
-            else if (t - t0 > TC_WAIT_NS) {
+            else if (t - t0 > limit) {
                 report(status, ST_MBAR_TIMEOUT, site, parity);
                 *abort_flag = 1;
                 return false;
@@ -34,10 +35,20 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile
 
 // The same for a whole converged warp: one lane polls.  32 polling lanes are 32 requests to the barrier unit, and those of the
 // epilogue warps stand in front of the MMA thread's own (a wait that was already over took it 190 ns instead of 30).
-__device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t site) {
+[[nodiscard]] __device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t site,
+                                                           unsigned long long limit = TC_WAIT_NS) {
     int ok = 0;
-    if ((threadIdx.x & 31) == 0) ok = tc_wait(bar, parity, abort_flag, status, site);
+    if ((threadIdx.x & 31) == 0) ok = tc_wait(bar, parity, abort_flag, status, site, limit);
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
+// After a wait has given up: let what is still under way to this block land before its memory is somebody else's.  Bounded, reports nothing.
+static __device__ __noinline__ void tc_drain(uint64_t* bar, uint32_t parity) {
+    const unsigned long long t0 = tc_ns();
+    uint32_t ok = 0;
+    while (!ok && tc_ns() - t0 <= TC_WAIT_NS)
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(tc_smem(bar)), "r"(parity) : "memory");
 }
 
 // shared-memory matrix descriptor of a K-major tile with 128-byte swizzle: rows of 128 bytes, 8-row

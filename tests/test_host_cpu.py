@@ -203,3 +203,18 @@ def test_load_hf_reads_a_sharded_checkpoint_end_to_end(tmp_path):
     (tmp_path / "model-00002-of-00002.safetensors").unlink()
     with pytest.raises(KeyError, match="model.layers.1"):
         weights.load_hf(str(tmp_path), layers=L, vocab=V)
+
+
+def test_no_bounded_wait_of_the_tensor_core_kernels_is_dropped():
+    """A bounded wait that gives up says so by its result: what comes behind it may not run as if it had ended.  A call whose
+    result nobody takes stands at the start of a statement."""
+    waits = re.compile(r"\b(tc_wait|tc_wait_warp|at_wait|at_wait_warp)\s*\(")
+    dropped, seen = [], 0
+    for path in sorted((ROOT / "qwen3-megakernel_b200" / "csrc").glob("*.cu*")):
+        code = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in waits.finditer(code):
+            before = code[:m.start()].rstrip()
+            seen += 1
+            if before[-1:] in ";{})":
+                dropped.append(f"{path.name}:{code.count(chr(10), 0, m.start()) + 1}")
+    assert seen > 20 and not dropped, dropped
