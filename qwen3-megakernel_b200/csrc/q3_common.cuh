@@ -106,6 +106,16 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
     return one != 0;
 }
+// A wait that one lane of a converged warp performs for all 32.  The shuffle hands over the answer but orders no memory: the
+// __syncwarp does, so that what the waiting lane has seen complete is complete for the others, too.
+template <typename Wait>
+__device__ __forceinline__ bool one_lane_waits(Wait&& wait) {
+    int ok = 0;
+    if ((threadIdx.x & 31) == 0) ok = wait();
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();
+    return ok != 0;
+}
 // the warp's index as a value the compiler knows to be uniform
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 

@@ -67,9 +67,7 @@ __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile
 }
 // One lane of a converged warp polls for all 32: the polls of 16 softmax warps, a request a lane, delay the MMA thread's own.
 __device__ __forceinline__ bool at_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t site) {
-    int ok = 0;
-    if ((threadIdx.x & 31) == 0) ok = at_wait(bar, parity, abort_flag, status, site);
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+    return one_lane_waits([&] { return at_wait(bar, parity, abort_flag, status, site); });
 }
 
 // K-major operand, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart (as in the GEMM)

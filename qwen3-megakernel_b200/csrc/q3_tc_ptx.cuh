@@ -37,9 +37,7 @@ __device__ __forceinline__ unsigned long long tc_ns() { unsigned long long t; as
 // epilogue warps stand in front of the MMA thread's own (a wait that was already over took it 190 ns instead of 30).
 [[nodiscard]] __device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t site,
                                                            unsigned long long limit = TC_WAIT_NS) {
-    int ok = 0;
-    if ((threadIdx.x & 31) == 0) ok = tc_wait(bar, parity, abort_flag, status, site, limit);
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+    return one_lane_waits([&] { return tc_wait(bar, parity, abort_flag, status, site, limit); });
 }
 
 // After a wait has given up: let what is still under way to this block land before its memory is somebody else's.  Bounded, reports nothing.

@@ -218,3 +218,13 @@ def test_no_bounded_wait_of_the_tensor_core_kernels_is_dropped():
             if before[-1:] in ";{})":
                 dropped.append(f"{path.name}:{code.count(chr(10), 0, m.start()) + 1}")
     assert seen > 20 and not dropped, dropped
+
+
+def test_a_wait_by_one_lane_orders_memory_for_its_warp():
+    """A shuffle passes the answer of the polling lane on but orders no memory; both polling helpers go through the one place
+    where a __syncwarp follows it."""
+    csrc = ROOT / "qwen3-megakernel_b200" / "csrc"
+    assert re.search(r"one_lane_waits\(Wait&& wait\) \{[^}]*__shfl_sync[^}]*__syncwarp\(\);[^}]*\}", (csrc / "q3_common.cuh").read_text())
+    for name, helper in (("q3_tc_ptx.cuh", "tc_wait_warp"), ("q3_prefill_attn_tc.cu", "at_wait_warp")):
+        body = re.search(rf"bool {helper}\([^{{]*\{{(.*?)\n\}}", (csrc / name).read_text(), re.S).group(1)
+        assert "one_lane_waits(" in body and "__shfl_sync" not in body, name
