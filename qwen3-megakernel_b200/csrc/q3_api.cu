@@ -66,6 +66,8 @@ static void drop_graphs(q3_engine* e) {
     v->clear();
 }
 
+constexpr int CHAIN_MAX_BATCH = 64;   // most sequences whose decode step runs as five launches per layer (chain_serves below)
+
 extern "C" const char* q3_version(void) { return "q3mk-b200 0.1 sm_100a"; }
 
 extern "C" const char* q3_last_error(const q3_engine* e) { return e ? e->err : g_create_error; }
@@ -96,6 +98,7 @@ extern "C" int q3_create(int device, const q3_config* cfg, q3_engine** out) {
     e->part_slots = (int)((B < 16 ? B : 16) * Q3_MAX_SPLITS > 2 * B ? (B < 16 ? B : 16) * Q3_MAX_SPLITS : 2 * B);
     const bool tc = e->cap >= Q3_TC_MIN_BATCH;
     const size_t cap_pad = (B + 127) / 128 * 128;
+    e->chain_rows = gemm_cluster_rows(cfg->max_batch < CHAIN_MAX_BATCH ? cfg->max_batch : CHAIN_MAX_BATCH);
     // one allocation for all of it: every cudaMalloc and cudaFree of an engine's life costs its caller about a millisecond
     struct Part { void** p; size_t bytes; };
     const Part parts[] = {
@@ -103,8 +106,8 @@ extern "C" int q3_create(int device, const q3_config* cfg, q3_engine** out) {
         {(void**)&e->part, (size_t)e->part_slots * Q_HEADS * ATTN_PART_STRIDE * 4},
         {(void**)&e->pval, (size_t)cfg->max_batch * e->lm_grid * 4}, {(void**)&e->pidx, (size_t)cfg->max_batch * e->lm_grid * 4},
         {(void**)&e->status, Q3_STATUS_WORDS * 4}, {(void**)&e->sync, Q3_SYNC_WORDS * 4}, {&e->pf_desc, 64 + B * 32},
-        {&e->planes, 3 * cap_pad * INTER * 2}, {&e->xplanes, 3 * cap_pad * HIDDEN * 2}, {(void**)&e->ssq, CL_SSQ_PARTS * cap_pad * 4},
-        {(void**)&e->logits_tc, (size_t)cfg->max_batch * cfg->vocab * 4},
+        {&e->planes, 3 * cap_pad * INTER * 2}, {&e->xplanes, (size_t)3 * e->chain_rows * HIDDEN * 2}, {(void**)&e->ssq, (size_t)CL_SSQ_PARTS * e->chain_rows * 4},
+        {(void**)&e->logits_tc, cfg->max_batch >= Q3_TC_MIN_BATCH ? (size_t)cfg->max_batch * cfg->vocab * 4 : 0},
         {(void**)&e->gate, tc ? B * INTER * 4 : 0}, {(void**)&e->up, tc ? B * INTER * 4 : 0}, {&e->lk_state, tc ? (size_t)LK_STATE_BYTES : 0}};
     auto padded = [](size_t n) { return (n + 1023) / 1024 * 1024; };
     size_t total = 0;
@@ -247,7 +250,6 @@ static int chunk_pad_for(int max_len, int ns) { return (((max_len + 1 + ns - 1) 
 
 // Decode steps of up to 64 sequences run as five launches per layer (q3_gemm_cl.h); larger ones, and engines without scratch
 // for the planes, keep one launch per phase.
-constexpr int CHAIN_MAX_BATCH = 64;
 static bool chain_serves(const q3_engine* e, int batch) { return e->xplanes != nullptr && batch <= CHAIN_MAX_BATCH; }
 constexpr int CHAIN_MAX_SPLITS = 8;   // the splits of a (sequence, kv head) are one cluster (16: one sequence at 5000 positions 897 us, 8: 793)
 
@@ -328,7 +330,7 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
     if (chain) {
         // q/k/v | attention | Wo | gate/up | down: each product finishes its rows and writes the planes of the next one, so
         // that nothing stands between them; the residual's planes and the others alternate between two buffers
-        const int rows = gemm_cluster_rows(B), ssq_ld = (e->cap + 127) / 128 * 128;
+        const int rows = gemm_cluster_rows(B), ssq_ld = e->chain_rows;
         bf16_raw* xp = reinterpret_cast<bf16_raw*>(e->xplanes);
         LAUNCH(launch_embed_planes(reinterpret_cast<const long long*>(a->token), bf(w.embed), V, e->x, bf(w.ln1), xp, rows, 3, e->ssq, ssq_ld, e->status, B, st,
                                    arg_keys, arg_tickets, a->seq_len, len_bound));

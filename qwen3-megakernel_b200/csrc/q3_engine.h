@@ -39,8 +39,9 @@ struct q3_engine {
     int cap;            // tokens the scratch is sized for: max(max_batch, max_tokens)
     int part_slots;     // (token, split) slots in `part`
     void* planes;       // bf16 [3][cap rounded up to 128][3072] activation planes
-    void* xplanes;      // bf16 [3][cap rounded up to 128][1024] planes of the residual rows (q3_gemm_cl.h)
-    float* ssq;         // [32][cap rounded up to 128] partial sums of squares of the residual rows
+    int chain_rows;     // rows of the following two: those of the largest decode batch the cluster products serve
+    void* xplanes;      // bf16 [3][chain_rows][1024] planes of the residual rows (q3_gemm_cl.h)
+    float* ssq;         // [32][chain_rows] partial sums of squares of the residual rows
     float* gate;        // [cap, 3072]
     float* up;          // [cap, 3072]
     float* logits_tc;   // [max_batch, vocab] when the caller passes no logits buffer

@@ -266,6 +266,21 @@ def test_a_short_bind_of_two_sequences_is_no_slower_than_one_after_the_other(ora
     assert best["auto"] <= 1.2 * best["persist"], best
 
 
+def test_prompt_capacity_pays_for_prompts_only():
+    """Scratch per token of prompt capacity: rows, projections, planes, gate and up, attention partials and a descriptor.
+    What only decode batches use is sized by the batch."""
+    def bytes_of(max_tokens):
+        before = torch.cuda.mem_get_info()[0]
+        mk = engine("auto", layers=1, vocab=512, max_tokens=max_tokens, max_positions=64)
+        used = before - torch.cuda.mem_get_info()[0]
+        del mk
+        return used
+
+    bytes_of(8192)
+    per_token = 4 * (1024 + 4096 + 2048 + 3 * 3072) + 3 * 2 * 3072 + 2 * 16 * 132 * 4 + 32
+    assert bytes_of(8192) - bytes_of(4096) <= 4096 * per_token + (4 << 20)      # (allocations come in pieces of 2 MB)
+
+
 @pytest.mark.parametrize("path", PATHS)
 def test_prefill_2048_then_greedy_decode(oracle, small, path):
     """The benchmark's third shape on a small model: a 2048-token prompt on the GPU, then chained greedy steps over
