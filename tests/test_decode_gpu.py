@@ -453,11 +453,13 @@ def _gate_batch_stream(oracle, w, toks0, kcs, vcs, got, outs, what):
         gate_teacher_forced(oracle, w, int(toks0[b]), kcs[b], vcs[b], got[:, b], outs, f"{what} seq {b}", seq=b)
 
 
-@pytest.mark.parametrize("batch,ctx,steps", [(8, 128, 72), (1, 1170, 40), (5, 30, 70)])
-def test_layered_graph_replay_follows_a_growing_cache(oracle, batch, ctx, steps):
-    """Chained launches with append and graph replay: the attention split count stays put while the padded chunk length,
-    which is part of the captured launch arguments, grows with the cache (batch 8 from 128 positions: at 161; batch 1:
-    at 1185).  A replayed graph must not keep the shorter chunk."""
+@pytest.mark.parametrize("path,batch,ctx,steps", [("layered", 8, 245, 24), ("layered", 1, 1270, 40), ("layered", 5, 24, 60),
+                                                  ("auto", 2, 500, 30), ("auto", 2, 56, 80), ("auto", 3, 250, 30)])
+def test_layered_graph_replay_follows_a_growing_cache(oracle, path, batch, ctx, steps):
+    """Chained launches with append and graph replay, across cache lengths where the attention split changes: the padded chunk
+    length, which is part of the captured launch arguments, at a fixed split count above one (batch 8 at 256 positions,
+    batch 1 at 1280, batch 2 at 512, batch 3 at 256), and the split count itself (batch 2 at 65, 96 and 128, batch 5 at 65).
+    Graphs are captured before and after each.  A replayed graph must not keep the shorter chunk."""
     from qwen3mk.kernel import SeqTable
 
     shp = oracle.Shape(layers=2, vocab=2048)
@@ -469,11 +471,93 @@ def test_layered_graph_replay_follows_a_growing_cache(oracle, batch, ctx, steps)
     kcs = [(torch.randn(2, n, 8, 128, generator=g) * 0.1).to(torch.bfloat16) for n in lens]
     vcs = [(torch.randn(2, n, 8, 128, generator=g) * 0.1).to(torch.bfloat16) for n in lens]
     room = lambda t: torch.cat([t, torch.zeros(2, steps, 8, 128, dtype=torch.bfloat16)], dim=1).cuda()
+    mk = engine(path, layers=2, vocab=2048, max_batch=batch, max_positions=4096)
+    dev = to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES})
+    # the split of the first step does not reach the last one's positions: the engine says so when a cache is longer than the host said
+    probe = SeqTable([room(k) for k in kcs], [room(v) for v in vcs], lens)
+    mk.bind_sequences(dev, toks.cuda(), probe)
+    probe.len[0] = ctx + steps - 1
+    mk.launch()
+    with pytest.raises(RuntimeError, match="device status: code 5"):
+        mk.status()
     seqs = SeqTable([room(k) for k in kcs], [room(v) for v in vcs], lens)
-    mk = engine("layered", layers=2, vocab=2048, max_batch=batch, max_positions=4096)
-    mk.bind_sequences(to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}), toks.cuda(), seqs, append=True, chained=True, graph=True)
+    mk.bind_sequences(dev, toks.cuda(), seqs, append=True, chained=True, graph=True)
     got, outs = run_chained(mk, steps)
-    _gate_batch_stream(oracle, w, toks, kcs, vcs, got.reshape(steps, batch), outs, f"batch {batch} from {ctx}")
+    _gate_batch_stream(oracle, w, toks, kcs, vcs, got.reshape(steps, batch), outs, f"{path} batch {batch} from {ctx}")
+
+
+@pytest.mark.parametrize("batch", [1, 3, 8, 33])
+def test_a_vocabulary_that_is_no_multiple_of_the_tile(oracle, batch):
+    """The launch chain's layers with the matrix-vector LM head."""
+    from qwen3mk.kernel import SeqTable
+
+    shp = oracle.Shape(layers=2, vocab=2000)
+    inp = oracle.synthetic(71, shp, context=8)
+    g = torch.Generator().manual_seed(batch)
+    lens = torch.randint(1, 300, (batch,), generator=g).tolist()
+    toks = torch.randint(0, 2000, (batch,), generator=g)
+    kcs = [(torch.randn(2, n, 8, 128, generator=g) * 0.1).to(torch.bfloat16) for n in lens]
+    vcs = [(torch.randn(2, n, 8, 128, generator=g) * 0.1).to(torch.bfloat16) for n in lens]
+    mk = engine("layered", layers=2, vocab=2000, max_batch=batch)
+    out = mk.bind_sequences(to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}), toks.cuda(), SeqTable([k.cuda() for k in kcs], [v.cuda() for v in vcs]))
+    mk.launch()
+    mk.status()
+    for b, ref in enumerate(oracle.decode_batch(oracle.to_fp32(inp), toks.tolist(), kcs, vcs)):
+        gate_step(oracle, {k: out[k][b] for k in out}, ref, f"seq {b} len {lens[b]}")
+
+
+@pytest.mark.parametrize("lens", [[32767], [32768], [33001, 40], [32900, 5, 700, 1, 64]])
+def test_caches_longer_than_a_cluster_of_splits(oracle, lens):
+    """A split takes at most 4096 positions and a cluster eight splits: from 32768 cached positions on, partials in memory and a
+    merge launch."""
+    from qwen3mk.kernel import SeqTable
+
+    shp = oracle.Shape(layers=1, vocab=512)
+    inp = oracle.synthetic(72, shp, context=8)
+    g = torch.Generator().manual_seed(len(lens))
+    toks = torch.randint(0, 512, (len(lens),), generator=g)
+    kcs = [torch.randn(1, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens]
+    vcs = [torch.randn(1, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens]
+    mk = engine("auto", layers=1, vocab=512, max_batch=len(lens), max_positions=33100)
+    out = mk.bind_sequences(to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}), toks.cuda(), SeqTable([k.cuda() for k in kcs], [v.cuda() for v in vcs]))
+    before = mk.launch_count
+    mk.launch()
+    mk.status()
+    # one layer: embedding, four products, the attention (and its merge), LM head, arg-max
+    assert mk.launch_count - before == (9 if max(lens) >= 32768 else 8)
+    for b, ref in enumerate(oracle.decode_batch(oracle.to_fp32(inp), toks.tolist(), kcs, vcs)):
+        gate_step(oracle, {k: out[k][b] for k in out}, ref, f"seq {b} len {lens[b]}")
+
+
+def test_engines_on_several_streams_at_once(oracle):
+    """Cluster products of three engines share the SMs: their blocks hold tensor memory while they wait for their cluster.  Every
+    step's rows are those of the engine running alone, bit by bit (the products add in a fixed order)."""
+    from qwen3mk.kernel import SeqTable
+
+    shp = oracle.Shape(layers=6, vocab=2048)
+    inp = oracle.synthetic(73, shp, context=8)
+    dev = to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES})
+    g = torch.Generator().manual_seed(1)
+    runs = []
+    for batch in (2, 8, 40):
+        lens = torch.randint(1, 400, (batch,), generator=g).tolist()
+        kcs = [torch.randn(6, n, 8, 128, generator=g).to(torch.bfloat16).cuda() for n in lens]
+        vcs = [torch.randn(6, n, 8, 128, generator=g).to(torch.bfloat16).cuda() for n in lens]
+        mk = engine("layered", layers=6, vocab=2048, max_batch=batch)
+        out = mk.bind_sequences(dev, torch.randint(0, 2048, (batch,), generator=g).cuda(), SeqTable(kcs, vcs))
+        mk.launch()
+        mk.status()
+        runs.append((mk, out, torch.cuda.Stream(), [out[n].clone() for n in ("k_write", "v_write")]))
+    for _, out, _, _ in runs:
+        out["k_write"].zero_()
+        out["v_write"].zero_()
+    torch.cuda.synchronize()
+    for _ in range(60):
+        for mk, _, stream, _ in runs:
+            mk.launch(stream.cuda_stream)
+    for mk, out, stream, alone in runs:
+        mk.status(stream.cuda_stream)
+        assert torch.equal(out["k_write"], alone[0]) and torch.equal(out["v_write"], alone[1])
 
 
 def test_a_wait_that_runs_out_is_reported_and_the_engine_recovers(oracle, small):
