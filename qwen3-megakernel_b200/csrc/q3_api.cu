@@ -66,8 +66,6 @@ static void drop_graphs(q3_engine* e) {
     v->clear();
 }
 
-constexpr int CHAIN_MAX_BATCH = 64;   // most sequences whose decode step runs as five launches per layer (chain_serves below)
-
 extern "C" const char* q3_version(void) { return "q3mk-b200 0.1 sm_100a"; }
 
 extern "C" const char* q3_last_error(const q3_engine* e) { return e ? e->err : g_create_error; }
@@ -98,7 +96,7 @@ extern "C" int q3_create(int device, const q3_config* cfg, q3_engine** out) {
     e->part_slots = (int)((B < 16 ? B : 16) * Q3_MAX_SPLITS > 2 * B ? (B < 16 ? B : 16) * Q3_MAX_SPLITS : 2 * B);
     const bool tc = e->cap >= Q3_TC_MIN_BATCH;
     const size_t cap_pad = (B + 127) / 128 * 128;
-    e->chain_rows = gemm_cluster_rows(cfg->max_batch < CHAIN_MAX_BATCH ? cfg->max_batch : CHAIN_MAX_BATCH);
+    e->chain_rows = gemm_cluster_rows(cfg->max_batch < CL_MAX_TOK ? cfg->max_batch : CL_MAX_TOK);
     // one allocation for all of it: every cudaMalloc and cudaFree of an engine's life costs its caller about a millisecond
     struct Part { void** p; size_t bytes; };
     const Part parts[] = {
@@ -248,10 +246,9 @@ extern "C" int q3_status(q3_engine* e, void* stream, uint32_t* words, int32_t n)
 // positions a split's block may take, rounded up to 32: with the split count it fixes the attention launch
 static int chunk_pad_for(int max_len, int ns) { return (((max_len + 1 + ns - 1) / ns) + 31) / 32 * 32; }
 
-// Decode steps of up to 64 sequences run as five launches per layer (q3_gemm_cl.h); larger ones, and engines without scratch
-// for the planes, keep one launch per phase.
-static bool chain_serves(const q3_engine* e, int batch) { return e->xplanes != nullptr && batch <= CHAIN_MAX_BATCH; }
-constexpr int CHAIN_MAX_SPLITS = 8;   // the splits of a (sequence, kv head) are one cluster (16: one sequence at 5000 positions 897 us, 8: 793)
+// Decode steps of up to CL_MAX_TOK sequences run as five launches per layer (q3_gemm_cl.h); larger ones, and a step without an
+// engine (q3_decode_noalloc, which has no planes), keep one launch per phase.
+static bool chain_serves(const q3_engine* e, int batch) { return e->xplanes != nullptr && batch <= CL_MAX_TOK; }
 
 static int splits_for(const q3_engine* e, int batch, int max_len, bool chain) {
     const double merge_us = chain ? 1.0 : 5.0;   // what more than one split costs beyond its blocks
@@ -274,7 +271,7 @@ static int splits_for(const q3_engine* e, int batch, int max_len, bool chain) {
     const double per_pos = big ? 0.023 : 0.006;
     double best = 1e30;
     int s = 1;
-    for (int c = 1; c <= (chain ? CHAIN_MAX_SPLITS : 16) && c <= by_len; ++c) {
+    for (int c = 1; c <= (chain ? ATTN_CLUSTER_MAX : 16) && c <= by_len; ++c) {
         const int waves = (pairs * c + slots - 1) / slots, per = (n + c - 1) / c;
         const double rounds = chain ? fmax(1.0, (double)pairs * c / slots) : waves;
         const double t = 4.0 * waves + per_pos * per * rounds + (c > 1 ? merge_us : 0.0);
@@ -332,11 +329,11 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
         // that nothing stands between them; the residual's planes and the others alternate between two buffers
         const int rows = gemm_cluster_rows(B), ssq_ld = e->chain_rows;
         bf16_raw* xp = reinterpret_cast<bf16_raw*>(e->xplanes);
-        LAUNCH(launch_embed_planes(reinterpret_cast<const long long*>(a->token), bf(w.embed), V, e->x, bf(w.ln1), xp, rows, 3, e->ssq, ssq_ld, e->status, B, st,
+        LAUNCH(launch_embed_planes(reinterpret_cast<const long long*>(a->token), bf(w.embed), V, e->x, bf(w.ln1), xp, rows, e->ssq, ssq_ld, e->status, B, st,
                                    arg_keys, arg_tickets, a->seq_len, len_bound));
         for (int l = 0; l < L; ++l) {
             ClusterGemmCall c{};
-            c.nsplit = 3; c.prow = rows; c.n_tok = B; c.ssq = e->ssq; c.ssq_ld = ssq_ld; c.status = e->status;
+            c.prow = rows; c.n_tok = B; c.ssq = e->ssq; c.ssq_ld = ssq_ld; c.status = e->status;
             ClusterGemmCall q = c;
             q.kind = CL_QKV; q.K = HIDDEN; q.in = xp; q.out = e->qkv;
             q.w[0] = bf(w.wq) + (size_t)l * Q_DIM * HIDDEN; q.w[1] = bf(w.wk) + (size_t)l * KV_DIM * HIDDEN; q.w[2] = bf(w.wv) + (size_t)l * KV_DIM * HIDDEN;
@@ -349,7 +346,7 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
             t.fused_prep = 1; t.qn = bf(w.qn); t.kn = bf(w.kn); t.rope = e->rope;
             t.k_write = reinterpret_cast<bf16_raw*>(a->k_write); t.v_write = reinterpret_cast<bf16_raw*>(a->v_write);
             t.n_layers = L; t.append = append; t.qp_planes = B < Q3_TC_MIN_BATCH ? 3 : 2;
-            if (ns <= CHAIN_MAX_SPLITS) {
+            if (ns <= ATTN_CLUSTER_MAX) {
                 t.planes_out = planes; t.plane_rows = rows; t.cluster = ns > 1; t.early = 1;
                 LAUNCH(launch_attn_split(t, B, st));
             } else {   // caches longer than a cluster's splits hold: partials in memory and a merge launch
@@ -564,7 +561,7 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
     // 1331 and 651 us; in plain launches, before a graph replays them, two at 16 positions 703 and 650 us; one sequence at 16 / 250 /
     // 1000 347 / 384 / 456 us against 567 and more).
     if (path == Q3_F_PATH_AUTO)
-        path = persist_supports(e, a) && (a->batch == 1 || !chain_serves(e, a->batch)) ? Q3_F_PATH_PERSIST : Q3_F_PATH_LAYERED;
+        path = a->batch == 1 && persist_supports(e, a) ? Q3_F_PATH_PERSIST : Q3_F_PATH_LAYERED;
     if (path == Q3_F_PATH_PERSIST) {
         if (!persist_supports(e, a))
             return fail(e, Q3_ERR_UNSUPPORTED, "q3_decode: the persistent kernel does not serve batch %d at length %d", a->batch, a->max_len);

@@ -25,10 +25,11 @@
 
 namespace q3 {
 
-// Two shapes of block.  Four warps (96 KB of stages, two blocks per SM) when the (sequence, kv head) pairs alone fill the
-// GPU: long runs per warp, few blocks.  Eight warps (192 KB, one block per SM) for smaller batches, preferably with ONE
+// Two shapes of block.  Four warps (96 KB of stages, two blocks per SM) in the launch chain, where a block of a neighbouring product
+// has to fit beside them and a cluster merges the splits, and wherever the (sequence, kv head) pairs alone fill the GPU: long runs
+// per warp, few blocks.  Eight warps (192 KB, one block per SM) for smaller batches outside the chain, preferably with ONE
 // split, so that the block writes the output planes itself and no merge launch follows.  Measured per decode step (28
-// launches): batch 64 x 1024 positions 2524 us with four warps and one split (2691 with three splits, 2705 with eight
+// launches) outside the chain: batch 64 x 1024 positions 2524 us with four warps and one split (2691 with three splits, 2705 with eight
 // warps); batch 8 x 1024 positions 1000 us with eight warps and one split, 1085 with two warps and five splits, 1153 with
 // four warps and one split; batch 16 x 2048 1446 against 1560.
 constexpr int AM_TILE = 16;                        // positions per stage
@@ -68,9 +69,8 @@ __device__ __forceinline__ void am_store_planes(const AttnArgs& a, int b, int co
     dst[(size_t)2 * a.plane_rows * Q_DIM] = f_to_bf(r1 - bf_to_f(m));
 }
 
-// CL: the splits of a (sequence, kv head) are the blocks of a cluster (at most AM_CLUSTER); every block sends its partial to the
+// CL: the splits of a (sequence, kv head) are the blocks of a cluster (at most ATTN_CLUSTER_MAX); every block sends its partial to the
 // first one through distributed shared memory and that one writes the output planes: no merge launch, no partials in global memory.
-constexpr int AM_CLUSTER = 16;
 constexpr int AM_PART = 2 * (HEAD_DIM + 2) * 4;     // bytes of a split's partial
 
 template <int AM_WARPS, bool CL, int PL>
@@ -393,8 +393,7 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
 
 template <int W, bool CL, int PL>
 static cudaError_t am_prepare() {
-    const cudaError_t e = cudaFuncSetAttribute(attn_mma_kernel<W, CL, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, W * AM_STAGES * AM_STAGE + (CL ? AM_CLUSTER * AM_PART : 0));
-    return e != cudaSuccess || !CL ? e : cudaFuncSetAttribute(attn_mma_kernel<W, CL, PL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return cudaFuncSetAttribute(attn_mma_kernel<W, CL, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, W * AM_STAGES * AM_STAGE + (CL ? ATTN_CLUSTER_MAX * AM_PART : 0));
 }
 
 template <int PL>
@@ -423,7 +422,7 @@ cudaError_t launch_attn_mma(const AttnArgs& a, int batch, cudaStream_t st) {
     const dim3 grid(a.n_splits, KV_HEADS, batch);
     const bool big = KV_HEADS * batch >= sm_count[dev];
     const int warps = big || a.early ? 4 : 8;
-    if (a.cluster && (a.n_splits > AM_CLUSTER || a.planes_out == nullptr)) return cudaErrorInvalidValue;
+    if (a.cluster && (a.n_splits > ATTN_CLUSTER_MAX || a.planes_out == nullptr)) return cudaErrorInvalidValue;
     return a.qp_planes == 3 ? am_launch<3>(a, grid, warps, st) : am_launch<2>(a, grid, warps, st);
 }
 

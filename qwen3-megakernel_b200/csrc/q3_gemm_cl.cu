@@ -1,4 +1,4 @@
-// The dense products of a layer for decode batches and short prompts: tcgen05 GEMMs whose k slices are the blocks of a
+// The dense products of a layer for decode batches of at most 64 sequences: tcgen05 GEMMs whose k slices are the blocks of a
 // cluster.
 //
 // With 1..64 tokens a layer's weights are a few megabytes per product, so what a launch costs is latency, and what a
@@ -25,10 +25,10 @@
 // 1.66e-6 (with one, and the LM head truncating as well, 2.16, 2.70 and 2.68e-6); the persistent kernel, one sequence after the other,
 // 1.23, 1.76 and 1.83e-6.  In larger batches the two planes of the attention leave 1.7e-5 whatever the products do.
 //
-// Measured (one B200, us per step, before -> after): 8 sequences x 1024 positions 984 -> 735, 64 x 1024 2333 -> 2075, one at
-// 5000 positions 1606 -> 793.  What bounds it: a launch is about 3.4 us of latencies in series (release of the wait to the first
-// plane 0.5, products 0.7, partial tile out 0.3, to the owners 0.5, finished row 0.6, end of the grid to the next release 0.7) beside
-// 1..2 us of weight bytes that overlap them.
+// Measured (one B200, us per step, before -> after): 8 sequences x 1024 positions 984 -> 720, 64 x 1024 2333 -> 2055, one at
+// 5000 positions 1606 -> 800.  What bounds it: a launch is about 3.4 us of latencies in series (8 sequences, medians of the blocks: release
+// of the wait to the first stage 0.6, products 1.0, partial tile out 0.3, to the owners 0.5, finished row 0.3, end of the grid to the
+// next release 1.0, each a little longer for the time stamps) beside 1..2 us of weight bytes that overlap them.
 //
 // Weight tiles are requested before the wait for the previous launch, so that their latency overlaps its tail.
 //
@@ -54,7 +54,7 @@ static_assert(Q3_TC_MIN_BATCH <= CL_FEW, "a batch below it fits");
 
 struct ClusterGemmParams {
     int kb_total;                 // k blocks of 64
-    int nsplit, prow, n_tok, stages;
+    int prow, n_tok, stages;
     int tiles_q, tiles_k;         // CL_QKV: tiles of the first two matrices
     float* out;
     int ldo;
@@ -75,19 +75,20 @@ __device__ __forceinline__ uint32_t cl_map(uint32_t smem_addr, int rank) {
 __device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
 __device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
-__device__ __forceinline__ void cl_store_planes(bf16_raw* p, size_t plane, int nsplit, float v) {
+__device__ __forceinline__ void cl_store_planes(bf16_raw* p, size_t plane, float v) {
     const bf16_raw h = f_to_bf(v);
     const float r1 = v - bf_to_f(h);
     const bf16_raw m = f_to_bf(r1), l = f_to_bf(r1 - bf_to_f(m));
     p[0] = h;
-    if (nsplit > 1) p[plane] = m;
-    if (nsplit > 2) p[2 * plane] = l;
+    p[plane] = m;
+    p[2 * plane] = l;
 }
 
 template <int KIND, int BN> struct ClShape {
     static constexpr int TM = KIND == CL_RESID ? 64 : 128;                                // rows of the weight tile
     static constexpr int C = KIND == CL_RESID ? 8 : 4;                                      // k slices = blocks of the cluster
     static constexpr int SLOTS = (BN + C - 1) / C;                                        // tokens a block owns
+    static constexpr uint32_t ACC_COLS = CL_PLANES * BN <= 64 ? 64 : 128;                 // TMEM columns of an accumulator
     static constexpr int RED_BYTES = C * SLOTS * TM * 4;                                  // partial tiles of the owned tokens
 };
 
@@ -107,10 +108,10 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int rank = blockIdx.x;                 // the cluster spans x
     const int tile = blockIdx.y, n0 = blockIdx.z * BN;
-    const int nsplit = p.nsplit, stages = p.stages;
+    const int stages = p.stages;
     const int base_kb = p.kb_total / C, rem_kb = p.kb_total % C;
     const int kb0 = rank * base_kb + min(rank, rem_kb), nkb = base_kb + (rank < rem_kb ? 1 : 0);
-    const uint32_t stage_bytes = A_BYTES + nsplit * B_BYTES;
+    constexpr uint32_t stage_bytes = A_BYTES + CL_PLANES * B_BYTES;
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(cl_raw) + 1023) & ~(uintptr_t)1023);
     float* red = reinterpret_cast<float*>(base + (size_t)stages * stage_bytes);      // [C][SLOTS][TM]: what the blocks send to this one
     auto slots_of = [&](int owner) { return max(0, (min(p.n_tok - n0, BN) - owner + C - 1) / C); };   // tokens of this tile that `owner` finishes
@@ -128,8 +129,8 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
             asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(&red_bar)), "r"((uint32_t)(C * my_slots * TM * 4)) : "memory");
         abort_flag = 0;
     }
-    // the planes of a stage lie side by side: nsplit * BN columns of one B operand (192 at most)
-    const uint32_t cols = (uint32_t)(nsplit * BN), acc_cols = cols <= 32 ? 32u : cols <= 64 ? 64u : cols <= 128 ? 128u : 256u, tmem_cols = NACC * acc_cols;
+    // the planes of a stage lie side by side: columns of one B operand
+    constexpr uint32_t cols = CL_PLANES * BN, acc_cols = S::ACC_COLS, tmem_cols = NACC * acc_cols;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_base_s)), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
         const bool live = TM == 128 || lane < 16;
         float* stage = reinterpret_cast<float*>(base) + (TM == 128 ? quad * 32 + lane : quad * 16 + (lane & 15));   // [C][SLOTS][TM]
         if constexpr (NACC > 1) {            // at most CL_FEW tokens: their columns of every accumulator and plane under one wait
-            uint32_t r[NACC][3][CL_FEW];
+            uint32_t r[NACC][CL_PLANES][CL_FEW];
 #pragma unroll
             for (int ac = 0; ac < NACC; ++ac)
 #pragma unroll
@@ -278,19 +279,17 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
             if constexpr (STEP == 16) {
                 tc_ld16(r, taddr);
-                if (nsplit > 1) tc_ld16(q1, taddr + BN);
-                if (nsplit > 2) tc_ld16(q2, taddr + 2 * BN);
+                tc_ld16(q1, taddr + BN);
+                tc_ld16(q2, taddr + 2 * BN);
             } else {
                 tc_ld32(r, taddr);
-                if (nsplit > 1) tc_ld32(q1, taddr + BN);
-                if (nsplit > 2) tc_ld32(q2, taddr + 2 * BN);
+                tc_ld32(q1, taddr + BN);
+                tc_ld32(q2, taddr + 2 * BN);
             }
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int j = 0; j < STEP; ++j) {
-                float v = __uint_as_float(r[j]);
-                if (nsplit > 1) v += __uint_as_float(q1[j]);
-                if (nsplit > 2) v += __uint_as_float(q2[j]);
+                const float v = __uint_as_float(r[j]) + __uint_as_float(q1[j]) + __uint_as_float(q2[j]);
                 if (live) stage[(((c0 + j) % C) * SLOTS + (c0 + j) / C) * TM] = v;
             }
         }
@@ -326,7 +325,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
             const float x = xr[i] + v;
             const size_t col = (size_t)tile * TM + orow;
             p.out[(size_t)t * p.ldo + col] = x;
-            cl_store_planes(p.planes + (size_t)t * p.ldp + col, plane, nsplit, x * gain);
+            cl_store_planes(p.planes + (size_t)t * p.ldp + col, plane, x * gain);
             const float ss = warp_sum(x * x);
             if (lane == 0) p.ssq[(size_t)(tile * 2 + (orow >> 5)) * p.ssq_ld + t] = ss;
         } else {
@@ -335,7 +334,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
             for (int c = 1; c < C; ++c) u += src[c * SLOTS * TM + TM / 2];
             const float g = v * s_r[s];
             u *= s_r[s];
-            cl_store_planes(p.planes + (size_t)t * p.ldp + tile * (TM / 2) + orow, plane, nsplit, (g / (1.f + expf(-g))) * u);
+            cl_store_planes(p.planes + (size_t)t * p.ldp + tile * (TM / 2) + orow, plane, (g / (1.f + expf(-g))) * u);
         }
     }
     cl_wait();
@@ -344,7 +343,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) gemm_cluster_kernel(const __gri
 
 // ---- embedding gather with the first layer's planes: one block per sequence ----------------------------------------
 __global__ void __launch_bounds__(256) embed_planes_kernel(const long long* __restrict__ token, const bf16_raw* __restrict__ embed, int vocab, float* __restrict__ x,
-                                                           const bf16_raw* __restrict__ gain, bf16_raw* __restrict__ planes, int prow, int nsplit,
+                                                           const bf16_raw* __restrict__ gain, bf16_raw* __restrict__ planes, int prow,
                                                            float* __restrict__ ssq, int ssq_ld, uint32_t* status, unsigned long long* argmax_keys,
                                                            unsigned* argmax_tickets, const int* __restrict__ seq_len, int len_bound) {
     pdl_launch();
@@ -362,7 +361,7 @@ __global__ void __launch_bounds__(256) embed_planes_kernel(const long long* __re
     reinterpret_cast<float4*>(x + (size_t)b * HIDDEN)[tid] = o;
     const float y[4] = {o.x * bf_lo(g.x), o.y * bf_hi(g.x), o.z * bf_lo(g.y), o.w * bf_hi(g.y)};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) cl_store_planes(planes + (size_t)b * HIDDEN + tid * 4 + i, (size_t)prow * HIDDEN, nsplit, y[i]);
+    for (int i = 0; i < 4; ++i) cl_store_planes(planes + (size_t)b * HIDDEN + tid * 4 + i, (size_t)prow * HIDDEN, y[i]);
     float ss = fmaf(o.x, o.x, fmaf(o.y, o.y, fmaf(o.z, o.z, o.w * o.w)));
 #pragma unroll
     for (int sh = 4; sh > 0; sh >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, sh);   // eight threads make a part of 32 elements
@@ -370,9 +369,9 @@ __global__ void __launch_bounds__(256) embed_planes_kernel(const long long* __re
 }
 
 cudaError_t launch_embed_planes(const long long* token, const bf16_raw* embed, int vocab, float* x, const bf16_raw* gain, bf16_raw* planes, int prow,
-                                int nsplit, float* ssq, int ssq_ld, uint32_t* status, int batch, cudaStream_t st, unsigned long long* argmax_keys,
+                                float* ssq, int ssq_ld, uint32_t* status, int batch, cudaStream_t st, unsigned long long* argmax_keys,
                                 unsigned* argmax_tickets, const int* seq_len, int len_bound) {
-    return launch_chain(embed_planes_kernel, dim3(batch), dim3(256), 0, st, token, embed, vocab, x, gain, planes, prow, nsplit, ssq, ssq_ld, status,
+    return launch_chain(embed_planes_kernel, dim3(batch), dim3(256), 0, st, token, embed, vocab, x, gain, planes, prow, ssq, ssq_ld, status,
                         argmax_keys, argmax_tickets, seq_len, len_bound);
 }
 
@@ -381,11 +380,8 @@ cudaError_t launch_embed_planes(const long long* token, const bf16_raw* embed, i
 // 64: 2419 / 2075 / 2349 us per step.
 static int cl_tile(int n_tok) { return n_tok <= 16 ? 16 : 32; }
 
-// (a plane's rows are a multiple of the LM head's token tile, which reads the last planes: 32 / 64 / 128)
-int gemm_cluster_rows(int n_tok) {
-    const int bn = n_tok <= 32 ? 32 : n_tok <= 64 ? 64 : 128;
-    return (n_tok + bn - 1) / bn * bn;
-}
+// (a plane's rows are the LM head's token tile, which reads the last planes)
+int gemm_cluster_rows(int n_tok) { return n_tok <= 32 ? 32 : CL_MAX_TOK; }
 
 template <int KIND, int BN, int NACC>
 static cudaError_t launch_cl(const CUtensorMap* tw, const CUtensorMap& tx, ClusterGemmParams p, int tiles, cudaStream_t st) {
@@ -399,7 +395,7 @@ static cudaError_t launch_cl(const CUtensorMap* tw, const CUtensorMap& tx, Clust
         if ((e = cudaFuncSetAttribute(gemm_cluster_kernel<KIND, BN, NACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM)) != cudaSuccess) return e;
         attr_set[dev] = true;
     }
-    const int stage_bytes = S::TM * TC_BK * 2 + p.nsplit * BN * TC_BK * 2;
+    constexpr int stage_bytes = S::TM * TC_BK * 2 + CL_PLANES * BN * TC_BK * 2;
     // Half of an SM's shared memory, so that the next launch's blocks find room while this one's are still there: they set up
     // and fetch their weights before they wait (batch 64 x 1024, 75 / 90 / 112 KB: 2118 / 2104 / 2075 us per step; 27 ragged
     // up to 2048: 1460 / 1437 / 1383 us).
@@ -417,9 +413,9 @@ static cudaError_t launch_cl(const CUtensorMap* tw, const CUtensorMap& tx, Clust
     // layer kernel (q3_layer_tc.cu), whose blocks wait for one another too, leaves room for one block of 128 columns beside its
     // 128.  The other kernels with TMEM wait for nothing but their predecessor in the stream, which has all its columns by then.
     constexpr int SM_SMEM = 228 * 1024, THIRD = 58 * 1024, HALF = 88 * 1024;
-    static_assert(4 * THIRD > SM_SMEM && 2 * HALF + THIRD > SM_SMEM && NACC * BN * 4 <= 256, "TMEM columns of an SM");
+    static_assert(4 * THIRD > SM_SMEM && 2 * HALF + THIRD > SM_SMEM && NACC * S::ACC_COLS <= 256, "TMEM columns of an SM");
     int smem = stages * stage_bytes + S::RED_BYTES + 1024;
-    const int least = NACC * p.nsplit * BN > 128 ? HALF : THIRD;
+    constexpr int least = NACC * S::ACC_COLS > 128 ? HALF : THIRD;
     if (smem < least) smem = least;
     return launch_chain_cluster(gemm_cluster_kernel<KIND, BN, NACC>, dim3(S::C, tiles, (p.n_tok + BN - 1) / BN), dim3(CL_THREADS), (size_t)smem, S::C, st,
                                 tw[0], tw[1], tw[2], tx, p);
@@ -427,20 +423,20 @@ static cudaError_t launch_cl(const CUtensorMap* tw, const CUtensorMap& tx, Clust
 
 template <int KIND>
 static cudaError_t launch_kind(const CUtensorMap* tw, const CUtensorMap& tx, const ClusterGemmParams& p, int tiles, int bn, cudaStream_t st) {
-    if (p.n_tok < Q3_TC_MIN_BATCH && p.nsplit == 3) return launch_cl<KIND, 16, 4>(tw, tx, p, tiles, st);
+    if (p.n_tok < Q3_TC_MIN_BATCH) return launch_cl<KIND, 16, 4>(tw, tx, p, tiles, st);
     if (bn == 16) return launch_cl<KIND, 16, 1>(tw, tx, p, tiles, st);
     return launch_cl<KIND, 32, 1>(tw, tx, p, tiles, st);
 }
 
 cudaError_t launch_gemm_cluster(const ClusterGemmCall& c, cudaStream_t st) {
     const int bn = cl_tile(c.n_tok);
-    if (c.n_tok < 1 || c.nsplit < 1 || c.nsplit > 3 || c.nsplit * bn > 256 || c.K % TC_BK || c.K < 8 * TC_BK || c.prow < gemm_cluster_rows(c.n_tok) || c.prow % bn)
+    if (c.n_tok < 1 || c.n_tok > CL_MAX_TOK || c.K % TC_BK || c.K < 8 * TC_BK || c.prow < gemm_cluster_rows(c.n_tok) || c.prow % bn)
         return cudaErrorInvalidValue;
     ClusterGemmParams p{};
-    p.kb_total = c.K / TC_BK; p.nsplit = c.nsplit; p.prow = c.prow; p.n_tok = c.n_tok;
+    p.kb_total = c.K / TC_BK; p.prow = c.prow; p.n_tok = c.n_tok;
     p.out = c.out; p.planes = c.planes; p.gain = c.gain; p.ssq = c.ssq; p.ssq_ld = c.ssq_ld; p.status = c.status;
     CUtensorMap tw[3], tx;
-    if (!tc_cached_map(c.in, (uint64_t)c.prow, (uint64_t)c.K, (uint32_t)bn, &tx, (uint64_t)c.nsplit)) return cudaErrorUnknown;
+    if (!tc_cached_map(c.in, (uint64_t)c.prow, (uint64_t)c.K, (uint32_t)bn, &tx, (uint64_t)CL_PLANES)) return cudaErrorUnknown;
     const int rows[3] = {c.kind == CL_QKV ? Q_DIM : c.kind == CL_RESID ? HIDDEN : INTER, c.kind == CL_QKV ? KV_DIM : INTER, KV_DIM};
     const int n_w = c.kind == CL_QKV ? 3 : c.kind == CL_RESID ? 1 : 2;
     const uint32_t box = c.kind == CL_QKV ? 128u : 64u;

@@ -16,6 +16,7 @@
 #include <cuda.h>
 
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "q3_engine.h"
@@ -30,11 +31,18 @@ static std::mutex& host_lock() { static std::mutex m; return m; }   // guards th
 constexpr int TC_THREADS = 192;    // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2..5: epilogue
 constexpr int TC_BM = 128;         // weight rows per tile (UMMA M)
 
-template <int BN, bool SCALE>   // SCALE: every token's column is multiplied by its RMS norm's scale (sums of squares in GemmTcParams::resid)
+// SCALE: every token's column is multiplied by its RMS norm's scale, rsqrt(sum of the 32 parts ssq[i * ssq_ld + t] / 1024 + eps)
+struct GemmTcScaledParams : GemmTcParams {
+    const float* ssq;
+    int ssq_ld;
+};
+template <bool SCALE> using TcParams = std::conditional_t<SCALE, GemmTcScaledParams, GemmTcParams>;
+
+template <int BN, bool SCALE>
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w0,
                                                                 const __grid_constant__ CUtensorMap tm_w1,
                                                                 const __grid_constant__ CUtensorMap tm_w2,
-                                                                const __grid_constant__ CUtensorMap tm_x, const GemmTcParams p) {
+                                                                const __grid_constant__ CUtensorMap tm_x, const TcParams<SCALE> p) {
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[8], empty_bar[8], acc_bar;
     __shared__ uint32_t tmem_base_s;
@@ -156,7 +164,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
             pdl_wait();
 #pragma unroll 4
             for (int j = warp - 2; j < BN; j += 4) {
-                const float ss = warp_sum(n0 + j < p.n_tok ? p.resid[(size_t)lane * p.ldr + n0 + j] : 0.f);
+                const float ss = warp_sum(n0 + j < p.n_tok ? p.ssq[(size_t)lane * p.ssq_ld + n0 + j] : 0.f);
                 if (lane == 0) s_scale[j] = rsqrtf(ss / (float)HIDDEN + EPS);
             }
             asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -551,7 +559,7 @@ static cudaError_t launch_persist(const CUtensorMap* tw, const CUtensorMap& tx, 
 }
 
 template <int BN, bool SCALE = false>
-static cudaError_t launch_bn(const CUtensorMap* tw, const CUtensorMap& tx, GemmTcParams p, int n_rows, int n_tok, int sm_count, cudaStream_t st) {
+static cudaError_t launch_bn(const CUtensorMap* tw, const CUtensorMap& tx, TcParams<SCALE> p, int n_rows, int n_tok, int sm_count, cudaStream_t st) {
     // n_rows: all weight rows of the launch (the sum over the groups); tw: three maps (unused ones repeat the first)
     const int nkb = p.K / TC_BK;
     const int tiles = ((n_rows + TC_BM - 1) / TC_BM) * ((n_tok + BN - 1) / BN);
@@ -653,11 +661,12 @@ cudaError_t launch_gemm_tc(const GemmTcCall& c, cudaStream_t st) {
     if (sm_count < 1) return cudaErrorInvalidDevice;
     const CUtensorMap maps[3] = {tw, tw, tw};
     if (c.ssq != nullptr) {
-        if (c.resid != nullptr) return cudaErrorInvalidValue;
-        p.resid = c.ssq; p.ldr = c.ssq_ld;
-        if (bn == 32) return launch_bn<32, true>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
-        if (bn == 64) return launch_bn<64, true>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
-        return launch_bn<128, true>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
+        if (c.resid != nullptr || bn > 64) return cudaErrorInvalidValue;
+        GemmTcScaledParams q{};
+        static_cast<GemmTcParams&>(q) = p;
+        q.ssq = c.ssq; q.ssq_ld = c.ssq_ld;
+        if (bn == 32) return launch_bn<32, true>(maps, tx, q, c.n_rows, c.n_tok, sm_count, st);
+        return launch_bn<64, true>(maps, tx, q, c.n_rows, c.n_tok, sm_count, st);
     }
     if (persist_serves(c.n_rows, c.n_tok, c.nsplit, c.plane_rows, sm_count)) {
         CUtensorMap txp;

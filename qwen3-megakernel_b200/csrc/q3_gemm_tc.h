@@ -12,8 +12,7 @@ enum { TC_EPI_STORE = 0, TC_EPI_RESID = 1, TC_EPI_ATOMIC = 2 };
 // device-side parameters
 struct GemmTcParams {
     float* out;            // [n_tok, ldo] fp32; element (t, n) at out[t * ldo + n]
-    const float* resid;    // TC_EPI_RESID: out = resid + acc (may alias out).  gemm_tc_kernel<., true>: the partial sums of squares, column t is
-                           // scaled by rsqrt(sum of the 32 parts resid[i * ldr + t] / 1024 + eps)
+    const float* resid;    // TC_EPI_RESID: out = resid + acc (may alias out)
     int ldo, ldr;
     int n_rows;            // weight rows (multiple of 128)
     int n_tok;             // valid tokens
@@ -41,7 +40,7 @@ struct GemmTcCall {
     int ldo, ldr;
     int n_rows, n_tok, K, nsplit, plane_rows;
     uint32_t* status;
-    const float* ssq;      // not null: the planes lack their RMS norm's scale, the epilogue applies it (never the persistent kernel)
+    const float* ssq;      // not null: the planes lack their RMS norm's scale, the epilogue applies it (at most 64 tokens, no residual)
     int ssq_ld;
 };
 

@@ -10,6 +10,7 @@ typedef unsigned short bf16_raw;
 enum { EPI_STORE = 0, EPI_RESID = 1, EPI_SILU = 2, EPI_LOGITS = 3 };
 
 // floats per (sequence, head, split) attention partial: [0] max, [1] sum, [4..132) unnormalised output
+constexpr int ATTN_CLUSTER_MAX = 8;      // splits that are one cluster (one sequence at 5000 positions with 8 / 16: 793 / 897 us a step)
 constexpr int ATTN_PART_STRIDE = 132;
 constexpr int ATTN_CHUNK_MAX = 4096;          // positions one block of the split-attention kernel takes (its scores live in shared memory)
 
@@ -80,7 +81,7 @@ struct AttnArgs {
     // [3][plane_rows][2048] the Wo GEMM reads
     bf16_raw* planes_out;
     int plane_rows;
-    int cluster;                      // the splits are a cluster of blocks (at most 16) that writes planes_out itself
+    int cluster;                      // the splits are a cluster of blocks (at most ATTN_CLUSTER_MAX) that writes planes_out itself
     int qp_planes;                    // bf16 planes q and the probabilities enter the products as: 3, or 2 (any other value)
     int early;                        // the predecessor lets this launch start only when everything before it has completed: lengths and
                                       // cached rows may be read before the wait (blocks of four warps, which fit beside its blocks)
