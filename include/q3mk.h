@@ -35,8 +35,8 @@ extern "C" {
 
 /* q3_decode_args.flags */
 #define Q3_F_APPEND_KV    0x1u  /* write the new K/V rows into cache slot seq_len[b], then seq_len[b] += 1 */
-#define Q3_F_PATH_AUTO    0x0u  /* engine picks: persistent kernel for small batches, layered otherwise    */
-#define Q3_F_PATH_LAYERED 0x10u /* one launch per phase (debug ladder, large batches)                      */
+#define Q3_F_PATH_AUTO    0x0u  /* engine picks: persistent kernel for one sequence it serves, layered otherwise */
+#define Q3_F_PATH_LAYERED 0x10u /* a chain of launches: five per layer up to 64 sequences, one per phase beyond */
 #define Q3_F_PATH_FUSED   0x30u /* layered, but batches of 4..64 run two launches per layer: split attention + one persistent
                                    kernel for Wo, norm, gate/up, SiLU, down, norm and the next layer's q/k/v (opt-in: measured
                                    slower than the launch chain so far) */
@@ -52,7 +52,8 @@ typedef struct q3_config {
     int32_t max_batch;      /* largest q3_decode_args.batch the scratch is sized for (>= 1)      */
     int32_t max_tokens;     /* largest q3_prefill_args.n_tokens the scratch is sized for (0: no prefill) */
     int32_t grid_limit;     /* 0 = one CTA per SM; otherwise cap the persistent grid (tests)     */
-    int32_t wait_limit_us;  /* patience of every device-side wait in microseconds; 0 = the default (200 ms).  Tests set it low to see a wait give up */
+    int32_t wait_limit_us;  /* patience of the persistent and the layer kernel's waits in microseconds; 0 = the default (200 ms).  Tests set it low
+                               to see a wait give up.  Waits inside the tensor-core products are fixed at 200 ms, at 400 for a cluster's partial tiles */
 } q3_config;
 
 /* The 13 weight tensors, device pointers to bf16.  Replaces slots 1..13 of the reference's
@@ -216,7 +217,8 @@ int64_t q3_launch_count(const q3_engine* e);
 int q3_grid_info(const q3_engine* e, int32_t* ctas, int32_t* threads, int32_t* smem_bytes);
 
 /* Engine-owned scratch for tools and tests: name in {"x","qkv","attn","hid","status","persist_acc"}; returns a
- * device pointer and its size in bytes, or Q3_ERR_INVALID.  "persist_acc" is the persistent kernel's four delta
+ * device pointer and its size in bytes, or Q3_ERR_INVALID.  Layered steps leave the residual rows in "x" and the last layer's
+ * projections in "qkv"; "attn" is written by the fused path only, "hid" by its steps of fewer than four sequences.  "persist_acc" is the persistent kernel's four delta
  * accumulators (64-bit words: contributions << 56 | fixed-point sum), all zero between launches. */
 int q3_scratch(const q3_engine* e, const char* name, void** ptr, int64_t* bytes);
 

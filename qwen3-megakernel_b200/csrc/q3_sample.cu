@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
 
     // ---- 2b. threshold: the k-th largest key (-inf keeps everything) ----
     float kth = -INFINITY;
-    // (`select` spelled out: nvcc 12.9 lost the branch when it reused the flag from above)
+    // (`select` spelled out: with `if (select)` nvcc 12.9 compiles this kernel so that every top-k test fails, kth staying -inf)
     if (top_k > 1 && top_k < vocab) {
         bool fits = true;
         int total = 0;

@@ -8,8 +8,8 @@
 // array, sized for at most Q3_NOALLOC_MAX_BATCH sequences, and every GPU that loads the library
 // holds those bytes until the process exits.
 //
-// The step itself is the layered path of q3_decode, kernel for kernel; only where the scratch comes
-// from differs.  All calls share the one array: it keeps the previous call's contents (every buffer is
+// The step itself is a layered one, one launch per phase with matrix-vector products: the engine's launch chain of cluster products
+// (q3_gemm_cl.h) needs planes of the activations, for which this scratch has no room.  All calls share the one array: it keeps the previous call's contents (every buffer is
 // fully rewritten before it is read, the status words are cleared on the stream at the start of each
 // call), and two calls that overlap on the GPU would race on it.
 #include <cstring>

@@ -154,7 +154,7 @@ def test_ragged_batch(oracle, path, batch):
 
 @pytest.mark.parametrize("batch", [1, 2, 15, 16, 17, 31, 32, 63, 64])
 def test_batches_at_the_edges_of_the_token_tiles(oracle, batch):
-    """The cluster GEMMs tile the tokens by 16, 32 and 64 and a row's owner is its index modulo the cluster size; the
+    """The cluster GEMMs tile the tokens by 16 and 32 and a row's owner is its index modulo the cluster size; the
     longest sequence decides the attention split, so the empty and the one-position cache get splits with nothing in
     them.  A layer's sums are added in a fixed order: a second launch repeats the first one's K and V rows bit by bit."""
     from qwen3mk.kernel import SeqTable

@@ -46,7 +46,7 @@ def test_noalloc_matches_engine_twice_in_a_row(oracle):
         assert rc == 0, lib.q3_last_error(None)
         torch.cuda.synchronize()
         assert nxt.tolist() == want["next_token"].tolist()
-        # same kernels, same order of operations: the tolerance of the parity tests is far more than needed
+        # other kernels (the engine runs its launch chain): the tolerance of the parity tests
         assert oracle.rel_l2(logits, want["logits"]) <= 1e-4
         assert oracle.bf16_ulps(kw, want["k_write"]) <= 2 and oracle.bf16_ulps(vw, want["v_write"]) <= 2
         # and against the CPU oracle, like every other path
