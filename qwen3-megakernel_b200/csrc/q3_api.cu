@@ -7,10 +7,13 @@
 #include <new>
 #include <vector>
 
+#include <cuda.h>
+
 #include "q3_engine.h"
 #include "q3_gemm_cl.h"
 #include "q3_gemm_tc.h"
 #include "q3_layer_tc.h"
+#include "q3_prompt.h"
 
 using namespace q3;
 
@@ -286,15 +289,16 @@ static int splits_for(const q3_engine* e, int batch, int max_len, bool chain) {
     return s;
 }
 
-int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, int tc_planes, const PrefillCtx* prompt, bool layer_kernel) {
-    const bool last_token_only = prompt != nullptr;
+int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, bool prompt, bool layer_kernel) {
+    const bool last_token_only = prompt;
     const int B = a->batch, L = e->cfg.n_layers, V = e->cfg.vocab;
     const q3_weights& w = e->w;
     const int append = (a->flags & Q3_F_APPEND_KV) ? 1 : 0;
-    const bool chain = prompt == nullptr && !layer_kernel && tc_planes == 3 && chain_serves(e, B);
+    const bool chain = !prompt && !layer_kernel && chain_serves(e, B);
     const int ns = splits_for(e, B, a->max_len, chain);
-    // From Q3_TC_MIN_BATCH tokens on, the projections are tensor-core GEMMs over bf16 planes of the
-    // activations (tc_planes = 3: exact to fp32); below that, CUDA-core matrix-vector kernels.
+    // From Q3_TC_MIN_BATCH tokens on, the projections are tensor-core GEMMs over three bf16 planes of the
+    // activations (exact to fp32); below that, CUDA-core matrix-vector kernels.
+    constexpr int tc_planes = 3;
     const bool tc = B >= Q3_TC_MIN_BATCH && e->planes != nullptr;
     const int tile = B <= 32 ? 32 : (B <= 64 ? 64 : 128);
     const int prow = (B + tile - 1) / tile * tile;
@@ -382,7 +386,7 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
     }
     // The fused path, decode batches of 4..64 sequences: two launches per layer, the split attention and the persistent layer kernel
     // (everything between two attentions: merge, Wo, norm, gate/up, SiLU, down, norm, q/k/v of the next layer).
-    const bool lk = layer_kernel && tc && prompt == nullptr && tc_planes == 3 && layer_tc_supports(e, B);
+    const bool lk = layer_kernel && tc && !prompt && layer_tc_supports(e, B);
     if (lk) LAUNCH(launch_layer_tc(e, LK_MODE_FIRST, 0, B, st));
     for (int l = 0; lk && l < L; ++l) {
         AttnArgs t{};
@@ -433,8 +437,7 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
         h.layer = l; h.n_layers = L; h.append = append; h.len_bound = len_bound;
         // A prompt's tokens attend rows that earlier tokens of the same launch append: those need the separate kernel.
         // A decode step prepares the heads inside the attention kernel (one launch less per layer).
-        const bool fused_prep = prompt == nullptr;
-        h.skip_k_store = (prompt != nullptr && B >= 64) ? 1 : 0;   // the tcgen05 attention of a long prompt reads K from the cache
+        const bool fused_prep = !prompt;
         if (!fused_prep) LAUNCH(launch_head_prep(h, B, st));
 
         AttnArgs t{};
@@ -444,13 +447,7 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
         t.chunk_pad = pad; t.len_bound = len_bound;
         t.fused_prep = fused_prep ? 1 : 0; t.qn = h.qn; t.kn = h.kn; t.rope = h.rope; t.k_write = h.k_write; t.v_write = h.v_write;
         t.n_layers = L; t.append = append;
-        if (prompt != nullptr && B >= 64) {
-            // a prompt: tiled causal attention over the rows head_prep has just written into the cache
-            const bf16_raw* kc = bf(prompt->kcache) + (size_t)l * prompt->layer_stride;
-            const bf16_raw* vc = bf(prompt->vcache) + (size_t)l * prompt->layer_stride;
-            // tcgen05 attention; it writes the Wo GEMM's input planes itself
-            LAUNCH(launch_prefill_attn_tc(e->qkv, kc, vc, (int)(prompt->layer_stride / KV_DIM), planes, prow, tc_planes, B, e->status, st));
-        } else if (tc && ns == 1 && fused_prep && tc_planes == 3) {
+        if (tc && ns == 1 && fused_prep) {
             // one split: the attention blocks write the Wo GEMM's input planes themselves, no merge launch (the padding rows of the
             // token tile keep whatever they held: their columns of the product are never stored)
             t.planes_out = planes; t.plane_rows = prow;
@@ -466,19 +463,6 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, i
         if (tc) {
             // x += attn @ wo^T
             LAUNCH(gemm(bf(w.wo) + (size_t)l * HIDDEN * Q_DIM, HIDDEN, Q_DIM, e->x, HIDDEN, e->x, HIDDEN));
-            // hid = silu(rms(x, ln2) @ wg^T) * (rms(x, ln2) @ wu^T)
-            // A long prompt: gate and up in one work item of the persistent GEMM, SiLU in its epilogue, the product written as
-            // the down GEMM's input plane into the second third of the plane buffer (one plane in use, so that third is free).
-            if (prompt != nullptr && tc_planes == 1 && gemm_tc_silu_fits(INTER, B)) {
-                LAUNCH(launch_act_split(e->x, HIDDEN, HIDDEN, bf(w.ln2) + (size_t)l * HIDDEN, planes, prow, tc_planes, B, st, nullptr));
-                bf16_raw* hplane = planes + (size_t)((e->cap + 127) / 128 * 128) * INTER;
-                GemmTcSiluCall c{bf(w.wg) + (size_t)l * INTER * HIDDEN, bf(w.wu) + (size_t)l * INTER * HIDDEN, planes, hplane,
-                                 INTER, B, HIDDEN, tc_planes, prow, prow, e->status};
-                LAUNCH(launch_gemm_tc_silu(c, st));
-                GemmTcCall d{bf(w.wd) + (size_t)l * HIDDEN * INTER, hplane, e->x, e->x, HIDDEN, HIDDEN, HIDDEN, B, INTER, 1, prow, e->status};
-                LAUNCH(launch_gemm_tc(d, st));
-                continue;
-            }
             // hid = silu(rms(x, ln2) @ wg^T) * (rms(x, ln2) @ wu^T)
             const ZeroRows zf{{e->gate, e->up}, {INTER, INTER}, {INTER, INTER}};
             LAUNCH(launch_act_split(e->x, HIDDEN, HIDDEN, bf(w.ln2) + (size_t)l * HIDDEN, planes, prow, tc_planes, B, st,
@@ -569,7 +553,7 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
     }
     if (path != Q3_F_PATH_LAYERED && path != Q3_F_PATH_FUSED) return fail(e, Q3_ERR_INVALID, "q3_decode: unknown path flag 0x%x", path);
     const bool layer_kernel = path == Q3_F_PATH_FUSED;
-    if (!(a->flags & Q3_F_GRAPH)) return decode_layered(e, a, st, 3, nullptr, layer_kernel);
+    if (!(a->flags & Q3_F_GRAPH)) return decode_layered(e, a, st, false, layer_kernel);
 
     // graph replay: the key is the argument block with max_len replaced by what it determines in the captured
     // launches: the split count and the padded chunk length (which also sizes the attention kernel's shared memory)
@@ -592,12 +576,12 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
         e->launches += hit->launches;
         return Q3_OK;
     }
-    if (hit->seen++ < plain_uses(a->batch)) return decode_layered(e, a, st, 3, nullptr, layer_kernel);
+    if (hit->seen++ < plain_uses(a->batch)) return decode_layered(e, a, st, false, layer_kernel);
     const int64_t before = e->launches;
     // capture on the engine's own stream (the legacy default stream cannot be captured); nothing runs during capture
     cudaStream_t cs = static_cast<cudaStream_t>(e->capture_stream);
     CU(e, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    const int rc = decode_layered(e, a, cs, 3, nullptr, layer_kernel);
+    const int rc = decode_layered(e, a, cs, false, layer_kernel);
     cudaGraph_t graph = nullptr;
     const cudaError_t end = cudaStreamEndCapture(cs, &graph);
     if (rc != Q3_OK) { if (graph) cudaGraphDestroy(graph); return rc; }
@@ -612,36 +596,113 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
     return Q3_OK;
 }
 
-// Activation planes of a prompt's GEMMs.  One: the activations enter the tensor cores rounded to bf16, like the weights and
-// like the cached K/V rows that the prompt's later positions attend anyway.  Measured at 2048 tokens, full model, against
-// the fp32 CPU checker: K/V rows rel-L2 6.6e-3 and logits 5.6e-3 with one plane, 4.0e-3 and 3.2e-3 with two (the cache
-// rounding dominates both; the gates are 1e-2 and 2e-2); 5.6 ms against 7.3 ms.
-constexpr int PREFILL_PLANES = 1;
+// A prompt: five launches a layer (q3_prompt.h).  The activations enter the tensor cores rounded to bf16, like the weights and like
+// the cached K/V rows that the prompt's later positions attend anyway.  Measured at 2048 tokens, full model, against the fp32 CPU
+// checker: K/V rows rel-L2 6.6e-3 and logits 5.6e-3 with one plane, 4.0e-3 and 3.2e-3 with two (the cache rounding dominates
+// both; the gates are 1e-2 and 2e-2).
+// From 64 tokens on the attention is the tiled one over cached rows; fewer tokens keep the split attention, whose own row and
+// probabilities are more precise than bf16.
+static int prefill_chain(q3_engine* e, const q3_prefill_args* a, const q3_decode_args& s, cudaStream_t st) {
+    const int T = a->n_tokens, L = e->cfg.n_layers, V = e->cfg.vocab;
+    const q3_weights& w = e->w;
+    const bool tiled = T >= 64;
+    auto bf = [](const void* p) { return reinterpret_cast<const bf16_raw*>(p); };
+    // one plane each of the residual rows, the FFN's hidden rows and the attention's output (three for the split attention, which writes
+    // them for its other callers); q's two planes take the place of the fp32 q/k/v rows
+    const size_t cap = (size_t)(e->cap + 127) / 128 * 128;
+    bf16_raw* xn = reinterpret_cast<bf16_raw*>(e->planes);
+    bf16_raw *hid = xn + cap * HIDDEN, *attn = hid + cap * INTER;
+    bf16_raw *q_hi = reinterpret_cast<bf16_raw*>(e->qkv), *q_lo = q_hi + (size_t)T * Q_DIM;
+    float* ssq = e->gate;
+    CUtensorMap m_xn, m_hid, m_attn, m_qh, m_ql, m_k, m_v;
+    bool ok = tc_make_map(&m_xn, xn, 0, T, HIDDEN, 1, 128) && tc_make_map(&m_hid, hid, 0, T, INTER, 1, 128) && tc_make_map(&m_attn, attn, 0, T, Q_DIM, 1, 128);
+    if (tiled)
+        ok = ok && tc_make_map(&m_qh, q_hi, 0, T, Q_DIM, 1, 64) && tc_make_map(&m_ql, q_lo, 0, T, Q_DIM, 1, 64) &&
+             tc_make_map(&m_k, a->kcache, L, T, KV_DIM, 1, 128, a->cache_capacity) && tc_make_map(&m_v, a->vcache, L, T, KV_DIM, 1, 128, a->cache_capacity);
+    if (!ok) return fail(e, Q3_ERR_CUDA, "q3_prefill: a tensor map could not be encoded");
+    const int ns = tiled ? 1 : splits_for(e, T, s.max_len, false);
+#define LAUNCH(call)                                                                                   \
+    do {                                                                                               \
+        cudaError_t err__ = (call);                                                                    \
+        ++e->launches;                                                                                 \
+        if (err__ != cudaSuccess) return fail(e, Q3_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(err__)); \
+    } while (0)
+    LAUNCH(launch_prompt_embed(reinterpret_cast<const long long*>(a->ids), bf(w.embed), V, e->x, bf(w.ln1), xn, ssq, T, e->status, T, st));
+    for (int l = 0; l < L; ++l) {
+        PromptGemmCall c{};
+        c.T = T; c.ssq = ssq; c.ssq_ld = T; c.status = e->status;
+        PromptGemmCall q = c;
+        q.kind = PR_QKV; q.K = HIDDEN; q.in = &m_xn;
+        q.w[0] = bf(w.wq) + (size_t)l * Q_DIM * HIDDEN; q.w[1] = bf(w.wk) + (size_t)l * KV_DIM * HIDDEN; q.w[2] = bf(w.wv) + (size_t)l * KV_DIM * HIDDEN;
+        if (tiled) { q.q_hi = q_hi; q.q_lo = q_lo; }
+        else q.qkv = e->qkv;
+        const size_t row0 = (size_t)l * a->cache_capacity * KV_DIM;
+        q.kc = reinterpret_cast<bf16_raw*>(a->kcache) + row0; q.vc = reinterpret_cast<bf16_raw*>(a->vcache) + row0;
+        q.qn = bf(w.qn) + (size_t)l * HEAD_DIM; q.kn = bf(w.kn) + (size_t)l * HEAD_DIM; q.rope = e->rope;
+        LAUNCH(launch_prompt_gemm(q, st));
 
-// Prefill: the T prompt tokens run through the layered path as T one-token "sequences" of the same
-// cache, token t at position t.  head_prep writes every K/V row into the cache before the attention
-// kernels run, so token t attends rows [0, t) from the cache (rounded to bf16, as a later decode step
-// will see them) and its own row in fp32: causal attention, the numerics of token-by-token decode.
-// The projections are tensor-core GEMMs over PREFILL_PLANES bf16 planes of the activations.
-static int prefill_batched(q3_engine* e, const q3_prefill_args* a, cudaStream_t st) {
+        if (tiled) {
+            LAUNCH(launch_prefill_attn_tc(m_qh, m_ql, m_k, m_v, l, attn, T, e->status, st));
+        } else {
+            AttnArgs t{};
+            t.qkv = e->qkv; t.seq_k = s.seq_k; t.seq_v = s.seq_v;
+            t.seq_layer_stride = reinterpret_cast<const long long*>(s.seq_layer_stride);
+            t.seq_len = s.seq_len; t.part = e->part; t.layer = l; t.n_splits = ns; t.chunk_pad = chunk_pad_for(s.max_len, ns); t.len_bound = s.max_len;
+            t.n_layers = L;
+            LAUNCH(launch_attn_planes(t, attn, T, 1, T, st));
+            ++e->launches;   // two kernels
+        }
+
+        PromptGemmCall o = c;
+        o.kind = PR_RESID; o.K = Q_DIM; o.in = &m_attn; o.x = e->x; o.xn = xn; o.gain = bf(w.ln2) + (size_t)l * HIDDEN;
+        o.w[0] = bf(w.wo) + (size_t)l * HIDDEN * Q_DIM;
+        LAUNCH(launch_prompt_gemm(o, st));
+        PromptGemmCall g = c;
+        g.kind = PR_SILU; g.K = HIDDEN; g.in = &m_xn; g.hid = hid;
+        g.w[0] = bf(w.wg) + (size_t)l * INTER * HIDDEN; g.w[1] = bf(w.wu) + (size_t)l * INTER * HIDDEN;
+        LAUNCH(launch_prompt_gemm(g, st));
+        PromptGemmCall d = c;
+        d.kind = PR_RESID; d.K = INTER; d.in = &m_hid; d.x = e->x; d.xn = xn;
+        d.gain = l + 1 < L ? bf(w.ln1) + (size_t)(l + 1) * HIDDEN : bf(w.fnorm);
+        d.w[0] = bf(w.wd) + (size_t)l * HIDDEN * INTER;
+        LAUNCH(launch_prompt_gemm(d, st));
+    }
+    // the last token's logits
+    GemvArgs g{};
+    g.seg[0] = {bf(w.embed), V};
+    g.x = e->x + (size_t)(T - 1) * HIDDEN; g.ldx = HIDDEN; g.gain = bf(w.fnorm);
+    g.out = s.logits; g.ldo = V; g.n_rows = V; g.batch = 1; g.pval = e->pval; g.pidx = e->pidx;
+    int lm_grid = (V + 15) / 16;
+    if (lm_grid > e->lm_grid) lm_grid = e->lm_grid;
+    LAUNCH(launch_gemv(1024, EPI_LOGITS, g, lm_grid, st));
+    LAUNCH(launch_argmax_final(e->pval, e->pidx, lm_grid, reinterpret_cast<long long*>(s.next_token), nullptr, 0, 1, st));
+#undef LAUNCH
+    return Q3_OK;
+}
+
+// A prompt of fewer than Q3_TC_MIN_BATCH tokens runs through the layered path as T one-token "sequences" of the same cache, token t at
+// position t, in fp32.  head_prep writes every K/V row into the cache before the attention kernels run, so token t attends rows [0, t)
+// from the cache (rounded to bf16, as a later decode step will see them) and its own row in fp32.
+static int prefill_any(q3_engine* e, const q3_prefill_args* a, cudaStream_t st) {
     const int T = a->n_tokens;
     char* d = reinterpret_cast<char*>(e->pf_desc);
     uint64_t* seq_k = reinterpret_cast<uint64_t*>(d + 64);
     uint64_t* seq_v = seq_k + e->cap;
     long long* stride = reinterpret_cast<long long*>(seq_v + e->cap);
     int* len = reinterpret_cast<int*>(stride + e->cap);
-    cudaError_t err = launch_prefill_desc(seq_k, seq_v, stride, len, reinterpret_cast<uint64_t>(a->kcache), reinterpret_cast<uint64_t>(a->vcache),
-                                          (long long)a->cache_capacity * KV_DIM, T, st);
-    ++e->launches;
-    if (err != cudaSuccess) return fail(e, Q3_ERR_CUDA, "prefill descriptors: %s", cudaGetErrorString(err));
     q3_decode_args s{};
     s.batch = T; s.max_len = T - 1; s.flags = Q3_F_APPEND_KV | Q3_F_PATH_LAYERED;
     s.token = a->ids;
     s.seq_k = seq_k; s.seq_v = seq_v; s.seq_layer_stride = reinterpret_cast<const int64_t*>(stride); s.seq_len = len;
     s.logits = a->last_logits;
     s.next_token = a->next_token ? a->next_token : reinterpret_cast<int64_t*>(d + 32);
-    const PrefillCtx ctx{a->kcache, a->vcache, (long long)a->cache_capacity * KV_DIM};
-    return decode_layered(e, &s, st, PREFILL_PLANES, &ctx);
+    if (T < 64) {   // the split attention takes a prompt's tokens as sequences of the same cache
+        cudaError_t err = launch_prefill_desc(seq_k, seq_v, stride, len, reinterpret_cast<uint64_t>(a->kcache), reinterpret_cast<uint64_t>(a->vcache),
+                                              (long long)a->cache_capacity * KV_DIM, T, st);
+        ++e->launches;
+        if (err != cudaSuccess) return fail(e, Q3_ERR_CUDA, "prefill descriptors: %s", cudaGetErrorString(err));
+    }
+    return T < Q3_TC_MIN_BATCH ? decode_layered(e, &s, st, true) : prefill_chain(e, a, s, st);
 }
 
 extern "C" int q3_linear_tc(const void* w, const float* x, float* out, const float* resid, int32_t n_rows, int32_t n_tok, int32_t K,
@@ -671,5 +732,5 @@ extern "C" int q3_prefill(q3_engine* e, const q3_prefill_args* a, void* stream) 
     if (a->n_tokens > e->rope_n) return fail(e, Q3_ERR_INVALID, "q3_prefill: RoPE table has %d rows, need %d", e->rope_n, a->n_tokens);
     if (!a->ids || !a->kcache || !a->vcache) return fail(e, Q3_ERR_INVALID, "q3_prefill: ids, kcache and vcache are required");
     CU(e, cudaSetDevice(e->device));
-    return prefill_batched(e, a, (cudaStream_t)stream);
+    return prefill_any(e, a, (cudaStream_t)stream);
 }

@@ -70,16 +70,8 @@ int persist_tp_attach(q3_engine* e, int rank, int size, const void* handles);
 int persist_recover(q3_engine* e);   // after a device-side wait gave up: clear the exchange buffers and accumulators
 int engine_fail(q3_engine* e, int code, const char* fmt, ...);
 // the layered decode step on engine `e` (one launch per phase); `e` supplies weights, RoPE table and scratch
-// prompt-mode extras of the layered step: one sequence, tokens at positions 0..T-1 of this cache
-struct PrefillCtx {
-    const void* kcache;   // bf16 [L, capacity, 8, 128]
-    const void* vcache;
-    long long layer_stride;
-};
+// prompt: a few prompt tokens as sequences of one cache, only the last one's logits
 // layer_kernel: decode batches the persistent layer kernel serves take it (two launches per layer); false keeps one
 // launch per phase
-int decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, int tc_planes = 3, const PrefillCtx* prompt = nullptr,
-                   bool layer_kernel = false);
-cudaError_t launch_prefill_attn_tc(const float* qkv, const void* kcache_layer, const void* vcache_layer, int cap_rows, void* planes,
-                                   int plane_rows, int nsplit, int T, uint32_t* status, cudaStream_t st);
+int decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, bool prompt = false, bool layer_kernel = false);
 }  // namespace q3

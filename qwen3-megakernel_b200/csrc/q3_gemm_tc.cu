@@ -247,27 +247,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
 //   * N = 256 per tcgen05.mma halves the shared-memory operand traffic per flop against N = 128.
 // Items are numbered with the weight tile fastest, so that the CTAs of a round share a few token tiles in L2.
 // ------------------------------------------------------------------------------------------------
-//
-// DUAL: the FFN's gate and up in one item - the same 128 rows of Wg and of Wu against a tile of 128 tokens, four
-// accumulators of 128 columns - and an epilogue that writes silu(gate) * up as the bf16 plane the down GEMM reads.  The
-// fp32 gate and up matrices (2 x 25 MB per layer at 2048 tokens) and the kernel that read them back are gone, and the
-// exponentials of the epilogue hide behind the next item's MMAs.
 constexpr int TP_BN = 256;
 constexpr int TP_THREADS = 64 + 256;   // warp 0: TMA, warp 1: MMA, warps 2..9: epilogue (two warps per TMEM lane quadrant, half the columns each)
 struct GemmPersistItems {
     int n_items, m_tiles, n_ttiles;   // items = token tiles x weight tiles
-    bf16_raw* silu_out;               // DUAL: [silu_rows][n_rows] bf16
-    int silu_rows;                    // rows of that plane (multiple of 128): rows past the prompt are written as zeros
 };
 
-template <bool DUAL>
 __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap tm_w0,
                                                                         const __grid_constant__ CUtensorMap tm_w1,
                                                                         const __grid_constant__ CUtensorMap tm_w2,
                                                                         const __grid_constant__ CUtensorMap tm_x, const GemmTcParams p,
                                                                         const GemmPersistItems w) {
-    constexpr int BN = DUAL ? 128 : TP_BN;          // tokens per item
-    constexpr int ACC = DUAL ? 2 * BN : BN;         // TMEM columns of one accumulator buffer (DUAL: gate | up)
+    constexpr int BN = TP_BN;                       // tokens per item
+    constexpr int ACC = BN;                         // TMEM columns of one accumulator buffer
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[8], empty_bar[8], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_s;
@@ -275,7 +267,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
 
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int nsplit = p.nsplit, stages = p.stages;
-    const uint32_t a_bytes = (DUAL ? 2 : 1) * TC_BM * TC_BK * 2, b_bytes = BN * TC_BK * 2;   // DUAL: the Wg tile, then the Wu tile
+    const uint32_t a_bytes = TC_BM * TC_BK * 2, b_bytes = BN * TC_BK * 2;
     const uint32_t stage_bytes = a_bytes + nsplit * b_bytes;
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
 
@@ -310,7 +302,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
         int tile = rem % w.m_tiles;
         r.n0 = (rem / w.m_tiles) * BN;
         r.grp = 0;
-        if (!DUAL && p.n_groups > 1) {
+        if (p.n_groups > 1) {
             if (tile >= p.g_tiles[0]) { tile -= p.g_tiles[0]; r.grp = 1; }
             if (r.grp == 1 && p.n_groups > 2 && tile >= p.g_tiles[1]) { tile -= p.g_tiles[1]; r.grp = 2; }
         }
@@ -335,9 +327,6 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(&full_bar[s])), "r"(stage_bytes) : "memory");
                     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                                  ::"r"(tc_smem(st)), "l"(tm_w), "r"((r.kb_begin + kb) * TC_BK), "r"(r.m0), "r"(tc_smem(&full_bar[s])) : "memory");
-                    if (DUAL)
-                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                     ::"r"(tc_smem(st + a_bytes / 2)), "l"(&tm_w1), "r"((r.kb_begin + kb) * TC_BK), "r"(r.m0), "r"(tc_smem(&full_bar[s])) : "memory");
                     for (int sp = 0; sp < nsplit; ++sp)
                         asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                                      ::"r"(tc_smem(st + a_bytes + sp * b_bytes)), "l"(&tm_x), "r"((r.kb_begin + kb) * TC_BK), "r"(sp * p.plane_rows + r.n0),
@@ -372,12 +361,6 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
                             asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                                          "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
                                          ::"r"(tmem_base + (uint32_t)(acc * ACC)), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
-                            if (DUAL) {
-                                const uint64_t du = tc_desc(sa + a_bytes / 2 + k * 32);
-                                asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                                             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                                             ::"r"(tmem_base + (uint32_t)(acc * ACC + BN)), "l"(du), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
-                            }
                         }
                     }
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&empty_bar[s])) : "memory");
@@ -400,30 +383,6 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = r.m0 + quad * 32 + lane;    // weight row = output column (every tile is a full 128 rows)
-            if (DUAL) {
-                // Reading TMEM while the MMAs of the next item run costs about a microsecond per round trip, whatever its width:
-                // two rounds of 64 tokens (gate and up requested together, one wait) instead of sixteen narrow ones
-                for (int c = half; c == half; ++c) {   // 64 tokens: this warp's half of the item
-                    if (r.n0 + c * 64 >= w.silu_rows) break;
-                    uint32_t g[64], u[64];
-                    const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * ACC + c * 64);
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-                                 : "=r"(g[0]), "=r"(g[1]), "=r"(g[2]), "=r"(g[3]), "=r"(g[4]), "=r"(g[5]), "=r"(g[6]), "=r"(g[7]), "=r"(g[8]), "=r"(g[9]), "=r"(g[10]), "=r"(g[11]), "=r"(g[12]), "=r"(g[13]), "=r"(g[14]), "=r"(g[15]), "=r"(g[16]), "=r"(g[17]), "=r"(g[18]), "=r"(g[19]), "=r"(g[20]), "=r"(g[21]), "=r"(g[22]), "=r"(g[23]), "=r"(g[24]), "=r"(g[25]), "=r"(g[26]), "=r"(g[27]), "=r"(g[28]), "=r"(g[29]), "=r"(g[30]), "=r"(g[31]), "=r"(g[32]), "=r"(g[33]), "=r"(g[34]), "=r"(g[35]), "=r"(g[36]), "=r"(g[37]), "=r"(g[38]), "=r"(g[39]), "=r"(g[40]), "=r"(g[41]), "=r"(g[42]), "=r"(g[43]), "=r"(g[44]), "=r"(g[45]), "=r"(g[46]), "=r"(g[47]), "=r"(g[48]), "=r"(g[49]), "=r"(g[50]), "=r"(g[51]), "=r"(g[52]), "=r"(g[53]), "=r"(g[54]), "=r"(g[55]), "=r"(g[56]), "=r"(g[57]), "=r"(g[58]), "=r"(g[59]), "=r"(g[60]), "=r"(g[61]), "=r"(g[62]), "=r"(g[63]) : "r"(taddr) : "memory");
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-                                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]), "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31]), "=r"(u[32]), "=r"(u[33]), "=r"(u[34]), "=r"(u[35]), "=r"(u[36]), "=r"(u[37]), "=r"(u[38]), "=r"(u[39]), "=r"(u[40]), "=r"(u[41]), "=r"(u[42]), "=r"(u[43]), "=r"(u[44]), "=r"(u[45]), "=r"(u[46]), "=r"(u[47]), "=r"(u[48]), "=r"(u[49]), "=r"(u[50]), "=r"(u[51]), "=r"(u[52]), "=r"(u[53]), "=r"(u[54]), "=r"(u[55]), "=r"(u[56]), "=r"(u[57]), "=r"(u[58]), "=r"(u[59]), "=r"(u[60]), "=r"(u[61]), "=r"(u[62]), "=r"(u[63]) : "r"(taddr + (uint32_t)BN) : "memory");
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    bf16_raw* dst = w.silu_out + (size_t)(r.n0 + c * 64) * p.n_rows + row;
-#pragma unroll
-                    for (int j = 0; j < 64; ++j) {
-                        const int t = r.n0 + c * 64 + j;
-                        if (t < w.silu_rows) {          // rows past the prompt are the token tile's padding: zeros
-                            const float a = __uint_as_float(g[j]), b = __uint_as_float(u[j]);
-                            const float x = t < p.n_tok ? __fdividef(a, 1.f + __expf(-a)) * b : 0.f;   // (a prompt's gates are 1e-2)
-                            dst[(size_t)j * p.n_rows] = f_to_bf(x);
-                        }
-                    }
-                }
-            } else
 #pragma unroll 1
             for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
                 if (r.n0 + c * 32 >= p.n_tok) break;    // the rest of the token tile is padding
@@ -484,14 +443,14 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// bf16 tensor [planes, rows, cols] row-major (two-dimensional when planes is 0), box [all planes, box_rows, 64 columns],
+// bf16 tensor [planes, rows, cols] row-major (two-dimensional when planes is 0), box [box_planes, box_rows, 64 columns],
 // 128-byte swizzle
-static bool make_map(CUtensorMap* m, const void* ptr, uint64_t planes, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+bool tc_make_map(CUtensorMap* m, const void* ptr, uint64_t planes, uint64_t rows, uint64_t cols, uint32_t box_planes, uint32_t box_rows, uint64_t plane_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t dims[3] = {cols, rows, planes};
-    const cuuint64_t strides[2] = {cols * 2, rows * cols * 2};
-    const cuuint32_t box[3] = {TC_BK, box_rows, (cuuint32_t)planes};
+    const cuuint64_t strides[2] = {cols * 2, (plane_rows ? plane_rows : rows) * cols * 2};
+    const cuuint32_t box[3] = {TC_BK, box_rows, box_planes};
     const cuuint32_t estr[3] = {1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, planes ? 3 : 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -520,18 +479,15 @@ static int k_slices(int n_rows, int n_tok, int bn, int nkb, int sm_count) {
 // 2.29 ms, 768 tokens 2.90 / 2.49 / 2.49, 1000 tokens 3.34 / 2.96 / 2.97, 300 tokens 2.05 / 2.05 / 2.13.  With K cut in
 // slices for the launches of few tiles (Wo, down) it was no faster than the one-tile-per-CTA kernel with three CTAs per
 // SM (19.1 / 23.1 us against 19.0 / 19.0), so those stay there.
-static bool persist_serves(int n_rows, int n_tok, int nsplit, int plane_rows, int sm_count) {
-    // one activation plane (what prompts use): with more the 256-token stages no longer fit four deep
-    (void)plane_rows;
+static bool persist_serves(int n_rows, int n_tok, int nsplit, int sm_count) {
+    // one activation plane: with more the 256-token stages no longer fit four deep
     return n_tok >= TP_BN && nsplit == 1 && (n_rows / TC_BM) * ((n_tok + TP_BN - 1) / TP_BN) * 10 >= sm_count * 6;
 }
 
-template <bool DUAL>
-static cudaError_t launch_persist(const CUtensorMap* tw, const CUtensorMap& tx, GemmTcParams p, int n_rows, int n_tok, int sm_count, cudaStream_t st,
-                                  bf16_raw* silu_out = nullptr, int silu_rows = 0) {
-    constexpr int BN = DUAL ? 128 : TP_BN;
+static cudaError_t launch_persist(const CUtensorMap* tw, const CUtensorMap& tx, GemmTcParams p, int n_rows, int n_tok, int sm_count, cudaStream_t st) {
+    constexpr int BN = TP_BN;
     p.kb_per_split = p.K / TC_BK;   // K is never cut here
-    const uint32_t stage_bytes = (DUAL ? 2 : 1) * TC_BM * TC_BK * 2 + p.nsplit * BN * TC_BK * 2;
+    const uint32_t stage_bytes = TC_BM * TC_BK * 2 + p.nsplit * BN * TC_BK * 2;
     int stages = (int)((200u * 1024u) / stage_bytes);
     if (stages > 8) stages = 8;
     if (stages < 2) return cudaErrorInvalidValue;
@@ -544,7 +500,7 @@ static cudaError_t launch_persist(const CUtensorMap* tw, const CUtensorMap& tx, 
         if (e != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return cudaErrorInvalidDevice;
         std::lock_guard<std::mutex> hold(host_lock());
         if (!attr_set[dev]) {
-            e = cudaFuncSetAttribute(gemm_tc_persist_kernel<DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+            e = cudaFuncSetAttribute(gemm_tc_persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
             if (e != cudaSuccess) return e;
             attr_set[dev] = true;
         }
@@ -553,9 +509,8 @@ static cudaError_t launch_persist(const CUtensorMap* tw, const CUtensorMap& tx, 
     w.m_tiles = n_rows / TC_BM;
     w.n_ttiles = (n_tok + BN - 1) / BN;
     w.n_items = w.m_tiles * w.n_ttiles;
-    w.silu_out = silu_out; w.silu_rows = silu_rows;
     const int grid = w.n_items < sm_count ? w.n_items : sm_count;
-    return launch_chain(gemm_tc_persist_kernel<DUAL>, dim3(grid), dim3(TP_THREADS), smem, st, tw[0], tw[1], tw[2], tx, p, w);
+    return launch_chain(gemm_tc_persist_kernel, dim3(grid), dim3(TP_THREADS), smem, st, tw[0], tw[1], tw[2], tx, p, w);
 }
 
 template <int BN, bool SCALE = false>
@@ -623,20 +578,19 @@ static bool cached_map(const void* ptr, uint64_t rows, uint64_t cols, uint32_t b
         if (e.k.p == ptr && e.k.planes == planes && e.k.rows == rows && e.k.cols == cols && e.k.box == box_rows) { *out = e.m; return true; }
     if (c.size() > 4096) c.clear();
     MapEntry e{{ptr, planes, rows, cols, box_rows}, {}};
-    if (!make_map(&e.m, ptr, planes, rows, cols, box_rows)) return false;
+    if (!tc_make_map(&e.m, ptr, planes, rows, cols, (uint32_t)planes, box_rows)) return false;
     c.push_back(e);
     *out = e.m;
     return true;
 }
 bool gemm_tc_splits_k(int n_rows, int n_tok, int K) {
-    // (the persistent kernel never cuts K; the callers that ask pass a prompt's single plane)
-    if (persist_serves(n_rows, n_tok, 1, 0, sm_count_of_current_device())) return false;
     const int bn = n_tok <= 32 ? 32 : (n_tok <= 64 ? 64 : 128);
     return k_slices(n_rows, n_tok, bn, K / TC_BK, sm_count_of_current_device()) > 1;
 }
 bool tc_cached_map(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out, uint64_t planes) {
     return cached_map(ptr, rows, cols, box_rows, out, planes);
 }
+int tc_sm_count() { return sm_count_of_current_device(); }
 static int sm_count_of_current_device() {
     static int sms[MAX_DEVICES] = {};
     int dev = 0;
@@ -668,10 +622,10 @@ cudaError_t launch_gemm_tc(const GemmTcCall& c, cudaStream_t st) {
         if (bn == 32) return launch_bn<32, true>(maps, tx, q, c.n_rows, c.n_tok, sm_count, st);
         return launch_bn<64, true>(maps, tx, q, c.n_rows, c.n_tok, sm_count, st);
     }
-    if (persist_serves(c.n_rows, c.n_tok, c.nsplit, c.plane_rows, sm_count)) {
+    if (persist_serves(c.n_rows, c.n_tok, c.nsplit, sm_count)) {
         CUtensorMap txp;
         if (!cached_map(c.x_planes, (uint64_t)c.nsplit * c.plane_rows, (uint64_t)c.K, (uint32_t)TP_BN, &txp)) return cudaErrorUnknown;
-        return launch_persist<false>(maps, txp, p, c.n_rows, c.n_tok, sm_count, st);
+        return launch_persist(maps, txp, p, c.n_rows, c.n_tok, sm_count, st);
     }
     if (bn == 32) return launch_bn<32>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
     if (bn == 64) return launch_bn<64>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
@@ -698,34 +652,14 @@ cudaError_t launch_gemm_tc_group(const GemmTcGroupCall& c, cudaStream_t st) {
     p.nsplit = c.nsplit; p.plane_rows = c.plane_rows; p.epi = TC_EPI_STORE; p.status = c.status; p.out_is_zero = c.out_is_zero;
     const int sm_count = sm_count_of_current_device();
     if (sm_count < 1) return cudaErrorInvalidDevice;
-    if (persist_serves(rows, c.n_tok, c.nsplit, c.plane_rows, sm_count)) {
+    if (persist_serves(rows, c.n_tok, c.nsplit, sm_count)) {
         CUtensorMap txp;
         if (!cached_map(c.x_planes, (uint64_t)c.nsplit * c.plane_rows, (uint64_t)c.K, (uint32_t)TP_BN, &txp)) return cudaErrorUnknown;
-        return launch_persist<false>(maps, txp, p, rows, c.n_tok, sm_count, st);
+        return launch_persist(maps, txp, p, rows, c.n_tok, sm_count, st);
     }
     if (bn == 32) return launch_bn<32>(maps, tx, p, rows, c.n_tok, sm_count, st);
     if (bn == 64) return launch_bn<64>(maps, tx, p, rows, c.n_tok, sm_count, st);
     return launch_bn<128>(maps, tx, p, rows, c.n_tok, sm_count, st);
-}
-
-bool gemm_tc_silu_fits(int n_rows, int n_tok) {
-    const int sm = sm_count_of_current_device();
-    return n_tok >= 128 && sm > 0 && (n_rows / TC_BM) * ((n_tok + 127) / 128) * 10 >= sm * 6;
-}
-
-cudaError_t launch_gemm_tc_silu(const GemmTcSiluCall& c, cudaStream_t st) {
-    if (c.K % TC_BK || c.n_rows % TC_BM || c.nsplit != 1 || c.n_tok < 1 || c.out_rows % 128 || c.out_rows < c.n_tok)
-        return cudaErrorInvalidValue;
-    CUtensorMap maps[3], tx;
-    if (!cached_map(c.wg, (uint64_t)c.n_rows, (uint64_t)c.K, TC_BM, &maps[0])) return cudaErrorUnknown;
-    if (!cached_map(c.wu, (uint64_t)c.n_rows, (uint64_t)c.K, TC_BM, &maps[1])) return cudaErrorUnknown;
-    maps[2] = maps[0];
-    if (!cached_map(c.x_planes, (uint64_t)c.nsplit * c.plane_rows, (uint64_t)c.K, 128u, &tx)) return cudaErrorUnknown;
-    GemmTcParams p{};
-    p.n_rows = c.n_rows; p.n_tok = c.n_tok; p.K = c.K; p.nsplit = c.nsplit; p.plane_rows = c.plane_rows; p.epi = TC_EPI_STORE; p.status = c.status;
-    const int sm_count = sm_count_of_current_device();
-    if (sm_count < 1) return cudaErrorInvalidDevice;
-    return launch_persist<true>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st, reinterpret_cast<bf16_raw*>(c.out_plane), c.out_rows);
 }
 
 }  // namespace q3

@@ -61,25 +61,15 @@ struct GemmTcGroupCall {
 };
 cudaError_t launch_gemm_tc_group(const GemmTcGroupCall& c, cudaStream_t st);
 
-// Prompts: out_plane = the bf16 plane of silu(x wg^T) * (x wu^T), both products in one work item of the persistent kernel,
-// for the down GEMM to read; no fp32 gate / up matrices.  gemm_tc_silu_fits: the items occupy at least 0.6 of the SMs.
-struct GemmTcSiluCall {
-    const void* wg;        // bf16 [n_rows, K]
-    const void* wu;        // bf16 [n_rows, K]
-    const void* x_planes;  // bf16 [nsplit, plane_rows, K]
-    void* out_plane;       // bf16 [out_rows, n_rows]; must not overlap x_planes; rows n_tok.. are written as zeros
-    int n_rows, n_tok, K, nsplit, plane_rows, out_rows;
-    uint32_t* status;
-};
-bool gemm_tc_silu_fits(int n_rows, int n_tok);
-cudaError_t launch_gemm_tc_silu(const GemmTcSiluCall& c, cudaStream_t st);
-
 // Whether a launch of n_rows weight rows (all groups together) against n_tok tokens will slice K, i.e. add partial tiles
 // into an output that must hold zeros (or the residual) beforehand.
 bool gemm_tc_splits_k(int n_rows, int n_tok, int K);
 
 // A cached tensor map of a row-major bf16 matrix [rows, cols]: boxes of 64 columns x box_rows rows, 128-byte swizzle,
 // out-of-range rows read as zeros.  (CUtensorMap is declared by <cuda.h>, which the caller includes.)
+bool tc_make_map(::CUtensorMap_st* m, const void* ptr, uint64_t planes, uint64_t rows, uint64_t cols, uint32_t box_planes, uint32_t box_rows,
+                 uint64_t plane_rows = 0);   // the same, not cached; plane_rows: rows from one plane to the next where that is more than `rows`
+int tc_sm_count();   // SMs of the current device
 bool tc_cached_map(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, ::CUtensorMap_st* out, uint64_t planes = 0);
 
 }  // namespace q3

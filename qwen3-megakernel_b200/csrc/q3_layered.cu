@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(256) head_prep_kernel(const HeadPrepArgs a) {
         const int d = (lane * 4 + i) & 63;
         v[i] = n * tab[d] + rot * tab[64 + d];
     }
-    if (is_q || !a.skip_k_store) *reinterpret_cast<float4*>(src) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(src) = make_float4(v[0], v[1], v[2], v[3]);
     if (!is_q) {
         const float4 vv = *reinterpret_cast<const float4*>(a.qkv + (size_t)b * QKV_DIM + Q_DIM + KV_DIM + g * HEAD_DIM + lane * 4);
         uint2 kb, vb;

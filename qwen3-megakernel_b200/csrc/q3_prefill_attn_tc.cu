@@ -23,7 +23,7 @@
 #include <cuda.h>
 
 #include "q3_engine.h"
-#include "q3_gemm_tc.h"
+#include "q3_prompt.h"
 
 namespace q3 {
 
@@ -123,19 +123,16 @@ __device__ __forceinline__ void at_ld32(uint32_t (&r)[32], uint32_t taddr) {
 }
 
 struct PrefillAttnTcArgs {
-    const float* qkv;     // [T, 4096] fp32 after head_prep (q normalised + RoPE, unscaled)
-    bf16_raw* planes;     // [nsplit][plane_rows][2048] bf16: the output, already split for the Wo GEMM (hi, then lo = what hi left)
-    int plane_rows, nsplit;
-    int T;
-    int paired;           // the grid has half as many blocks as query tiles
-    int heavy_first;      // a one-dimensional grid of (query tile, kv group) blocks, the tiles with the most key tiles first
+    bf16_raw* plane;      // [T][2048] bf16: the output, as the Wo GEMM reads it
+    int T, layer;
     uint32_t* status;
 };
 
-__global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k,
-                                                                        const __grid_constant__ CUtensorMap tm_v, const PrefillAttnTcArgs a) {
+__global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_constant__ CUtensorMap tm_ql,
+                                                                        const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                                                                        const PrefillAttnTcArgs a) {
     extern __shared__ __align__(1024) unsigned char at_raw[];
-    __shared__ __align__(8) uint64_t k_full[AT_STAGES], v_full[AT_STAGES], k_empty[AT_STAGES], v_empty[AT_STAGES], s_full[2], p_full, o_full[2];
+    __shared__ __align__(8) uint64_t k_full[AT_STAGES], v_full[AT_STAGES], k_empty[AT_STAGES], v_empty[AT_STAGES], q_full, s_full[2], p_full, o_full[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_flag;
     // Per-row partial maxima of the four column parts, exchanged once per key tile with ONE barrier: two buffers, picked by the
@@ -146,7 +143,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
     float (*pm)[128] = reinterpret_cast<float (*)[128]>(&pm16[0][0][0]);
 
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
-    const int g = a.heavy_first ? (int)blockIdx.x % KV_HEADS : (int)blockIdx.y;   // kv head; query heads 2g and 2g + 1
+    const int g = (int)blockIdx.x % KV_HEADS;       // kv head; query heads 2g and 2g + 1
     unsigned char* sQh = at_raw;
     unsigned char* sQl = sQh + AT_Q_BYTES;
     unsigned char* sP = sQl + AT_Q_BYTES;
@@ -163,6 +160,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&s_full[b])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&o_full[b])) : "memory");
         }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&q_full)) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(at_smem(&p_full)), "r"(AT_SOFT) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         abort_flag = 0;
@@ -176,52 +174,42 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
 
-    const int n_qt = (a.T + AT_QT - 1) / AT_QT;
-    int it0 = 0;                                    // key tiles consumed before this pass: every barrier's phase is counted on it
-    for (int pass = 0; pass < 2; ++pass) {
-        const int qt = a.heavy_first ? n_qt - 1 - (int)blockIdx.x / KV_HEADS : (pass ? n_qt - 1 - (int)blockIdx.x : (int)blockIdx.x);
-        if (pass && (a.heavy_first || !a.paired || qt <= (int)blockIdx.x)) break;
-        const int q0 = qt * AT_QT;
-        const int n_kt = (q0 + AT_QT - 1) / AT_KT + 1;          // key tiles up to and including the diagonal one
+    pdl_launch();
 
-        // ---- Q of both heads, scaled, as hi + lo bf16 planes in the operand layout (all 320 threads) ----
-        for (int i = tid; i < 128 * 32; i += AT_THREADS) {       // 128 rows x 32 groups of 4 dims
-            const int row = i >> 5, c4 = (i & 31) * 4;
-            const int pos = min(q0 + (row & 63), a.T - 1), head = 2 * g + (row >> 6);
-            const float4 v = *reinterpret_cast<const float4*>(a.qkv + (size_t)pos * QKV_DIM + head * HEAD_DIM + c4);
-            constexpr float QS = ATTN_SCALE * 1.4426950408889634f;   // scores in units of log2: probabilities are ex2(s - m)
-            const float x[4] = {v.x * QS, v.y * QS, v.z * QS, v.w * QS};
-            bf16_raw h[4], l[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { h[j] = f_to_bf(x[j]); l[j] = f_to_bf(x[j] - bf_to_f(h[j])); }
-            const uint32_t off = at_swz(row, c4);
-            *reinterpret_cast<uint2*>(sQh + off) = make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
-            *reinterpret_cast<uint2*>(sQl + off) = make_uint2((uint32_t)l[0] | ((uint32_t)l[1] << 16), (uint32_t)l[2] | ((uint32_t)l[3] << 16));
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-
+    const int q0 = ((a.T + AT_QT - 1) / AT_QT - 1 - (int)blockIdx.x / KV_HEADS) * AT_QT;   // the query tiles with the most key tiles come first
+    const int n_kt = (q0 + AT_QT - 1) / AT_KT + 1;          // key tiles up to and including the diagonal one
+    {
         if (warp == AT_SOFT / 32) {
             // ------------------------------------------------------------------ TMA producer
             if (elect_one()) {
+                pdl_wait();
+                // Q of both heads, hi and lo: boxes of 64 positions x 64 dims, rows past the prompt read as zeros
+                asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"(2 * AT_Q_BYTES) : "memory");
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int plane = i >> 2, head = (i >> 1) & 1, b = i & 1;
+                    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                                 ::"r"(at_smem((plane ? sQl : sQh) + b * AT_BOX + head * (AT_BOX / 2))), "l"(plane ? &tm_ql : &tm_qh),
+                                   "r"((2 * g + head) * HEAD_DIM + 64 * b), "r"(q0), "r"(at_smem(&q_full)) : "memory");
+                }
                 // K and V of a tile share a stage but are released separately: the K half is free as soon as S of its tile has
                 // been computed, a whole tile before the V half (after PV), so the next K is on its way that much earlier
                 for (int t = 0; t < n_kt; ++t) {
-                    const int it = it0 + t, s = it % AT_STAGES;
+                    const int it = t, s = it % AT_STAGES;
                     unsigned char* sk = sKV + (size_t)s * 2 * AT_KV_BYTES;
                     unsigned char* sv = sk + AT_KV_BYTES;
                     if (it >= AT_STAGES && !at_wait(&k_empty[s], ((it / AT_STAGES) - 1) & 1, &abort_flag, a.status, 40)) break;
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&k_full[s])), "r"(AT_KV_BYTES) : "memory");
 #pragma unroll
                     for (int b = 0; b < 2; ++b)        // the two 64-dim halves of the head
-                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                     ::"r"(at_smem(sk + b * AT_BOX)), "l"(&tm_k), "r"(g * HEAD_DIM + 64 * b), "r"(t * AT_KT), "r"(at_smem(&k_full[s])) : "memory");
+                        asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                                     ::"r"(at_smem(sk + b * AT_BOX)), "l"(&tm_k), "r"(g * HEAD_DIM + 64 * b), "r"(t * AT_KT), "r"(a.layer), "r"(at_smem(&k_full[s])) : "memory");
                     if (it >= AT_STAGES && !at_wait(&v_empty[s], ((it / AT_STAGES) - 1) & 1, &abort_flag, a.status, 47)) break;
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&v_full[s])), "r"(AT_KV_BYTES) : "memory");
 #pragma unroll
                     for (int b = 0; b < 2; ++b)
-                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                     ::"r"(at_smem(sv + b * AT_BOX)), "l"(&tm_v), "r"(g * HEAD_DIM + 64 * b), "r"(t * AT_KT), "r"(at_smem(&v_full[s])) : "memory");
+                        asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                                     ::"r"(at_smem(sv + b * AT_BOX)), "l"(&tm_v), "r"(g * HEAD_DIM + 64 * b), "r"(t * AT_KT), "r"(a.layer), "r"(at_smem(&v_full[s])) : "memory");
                 }
             }
         } else if (warp == AT_SOFT / 32 + 1) {
@@ -231,7 +219,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                 const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
                 const uint32_t idesc_o = idesc_s | (1u << 16);
                 auto issue_s = [&](int t) -> bool {    // S = (Q hi + Q lo) K^T of key tile t, into S buffer it & 1
-                    const int it = it0 + t, s = it % AT_STAGES;
+                    const int it = t, s = it % AT_STAGES;
                     if (!at_wait(&k_full[s], (it / AT_STAGES) & 1, &abort_flag, a.status, 41)) return false;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t sk = at_smem(sKV + (size_t)s * 2 * AT_KV_BYTES);
@@ -252,9 +240,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(at_smem(&k_empty[s])) : "memory");
                     return true;
                 };
-                bool ok = issue_s(0);
+                bool ok = at_wait(&q_full, 0, &abort_flag, a.status, 48) && issue_s(0);
                 for (int t = 0; t < n_kt && ok; ++t) {
-                    const int it = it0 + t, s = it % AT_STAGES;
+                    const int it = t, s = it % AT_STAGES;
                     // S of the next tile first: its buffer was read before P of tile t - 1 was posted, and the exponentials of
                     // tile t can be followed by those of tile t + 1 without waiting for the tensor pipe
                     if (t + 1 < n_kt) ok = issue_s(t + 1);
@@ -297,7 +285,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                 return true;
             };
             for (int t = 0; t < n_kt && ok; ++t) {
-                const int it = it0 + t;
+                const int it = t;
                 ok = at_wait_warp(&s_full[it & 1], (it >> 1) & 1, &abort_flag, a.status, 44);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -346,7 +334,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                 if (t > 0) ok = fold(it - 1, c_prev);
                 c_prev = c;
             }
-            if (ok) ok = fold(it0 + n_kt - 1, c_prev);
+            if (ok) ok = fold(n_kt - 1, c_prev);
             // the row sum is split over the parts' key ranges
             asm volatile("bar.sync 1, %0;" ::"n"(AT_SOFT) : "memory");   // the last tile's maxima have been read
             pm[part][row] = lsum;
@@ -355,24 +343,14 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
 #pragma unroll
             for (int q = 0; q < AT_PARTS; ++q) ltot += pm[q][row];
             const float inv = 1.f / ltot;
-            if (ok && qpos < a.T) {   // 32 dims = 64 contiguous bytes per plane
-                const size_t off = (size_t)qpos * Q_DIM + (2 * g + (row >> 6)) * HEAD_DIM + part * 32;
+            if (ok && qpos < a.T) {   // 32 dims = 64 contiguous bytes
+                bf16_raw* dst = a.plane + (size_t)qpos * Q_DIM + (2 * g + (row >> 6)) * HEAD_DIM + part * 32;
 #pragma unroll
-                for (int j = 0; j < 32; j += 8) {
-                    uint32_t hi[4], lo[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const float x = o[j + 2 * q] * inv, y = o[j + 2 * q + 1] * inv;
-                        hi[q] = at_pack_bf16(x, y);
-                        lo[q] = at_pack_bf16(x - bf_lo(hi[q]), y - bf_hi(hi[q]));
-                    }
-                    *reinterpret_cast<uint4*>(a.planes + off + j) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                    if (a.nsplit > 1) *reinterpret_cast<uint4*>(a.planes + (size_t)a.plane_rows * Q_DIM + off + j) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                }
+                for (int j = 0; j < 32; j += 8)
+                    *reinterpret_cast<uint4*>(dst + j) = make_uint4(at_pack_bf16(o[j] * inv, o[j + 1] * inv), at_pack_bf16(o[j + 2] * inv, o[j + 3] * inv),
+                                                                    at_pack_bf16(o[j + 4] * inv, o[j + 5] * inv), at_pack_bf16(o[j + 6] * inv, o[j + 7] * inv));
             }
         }
-        it0 += n_kt;
-        __syncthreads();   // every MMA of this pass has completed (the last O was read): Q and P may be rewritten
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -382,13 +360,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
     }
 }
 
-cudaError_t launch_prefill_attn_tc(const float* qkv, const void* kcache_layer, const void* vcache_layer, int cap_rows, void* planes,
-                                   int plane_rows, int nsplit, int T, uint32_t* status, cudaStream_t st) {
-    if (nsplit < 1 || nsplit > 2) return cudaErrorInvalidValue;
-    CUtensorMap tk, tv;
-    // the layer's cache as a [cap_rows, 1024] bf16 matrix; boxes of 64 columns x 128 rows (keys past the cache read as zeros)
-    if (!tc_cached_map(kcache_layer, (uint64_t)cap_rows, (uint64_t)KV_DIM, AT_KT, &tk)) return cudaErrorUnknown;
-    if (!tc_cached_map(vcache_layer, (uint64_t)cap_rows, (uint64_t)KV_DIM, AT_KT, &tv)) return cudaErrorUnknown;
+cudaError_t launch_prefill_attn_tc(const CUtensorMap& q_hi, const CUtensorMap& q_lo, const CUtensorMap& k, const CUtensorMap& v, int layer, void* plane, int T,
+                                   uint32_t* status, cudaStream_t st) {
     {
         static bool attr_set[64] = {};
         int dev = 0;
@@ -400,15 +373,10 @@ cudaError_t launch_prefill_attn_tc(const float* qkv, const void* kcache_layer, c
             attr_set[dev] = true;
         }
     }
-    const int n_qt = (T + AT_QT - 1) / AT_QT;
-    // More blocks than SMs: one block per (query tile, kv group), dispatched in the order of their work (a query tile has
-    // 1..n key tiles), so that the SMs that finish early pick up the light tiles: greedy longest-first over all 148 SMs,
-    // where pairing a light with a heavy tile per CTA used 128 of them (measured at 2048 tokens: see the profile).
-    const int heavy_first = n_qt * KV_HEADS > 148 ? 1 : 0, paired = 0;
-    PrefillAttnTcArgs a{qkv, reinterpret_cast<bf16_raw*>(planes), plane_rows, nsplit, T, paired, heavy_first, status};
-    const dim3 grid = heavy_first ? dim3(n_qt * KV_HEADS) : dim3(paired ? (n_qt + 1) / 2 : n_qt, KV_HEADS);
-    prefill_attn_tc_kernel<<<grid, AT_THREADS, AT_SMEM, st>>>(tk, tv, a);
-    return cudaGetLastError();
+    // one block per (query tile, kv group), dispatched in the order of their work (a query tile has 1..n key tiles), so that the
+    // SMs that finish early pick up the light tiles: greedy longest-first over all SMs
+    PrefillAttnTcArgs a{reinterpret_cast<bf16_raw*>(plane), T, layer, status};
+    return launch_chain(prefill_attn_tc_kernel, dim3((T + AT_QT - 1) / AT_QT * KV_HEADS), dim3(AT_THREADS), AT_SMEM, st, q_hi, q_lo, k, v, a);
 }
 
 }  // namespace q3

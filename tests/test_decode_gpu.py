@@ -393,6 +393,28 @@ def test_prefill_matches_oracle(oracle, small, T):
         print(f"prefill T={T}: arg-max {top} against {want} on a near-tie (margin {margin:.3e})")
 
 
+@pytest.mark.parametrize("T", [4, 63, 65, 128, 129, 256, 257, 385, 512, 513, 1025])
+def test_prompt_products_at_the_edges_of_their_tiles(oracle, small, T):
+    """Prompt lengths around the tiles of the prompt's products (128 tokens a block, 256 a pair, every cut of K and the pair kernel) on an
+    engine with more room than the prompt needs, twice: no atomics, so the same bits."""
+    from qwen3mk import Megakernel, prefill
+
+    shp, inp, w = small
+    g = torch.Generator().manual_seed(T)
+    ids = torch.randint(0, 4096, (T,), generator=g).tolist()
+    wdev = to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES})
+    mk = Megakernel("cuda", layers=2, vocab=4096, max_tokens=1100, max_positions=1200)
+    kc, vc, last = prefill.prefill(wdev, ids, "cuda", capacity=T + 3, engine=mk)
+    mk.status()
+    rk, rv, rlast = oracle.prefill(w, ids)
+    for got, want in ((kc, rk), (vc, rv)):
+        assert oracle.max_rel(got[:, :T], want) <= GATE_MAX_REL and oracle.rel_l2(got[:, :T], want) <= GATE_KV_REL_L2
+        assert float(got[:, T:].abs().max()) == 0.0
+    assert oracle.max_rel(last, rlast) <= GATE_MAX_REL
+    again = prefill.prefill(wdev, ids, "cuda", capacity=T + 3, engine=mk)
+    assert torch.equal(again[0], kc) and torch.equal(again[1], vc) and torch.equal(again[2], last)
+
+
 def test_error_paths():
     from qwen3mk import Megakernel, weights
     from qwen3mk.kernel import SeqTable
