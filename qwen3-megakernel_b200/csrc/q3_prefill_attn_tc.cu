@@ -6,18 +6,22 @@
 // the key tiles (128 keys) up to its diagonal:
 //     S  = Q K^T      M 128 x N 128 keys x K 128 dims: Q as TWO bf16 planes (hi + lo, so the scores carry fp32-grade
 //                     accuracy into the exponent), both K-major operands      -> TMEM columns [0, 128) / [128, 256)
-//     P  = exp(S - m) sixteen warps, four threads per row (32 keys each): tcgen05.ld, causal mask on the diagonal tile,
-//                     running max / sum, P rounded to bf16 into shared memory in the K-major swizzled operand layout
-//     PV = P V        M 128 x N 128 dims x K 128 keys; V is the MN-major B operand straight from its TMA tile
-//                                                                             -> TMEM columns [256, 384) / [384, 512)
-//     O  = O c + PV   in registers (32 dims per thread), rescaled by c = exp(m_old - m_new); written at the end as the
-//                     bf16 plane(s) the Wo GEMM reads, so no fp32 round trip and no separate splitting kernel
-// S and PV are double-buffered in TMEM (all 512 columns): the MMA thread issues S of tile t + 1 before it waits for P
-// of tile t, and the softmax warps fold PV of tile t - 1 into O after they have posted P of tile t, so the exponentials
-// (the bottleneck: 16 K of them per tile on the SFUs) run back to back while the tensor pipe works beside them.
-// Long prompts launch one block per (query tile, kv group) in order of work (a query tile has 1..n key tiles), so that
-// the SMs that finish early pick up the light tiles; short ones a (query tile, kv group) grid.  Every mbarrier wait is
-// bounded.
+//     P  = exp(S - m) two groups of eight warps, two threads per row (64 keys each); group g takes the key tiles t with t % 2 == g, so that
+//                     one group's exponentials run while the tensor pipe and the hand-offs of the other's tile do.  P, rounded to
+//                     bf16, takes the place of S in TMEM: the A operand of the second product
+//     O += P V        M 128 x N 128 dims x K 128 keys; V is the MN-major B operand straight from its TMA tile.  Each group has an O of its own
+//                     -> TMEM columns [256, 384) / [384, 512), summed by the tensor pipe over the group's tiles
+// A group keeps its own running maximum and sum.  Its maximum is raised, and its O rescaled, only when a score exceeds it by 2^8: P
+// then reaches at most 2^8, its bf16 rounding stays the same relative error and the fp32 sums have room.  At the end the two groups'
+// O are combined under one maximum and written as the bf16 plane the Wo GEMM reads.
+// The MMA thread issues S of tile t + 2 right behind the product of tile t, whose P it overwrites (the pipe works in order).
+// One block per (query tile, kv group) in order of work (a query tile has 1..n key tiles), so that the SMs that finish early pick up the
+// light tiles.  Every mbarrier wait is bounded.
+//
+// What bounds it: a key tile is 24 products of 128 x 128 x 16 (0.8 us at the measured bf16 rate) and 16 K exponentials and 8 K conversions on
+// the XU pipe (0.8 us).  A tile takes 1.2 us: the products wait
+// for the slowest of a group's warps (0.3 us) and for the exponentials that no other tile covers.  Measured, us a launch at 512 / 777 / 2048 tokens: sixteen
+// warps on every tile with P in shared memory and O in registers 12.6 / 16.8 / 37.6, two groups 11.4 / 14.5 / 32.1.
 //
 // Replaces the [16, T, T] masked score matrix of the reference's prefill (qwen3mk/prefill.py:71-75).
 #include <cuda.h>
@@ -27,17 +31,15 @@
 
 namespace q3 {
 
-constexpr int AT_PARTS = 4;               // threads per row in the softmax: each takes 128 / AT_PARTS columns of S and of O
-constexpr int AT_SOFT = 128 * AT_PARTS;   // softmax / output threads: warps 0..15
+constexpr int AT_SOFT = 512;              // softmax / output threads: warps 0..15, group 0 the first eight
 constexpr int AT_THREADS = AT_SOFT + 64;  // + warp 16 TMA producer, warp 17 MMA issuer and TMEM owner
 constexpr int AT_QT = 64;                 // query positions per CTA pass
 constexpr int AT_KT = 128;                // keys per tile
 constexpr int AT_STAGES = 2;
 constexpr uint32_t AT_BOX = 128 * 128;    // bytes of one [128 rows x 64 columns] bf16 box, 128-byte swizzle
-constexpr uint32_t AT_Q_BYTES = 2 * AT_BOX, AT_P_BYTES = 2 * AT_BOX, AT_KV_BYTES = 2 * AT_BOX;   // 128 x 128 bf16 = two boxes
-// Q hi, Q lo, P, stages x (K, V) = 224 KB; with the 3 KB of static shared memory below that is all an SM has, so the
-// dynamic part must start 1024-aligned by itself (the extern array is declared so) and the static part must stay <= 3 KB
-constexpr size_t AT_SMEM = 2 * AT_Q_BYTES + AT_P_BYTES + AT_STAGES * 2 * AT_KV_BYTES;
+constexpr uint32_t AT_Q_BYTES = 2 * AT_BOX, AT_KV_BYTES = 2 * AT_BOX;   // 128 x 128 bf16 = two boxes
+constexpr size_t AT_SMEM = 2 * AT_Q_BYTES + AT_STAGES * 2 * AT_KV_BYTES;   // Q hi, Q lo, stages x (K, V) = 192 KB
+constexpr float AT_LAG = 8.f;             // how far (in log2) scores may exceed the maximum that P is taken under
 constexpr unsigned long long AT_WAIT_NS = 200ull * 1000 * 1000;
 
 __device__ __forceinline__ uint32_t at_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -91,12 +93,6 @@ __device__ __forceinline__ uint64_t at_desc_mn(uint32_t smem_addr) {
     d |= (uint64_t)2 << 61;
     return d;
 }
-// byte offset of element (row, col) of a [128 x 128] bf16 operand stored as two swizzled boxes of 64 columns
-__device__ __forceinline__ uint32_t at_swz(int row, int col) {
-    const int box = col >> 6, c = col & 63;
-    return (uint32_t)box * AT_BOX + (uint32_t)row * 128u + (uint32_t)((((c >> 3) ^ (row & 7)) << 4) + ((c & 7) << 1));
-}
-
 // The special-function pipe (16 results a cycle and SM) is this kernel's bottleneck: a tile needs 16 K exponentials and
 // the conversion of 16 K probabilities to bf16.  So: one ex2 per element (log2(e) is folded into the scale of Q) and one
 // conversion per PAIR of elements.
@@ -122,6 +118,18 @@ __device__ __forceinline__ void at_ld32(uint32_t (&r)[32], uint32_t taddr) {
                  : "r"(taddr) : "memory");
 }
 
+__device__ __forceinline__ void at_ld16(uint32_t* r, uint32_t taddr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void at_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+                 ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
+}
+
 struct PrefillAttnTcArgs {
     bf16_raw* plane;      // [T][2048] bf16: the output, as the Wo GEMM reads it
     int T, layer;
@@ -132,22 +140,17 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                                                                         const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                                                                         const PrefillAttnTcArgs a) {
     extern __shared__ __align__(1024) unsigned char at_raw[];
-    __shared__ __align__(8) uint64_t k_full[AT_STAGES], v_full[AT_STAGES], k_empty[AT_STAGES], v_empty[AT_STAGES], q_full, s_full[2], p_full, o_full[2];
+    __shared__ __align__(8) uint64_t k_full[AT_STAGES], v_full[AT_STAGES], k_empty[AT_STAGES], v_empty[AT_STAGES], q_full, s_full[2], p_full[2], o_full[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_flag;
-    // Per-row partial maxima of the four column parts, exchanged once per key tile with ONE barrier: two buffers, picked by the
-    // tile's parity, so that a warp that is a tile ahead never overwrites what a slower one has yet to read.  Stored as bf16
-    // rounded UP (the shared maximum only has to be an upper bound that every thread of the row agrees on), which keeps the
-    // two buffers in the 2 KB the kernel has left.  The same bytes hold the fp32 partial sums at the end.
-    __shared__ __align__(16) unsigned short pm16[2][AT_PARTS][128];
-    float (*pm)[128] = reinterpret_cast<float (*)[128]>(&pm16[0][0][0]);
+    __shared__ float s_max[2][2][128];              // per group: the tile's maximum of a row's two halves
+    __shared__ float s_m[2][128], s_l[2][2][128];   // at the end: per group, a row's maximum and the two halves of its sum
 
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int g = (int)blockIdx.x % KV_HEADS;       // kv head; query heads 2g and 2g + 1
     unsigned char* sQh = at_raw;
     unsigned char* sQl = sQh + AT_Q_BYTES;
-    unsigned char* sP = sQl + AT_Q_BYTES;
-    unsigned char* sKV = sP + AT_P_BYTES;           // stage s: K at s * 2 * AT_KV_BYTES, V right after it
+    unsigned char* sKV = sQl + AT_Q_BYTES;          // stage s: K at s * 2 * AT_KV_BYTES, V right after it
 
     if (tid == 0) {
         for (int s = 0; s < AT_STAGES; ++s) {
@@ -159,9 +162,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
         for (int b = 0; b < 2; ++b) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&s_full[b])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&o_full[b])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(at_smem(&p_full[b])) : "memory");   // the group's warps
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&q_full)) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(at_smem(&p_full)), "r"(AT_SOFT) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         abort_flag = 0;
     }
@@ -195,16 +198,16 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                 // K and V of a tile share a stage but are released separately: the K half is free as soon as S of its tile has
                 // been computed, a whole tile before the V half (after PV), so the next K is on its way that much earlier
                 for (int t = 0; t < n_kt; ++t) {
-                    const int it = t, s = it % AT_STAGES;
+                    const int s = t % AT_STAGES;
                     unsigned char* sk = sKV + (size_t)s * 2 * AT_KV_BYTES;
                     unsigned char* sv = sk + AT_KV_BYTES;
-                    if (it >= AT_STAGES && !at_wait(&k_empty[s], ((it / AT_STAGES) - 1) & 1, &abort_flag, a.status, 40)) break;
+                    if (t >= AT_STAGES && !at_wait(&k_empty[s], ((t / AT_STAGES) - 1) & 1, &abort_flag, a.status, 40)) break;
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&k_full[s])), "r"(AT_KV_BYTES) : "memory");
 #pragma unroll
                     for (int b = 0; b < 2; ++b)        // the two 64-dim halves of the head
                         asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                                      ::"r"(at_smem(sk + b * AT_BOX)), "l"(&tm_k), "r"(g * HEAD_DIM + 64 * b), "r"(t * AT_KT), "r"(a.layer), "r"(at_smem(&k_full[s])) : "memory");
-                    if (it >= AT_STAGES && !at_wait(&v_empty[s], ((it / AT_STAGES) - 1) & 1, &abort_flag, a.status, 47)) break;
+                    if (t >= AT_STAGES && !at_wait(&v_empty[s], ((t / AT_STAGES) - 1) & 1, &abort_flag, a.status, 47)) break;
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&v_full[s])), "r"(AT_KV_BYTES) : "memory");
 #pragma unroll
                     for (int b = 0; b < 2; ++b)
@@ -218,137 +221,149 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                 // D fp32, A and B bf16, M 128, N 128; bit 16: B is MN-major (V)
                 const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
                 const uint32_t idesc_o = idesc_s | (1u << 16);
-                auto issue_s = [&](int t) -> bool {    // S = (Q hi + Q lo) K^T of key tile t, into S buffer it & 1
-                    const int it = t, s = it % AT_STAGES;
-                    if (!at_wait(&k_full[s], (it / AT_STAGES) & 1, &abort_flag, a.status, 41)) return false;
+                // (descriptors count 16-byte units; what a step adds to them is a constant)
+                constexpr uint64_t BOX = AT_BOX >> 4, STAGE = 2 * AT_KV_BYTES >> 4;
+                const uint64_t dq = at_desc_k(at_smem(sQh)), dk = at_desc_k(at_smem(sKV)), dv = at_desc_mn(at_smem(sKV + AT_KV_BYTES));
+                static_assert(AT_STAGES == 2, "a tile's stage is its parity");
+                auto issue_s = [&](int t) -> bool {    // S = (Q hi + Q lo) K^T of key tile t, into S buffer t & 1
+                    const int s = t % AT_STAGES;
+                    if (!at_wait(&k_full[s], (t / AT_STAGES) & 1, &abort_flag, a.status, 41)) return false;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t sk = at_smem(sKV + (size_t)s * 2 * AT_KV_BYTES);
+                    const uint64_t dks = dk + (uint64_t)s * STAGE;
 #pragma unroll
                     for (int plane = 0; plane < 2; ++plane) {
-                        const uint32_t sq = at_smem(plane ? sQl : sQh);
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {  // 16 dims a step: four steps per 64-dim box
-                            const uint32_t o = (uint32_t)(k >> 2) * AT_BOX + (uint32_t)(k & 3) * 32u;
-                            const uint64_t da = at_desc_k(sq + o), db = at_desc_k(sk + o);
+                            const uint64_t o = (uint64_t)(k >> 2) * BOX + (uint64_t)(k & 3) * 2;
+                            const uint64_t da = dq + (uint64_t)plane * (AT_Q_BYTES >> 4) + o, db = dks + o;
                             const uint32_t acc = (plane | k) ? 1u : 0u;
                             asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                                          "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                                         ::"r"(tmem_base + (uint32_t)(it & 1) * 128u), "l"(da), "l"(db), "r"(idesc_s), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
+                                         ::"r"(tmem_base + (uint32_t)(t & 1) * 128u), "l"(da), "l"(db), "r"(idesc_s), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
                         }
                     }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(at_smem(&s_full[it & 1])) : "memory");
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(at_smem(&s_full[t & 1])) : "memory");
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(at_smem(&k_empty[s])) : "memory");
                     return true;
                 };
-                bool ok = at_wait(&q_full, 0, &abort_flag, a.status, 48) && issue_s(0);
+                bool ok = at_wait(&q_full, 0, &abort_flag, a.status, 48) && issue_s(0) && (n_kt == 1 || issue_s(1));
                 for (int t = 0; t < n_kt && ok; ++t) {
-                    const int it = t, s = it % AT_STAGES;
-                    // S of the next tile first: its buffer was read before P of tile t - 1 was posted, and the exponentials of
-                    // tile t can be followed by those of tile t + 1 without waiting for the tensor pipe
-                    if (t + 1 < n_kt) ok = issue_s(t + 1);
-                    ok = ok && at_wait(&p_full, it & 1, &abort_flag, a.status, 42) && at_wait(&v_full[s], (it / AT_STAGES) & 1, &abort_flag, a.status, 43);
+                    const int b = t & 1, s = t % AT_STAGES;
+                    ok = at_wait(&p_full[b], (t >> 1) & 1, &abort_flag, a.status, 42) && at_wait(&v_full[s], (t / AT_STAGES) & 1, &abort_flag, a.status, 43);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t sv = at_smem(sKV + (size_t)s * 2 * AT_KV_BYTES + AT_KV_BYTES), sp = at_smem(sP);
+                    const uint64_t dvs = dv + (uint64_t)s * STAGE;
+                    const uint32_t tp = tmem_base + (uint32_t)b * 128u;
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {      // 16 keys a step; PV buffer it & 1 (its previous tenant, tile t - 2, was folded into O before P of tile t was posted)
-                        const uint64_t da = at_desc_k(sp + (uint32_t)(k >> 2) * AT_BOX + (uint32_t)(k & 3) * 32u);
-                        const uint64_t db = at_desc_mn(sv + (uint32_t)k * 2048u);
+                    for (int k = 0; k < 8; ++k) {      // 16 keys a step: eight columns of P (two bf16 each)
+                        const uint64_t db = dvs + (uint64_t)k * (2048 >> 4);
                         asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                                     ::"r"(tmem_base + 256u + (uint32_t)(it & 1) * 128u), "l"(da), "l"(db), "r"(idesc_o), "r"(k ? 1u : 0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
+                                     "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+                                     ::"r"(tp + 256u), "r"(tp + (uint32_t)k * 8u), "l"(db), "r"(idesc_o), "r"((t >= 2 || k) ? 1u : 0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
                     }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(at_smem(&o_full[it & 1])) : "memory");
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(at_smem(&o_full[b])) : "memory");
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(at_smem(&v_empty[s])) : "memory");
+                    if (t + 2 < n_kt) ok = issue_s(t + 2);
                 }
             }
         } else {
-            // ------------------------------------------------------------------ softmax and output: row = TMEM lane, part = 32 columns
-            const int row = (warp & 3) * 32 + lane, part = warp >> 2;
+            // ------------------------------------------------------------------ softmax and output: row = TMEM lane
+            const int quad = warp & 3, row = quad * 32 + lane, grp = warp >> 3, part = (warp >> 2) & 1;   // part: 64 keys of a tile
             const int qpos = q0 + (row & 63);
-            const uint32_t trow = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(part * 32);
-            float o[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) o[j] = 0.f;
-            float m = -INFINITY, lsum = 0.f, c_prev = 1.f;
+            const uint32_t trow = tmem_base + ((uint32_t)(quad * 32) << 16);
+            const uint32_t ts = trow + (uint32_t)(grp * 128), to = trow + 256u + (uint32_t)(grp * 128 + part * 64);
+            float m = -INFINITY, lsum = 0.f;
             bool ok = true;
-            // O = O c + PV of tile `it` (this thread's 32 dims), once its MMAs have completed
-            auto fold = [&](int it, float c) -> bool {
-                if (!at_wait_warp(&o_full[it & 1], (it >> 1) & 1, &abort_flag, a.status, 45)) return false;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                uint32_t v0[32];
-                at_ld32(v0, trow + 256u + (uint32_t)(it & 1) * 128u);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int j = 0; j < 32; ++j) o[j] = fmaf(o[j], c, __uint_as_float(v0[j]));
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                return true;
-            };
-            for (int t = 0; t < n_kt && ok; ++t) {
-                const int it = t;
-                ok = at_wait_warp(&s_full[it & 1], (it >> 1) & 1, &abort_flag, a.status, 44);
+            for (int t = grp, i = 0; t < n_kt; t += 2, ++i) {
+                ok = at_wait_warp(&s_full[grp], i & 1, &abort_flag, a.status, 44);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                uint32_t r0[32];
-                at_ld32(r0, trow + (uint32_t)(it & 1) * 128u);
+                uint32_t r[2][32];
+                at_ld32(r[0], ts + (uint32_t)(part * 64));
+                at_ld32(r[1], ts + (uint32_t)(part * 64 + 32));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                const int key0 = t * AT_KT + part * 32;
                 if (t == n_kt - 1) {   // the diagonal tile: causal mask (it also hides keys past the prompt)
+                    const int key0 = t * AT_KT + part * 64;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (key0 + j > qpos) r0[j] = 0xff800000u;            // -inf
+                    for (int j = 0; j < 32; ++j) {
+                        if (key0 + j > qpos) r[0][j] = 0xff800000u;            // -inf
+                        if (key0 + 32 + j > qpos) r[1][j] = 0xff800000u;
+                    }
                 }
-                float tmax = -INFINITY;
+                float x[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-                for (int j = 0; j < 32; ++j) tmax = fmaxf(tmax, __uint_as_float(r0[j]));
-                {
-                    const uint32_t tb = __float_as_uint(tmax);   // towards +inf: truncation for negative values, carry for positive ones
-                    pm16[it & 1][part][row] = (unsigned short)((tb & 0x80000000u) ? (tb >> 16) : ((tb + 0xffffu) >> 16));
+                for (int j = 0; j < 32; ++j) { x[j & 1] = fmaxf(x[j & 1], __uint_as_float(r[0][j])); x[2 + (j & 1)] = fmaxf(x[2 + (j & 1)], __uint_as_float(r[1][j])); }
+                const float x0 = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
+                // the row's other half is a thread of the warp four further; behind the barrier both have read their part of S, too
+                s_max[grp][part][row] = x0;
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + grp * 4 + quad) : "memory");
+                const float top = fmaxf(x0, s_max[grp][part ^ 1][row]);   // finite: the first key of a tile is visible to every row
+                const bool raise = top > m + AT_LAG;
+                if (__any_sync(0xffffffffu, raise)) {
+                    const float mn = raise ? top : m, c = at_ex2(m - mn);
+                    m = mn;
+                    if (i > 0) {           // O of the tiles so far, once the last of them has been added
+                        ok = at_wait_warp(&o_full[grp], (i - 1) & 1, &abort_flag, a.status, 45);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        lsum *= c;
+#pragma unroll 1
+                        for (int h = 0; h < 64; h += 16) {
+                            uint32_t o[16];
+                            at_ld16(o, to + (uint32_t)h);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * c);
+                            at_st16(to + (uint32_t)h, o);
+                        }
+                    }
                 }
-                asm volatile("bar.sync 1, %0;" ::"n"(AT_SOFT) : "memory");
-                float mn = m;                                   // finite from the first tile on: key 0 is visible to every row
+                float psum0 = 0.f, psum1 = 0.f;
 #pragma unroll
-                for (int q = 0; q < AT_PARTS; ++q) mn = fmaxf(mn, __uint_as_float((uint32_t)pm16[it & 1][q][row] << 16));
-                const float c = at_ex2(m - mn);
-                m = mn;
-                float psum = 0.f;
-                uint32_t pk[16];
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t pk[16];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float e0 = at_ex2(__uint_as_float(r0[2 * j]) - mn), e1 = at_ex2(__uint_as_float(r0[2 * j + 1]) - mn);
-                    psum += e0 + e1;
-                    pk[j] = at_pack_bf16(e0, e1);
+                    for (int j = 0; j < 16; ++j) {
+                        const float e0 = at_ex2(__uint_as_float(r[h][2 * j]) - m), e1 = at_ex2(__uint_as_float(r[h][2 * j + 1]) - m);
+                        psum0 += e0; psum1 += e1;
+                        pk[j] = at_pack_bf16(e0, e1);
+                    }
+                    at_st16(ts + (uint32_t)(part * 32 + h * 16), pk);
                 }
-                lsum = lsum * c + psum;
-                // the P buffer is free once PV of the previous tile has completed (long ago in practice)
-                if (t > 0 && !at_wait_warp(&o_full[(it - 1) & 1], ((it - 1) >> 1) & 1, &abort_flag, a.status, 46)) { ok = false; break; }
-                // P[row][32 part .. 32 part + 31]: four 16-byte chunks of box part / 2, chunk slots 4 (part & 1) + ch
-#pragma unroll
-                for (int ch = 0; ch < 4; ++ch)
-                    *reinterpret_cast<uint4*>(sP + (uint32_t)(part >> 1) * AT_BOX + (uint32_t)row * 128u + (uint32_t)((((part & 1) * 4 + ch) ^ (row & 7)) << 4)) =
-                        make_uint4(pk[4 * ch], pk[4 * ch + 1], pk[4 * ch + 2], pk[4 * ch + 3]);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                lsum += psum0 + psum1;
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(at_smem(&p_full)) : "memory");
-                // fold the PREVIOUS tile's PV into O while the tensor pipe works on this one
-                if (t > 0) ok = fold(it - 1, c_prev);
-                c_prev = c;
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(at_smem(&p_full[grp])) : "memory");
             }
-            if (ok) ok = fold(n_kt - 1, c_prev);
-            // the row sum is split over the parts' key ranges
-            asm volatile("bar.sync 1, %0;" ::"n"(AT_SOFT) : "memory");   // the last tile's maxima have been read
-            pm[part][row] = lsum;
-            asm volatile("bar.sync 1, %0;" ::"n"(AT_SOFT) : "memory");
-            float ltot = 0.f;
+            const int mine = (n_kt - grp + 1) / 2;      // tiles of this group
+            if (ok && mine > 0) ok = at_wait_warp(&o_full[grp], (mine - 1) & 1, &abort_flag, a.status, 46);
+            if (part == 0) s_m[grp][row] = m;
+            s_l[grp][part][row] = lsum;
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            asm volatile("bar.sync 9, %0;" ::"n"(AT_SOFT) : "memory");
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const float m0 = s_m[0][row], m1 = s_m[1][row], mx = fmaxf(m0, m1);      // (a block of one tile has no second group: m1 is -inf)
+            const float f0 = at_ex2(m0 - mx), f1 = at_ex2(m1 - mx);
+            const float inv = 1.f / ((s_l[0][0][row] + s_l[0][1][row]) * f0 + (s_l[1][0][row] + s_l[1][1][row]) * f1);
+            const float w0 = f0 * inv, w1 = f1 * inv;
+            const int dim0 = (warp >> 2) * 32;          // a quarter of the row's dims
+            uint32_t o0[32], o1[32];
+            at_ld32(o0, trow + 256u + (uint32_t)dim0);
+            at_ld32(o1, trow + 384u + (uint32_t)dim0);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (!abort_flag && qpos < a.T) {   // 32 dims = 64 contiguous bytes
+                float o[32];
 #pragma unroll
-            for (int q = 0; q < AT_PARTS; ++q) ltot += pm[q][row];
-            const float inv = 1.f / ltot;
-            if (ok && qpos < a.T) {   // 32 dims = 64 contiguous bytes
-                bf16_raw* dst = a.plane + (size_t)qpos * Q_DIM + (2 * g + (row >> 6)) * HEAD_DIM + part * 32;
+                for (int j = 0; j < 32; ++j) {
+                    o[j] = __uint_as_float(o0[j]) * w0;
+                    if (n_kt > 1) o[j] = fmaf(__uint_as_float(o1[j]), w1, o[j]);   // (TMEM that nothing was added to may hold anything)
+                }
+                bf16_raw* dst = a.plane + (size_t)qpos * Q_DIM + (2 * g + (row >> 6)) * HEAD_DIM + dim0;
 #pragma unroll
                 for (int j = 0; j < 32; j += 8)
-                    *reinterpret_cast<uint4*>(dst + j) = make_uint4(at_pack_bf16(o[j] * inv, o[j + 1] * inv), at_pack_bf16(o[j + 2] * inv, o[j + 3] * inv),
-                                                                    at_pack_bf16(o[j + 4] * inv, o[j + 5] * inv), at_pack_bf16(o[j + 6] * inv, o[j + 7] * inv));
+                    *reinterpret_cast<uint4*>(dst + j) = make_uint4(at_pack_bf16(o[j], o[j + 1]), at_pack_bf16(o[j + 2], o[j + 3]),
+                                                                    at_pack_bf16(o[j + 4], o[j + 5]), at_pack_bf16(o[j + 6], o[j + 7]));
             }
         }
     }
