@@ -7,23 +7,25 @@
 // A CLUSTER of blocks per row: block r of C owns a contiguous slice of the row, warp w of it a contiguous run of the
 // slice, so that sums over (block, warp, group of 32) follow the index order and every load is coalesced.  What the
 // blocks of a row have to agree on travels through distributed shared memory, one cluster barrier each:
-//   1. every block finds its maximum (lowest index on ties);
+//   1. every block finds its maximum.  Where the whole vocabulary takes part, it sums its weights exp((l_i - max) / T) under its own maximum,
+//      in the same pass over memory where a thread's words do not fit its registers (a thread's sum is scaled when its maximum
+//      grows); maxima and sums are exchanged together and the blocks' sums scaled to the row's maximum;
 //   2. top-k: a block whose threads have at least k elements bins its THREADS' maxima linearly between the smallest and
 //      the largest of them; the bins that hold the k largest maxima bound its own k largest elements from below, so the
 //      few elements at or above that bound (about 1.1 k of them) are the block's candidates.  The union of all blocks'
-//      candidates contains the row's k largest; every block selects the k-th largest key among them (binary search over
-//      the bits of the keys, held in registers).  A row whose candidates do not fit (large k, many equal values) goes
+//      candidates contains every word that is kept; every block finds the threshold among them (binary search over the bits of
+//      the keys, held in registers, below the bits they share and until exactly k are above it) and adds up the weights of the kept
+//      ones, in the same order as every other block.  A row whose candidates do not fit (large k, many equal values) goes
 //      through a radix select instead: three passes of 11, 11 and 10 bits over the order-preserving integer image of the
-//      floats, histograms summed over the cluster.  Every logit >= the k-th value is kept, so ties are all kept;
-//   3. weights w_i = exp((l_i - max) / T) of the kept logits, summed per warp, per block and over the row;
-//   4. the token is the first index whose inclusive prefix sum exceeds u * total, u in [0, 1) supplied per row
-//      by the caller (a seeded generator on the host side keeps runs reproducible); the block whose warps' runs
-//      bracket the target walks that run, a thread an element.
+//      floats, histograms summed over the cluster, then the weights' sums.  Every logit >= the k-th value is kept, so ties are all kept;
+//   3. the token is the first index whose inclusive prefix sum exceeds u * total, u in [0, 1) supplied per row
+//      by the caller (a seeded generator on the host side keeps runs reproducible); the block whose words
+//      bracket the target finds it among its candidates, a thread each, or walks the run of the warp that brackets it.
 // T <= 0 or k == 1 degenerate to the arg-max (ties -> lowest index), like the decode kernels.
 //
-// A single row is bound by latency (0.6 MB, but a dozen dependent block-wide steps), a full batch by the row's bytes.  One
-// block of 1024 threads per row, as this kernel was before, left 147 SMs idle at one row and walked the 2048 bins of each
-// radix pass with one thread: 1 row, k = 50: 165 us, now 14; 64 rows, whole vocabulary: 70 us, now 25.
+// A single row is bound by latency (0.6 MB, but a dozen dependent block-wide steps), a full batch by the row's bytes and the same steps.
+// Measured, us, before the sums under a block's own maximum and the draw from the candidates -> now: 1 row, k = 50: 14.7 -> 12.0; 64 rows, k = 50:
+// 32.8 -> 24.6; 64 rows, whole vocabulary: 24.7 -> 20.5 (the second pass over the row is gone).
 #include <cooperative_groups.h>
 
 #include <cfloat>
@@ -63,7 +65,9 @@ struct SampleShared {
     unsigned wcount[2][SAMPLE_WARPS];
     unsigned hist[SAMPLE_BINS];
     unsigned cand[SAMPLE_CAND];             // keys
-    unsigned sel, need, cand_n;
+    int candi[SAMPLE_CAND];                 // and where they are
+    unsigned sel, need, cand_n, cmin;
+    float bracket[2];                       // the block's share of the weights' running sum
 };
 
 // Block-wide: the bin, counted from the largest, in which the running count of hist[] reaches `need`, and what is still
@@ -107,8 +111,11 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     // warp w of block r: elements [i0, i1), `per` of them but for the last runs of the row
     const int per = sample_run(vocab, C);
     const int i0 = (int)min((long long)vocab, (long long)(rank * SAMPLE_WARPS + warp) * per), i1 = min(vocab, i0 + per);
-    const bool greedy = !(temperature > 0.f) || top_k == 1;
-    const bool select = !greedy && top_k > 1 && top_k < vocab;
+    // 0: the arg-max, 1: the k largest words take part, 2: all do.  (Opaque to the compiler: nvcc 12.9 mixes up the flags of this kernel when
+    // it can see what they are made of.)
+    int mode = !(temperature > 0.f) || top_k == 1 ? 0 : top_k > 1 && top_k < vocab ? 1 : 2;
+    asm volatile("" : "+r"(mode));
+    const bool greedy = mode == 0, select = mode == 1;
     const bool vec = ((vocab & 3) | (int)(reinterpret_cast<uintptr_t>(logits) & 15)) == 0;
     cluster.barrier_arrive();   // (a peer's shared memory may be written once the peer runs: waited for before the first exchange)
 
@@ -149,15 +156,40 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
 
     // ---- 1. the block's maximum, and the smallest of its threads' maxima ----
     const bool any = i0 + 4 * lane < i1;
-    float mine = -INFINITY;
-    each([&](int, float v) { mine = fmaxf(mine, v); });
+    const float inv_t = 1.f / temperature;
+    const bool whole_row = mode == 2;
+    float mine = -INFINITY, wsum = 0.f;
+    bool nan = false;
+    // (a logit that is no number makes a sum one, too: below; a word masked with -inf weighs nothing at any temperature, and so does what
+    // lies past the end of a run: with 1 / T = 0 the exponential of the product would be NaN, not 0)
+    auto weight = [&](float v, float top) { return v < -FLT_MAX ? 0.f : __expf((v - top) * inv_t); };
+    if (NQ == 0 && whole_row) {
+        // maximum and sum of weights in one pass over memory: the sum is taken under the running maximum and scaled when that grows
+        auto raise = [&](float top) {
+            if (top > mine) { if (mine > -INFINITY) wsum *= __expf((mine - top) * inv_t); mine = top; }
+        };
+        auto top4 = [&](const float4& v) { return fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); };
+        auto add4 = [&](const float4& v) { wsum += (weight(v.x, mine) + weight(v.y, mine)) + (weight(v.z, mine) + weight(v.w, mine)); };
+        int j = 0;
+        for (; j + 4 <= whole; j += 4) {
+            float4 v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = *reinterpret_cast<const float4*>(row + i0 + 128 * (j + q) + 4 * lane);
+            raise(fmaxf(fmaxf(top4(v[0]), top4(v[1])), fmaxf(top4(v[2]), top4(v[3]))));
+#pragma unroll
+            for (int q = 0; q < 4; ++q) add4(v[q]);
+        }
+        for (; j < groups; ++j) { const float4 v = fetch(j); raise(top4(v)); add4(v); }
+    } else {
+        each([&](int, float v) { mine = fmaxf(mine, v); nan = nan || v != v; });
+    }
     {
         const float bv = warp_max(mine), lo = -warp_max(any ? -mine : -INFINITY);
         if (lane == 0) { sh.wf[warp] = bv; sh.wg[warp] = lo; }
     }
     if (select)
         for (int b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) sh.hist[b] = 0u;
-    if (tid == 0) { sh.cand_n = 0u; sh.need = 0x7fffffffu; }
+    if (tid == 0) { sh.cand_n = 0u; sh.need = 0x7fffffffu; sh.cmin = 0xffffffffu; }
     const int n_thr = __syncthreads_count(any);     // threads that have an element
     const float bmax = warp_max(sh.wf[lane]), blo = -warp_max(-sh.wg[lane]);
 
@@ -177,24 +209,46 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
             if (any && bin(mine) <= last)           // (a thread whose maximum is below the bound has no candidate)
                 each([&](int i, float v) {
                     if (bin(v) <= last && i < i1) {
-                        const unsigned n = atomicAdd(&sh.cand_n, 1u);
-                        if (n < SAMPLE_CAND) sh.cand[n] = ordered_key(v);
+                        const unsigned n = atomicAdd(&sh.cand_n, 1u), key = ordered_key(v);
+                        if (n < SAMPLE_CAND) { sh.cand[n] = key; sh.candi[n] = i; }
+                        atomicMin(&sh.cmin, key);
                     }
                 });
         } else {
             // fewer threads with elements than k: every element is a candidate, if they fit
             const int s0 = rank * SAMPLE_WARPS * per, slice = min(vocab, s0 + SAMPLE_WARPS * per) - min(vocab, s0);
             if (slice <= SAMPLE_CAND)
-                each([&](int i, float v) { if (i < i1) sh.cand[i - s0] = ordered_key(v); });
-            if (tid == 0) sh.cand_n = (unsigned)slice;
+                each([&](int i, float v) { if (i < i1) { sh.cand[i - s0] = ordered_key(v); sh.candi[i - s0] = i; } });
+            if (tid == 0) { sh.cand_n = (unsigned)slice; sh.cmin = 0u; }
         }
         __syncthreads();
         n_cand = sh.cand_n <= SAMPLE_CAND ? (int)sh.cand_n : -1;
     }
+    // ---- the block's sum of weights: over all its words under its own maximum, or (select) whether it has a NaN ----
+    float lo = 0.f, hi = 0.f, bsum = 0.f;           // this warp's bracket inside the block, and the block's sum
+    auto warp_sums = [&](float ws) {
+        ws = warp_sum(ws);
+        __syncthreads();
+        if (lane == 0) sh.wf[warp] = ws;
+        __syncthreads();
+        bsum = 0.f;
+        for (int w = 0; w < SAMPLE_WARPS; ++w) {    // (the same order everywhere: brackets meet without gaps)
+            if (w == warp) lo = bsum;
+            bsum += sh.wf[w];
+            if (w == warp) hi = bsum;
+        }
+    };
+    if (whole_row) {
+        if constexpr (NQ > 0) each([&](int, float v) { wsum += weight(v, bmax); });
+        else if (mine > -INFINITY) wsum *= __expf((mine - bmax) * inv_t);
+        warp_sums(wsum);
+    } else if (select) {
+        bsum = __syncthreads_or(nan) ? NAN : 0.f;
+    }
     cluster.barrier_wait();
     if (tid < C) {
         SampleShared* peer = cluster.map_shared_rank(&sh, tid);
-        peer->bmax[rank] = bmax; peer->ncand[rank] = n_cand;
+        peer->bmax[rank] = bmax; peer->ncand[rank] = n_cand; peer->bsum[rank] = bsum;
     }
     cluster.sync();
     float vmax = sh.bmax[0];
@@ -220,14 +274,18 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     };
     if (greedy) { write_argmax(); return; }
 
-    // ---- 2b. threshold: the k-th largest key (-inf keeps everything) ----
-    float kth = -INFINITY;
-    // (`select` spelled out: with `if (select)` nvcc 12.9 compiles this kernel so that every top-k test fails, kth staying -inf)
-    if (top_k > 1 && top_k < vocab) {
+    const float u = uniform[row_id];
+    float least = -FLT_MAX, base = 0.f, next = 0.f, total = 0.f, scale = 1.f;      // the block's bracket and the total; what its own sums are scaled by
+    if (select) {
+        // ---- 2b. threshold: the k-th largest key ----
         bool fits = true;
-        int total = 0;
-        for (int r = 0; r < C; ++r) { fits = fits && sh.ncand[r] >= 0; total += max(sh.ncand[r], 0); }
-        fits = fits && total <= SAMPLE_KEYS * SAMPLE_THREADS;
+        int count = 0, mine0 = 0;                   // candidates of all blocks, and of those before this one
+        float odd = 0.f;
+        for (int r = 0; r < C; ++r) {
+            if (r == rank) mine0 = count;
+            fits = fits && sh.ncand[r] >= 0; count += max(sh.ncand[r], 0); odd += sh.bsum[r];
+        }
+        fits = fits && count <= SAMPLE_KEYS * SAMPLE_THREADS;
         if (fits) {
             // this thread's share of the union: the blocks' lists one after the other (0 is below every key of a number)
             unsigned key[SAMPLE_KEYS];
@@ -235,14 +293,20 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
             for (int q = 0; q < SAMPLE_KEYS; ++q) {
                 int e = q * SAMPLE_THREADS + tid, r = 0;
                 key[q] = 0u;
-                if (e < total) {
+                if (e < count) {
                     while (e >= sh.ncand[r]) e -= sh.ncand[r++];
                     key[q] = cluster.map_shared_rank(&sh, r)->cand[e];
                 }
             }
-            const bool one = total <= SAMPLE_THREADS;
-            unsigned t = 0u;
-            for (int bit = 31; bit >= 0; --bit) {   // the largest t with at least k keys >= t
+            // Every block has read every list when it may leave; this one's own lists stay until then.
+            cluster.barrier_arrive();
+            const bool one = count <= SAMPLE_THREADS;
+            // The largest t with at least k keys >= t, or any t with exactly k of them.  This block's candidates are at least k, so the k-th
+            // largest key lies between the smallest of them and the maximum: only the bits below their common ones are searched.
+            const unsigned diff = ordered_key(vmax) ^ sh.cmin;
+            int bit = diff ? 31 - __clz(diff) : -1;
+            unsigned t = bit < 0 ? sh.cmin : bit == 31 ? 0u : sh.cmin & ~((2u << bit) - 1u);
+            for (; bit >= 0; --bit) {
                 const unsigned trial = t | (1u << bit);
                 unsigned n;
                 if (one) n = (unsigned)__syncthreads_count(key[0] >= trial);
@@ -256,8 +320,67 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
                     n = __reduce_add_sync(0xffffffffu, sh.wcount[bit & 1][lane]);
                 }
                 if (n >= (unsigned)top_k) t = trial;
+                if (n == (unsigned)top_k) break;
             }
-            kth = key_value(t);
+            // ---- 3. and 4. from the candidates alone: all kept words are among them, and every block adds the same weights in the same order, so
+            // the blocks' brackets meet without another exchange ----
+            auto key_weight = [&](unsigned k) { return k >= t ? weight(key_value(k), vmax) : 0.f; };
+            float run = 0.f;
+#pragma unroll
+            for (int q = 0; q < SAMPLE_KEYS; ++q) {
+                if (q * SAMPLE_THREADS < count) {
+                    const int e = q * SAMPLE_THREADS + tid;
+                    const float w = e < count ? key_weight(key[q]) : 0.f;
+                    float incl = w;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const float p = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += p;
+                    }
+                    __syncthreads();
+                    if (lane == 31) sh.wf[warp] = incl;
+                    float before = __shfl_up_sync(0xffffffffu, incl, 1);
+                    __syncthreads();
+                    float all = sh.wf[lane];
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const float p = __shfl_up_sync(0xffffffffu, all, o);
+                        if (lane >= o) all += p;
+                    }
+                    const float warps = warp ? __shfl_sync(0xffffffffu, all, warp - 1) : 0.f;
+                    before = run + (warps + (lane ? before : 0.f));
+                    if (e == mine0) sh.bracket[0] = before;
+                    if (e == mine0 + n_cand) sh.bracket[1] = before;
+                    run += __shfl_sync(0xffffffffu, all, 31);
+                }
+            }
+            if (tid == 0) { sh.need = 0xffffffffu; sh.cand_n = 0u; }
+            __syncthreads();
+            base = sh.bracket[0]; next = mine0 + n_cand == count ? run : sh.bracket[1]; total = run + odd;
+            // Weights that are not numbers (infinite logits, or a NaN in the row), or a u outside [0, 1): no draw, the arg-max.
+            if (!(total > 0.f && total < INFINITY && u >= 0.f && u < 1.f)) { cluster.barrier_wait(); write_argmax(); return; }
+            float target = u * total;
+            if (!(target < total)) target = __uint_as_float(__float_as_uint(total) - 1u);   // u * total rounded up to the total: the last word with a weight
+            if (n_cand > 0 && base <= target && target < next) {
+                // the first of this block's kept words, in the order of their indices, whose inclusive prefix sum exceeds the target
+                float* const w = reinterpret_cast<float*>(sh.hist);
+                const float own = tid < n_cand ? key_weight(sh.cand[tid]) : 0.f;
+                const int at = tid < n_cand ? sh.candi[tid] : 0;
+                if (tid < n_cand) w[tid] = own;
+                __syncthreads();
+                if (own > 0.f) {
+                    float p = 0.f;
+                    for (int j = 0; j < n_cand; ++j)
+                        if (sh.candi[j] <= at) p += w[j];
+                    if (base + p > target) atomicMin(&sh.need, (unsigned)at);
+                    atomicMax(&sh.cand_n, (unsigned)at);
+                }
+                __syncthreads();
+                // rounding may leave the target a hair beyond the block's own sum: then its last word with a weight
+                if (tid == 0) out[row_id] = sh.need != 0xffffffffu ? (long long)sh.need : (long long)sh.cand_n;
+            }
+            cluster.barrier_wait();
+            return;
         } else {
             unsigned prefix = 0u, need = (unsigned)top_k;
             for (int pass = 0; pass < 3; ++pass) {
@@ -280,45 +403,40 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
                 need = sh.need;
                 cluster.sync();                     // every block has read this pass's histograms
             }
-            kth = key_value(prefix);
+            least = fmaxf(key_value(prefix), -FLT_MAX);
         }
-    }
-
-    // ---- 3. weights of the kept logits: sums per warp, per block, over the row, in index order ----
-    // (a logit that is no number makes the total one, too: below; a word masked with -inf weighs nothing at any temperature, and so does what lies past the end of a run: with 1 / T = 0 the
-    // exponential of the product would be NaN, not 0)
-    const float inv_t = 1.f / temperature;
-    const float least = fmaxf(kth, -FLT_MAX);
-    float ws = 0.f;
-    each([&](int, float v) { if (!(v < least)) ws += __expf((v - vmax) * inv_t); });
-    ws = warp_sum(ws);
-    __syncthreads();
-    if (lane == 0) sh.wf[warp] = ws;
-    __syncthreads();
-    float lo = 0.f, hi = 0.f, bsum = 0.f;           // this warp's bracket inside the block, and the block's sum
-    for (int w = 0; w < SAMPLE_WARPS; ++w) {        // (the same order everywhere: brackets meet without gaps)
-        if (w == warp) lo = bsum;
-        bsum += sh.wf[w];
-        if (w == warp) hi = bsum;
-    }
-    if (tid < C) cluster.map_shared_rank(&sh, tid)->bsum[rank] = bsum;
-    cluster.sync();
-    float base = 0.f, next = 0.f, total = 0.f;      // the block's bracket and the total
-    for (int r = 0; r < C; ++r) {
-        if (r == rank) base = total;
-        total += sh.bsum[r];
-        if (r == rank) next = total;
+        // ---- 3. weights of the kept logits: sums per warp, per block, over the row, in index order ----
+        float ws = 0.f;
+        each([&](int, float v) { if (!(v < least)) ws += __expf((v - vmax) * inv_t); });
+        warp_sums(ws);
+        if (tid < C) cluster.map_shared_rank(&sh, tid)->bsum[rank] = bsum;
+        cluster.sync();
+        for (int r = 0; r < C; ++r) {
+            if (r == rank) base = total;
+            total += sh.bsum[r];
+            if (r == rank) next = total;
+        }
+    } else {
+        // ---- 3. every block's sum was taken under its own maximum ----
+        const float own = lane < C ? sh.bsum[lane] : 0.f, f = own == 0.f ? 0.f : __expf((sh.bmax[lane < C ? lane : 0] - vmax) * inv_t);
+        const float part = __fmul_rn(f, own);       // a lane per block
+        scale = __shfl_sync(0xffffffffu, f, rank);
+        for (int r = 0; r < C; ++r) {
+            if (r == rank) base = total;
+            total = __fadd_rn(total, __shfl_sync(0xffffffffu, part, r));
+            if (r == rank) next = total;
+        }
     }
     // ---- 4. the first index whose inclusive prefix exceeds u * total ----
     // Weights that are not numbers (infinite logits, or a NaN among them), or a u outside [0, 1): no draw, the arg-max.
-    const float u = uniform[row_id];
     if (!(total > 0.f && total < INFINITY && u >= 0.f && u < 1.f)) { write_argmax(); return; }
     float target = u * total;
     if (!(target < total)) target = __uint_as_float(__float_as_uint(total) - 1u);   // u * total rounded up to the total: the last word with a weight
     if (!(base <= target && target < next)) return;
-    // Inside the block: base + lo of the first warp is base, base + hi of the last one is next, and both are the same sums for
+    // Inside the block: `from` of the first warp is base, `to` of the last one is next (the same roundings), and both are the same sums for
     // the neighbouring warps, so exactly one warp's run takes it.  The whole block walks that run, 1024 elements a round.
-    if (lane == 0 && base + lo <= target && target < base + hi) { sh.sel = (unsigned)warp; sh.wg[0] = base + lo; }
+    const float from = __fadd_rn(base, __fmul_rn(scale, lo)), to = __fadd_rn(base, __fmul_rn(scale, hi));
+    if (lane == 0 && from <= target && target < to) { sh.sel = (unsigned)warp; sh.wg[0] = from; }
     if (tid == 0) { sh.need = 0xffffffffu; sh.cand_n = 0u; }
     __syncthreads();
     const int r0 = (rank * SAMPLE_WARPS + (int)sh.sel) * per, r1 = min(vocab, r0 + per);
@@ -377,11 +495,11 @@ extern "C" int q3_sample(const float* logits, int32_t batch, int32_t vocab, floa
     if (batch < 1 || vocab < 1 || top_k < 0) return q3::engine_fail(nullptr, Q3_ERR_INVALID, "q3_sample: batch=%d vocab=%d top_k=%d out of range", batch, vocab, top_k);
     if (temperature > 0.f && top_k != 1 && !uniform) return q3::engine_fail(nullptr, Q3_ERR_INVALID, "q3_sample: sampling needs one uniform number per row");
     // Blocks per row: as many as keep all rows' clusters resident at once, and at least 1024 words a block.  Measured with the
-    // full vocabulary and a cold L2, us with clusters of 1 / 2 / 4 / 8 / 16 blocks: 1 row, k = 50: 42.9 / 32.8 / 24.8 / 18.5 /
-    // 18.5; 8 rows, k = 50: 45 / 33 / 26.5 / 20.4 / 30.7; 16 rows, k = 50: 47 / 35 / 26.6 / 32.7 / 43; 33 rows, all words:
-    // 37 / 27 / 22.5 / 28.7 / 41; 64 rows, all words: 39 / 30.7 / 30.8 / 43 / 72; 64 rows, k = 50: 49 / 38.7 / 41 / 70 / 125.
+    // full vocabulary, us with clusters of 1 / 2 / 4 / 8 / 16 blocks: 1 row, k = 50: 24.4 / 18.5 / 15.8 / 12.3 / 12.1; 8 rows, k = 50:
+    // 24.7 / 19.1 / 16.4 / 12.3 / 20.2; 16 rows, k = 50: 25.3 / 19.5 / 16.4 / 20.5 / 29.1; 33 rows, all words: 25.1 / 18.5 / 14.4 / 20.5 / 32.8;
+    // 40 rows, all words: 26.7 / 19.2 / 20.7 / 22.6; 64 rows, all words: 27.5 / 20.5 / 21.6 / 35.0; 64 rows, k = 50: 30.7 / 24.6 / 26.6 / 48.1.
     // A thread keeps its elements in registers where it has at most three groups of four, or five.
-    int cluster = batch <= 4 ? 16 : batch <= 14 ? 8 : batch <= 48 ? 4 : batch <= 148 ? 2 : 1;
+    int cluster = batch <= 4 ? 16 : batch <= 14 ? 8 : batch <= 36 ? 4 : batch <= 148 ? 2 : 1;
     while (cluster > 1 && vocab < cluster * q3::SAMPLE_THREADS) cluster /= 2;
     const int groups = q3::sample_run(vocab, cluster) / 128;
     cudaStream_t st = (cudaStream_t)stream;

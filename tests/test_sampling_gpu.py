@@ -212,3 +212,31 @@ def test_numbers_that_are_no_draw_give_the_argmax(vocab, top_k):
     logits[5, int(want[5]) - 1] = float("nan")
     out = torch.full((6,), -1, dtype=torch.int64, device="cuda")
     assert sampling.sample(logits.cuda(), 0.9, top_k, u=u.cuda(), out=out).tolist() == want.tolist()
+
+
+@pytest.mark.parametrize("batch,vocab,top_k", [(1, 151936, 50), (5, 151936, 200), (16, 50001, 20), (36, 151936, 50), (37, 151936, 50), (37, 151936, 0),
+                                               (64, 151936, 0), (64, 1001, 0), (149, 50001, 0), (149, 50001, 7), (2, 1030, 1029)])
+@pytest.mark.parametrize("temperature", [0.5, 1e-3, 1e30])
+def test_draws_over_every_number_of_blocks_a_row(batch, vocab, top_k, temperature):
+    """Rows whose largest words, masked words and ties lie in different blocks of a cluster: the chosen word is kept and its interval of the exact
+    distribution holds u."""
+    from qwen3mk import sampling
+
+    g = torch.Generator().manual_seed(batch + vocab + top_k)
+    logits = torch.randn(batch, vocab, generator=g) * 4.0
+    logits[:, : vocab // 3] = float("-inf")              # whole blocks without a weight
+    logits[::2, vocab // 2] = logits[::2, -1]            # equal words far apart
+    u = torch.rand(batch, generator=g)
+    u[0] = 0.0
+    got = sampling.sample(logits.cuda(), temperature, top_k, u=u.cuda()).cpu()
+    rows = logits.double()
+    keep = rows > float("-inf")
+    if 0 < top_k < vocab:
+        keep &= rows >= rows.topk(top_k, dim=-1).values[:, -1:]
+    w = torch.where(keep, torch.exp((rows - rows.max(dim=-1, keepdim=True).values) / temperature), torch.zeros_like(rows))
+    cdf = (w / w.sum(dim=-1, keepdim=True)).cumsum(dim=-1)
+    for b in range(batch):
+        j = int(got[b])
+        assert bool(keep[b, j]) and float(w[b, j]) > 0.0, (b, j)
+        lo = float(cdf[b, j - 1]) if j else 0.0
+        assert lo - CDF_TOL <= float(u[b]) <= float(cdf[b, j]) + CDF_TOL, (b, j, float(u[b]), lo, float(cdf[b, j]))
