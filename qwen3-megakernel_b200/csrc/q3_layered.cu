@@ -537,7 +537,7 @@ cudaError_t launch_head_prep(const HeadPrepArgs& a, int batch, cudaStream_t st) 
 static cudaError_t launch_split(const AttnArgs& a, int batch, cudaStream_t st) { return launch_attn_mma(a, batch, st); }
 
 cudaError_t launch_attn_split(const AttnArgs& a, int batch, cudaStream_t st) {
-    if (a.chunk_pad < 32 || a.chunk_pad % 32 || a.chunk_pad > ATTN_CHUNK_MAX || !a.fused_prep) return cudaErrorInvalidValue;
+    if (a.chunk_pad < 32 || a.chunk_pad % 32 || a.chunk_pad > ATTN_CHUNK_MAX) return cudaErrorInvalidValue;
     return launch_split(a, batch, st);
 }
 

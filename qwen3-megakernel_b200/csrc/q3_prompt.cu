@@ -784,8 +784,9 @@ cudaError_t launch_prompt_gemm(const PromptGemmCall& c, cudaStream_t st) {
     //   q/k/v    128 tokens 14.2 / 11.8 / 11.7 / 10.6;  512: 14.5 / 13.1 / 11.7 / 20.5;  1024: 14.2 / 13.6;  1280: 19.7 / 22.5
     //   Wo       128 tokens 14.1 / 13.2 / 9.0 / 8.1 / 7.0;  512: 14.5 / 13.2 / 9.6 / 8.8 / 14.0;  777: 14.6 / 13.2 / 10.0 / 14.9;  2048: 14.8 / 14.4
     //   down     128 tokens 17.9 / 17.6 / 11.2 / 9.5 / 7.5;  512: 18.4 / 17.2 / 11.6 / 10.1 / 15.6;  777: 18.6 / 17.0 / 12.4 / 17.4;  2048: 18.7 / 19.5
-    //   gate/up  128 tokens 11.0 / 9.7 / 8.9;  512: 11.4 / 9.8 / 16.1;  640: 11.2 / 17.1;  2048: 22.1 / 36.5
-    const int blocks = (c.kind == PR_QKV ? 32 : c.kind == PR_RESID ? 16 : 64) * mt, most = c.kind == PR_QKV ? 4 : c.kind == PR_RESID ? 8 : 2;
+    //   gate/up  64 tokens 10.6 / 8.6 / 7.3 / 6.6;  128: 11.0 / 9.7 / 8.6 / 9.2;  512: 11.4 / 9.8 / 16.1;  640: 11.2 / 17.1;  2048: 22.1 / 36.5
+    // (four slices of gate/up exchange three quarters of a tile: up to 64 tokens that is less than the two waits for its ring that it saves)
+    const int blocks = (c.kind == PR_QKV ? 32 : c.kind == PR_RESID ? 16 : 64) * mt, most = c.kind == PR_QKV ? 4 : c.kind == PR_RESID ? 8 : c.T <= 64 ? 4 : 2;
     const bool pair = blocks > 2 * sm;
     int cut = 1;
     while (cut < most && 2 * cut * blocks <= 2 * sm) cut *= 2;
@@ -811,6 +812,7 @@ cudaError_t launch_prompt_gemm(const PromptGemmCall& c, cudaStream_t st) {
             return launch_split<PR_RESID, 1>(tw, *c.in, p, st);
         case PR_SILU:
             if (pair) return launch_pair<PR_SILU, 256>(tw, *c.in, p, sm, st);
+            if (cut == 4) return launch_split<PR_SILU, 4>(tw, *c.in, p, st);
             if (cut == 2) return launch_split<PR_SILU, 2>(tw, *c.in, p, st);
             return launch_split<PR_SILU, 1>(tw, *c.in, p, st);
     }
