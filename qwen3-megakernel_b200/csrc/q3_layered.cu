@@ -490,22 +490,28 @@ cudaError_t launch_argmax_rows(const float* logits, int vocab, long long* next_t
 // ------------------------------------------------------------------------------------------------
 // host-side launchers
 // ------------------------------------------------------------------------------------------------
-template <int K, int EPI>
-static cudaError_t launch_gemv_k(const GemvArgs& a, int grid_x, cudaStream_t st) {
-    if (a.batch == 1) {
-        gemv_kernel<K, EPI, 1><<<dim3(grid_x, 1), 256, K * sizeof(float), st>>>(a);
-    } else {
-        constexpr int BT = 4;
-        const size_t smem = (size_t)BT * K * sizeof(float);
+template <int K, int EPI, int BT>
+static cudaError_t launch_gemv_bt(const GemvArgs& a, int grid_x, cudaStream_t st) {
+    constexpr size_t smem = (size_t)BT * K * sizeof(float);
+    if constexpr (smem > 48 * 1024) {
         static bool attr_done = false;  // > 48 KB needs the opt-in once per function
         if (!attr_done) {
             cudaError_t e = cudaFuncSetAttribute(gemv_kernel<K, EPI, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
             attr_done = true;
         }
-        gemv_kernel<K, EPI, BT><<<dim3(grid_x, (a.batch + BT - 1) / BT), 256, smem, st>>>(a);
     }
+    gemv_kernel<K, EPI, BT><<<dim3(grid_x, (a.batch + BT - 1) / BT), 256, smem, st>>>(a);
     return cudaGetLastError();
+}
+template <int K, int EPI>
+static cudaError_t launch_gemv_k(const GemvArgs& a, int grid_x, cudaStream_t st) {
+    // A tile of exactly the batch: beyond one sequence the kernel is bound by the activations it reads from shared memory, a padding
+    // sequence's as well (LM head of 2 / 3 sequences with tiles of four 80 us, of two and three 64 / 60)
+    if (a.batch == 1) return launch_gemv_bt<K, EPI, 1>(a, grid_x, st);
+    if (a.batch == 2) return launch_gemv_bt<K, EPI, 2>(a, grid_x, st);
+    if (a.batch == 3) return launch_gemv_bt<K, EPI, 3>(a, grid_x, st);
+    return launch_gemv_bt<K, EPI, 4>(a, grid_x, st);
 }
 
 cudaError_t launch_gemv(int K, int epi, const GemvArgs& a, int grid_x, cudaStream_t st) {
