@@ -376,8 +376,7 @@ int q3::decode_layered(q3_engine* e, const q3_decode_args* a, cudaStream_t st, b
         // 64 additions into one accumulator, each truncated, leave logits 9.8e-7 from fp64, fp32 FMAs 1.2e-7 (19 us a step more for three).
         if (V % 128 == 0 && B >= Q3_TC_MIN_BATCH) {
             float* logits = a->logits ? a->logits : e->logits_tc;
-            GemmTcCall h{bf(w.embed), xp, logits, nullptr, V, 0, V, B, HIDDEN, 3, rows, e->status, e->ssq, ssq_ld};
-            LAUNCH(launch_gemm_tc(h, st));
+            LAUNCH(launch_lm_head(LmHeadCall{bf(w.embed), xp, rows, B, V, e->ssq, ssq_ld, logits, e->status}, st));
             LAUNCH(launch_argmax_rows(logits, V, reinterpret_cast<long long*>(a->next_token), a->seq_len, append, B, st, arg_keys, arg_tickets));
             return Q3_OK;
         }

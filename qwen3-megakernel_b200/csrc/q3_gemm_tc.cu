@@ -16,7 +16,6 @@
 #include <cuda.h>
 
 #include <mutex>
-#include <type_traits>
 #include <vector>
 
 #include "q3_engine.h"
@@ -31,23 +30,15 @@ static std::mutex& host_lock() { static std::mutex m; return m; }   // guards th
 constexpr int TC_THREADS = 192;    // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2..5: epilogue
 constexpr int TC_BM = 128;         // weight rows per tile (UMMA M)
 
-// SCALE: every token's column is multiplied by its RMS norm's scale, rsqrt(sum of the 32 parts ssq[i * ssq_ld + t] / 1024 + eps)
-struct GemmTcScaledParams : GemmTcParams {
-    const float* ssq;
-    int ssq_ld;
-};
-template <bool SCALE> using TcParams = std::conditional_t<SCALE, GemmTcScaledParams, GemmTcParams>;
-
-template <int BN, bool SCALE>
+template <int BN>
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w0,
                                                                 const __grid_constant__ CUtensorMap tm_w1,
                                                                 const __grid_constant__ CUtensorMap tm_w2,
-                                                                const __grid_constant__ CUtensorMap tm_x, const TcParams<SCALE> p) {
+                                                                const __grid_constant__ CUtensorMap tm_x, const GemmTcParams p) {
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[8], empty_bar[8], acc_bar;
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_flag;
-    __shared__ float s_scale[SCALE ? BN : 1];
 
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     // which weight matrix this tile belongs to (grouped launches), and its first row inside that matrix
@@ -160,15 +151,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     } else {
         // ------------------------------------------------------------------ epilogue: TMEM -> registers -> global
         const int quad = warp & 3;                      // TMEM lanes [32 quad, 32 quad + 32) belong to this warp
-        if constexpr (SCALE) {                          // the planes lack their norm's scale: one per token, while the MMAs run
-            pdl_wait();
-#pragma unroll 4
-            for (int j = warp - 2; j < BN; j += 4) {
-                const float ss = warp_sum(n0 + j < p.n_tok ? p.ssq[(size_t)lane * p.ssq_ld + n0 + j] : 0.f);
-                if (lane == 0) s_scale[j] = rsqrtf(ss / (float)HIDDEN + EPS);
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-        }
         const bool ok = tc_wait_warp(&acc_bar, 0, &abort_flag, p.status, 32);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         pdl_wait();   // before the first store (the output may be something the predecessor still reads)
@@ -215,7 +197,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
                         const int t = n0 + c * 32 + j;
                         if (t < p.n_tok) {
                             float v = __uint_as_float(r[j]);
-                            if constexpr (SCALE) v *= s_scale[c * 32 + j];
                             float* dst = out + (size_t)t * ldo + row;
                             if (p.epi == TC_EPI_ATOMIC) {
                                 atomicAdd(dst, v);   // split-K: `out` already holds zero or the residual
@@ -426,6 +407,161 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
 }
 
 // ------------------------------------------------------------------------------------------------
+// The LM head of a decode batch of 4..64 sequences: logits[t, n] = (planes[t] . W[n]) * rsqrt(sum of the 32 parts ssq[i * ssq_ld + t] /
+// 1024 + eps).  PERSISTENT: a block per SM walks tiles of 128 words; a TMA ring of five to seven stages (the weight tile's 64 columns and
+// the three planes' of all sequences, one B operand) never drains between tiles, and two accumulators let the epilogue of a tile
+// run while the products of the next do.
+//
+// Bound by the weights' bytes: 311 MB, 48 us at the copy bandwidth.  The one-tile-per-block kernel this replaced had two stages a
+// block, so a tile was two waits for memory, its products and its epilogue in series.  A one-layer step (LM head, arg-max and about 25 us
+// of a layer) of 8 / 27 / 64 sequences, us: 88.9 / 98.8 / 139.9 before, 81.8 / 92.8 / 113.8 now.
+// ------------------------------------------------------------------------------------------------
+struct LmHeadParams {
+    const float* ssq;
+    int ssq_ld, n_tok, n_tiles;
+    float* out;
+    int ldo;
+    uint32_t* status;
+};
+template <int BN> struct LmShape {
+    static constexpr uint32_t A_BYTES = TC_BM * TC_BK * 2, STAGE = A_BYTES + 3 * BN * TC_BK * 2;
+    static constexpr int STAGES = 200 * 1024 / STAGE;              // 7 or 5
+    static constexpr int KB = HIDDEN / TC_BK;
+    static constexpr uint32_t ACC = BN == 32 ? 128 : 256;          // TMEM columns of an accumulator
+    static constexpr int EPI_WARPS = BN / 8;                       // a warp takes 32 words x 32 sequences
+    static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+};
+
+template <int BN>
+__global__ void __launch_bounds__(LmShape<BN>::THREADS, 1) lm_head_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
+                                                                          const LmHeadParams p) {
+    using S = LmShape<BN>;
+    extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
+    __shared__ __align__(8) uint64_t full_bar[S::STAGES], empty_bar[S::STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_base_s;
+    __shared__ volatile int abort_flag;
+    __shared__ float s_scale[BN];
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S::STAGES; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&full_bar[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&empty_bar[s])) : "memory");
+        }
+        for (int b = 0; b < 2; ++b) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&acc_full[b])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(&acc_empty[b])), "r"(S::EPI_WARPS) : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        abort_flag = 0;
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_base_s)), "r"(2 * S::ACC) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = tmem_base_s;
+    pdl_launch();
+
+    if (warp == 0) {
+        // ------------------------------------------------------------------ TMA producer
+        int armed = 0;                                       // stages requested
+        if (elect_one()) {
+            const uint32_t st0 = tc_smem(base);
+            auto weights = [&](int tile, int kb, int s) {
+                asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(&full_bar[s])), "r"(S::STAGE) : "memory");
+                tc_load_box(st0 + s * S::STAGE, &tm_w, kb * TC_BK, tile * TC_BM, &full_bar[s]);
+                ++armed;
+            };
+            for (int kb = 0; kb < S::STAGES; ++kb) weights(blockIdx.x, kb, kb);      // (KB > STAGES: the first tile's)
+            pdl_wait();
+            int s = 0, turn = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < p.n_tiles && ok; tile += gridDim.x)
+                for (int kb = 0; kb < S::KB; ++kb, ++s) {
+                    if (s == S::STAGES) { s = 0; ++turn; }
+                    if (turn > 0) {
+                        ok = tc_wait(&empty_bar[s], (turn - 1) & 1, &abort_flag, p.status, 70);
+                        if (!ok) break;
+                        weights(tile, kb, s);
+                    }
+                    tc_load_planes(st0 + s * S::STAGE + S::A_BYTES, &tm_x, kb * TC_BK, 0, &full_bar[s]);
+                }
+            if (abort_flag)                                  // (what is under way lands before this memory is somebody else's)
+                for (int k = max(0, armed - S::STAGES); k < armed; ++k) tc_drain(&full_bar[k % S::STAGES], (k / S::STAGES) & 1);
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // ------------------------------------------------------------------ MMA issuer
+        if (elect_one()) {
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(3 * BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+            const uint64_t da0 = tc_desc(tc_smem(base)), db0 = tc_desc(tc_smem(base) + S::A_BYTES);
+            uint64_t ds = 0;
+            int s = 0, phase = 0, li = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < p.n_tiles && ok; tile += gridDim.x, ++li) {
+                const int acc = li & 1;
+                if (li >= 2) ok = tc_wait(&acc_empty[acc], ((li >> 1) - 1) & 1, &abort_flag, p.status, 71);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int kb = 0; kb < S::KB && ok; ++kb, ++s, ds += S::STAGE >> 4) {
+                    if (s == S::STAGES) { s = 0; phase ^= 1; ds = 0; }
+                    ok = tc_wait(&full_bar[s], phase, &abort_flag, p.status, 72);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                    for (int k = 0; k < TC_BK / 16; ++k)
+                        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+                                     ::"r"(tmem_base + (uint32_t)acc * S::ACC), "l"(da0 + ds + 2 * k), "l"(db0 + ds + 2 * k), "r"(idesc), "r"((uint32_t)(kb | k)), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&empty_bar[s])) : "memory");
+                }
+                // (also after a wait that gave up: whoever waits for the accumulator sees the flag, and the products end before the columns go)
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&acc_full[acc])) : "memory");
+                if (!ok) tc_drain(&acc_full[acc], (li >> 1) & 1);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------------ epilogue
+        const int quad = warp & 3, t0 = ((warp - 2) >> 2) * 32;     // TMEM lanes [32 quad, + 32), sequences [t0, t0 + 32)
+        pdl_wait();
+        for (int j = warp - 2; j < BN; j += S::EPI_WARPS) {
+            const float ss = warp_sum(j < p.n_tok ? p.ssq[(size_t)lane * p.ssq_ld + j] : 0.f);
+            if (lane == 0) s_scale[j] = rsqrtf(ss / (float)HIDDEN + EPS);
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * S::EPI_WARPS) : "memory");
+        int li = 0;
+        for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x, ++li) {
+            const int acc = li & 1;
+            if (!tc_wait_warp(&acc_full[acc], (li >> 1) & 1, &abort_flag, p.status, 73) || __any_sync(0xffffffffu, abort_flag)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint32_t r[32], q1[32], q2[32];                  // the planes' columns of the same sequences, under one wait
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * S::ACC + (uint32_t)t0;
+            tc_ld32(r, taddr);
+            tc_ld32(q1, taddr + BN);
+            tc_ld32(q2, taddr + 2 * BN);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(tc_smem(&acc_empty[acc])) : "memory");
+            float* dst = p.out + (size_t)t0 * p.ldo + tile * TC_BM + quad * 32 + lane;
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                if (t0 + j < p.n_tok) dst[(size_t)j * p.ldo] = (__uint_as_float(r[j]) + __uint_as_float(q1[j]) + __uint_as_float(q2[j])) * s_scale[t0 + j];
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * S::ACC) : "memory");
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -513,8 +649,8 @@ static cudaError_t launch_persist(const CUtensorMap* tw, const CUtensorMap& tx, 
     return launch_chain(gemm_tc_persist_kernel, dim3(grid), dim3(TP_THREADS), smem, st, tw[0], tw[1], tw[2], tx, p, w);
 }
 
-template <int BN, bool SCALE = false>
-static cudaError_t launch_bn(const CUtensorMap* tw, const CUtensorMap& tx, TcParams<SCALE> p, int n_rows, int n_tok, int sm_count, cudaStream_t st) {
+template <int BN>
+static cudaError_t launch_bn(const CUtensorMap* tw, const CUtensorMap& tx, GemmTcParams p, int n_rows, int n_tok, int sm_count, cudaStream_t st) {
     // n_rows: all weight rows of the launch (the sum over the groups); tw: three maps (unused ones repeat the first)
     const int nkb = p.K / TC_BK;
     const int tiles = ((n_rows + TC_BM - 1) / TC_BM) * ((n_tok + BN - 1) / BN);
@@ -555,13 +691,13 @@ static cudaError_t launch_bn(const CUtensorMap* tw, const CUtensorMap& tx, TcPar
         if (e != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return cudaErrorInvalidDevice;
         std::lock_guard<std::mutex> hold(host_lock());
         if (!attr_set[dev]) {
-            e = cudaFuncSetAttribute(gemm_tc_kernel<BN, SCALE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+            e = cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
             if (e != cudaSuccess) return e;
             attr_set[dev] = true;
         }
     }
     dim3 grid((n_rows + TC_BM - 1) / TC_BM, (n_tok + BN - 1) / BN, ksplit);
-    return launch_chain(gemm_tc_kernel<BN, SCALE>, grid, dim3(TC_THREADS), smem, st, tw[0], tw[1], tw[2], tx, p);
+    return launch_chain(gemm_tc_kernel<BN>, grid, dim3(TC_THREADS), smem, st, tw[0], tw[1], tw[2], tx, p);
 }
 
 // Encoding a tensor map costs a few microseconds of host time; a step issues hundreds of GEMMs over the
@@ -600,6 +736,35 @@ static int sm_count_of_current_device() {
     return sms[dev];
 }
 
+template <int BN>
+static cudaError_t launch_lm(const CUtensorMap& tw, const CUtensorMap& tx, const LmHeadParams& p, int sm_count, cudaStream_t st) {
+    using S = LmShape<BN>;
+    constexpr size_t smem = (size_t)S::STAGES * S::STAGE + 1024;
+    static bool attr_set[MAX_DEVICES] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return cudaErrorInvalidDevice;
+    {
+        std::lock_guard<std::mutex> hold(host_lock());
+        if (!attr_set[dev]) {
+            e = cudaFuncSetAttribute(lm_head_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+            attr_set[dev] = true;
+        }
+    }
+    return launch_chain(lm_head_kernel<BN>, dim3(p.n_tiles < sm_count ? p.n_tiles : sm_count), dim3(S::THREADS), smem, st, tw, tx, p);
+}
+
+cudaError_t launch_lm_head(const LmHeadCall& c, cudaStream_t st) {
+    const int bn = c.n_tok <= 32 ? 32 : 64, sm = sm_count_of_current_device();
+    if (sm < 1) return cudaErrorInvalidDevice;
+    if (c.vocab < TC_BM || c.vocab % TC_BM || c.n_tok < 1 || c.n_tok > 64 || c.prow < bn) return cudaErrorInvalidValue;
+    CUtensorMap tw, tx;
+    if (!cached_map(c.w, (uint64_t)c.vocab, (uint64_t)HIDDEN, TC_BM, &tw) || !cached_map(c.planes, (uint64_t)c.prow, (uint64_t)HIDDEN, (uint32_t)bn, &tx, 3)) return cudaErrorUnknown;
+    const LmHeadParams p{c.ssq, c.ssq_ld, c.n_tok, c.vocab / TC_BM, c.out, c.vocab, c.status};
+    return bn == 32 ? launch_lm<32>(tw, tx, p, sm, st) : launch_lm<64>(tw, tx, p, sm, st);
+}
+
 cudaError_t launch_gemm_tc(const GemmTcCall& c, cudaStream_t st) {
     if (c.K % TC_BK || c.n_rows % TC_BM || c.nsplit < 1 || c.nsplit > 3 || c.n_tok < 1) return cudaErrorInvalidValue;
     // token tile: the smallest of 32 / 64 / 128 that covers the batch, 128 for long prompts
@@ -614,14 +779,6 @@ cudaError_t launch_gemm_tc(const GemmTcCall& c, cudaStream_t st) {
     const int sm_count = sm_count_of_current_device();
     if (sm_count < 1) return cudaErrorInvalidDevice;
     const CUtensorMap maps[3] = {tw, tw, tw};
-    if (c.ssq != nullptr) {
-        if (c.resid != nullptr || bn > 64) return cudaErrorInvalidValue;
-        GemmTcScaledParams q{};
-        static_cast<GemmTcParams&>(q) = p;
-        q.ssq = c.ssq; q.ssq_ld = c.ssq_ld;
-        if (bn == 32) return launch_bn<32, true>(maps, tx, q, c.n_rows, c.n_tok, sm_count, st);
-        return launch_bn<64, true>(maps, tx, q, c.n_rows, c.n_tok, sm_count, st);
-    }
     if (persist_serves(c.n_rows, c.n_tok, c.nsplit, sm_count)) {
         CUtensorMap txp;
         if (!cached_map(c.x_planes, (uint64_t)c.nsplit * c.plane_rows, (uint64_t)c.K, (uint32_t)TP_BN, &txp)) return cudaErrorUnknown;

@@ -40,11 +40,21 @@ struct GemmTcCall {
     int ldo, ldr;
     int n_rows, n_tok, K, nsplit, plane_rows;
     uint32_t* status;
-    const float* ssq;      // not null: the planes lack their RMS norm's scale, the epilogue applies it (at most 64 tokens, no residual)
-    int ssq_ld;
 };
 
 cudaError_t launch_gemm_tc(const GemmTcCall& c, cudaStream_t st);
+
+// The LM head of a decode batch: three planes that lack their RMS norm's scale, taken from 32 partial sums of squares a row
+struct LmHeadCall {
+    const void* w;         // bf16 [vocab][1024], vocab a multiple of 128
+    const void* planes;    // bf16 [3][prow][1024]
+    int prow, n_tok, vocab;
+    const float* ssq;      // [32][ssq_ld]
+    int ssq_ld;
+    float* out;            // [n_tok][vocab]
+    uint32_t* status;
+};
+cudaError_t launch_lm_head(const LmHeadCall& c, cudaStream_t st);
 
 // Up to three weight matrices with the same K against the same activation planes in ONE launch (q/k/v, gate/up):
 // group g writes out[g][t * ldo[g] + n] for its own rows n.  Plain stores or split-K atomics onto zeros; no residual.
