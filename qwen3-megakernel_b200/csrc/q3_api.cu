@@ -597,7 +597,7 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
 
 // A prompt: five launches a layer (q3_prompt.h).  The activations enter the tensor cores rounded to bf16, like the weights and like
 // the cached K/V rows that the prompt's later positions attend anyway.  Measured at 2048 tokens, full model, against the fp32 CPU
-// checker: K/V rows rel-L2 6.6e-3 and logits 5.6e-3 with one plane, 4.0e-3 and 3.2e-3 with two (the cache rounding dominates
+// oracle: K/V rows rel-L2 6.6e-3 and logits 5.6e-3 with one plane, 4.0e-3 and 3.2e-3 with two (the cache rounding dominates
 // both; the gates are 1e-2 and 2e-2).
 // From 64 tokens on the attention is the tiled one over cached rows; fewer tokens keep the split attention, whose own row and
 // probabilities are more precise than bf16.

@@ -1,4 +1,5 @@
-// Tensor-core GEMM for prefill and large-batch decode: out[t, n] (+)= sum_k W[n, k] * X[t, k].
+// Tensor-core GEMM for decode batches of more than 64 sequences and for q3_linear_tc: out[t, n] (+)= sum_k W[n, k] * X[t, k]; and the
+// LM head of smaller decode batches.  (A prompt's products: q3_prompt.cu.)
 //
 // Blackwell path: TMA (cp.async.bulk.tensor, 128-byte swizzle) stages W and X tiles in shared memory,
 // one elected thread issues tcgen05.mma (kind::f16, bf16 operands, fp32 accumulator in TMEM), four
@@ -9,10 +10,7 @@
 // Exact activations: the fp32 activations are passed as up to three bf16 planes (hi, mid, lo with
 // X = hi + mid + lo); each W tile is multiplied with every plane into the same accumulator.  With
 // three planes the result equals the fp32 product of the bf16 weights up to accumulation order;
-// large-batch decode uses that (the extra MMAs are free while the weights stream from HBM), prefill
-// uses one or two planes.
-//
-// Replaces the dense `xn @ w.T` products of the reference's PyTorch prefill (qwen3mk/prefill.py:61-80).
+// large-batch decode uses that (the extra MMAs are free while the weights stream from HBM).
 #include <cuda.h>
 
 #include <mutex>
@@ -219,7 +217,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
 }
 
 // ------------------------------------------------------------------------------------------------
-// The same GEMM for prompts as a PERSISTENT kernel: one CTA per SM walks a list of work items (a tile of 128 weight rows x
+// The same GEMM for many tokens of one plane as a PERSISTENT kernel: one CTA per SM walks a list of work items (a tile of 128 weight rows x
 // 256 tokens).  What the one-tile-per-CTA kernel does in
 // series - fill the pipeline, the MMAs, the read-back of 128 KB of accumulator - overlaps here:
 //   * the TMA ring never drains between items (the producer runs ahead into the next item's k blocks),
@@ -234,9 +232,7 @@ struct GemmPersistItems {
     int n_items, m_tiles, n_ttiles;   // items = token tiles x weight tiles
 };
 
-__global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap tm_w0,
-                                                                        const __grid_constant__ CUtensorMap tm_w1,
-                                                                        const __grid_constant__ CUtensorMap tm_w2,
+__global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap tm_w,
                                                                         const __grid_constant__ CUtensorMap tm_x, const GemmTcParams p,
                                                                         const GemmPersistItems w) {
     constexpr int BN = TP_BN;                       // tokens per item
@@ -274,24 +270,10 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
     const uint32_t tmem_base = tmem_base_s;
     pdl_launch();
 
-    // item -> (k slice, token tile, weight tile -> matrix of a grouped launch and row inside it)
-    struct Item { int grp, m0, n0, kb_begin, nkb; };
-    auto decode = [&](int it) {
-        Item r;
-        const int per_slice = w.m_tiles * w.n_ttiles;
-        const int ks = it / per_slice, rem = it - ks * per_slice;
-        int tile = rem % w.m_tiles;
-        r.n0 = (rem / w.m_tiles) * BN;
-        r.grp = 0;
-        if (p.n_groups > 1) {
-            if (tile >= p.g_tiles[0]) { tile -= p.g_tiles[0]; r.grp = 1; }
-            if (r.grp == 1 && p.n_groups > 2 && tile >= p.g_tiles[1]) { tile -= p.g_tiles[1]; r.grp = 2; }
-        }
-        r.m0 = tile * TC_BM;
-        r.kb_begin = ks * p.kb_per_split;
-        r.nkb = min(p.K / TC_BK - r.kb_begin, p.kb_per_split);
-        return r;
-    };
+    // item -> (token tile, weight tile)
+    struct Item { int m0, n0; };
+    auto decode = [&](int it) { return Item{it % w.m_tiles * TC_BM, it / w.m_tiles * BN}; };
+    const int nkb = p.K / TC_BK;
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
@@ -300,17 +282,16 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
             int s = 0, turn = 0;
             for (int it = blockIdx.x; it < w.n_items && !abort_flag; it += gridDim.x) {
                 const Item r = decode(it);
-                const CUtensorMap* tm_w = r.grp == 0 ? &tm_w0 : (r.grp == 1 ? &tm_w1 : &tm_w2);
-                for (int kb = 0; kb < r.nkb; ++kb, ++s) {
+                for (int kb = 0; kb < nkb; ++kb, ++s) {
                     if (s == stages) { s = 0; ++turn; }
                     if (turn > 0 && !tc_wait(&empty_bar[s], (turn - 1) & 1, &abort_flag, p.status, 36)) break;
                     unsigned char* st = base + (size_t)s * stage_bytes;
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(&full_bar[s])), "r"(stage_bytes) : "memory");
                     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                 ::"r"(tc_smem(st)), "l"(tm_w), "r"((r.kb_begin + kb) * TC_BK), "r"(r.m0), "r"(tc_smem(&full_bar[s])) : "memory");
+                                 ::"r"(tc_smem(st)), "l"(&tm_w), "r"(kb * TC_BK), "r"(r.m0), "r"(tc_smem(&full_bar[s])) : "memory");
                     for (int sp = 0; sp < nsplit; ++sp)
                         asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                     ::"r"(tc_smem(st + a_bytes + sp * b_bytes)), "l"(&tm_x), "r"((r.kb_begin + kb) * TC_BK), "r"(sp * p.plane_rows + r.n0),
+                                     ::"r"(tc_smem(st + a_bytes + sp * b_bytes)), "l"(&tm_x), "r"(kb * TC_BK), "r"(sp * p.plane_rows + r.n0),
                                        "r"(tc_smem(&full_bar[s])) : "memory");
                 }
             }
@@ -322,12 +303,11 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
             int s = 0, phase = 0, li = 0;
             bool ok = true;
             for (int it = blockIdx.x; it < w.n_items && ok; it += gridDim.x, ++li) {
-                const Item r = decode(it);
                 const int acc = li & 1;
                 // the accumulator is free once the epilogue warps have read its previous tenant out
                 if (li >= 2) ok = tc_wait(&acc_empty[acc], ((li >> 1) - 1) & 1, &abort_flag, p.status, 37);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int kb = 0; kb < r.nkb && ok; ++kb, ++s) {
+                for (int kb = 0; kb < nkb && ok; ++kb, ++s) {
                     if (s == stages) { s = 0; phase ^= 1; }
                     ok = tc_wait(&full_bar[s], phase, &abort_flag, p.status, 38);
                     if (!ok) break;
@@ -358,8 +338,6 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
         for (int it = blockIdx.x; it < w.n_items && ok; it += gridDim.x, ++li) {
             const Item r = decode(it);
             const int acc = li & 1;
-            float* const out = p.n_groups > 1 ? (r.grp == 0 ? p.g_out[0] : r.grp == 1 ? p.g_out[1] : p.g_out[2]) : p.out;
-            const int ldo = p.n_groups > 1 ? (r.grp == 0 ? p.g_ldo[0] : r.grp == 1 ? p.g_ldo[1] : p.g_ldo[2]) : p.ldo;
             ok = tc_wait_warp(&acc_full[acc], (li >> 1) & 1, &abort_flag, p.status, 39);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -383,13 +361,9 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
                     const int t = r.n0 + c * 32 + j;
                     if (t < p.n_tok) {
                         float x = __uint_as_float(v[j]);
-                        float* dst = out + (size_t)t * ldo + row;
-                        if (p.epi == TC_EPI_ATOMIC) {
-                            atomicAdd(dst, x);   // split-K: `out` already holds zero or the residual
-                        } else {
-                            if (p.epi == TC_EPI_RESID) x += p.resid[(size_t)t * p.ldr + row];
-                            *dst = x;
-                        }
+                        float* dst = p.out + (size_t)t * p.ldo + row;
+                        if (p.epi == TC_EPI_RESID) x += p.resid[(size_t)t * p.ldr + row];
+                        *dst = x;
                     }
                 }
             }
@@ -609,20 +583,16 @@ static int k_slices(int n_rows, int n_tok, int bn, int nkb, int sm_count) {
     return ksplit < 1 ? 1 : ksplit;
 }
 
-// A prompt's GEMM takes the persistent kernel when its 128 x 256 items occupy at least 0.6 of the SMs (q/k/v from about
-// 520 tokens on, gate + up from about 420).  Measured inside a prefill of 2048 tokens: q/k/v 23.9 us against 32.3 us,
-// gate/up 32.7 against 36.3; whole prefills with the threshold at 1.0 / 0.6 / 0.4 of the SMs: 512 tokens 2.39 / 2.28 /
-// 2.29 ms, 768 tokens 2.90 / 2.49 / 2.49, 1000 tokens 3.34 / 2.96 / 2.97, 300 tokens 2.05 / 2.05 / 2.13.  With K cut in
-// slices for the launches of few tiles (Wo, down) it was no faster than the one-tile-per-CTA kernel with three CTAs per
-// SM (19.1 / 23.1 us against 19.0 / 19.0), so those stay there.
+// One plane and 128 x 256 items that occupy at least 0.6 of the SMs take the persistent kernel.  Measured when prompts ran on it, 2048 tokens: 4096
+// weight rows of K = 1024 23.9 us against 32.3; a threshold of 1.0 / 0.6 / 0.4 of the SMs, whole prompts of 512 tokens 2.39 / 2.28 / 2.29 ms,
+// 768 2.90 / 2.49 / 2.49.
 static bool persist_serves(int n_rows, int n_tok, int nsplit, int sm_count) {
     // one activation plane: with more the 256-token stages no longer fit four deep
     return n_tok >= TP_BN && nsplit == 1 && (n_rows / TC_BM) * ((n_tok + TP_BN - 1) / TP_BN) * 10 >= sm_count * 6;
 }
 
-static cudaError_t launch_persist(const CUtensorMap* tw, const CUtensorMap& tx, GemmTcParams p, int n_rows, int n_tok, int sm_count, cudaStream_t st) {
+static cudaError_t launch_persist(const CUtensorMap& tw, const CUtensorMap& tx, GemmTcParams p, int n_rows, int n_tok, int sm_count, cudaStream_t st) {
     constexpr int BN = TP_BN;
-    p.kb_per_split = p.K / TC_BK;   // K is never cut here
     const uint32_t stage_bytes = TC_BM * TC_BK * 2 + p.nsplit * BN * TC_BK * 2;
     int stages = (int)((200u * 1024u) / stage_bytes);
     if (stages > 8) stages = 8;
@@ -646,7 +616,7 @@ static cudaError_t launch_persist(const CUtensorMap* tw, const CUtensorMap& tx, 
     w.n_ttiles = (n_tok + BN - 1) / BN;
     w.n_items = w.m_tiles * w.n_ttiles;
     const int grid = w.n_items < sm_count ? w.n_items : sm_count;
-    return launch_chain(gemm_tc_persist_kernel, dim3(grid), dim3(TP_THREADS), smem, st, tw[0], tw[1], tw[2], tx, p, w);
+    return launch_chain(gemm_tc_persist_kernel, dim3(grid), dim3(TP_THREADS), smem, st, tw, tx, p, w);
 }
 
 template <int BN>
@@ -782,7 +752,7 @@ cudaError_t launch_gemm_tc(const GemmTcCall& c, cudaStream_t st) {
     if (persist_serves(c.n_rows, c.n_tok, c.nsplit, sm_count)) {
         CUtensorMap txp;
         if (!cached_map(c.x_planes, (uint64_t)c.nsplit * c.plane_rows, (uint64_t)c.K, (uint32_t)TP_BN, &txp)) return cudaErrorUnknown;
-        return launch_persist(maps, txp, p, c.n_rows, c.n_tok, sm_count, st);
+        return launch_persist(tw, txp, p, c.n_rows, c.n_tok, sm_count, st);
     }
     if (bn == 32) return launch_bn<32>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
     if (bn == 64) return launch_bn<64>(maps, tx, p, c.n_rows, c.n_tok, sm_count, st);
@@ -809,11 +779,6 @@ cudaError_t launch_gemm_tc_group(const GemmTcGroupCall& c, cudaStream_t st) {
     p.nsplit = c.nsplit; p.plane_rows = c.plane_rows; p.epi = TC_EPI_STORE; p.status = c.status; p.out_is_zero = c.out_is_zero;
     const int sm_count = sm_count_of_current_device();
     if (sm_count < 1) return cudaErrorInvalidDevice;
-    if (persist_serves(rows, c.n_tok, c.nsplit, sm_count)) {
-        CUtensorMap txp;
-        if (!cached_map(c.x_planes, (uint64_t)c.nsplit * c.plane_rows, (uint64_t)c.K, (uint32_t)TP_BN, &txp)) return cudaErrorUnknown;
-        return launch_persist(maps, txp, p, rows, c.n_tok, sm_count, st);
-    }
     if (bn == 32) return launch_bn<32>(maps, tx, p, rows, c.n_tok, sm_count, st);
     if (bn == 64) return launch_bn<64>(maps, tx, p, rows, c.n_tok, sm_count, st);
     return launch_bn<128>(maps, tx, p, rows, c.n_tok, sm_count, st);
