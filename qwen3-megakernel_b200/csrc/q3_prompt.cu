@@ -120,6 +120,10 @@ __device__ __forceinline__ void pr_expect(uint64_t* bar, uint32_t bytes) {
 // tiles while this launch ends.  A partial tile is [row][BN] fp32 with the 16-byte chunks of a row XORed by row & 7, so
 // that a thread per row writes it and half a warp per row reads it without bank conflicts; it overlays the stages.
 //
+// Tensor memory of an SM: a block waits for its cluster while it holds its columns, so the blocks that fit on an SM may not ask for more than 512
+// together (q3_gemm_cl.cu).  Two of these are 256 and leave no room for a decode product's 58 KB; one of them and two decode products are 384.
+// A block of the pair kernel (512 columns) has more shared memory than any of them leaves.
+//
 // A wait that gives up: as in q3_gemm_cl.cu (a block without its sums sends and stores nothing, everyone meets at every cluster
 // barrier, and what was under way is drained before the block leaves).
 // ------------------------------------------------------------------------------------------------------------------------------
