@@ -66,8 +66,8 @@ struct SampleShared {
     unsigned hist[SAMPLE_BINS];
     unsigned cand[SAMPLE_CAND];             // keys
     int candi[SAMPLE_CAND];                 // and where they are
+    float weight[SAMPLE_KEYS * SAMPLE_THREADS];   // weights of all blocks' candidates, the lists one after the other
     unsigned sel, need, cand_n, cmin;
-    float bracket[2];                       // the block's share of the weights' running sum
 };
 
 // Block-wide: the bin, counted from the largest, in which the running count of hist[] reaches `need`, and what is still
@@ -323,51 +323,42 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
                 if (n == (unsigned)top_k) break;
             }
             // ---- 3. and 4. from the candidates alone: all kept words are among them, and every block adds the same weights in the same order, so
-            // the blocks' brackets meet without another exchange ----
+            // the blocks' brackets meet without another exchange.  A warp sums a list, and the lists' sums follow one another: a list without a
+            // kept word adds exactly nothing, its block's bracket is empty (prefix sums of one scan over all lists would differ in the
+            // last place where nothing but zeros lies between them) ----
             auto key_weight = [&](unsigned k) { return k >= t ? weight(key_value(k), vmax) : 0.f; };
-            float run = 0.f;
 #pragma unroll
             for (int q = 0; q < SAMPLE_KEYS; ++q) {
-                if (q * SAMPLE_THREADS < count) {
-                    const int e = q * SAMPLE_THREADS + tid;
-                    const float w = e < count ? key_weight(key[q]) : 0.f;
-                    float incl = w;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const float p = __shfl_up_sync(0xffffffffu, incl, o);
-                        if (lane >= o) incl += p;
-                    }
-                    __syncthreads();
-                    if (lane == 31) sh.wf[warp] = incl;
-                    float before = __shfl_up_sync(0xffffffffu, incl, 1);
-                    __syncthreads();
-                    float all = sh.wf[lane];
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const float p = __shfl_up_sync(0xffffffffu, all, o);
-                        if (lane >= o) all += p;
-                    }
-                    const float warps = warp ? __shfl_sync(0xffffffffu, all, warp - 1) : 0.f;
-                    before = run + (warps + (lane ? before : 0.f));
-                    if (e == mine0) sh.bracket[0] = before;
-                    if (e == mine0 + n_cand) sh.bracket[1] = before;
-                    run += __shfl_sync(0xffffffffu, all, 31);
-                }
+                const int e = q * SAMPLE_THREADS + tid;
+                if (e < count) sh.weight[e] = key_weight(key[q]);
             }
             if (tid == 0) { sh.need = 0xffffffffu; sh.cand_n = 0u; }
             __syncthreads();
-            base = sh.bracket[0]; next = mine0 + n_cand == count ? run : sh.bracket[1]; total = run + odd;
+            if (warp < C) {
+                int first = 0;
+                for (int r = 0; r < warp; ++r) first += sh.ncand[r];
+                float ws = 0.f;
+                for (int j = lane; j < sh.ncand[warp]; j += 32) ws += sh.weight[first + j];
+                ws = warp_sum(ws);
+                if (lane == 0) sh.wf[warp] = ws;
+            }
+            __syncthreads();
+            for (int r = 0; r < C; ++r) {
+                if (r == rank) base = total;
+                total += sh.wf[r];
+                if (r == rank) next = total;
+            }
+            total += odd;
             // Weights that are not numbers (infinite logits, or a NaN in the row), or a u outside [0, 1): no draw, the arg-max.
             if (!(total > 0.f && total < INFINITY && u >= 0.f && u < 1.f)) { cluster.barrier_wait(); write_argmax(); return; }
             float target = u * total;
             if (!(target < total)) target = __uint_as_float(__float_as_uint(total) - 1u);   // u * total rounded up to the total: the last word with a weight
-            if (n_cand > 0 && base <= target && target < next) {
-                // the first of this block's kept words, in the order of their indices, whose inclusive prefix sum exceeds the target
-                float* const w = reinterpret_cast<float*>(sh.hist);
-                const float own = tid < n_cand ? key_weight(sh.cand[tid]) : 0.f;
+            if (base <= target && target < next) {
+                // the first of this block's kept words, in the order of their indices, whose inclusive prefix sum exceeds the target.  (next > base:
+                // one of them has a weight)
+                const float* const w = sh.weight + mine0;
+                const float own = tid < n_cand ? w[tid] : 0.f;
                 const int at = tid < n_cand ? sh.candi[tid] : 0;
-                if (tid < n_cand) w[tid] = own;
-                __syncthreads();
                 if (own > 0.f) {
                     float p = 0.f;
                     for (int j = 0; j < n_cand; ++j)

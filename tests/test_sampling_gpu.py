@@ -240,3 +240,39 @@ def test_draws_over_every_number_of_blocks_a_row(batch, vocab, top_k, temperatur
         assert bool(keep[b, j]) and float(w[b, j]) > 0.0, (b, j)
         lo = float(cdf[b, j - 1]) if j else 0.0
         assert lo - CDF_TOL <= float(u[b]) <= float(cdf[b, j]) + CDF_TOL, (b, j, float(u[b]), lo, float(cdf[b, j]))
+
+
+def block_ends(vocab, blocks):
+    """Where the kernel's blocks end that share a row: 32 warps a block, a run of whole groups of 128 words a warp."""
+    run = (-(-vocab // (blocks * 32)) + 127) // 128 * 128
+    return [min(vocab, (r + 1) * 32 * run) for r in range(blocks)]
+
+
+def beside(u, ulps=range(-8, 9)):
+    """Uniform numbers a few units in the last place around u, all in [0, 1)."""
+    return [(u.double() * (1.0 + n * 2.0 ** -24)).float().clamp(0.0, 1.0 - 2.0 ** -24) for n in ulps]
+
+
+@pytest.mark.parametrize("batch,blocks", [(4, 16), (14, 8), (36, 4), (64, 2)])
+@pytest.mark.parametrize("top_k", [2, 20, 50, 200])
+@pytest.mark.parametrize("part", [10, 4])
+def test_a_word_that_is_not_kept_is_never_drawn(batch, blocks, top_k, part):
+    """The k largest words lie in the first tenth or quarter of the row, so most of its blocks keep none, and the uniform numbers lie on the
+    ends of the blocks' shares of the distribution, a few units in the last place beside them, and at both ends of [0, 1)."""
+    from qwen3mk import sampling
+
+    vocab = 151936
+    g = torch.Generator(device="cuda").manual_seed(1000 * batch + 10 * top_k + part)
+    logits = torch.randn((batch, vocab), generator=g, device="cuda") * 3.0
+    logits[:, vocab // part:] -= 30.0
+    rows = logits.double()
+    keep = rows >= rows.topk(top_k, dim=-1).values[:, -1:]
+    assert not bool(keep[:, vocab // part:].any())
+    w = torch.where(keep, torch.exp((rows - rows.amax(dim=-1, keepdim=True)) / 0.8), torch.zeros_like(rows))
+    cdf = w.cumsum(dim=-1)
+    ends = (cdf / cdf[:, -1:])[:, [e - 1 for e in block_ends(vocab, blocks)]]
+    zero = torch.zeros(batch, device="cuda")
+    for u in [zero] + [v for r in range(blocks) for v in beside(ends[:, r])]:
+        got = sampling.sample(logits, 0.8, top_k, u=u)
+        bad = (~keep.gather(1, got[:, None])[:, 0]).nonzero().flatten().tolist()
+        assert not bad, f"{len(bad)} rows drew words that are not kept: row {bad[0]}, word {int(got[bad[0]])}, u = 1 - {(1 - float(u[bad[0]])) * 2 ** 24} / 2^24"
