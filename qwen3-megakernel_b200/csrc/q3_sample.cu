@@ -430,11 +430,15 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     if (lane == 0 && from <= target && target < to) { sh.sel = (unsigned)warp; sh.wg[0] = from; }
     if (tid == 0) { sh.need = 0xffffffffu; sh.cand_n = 0u; }
     __syncthreads();
-    const int r0 = (rank * SAMPLE_WARPS + (int)sh.sel) * per, r1 = min(vocab, r0 + per);
+    // The run was chosen by weights under the block's own maximum, its words are weighed under the row's: where those underflow the run may have no
+    // word with a weight.  Then it is the next one behind the run, or the block's first: its maximum has a weight, or its sum would be nothing.
+    auto run_start = [&](int w) { return (int)min((long long)vocab, (long long)(rank * SAMPLE_WARPS + w) * per); };
+    const int s0 = run_start(0), s1 = run_start(SAMPLE_WARPS), r0 = run_start((int)sh.sel), r1 = run_start((int)sh.sel + 1);
     float run = sh.wg[0];
-    for (int first = r0; first < r1; first += SAMPLE_THREADS) {
+    int first = r0, end = r1, span = 0;             // 0: the run, 1: what follows it, 2: what is before it
+    for (;;) {
         const int i = first + tid;
-        const float v = i < r1 ? row[i] : -INFINITY;
+        const float v = i < end ? row[i] : -INFINITY;
         // (the scan adds the same weights in another order for every lane, so a word without weight may see a larger prefix than the
         // word before it: only one with a weight is a candidate)
         const float own = v >= least ? __expf((v - vmax) * inv_t) : 0.f;
@@ -452,14 +456,20 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
             if (w == warp) before = run;
             run += sh.wf[w];
         }
-        const unsigned hit = __ballot_sync(0xffffffffu, kept && before + incl > target), all = __ballot_sync(0xffffffffu, kept);
+        const unsigned hit = __ballot_sync(0xffffffffu, kept && (span > 0 || before + incl > target)), all = __ballot_sync(0xffffffffu, kept);
         if (lane == 0 && hit) atomicMin(&sh.need, (unsigned)(first + 32 * warp + __ffs(hit) - 1));
-        if (lane == 0 && all) atomicMax(&sh.cand_n, (unsigned)(first + 32 * warp + 31 - __clz(all)));
+        if (lane == 0 && all) atomicMax(&sh.cand_n, (unsigned)(first + 32 * warp + 32 - __clz(all)));   // (0: none so far)
         __syncthreads();
         if (sh.need != 0xffffffffu) break;
+        first += SAMPLE_THREADS;
+        if (first >= end) {
+            if (sh.cand_n > 0u || span == 2) break;
+            ++span;
+            first = span == 1 ? r1 : s0; end = span == 1 ? s1 : r0;
+        }
     }
     // rounding may leave the target a hair beyond the run's own sum: then its last element with a weight
-    if (tid == 0) out[row_id] = sh.need != 0xffffffffu ? (long long)sh.need : (long long)sh.cand_n;
+    if (tid == 0) out[row_id] = sh.need != 0xffffffffu ? (long long)sh.need : (long long)sh.cand_n - 1;
 }
 
 template <int NQ>

@@ -276,3 +276,22 @@ def test_a_word_that_is_not_kept_is_never_drawn(batch, blocks, top_k, part):
         got = sampling.sample(logits, 0.8, top_k, u=u)
         bad = (~keep.gather(1, got[:, None])[:, 0]).nonzero().flatten().tolist()
         assert not bad, f"{len(bad)} rows drew words that are not kept: row {bad[0]}, word {int(got[bad[0]])}, u = 1 - {(1 - float(u[bad[0]])) * 2 ** 24} / 2^24"
+
+
+@pytest.mark.parametrize("batch,blocks", [(4, 16), (14, 8), (36, 4), (64, 2), (149, 1)])
+def test_a_word_whose_weight_underflows_is_never_drawn(batch, blocks):
+    """Whole vocabulary, u = 0, low temperature: the first block's largest word weighs about the smallest number there is beside the row's maximum,
+    the thousands of words before it weigh nothing each, although their sum under the block's own maximum does weigh something."""
+    from qwen3mk import sampling
+
+    vocab, temperature = 151936, 0.01
+    end = block_ends(vocab, blocks)[0]
+    gap = torch.linspace(0.95, 1.03, batch)
+    logits = torch.full((batch, vocab), -5.0)
+    logits[:, : end // 2] = -gap[:, None] - 0.1                 # exp(-105) and less: below half of the smallest denormal, exp(-103.28)
+    logits[torch.arange(batch), torch.randint(end // 2, end, (batch,), generator=torch.Generator().manual_seed(batch))] = -gap
+    logits[:, -1] = 0.0
+    got = sampling.sample(logits.cuda(), temperature, 0, u=torch.zeros(batch, device="cuda")).cpu()
+    # (0.25: rounding of (logit - maximum) / temperature, and of the exponential's argument)
+    nats = -logits.gather(1, got[:, None])[:, 0] / temperature
+    assert float(nats.max()) <= 103.28 + 0.25, nats.tolist()
