@@ -12,7 +12,7 @@
 //      grows); maxima and sums are exchanged together and the blocks' sums scaled to the row's maximum;
 //   2. top-k: a block whose threads have at least k elements bins its THREADS' maxima linearly between the smallest and
 //      the largest of them; the bins that hold the k largest maxima bound its own k largest elements from below, so the
-//      few elements at or above that bound (about 1.1 k of them) are the block's candidates.  The union of all blocks'
+//      few elements at or above that bound (about 1.1 k of them) are the block's candidates, in the order of their indices.  The union of all blocks'
 //      candidates contains every word that is kept; every block finds the threshold among them (binary search over the bits of
 //      the keys, held in registers, below the bits they share and until exactly k are above it) and adds up the weights of the kept
 //      ones, in the same order as every other block.  A row whose candidates do not fit (large k, many equal values) goes
@@ -66,7 +66,7 @@ struct SampleShared {
     unsigned hist[SAMPLE_BINS];
     unsigned cand[SAMPLE_CAND];             // keys
     int candi[SAMPLE_CAND];                 // and where they are
-    float weight[SAMPLE_KEYS * SAMPLE_THREADS];   // weights of all blocks' candidates, the lists one after the other
+    float weight[SAMPLE_KEYS * SAMPLE_THREADS];   // weights of all blocks' candidates, the lists one after the other (before that, the block's own list unordered)
     unsigned sel, need, cand_n, cmin;
 };
 
@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
             return d >= 0.f ? (int)fminf(d, (float)(SAMPLE_BINS - 1)) : 0;
         };
         if (top_k <= n_thr) {
+            unsigned* const raw = reinterpret_cast<unsigned*>(sh.weight);    // the candidates as they come: keys, then indices
             if (any) atomicAdd(&sh.hist[bin(mine)], 1u);
             __syncthreads();
             find_bin(sh, sh.hist[2 * tid], sh.hist[2 * tid + 1], (unsigned)top_k, false);
@@ -210,19 +211,29 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
                 each([&](int i, float v) {
                     if (bin(v) <= last && i < i1) {
                         const unsigned n = atomicAdd(&sh.cand_n, 1u), key = ordered_key(v);
-                        if (n < SAMPLE_CAND) { sh.cand[n] = key; sh.candi[n] = i; }
+                        if (n < SAMPLE_CAND) { raw[n] = key; raw[SAMPLE_CAND + n] = (unsigned)i; }
                         atomicMin(&sh.cmin, key);
                     }
                 });
+            __syncthreads();
+            // In the order of their indices: sums of weights must not depend on which thread came first.  (A list is about 1.1 k words long.)
+            const int n = (int)sh.cand_n;
+            if (n <= SAMPLE_CAND && tid < n) {
+                const unsigned at = raw[SAMPLE_CAND + tid];
+                int place = 0;
+#pragma unroll 8
+                for (int j = 0; j < n; ++j) place += raw[SAMPLE_CAND + j] < at;
+                sh.cand[place] = raw[tid]; sh.candi[place] = (int)at;
+            }
+            n_cand = n <= SAMPLE_CAND ? n : -1;
         } else {
             // fewer threads with elements than k: every element is a candidate, if they fit
             const int s0 = rank * SAMPLE_WARPS * per, slice = min(vocab, s0 + SAMPLE_WARPS * per) - min(vocab, s0);
             if (slice <= SAMPLE_CAND)
                 each([&](int i, float v) { if (i < i1) { sh.cand[i - s0] = ordered_key(v); sh.candi[i - s0] = i; } });
-            if (tid == 0) { sh.cand_n = (unsigned)slice; sh.cmin = 0u; }
+            if (tid == 0) sh.cmin = 0u;
+            n_cand = slice <= SAMPLE_CAND ? slice : -1;
         }
-        __syncthreads();
-        n_cand = sh.cand_n <= SAMPLE_CAND ? (int)sh.cand_n : -1;
     }
     // ---- the block's sum of weights: over all its words under its own maximum, or (select) whether it has a NaN ----
     float lo = 0.f, hi = 0.f, bsum = 0.f;           // this warp's bracket inside the block, and the block's sum
@@ -279,10 +290,11 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     if (select) {
         // ---- 2b. threshold: the k-th largest key ----
         bool fits = true;
-        int count = 0, mine0 = 0;                   // candidates of all blocks, and of those before this one
+        int count = 0, mine0 = 0, list0 = 0;        // candidates of all blocks, of those before this one, and before the one that this warp sums below
         float odd = 0.f;
         for (int r = 0; r < C; ++r) {
             if (r == rank) mine0 = count;
+            if (r == warp) list0 = count;
             fits = fits && sh.ncand[r] >= 0; count += max(sh.ncand[r], 0); odd += sh.bsum[r];
         }
         fits = fits && count <= SAMPLE_KEYS * SAMPLE_THREADS;
@@ -335,10 +347,8 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
             if (tid == 0) { sh.need = 0xffffffffu; sh.cand_n = 0u; }
             __syncthreads();
             if (warp < C) {
-                int first = 0;
-                for (int r = 0; r < warp; ++r) first += sh.ncand[r];
                 float ws = 0.f;
-                for (int j = lane; j < sh.ncand[warp]; j += 32) ws += sh.weight[first + j];
+                for (int j = lane; j < sh.ncand[warp]; j += 32) ws += sh.weight[list0 + j];
                 ws = warp_sum(ws);
                 if (lane == 0) sh.wf[warp] = ws;
             }
@@ -358,11 +368,10 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
                 // one of them has a weight)
                 const float* const w = sh.weight + mine0;
                 const float own = tid < n_cand ? w[tid] : 0.f;
-                const int at = tid < n_cand ? sh.candi[tid] : 0;
                 if (own > 0.f) {
+                    const int at = sh.candi[tid];
                     float p = 0.f;
-                    for (int j = 0; j < n_cand; ++j)
-                        if (sh.candi[j] <= at) p += w[j];
+                    for (int j = 0; j <= tid; ++j) p += w[j];
                     if (base + p > target) atomicMin(&sh.need, (unsigned)at);
                     atomicMax(&sh.cand_n, (unsigned)at);
                 }

@@ -295,3 +295,27 @@ def test_a_word_whose_weight_underflows_is_never_drawn(batch, blocks):
     # (0.25: rounding of (logit - maximum) / temperature, and of the exponential's argument)
     nats = -logits.gather(1, got[:, None])[:, 0] / temperature
     assert float(nats.max()) <= 103.28 + 0.25, nats.tolist()
+
+
+@pytest.mark.parametrize("batch,blocks", [(4, 16), (14, 8), (36, 4), (64, 2), (149, 1)])
+@pytest.mark.parametrize("top_k", [20, 50, 200])
+def test_the_same_numbers_draw_the_same_words(batch, blocks, top_k):
+    """The uniform numbers lie on boundaries between kept words and a few units in the last place beside them, where the order of the additions
+    decides: every run draws the same."""
+    from qwen3mk import sampling
+
+    vocab = 151936
+    g = torch.Generator(device="cuda").manual_seed(batch + top_k)
+    logits = torch.randn((batch, vocab), generator=g, device="cuda") * 3.0
+    rows = logits.double()
+    keep = rows >= rows.topk(top_k, dim=-1).values[:, -1:]
+    w = torch.where(keep, torch.exp((rows - rows.amax(dim=-1, keepdim=True)) / 0.8), torch.zeros_like(rows))
+    cdf = w.cumsum(dim=-1)
+    cdf /= cdf[:, -1:].clone()
+    kept = [torch.nonzero(keep[b]).flatten() for b in range(batch)]
+    for trial in range(8):
+        edge = torch.stack([cdf[b, kept[b][(7 * trial + b) % (len(kept[b]) - 1)]] for b in range(batch)])
+        for u in beside(edge, range(-4, 5)):
+            want = sampling.sample(logits, 0.8, top_k, u=u)
+            again = torch.stack([sampling.sample(logits, 0.8, top_k, u=u) for _ in range(6)])
+            assert bool((again == want).all()), f"trial {trial}: rows {(again != want).any(0).nonzero().flatten().tolist()}"
