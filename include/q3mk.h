@@ -143,7 +143,8 @@ int q3_tp_attach(q3_engine* e, int32_t rank, int32_t size, const void* handles);
 
 /* RoPE table: device fp32 [n_positions][128], row p = cos(p * f_0..f_63) then sin(p * f_0..f_63),
  * f_i = 1e6^(-2i/128).  Generalises the reference's single-position table
- * (qwen3mk/kernel.py:102-106).  Borrowed. */
+ * (qwen3mk/kernel.py:102-106).  Any address a float may have serves; the persistent kernel
+ * only takes a 16-byte aligned table, one sequence takes the launch chain otherwise.  Borrowed. */
 int q3_set_rope(q3_engine* e, const float* table, int32_t n_positions);
 
 /* Enqueue one decode step on `stream` (a cudaStream_t; NULL = default stream).  No host sync.

@@ -547,7 +547,7 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
         path = a->batch == 1 && persist_supports(e, a) ? Q3_F_PATH_PERSIST : Q3_F_PATH_LAYERED;
     if (path == Q3_F_PATH_PERSIST) {
         if (!persist_supports(e, a))
-            return fail(e, Q3_ERR_UNSUPPORTED, "q3_decode: the persistent kernel does not serve batch %d at length %d", a->batch, a->max_len);
+            return fail(e, Q3_ERR_UNSUPPORTED, "q3_decode: the persistent kernel does not serve batch %d at length %d with a RoPE table at %p", a->batch, a->max_len, (const void*)e->rope);
         return persist_decode(e, a, st);
     }
     if (path != Q3_F_PATH_LAYERED && path != Q3_F_PATH_FUSED) return fail(e, Q3_ERR_INVALID, "q3_decode: unknown path flag 0x%x", path);

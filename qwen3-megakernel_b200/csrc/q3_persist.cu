@@ -1485,6 +1485,7 @@ void persist_teardown(q3_engine* e) {
 bool persist_supports(const q3_engine* e, const q3_decode_args* a) {
     const PersistState* s = static_cast<const PersistState*>(e->p_state);
     if (s == nullptr || a->batch < 1) return false;
+    if (reinterpret_cast<uintptr_t>(e->rope) & 15) return false;   // the kernel reads the table 16 bytes at a time (a test of it there: 3 us a step)
     if (s->tp_size > 1) return a->batch == 1 && a->max_len <= mode_max_len(N_MODES - 2);   // one sequence, local attention
     return a->batch <= PERSIST_MAX_BATCH && a->max_len <= PERSIST_MAX_LEN;
 }

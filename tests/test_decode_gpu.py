@@ -415,6 +415,46 @@ def test_prompt_products_at_the_edges_of_their_tiles(oracle, small, T):
     assert torch.equal(again[0], kc) and torch.equal(again[1], vc) and torch.equal(again[2], last)
 
 
+@pytest.mark.parametrize("floats", [1, 2, 3])
+def test_rope_table_at_any_address(oracle, small, floats):
+    """A RoPE table that is not 16-byte aligned gives the results of one that is: prompts (matrix-vector kernels, k slices with either
+    attention, the pair kernel) and one sequence, which leaves the persistent kernel for the launch chain."""
+    from qwen3mk import Megakernel, prefill
+
+    shp, inp, w = small
+    dev = to_dev(inp)
+    wdev = {k: dev[k] for k in oracle.WEIGHT_NAMES}
+    g = torch.Generator().manual_seed(floats)
+    mk = Megakernel("cuda", layers=2, vocab=4096, max_tokens=1300, max_positions=1400)
+    chain = Megakernel("cuda", layers=2, vocab=4096, max_positions=1400, path="layered")
+    odd = torch.empty(mk.rope.numel() + 4, device="cuda")[floats:floats + mk.rope.numel()].view_as(mk.rope).copy_(mk.rope)
+    assert mk.rope.data_ptr() % 16 == 0 and odd.data_ptr() % 16 == 4 * floats
+    prompts = [torch.randint(0, 4096, (T,), generator=g).tolist() for T in (2, 37, 128, 1300)]
+
+    def all_of_it(table):
+        for e in (mk, chain):
+            assert e.lib.q3_set_rope(e.handle, table.data_ptr(), table.shape[0]) == 0
+        got = [prefill.prefill(wdev, ids, "cuda", engine=mk) for ids in prompts]
+        steps = [{k: v.clone() for k, v in e.step(dev).items()} for e in (mk, chain)]
+        mk.status()
+        chain.status()
+        return got, steps
+
+    want, got = all_of_it(mk.rope), all_of_it(odd)
+    persist = Megakernel("cuda", layers=2, vocab=4096, path="persist")
+    persist.step(dev)
+    assert persist.lib.q3_set_rope(persist.handle, odd.data_ptr(), odd.shape[0]) == 0
+    with pytest.raises(RuntimeError, match="persistent kernel"):
+        persist.step(dev)
+    for a, b in zip(want[0], got[0]):
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
+    for a, b in zip(want[1], got[1]):
+        assert int(a["next_token"]) == int(b["next_token"])
+        assert oracle.rel_l2(a["logits"], b["logits"]) <= 1e-5      # (two kernels within 1e-6 of fp64 each)
+        for n in ("k_write", "v_write"):
+            assert oracle.bf16_ulps(a[n], b[n]) <= GATE_KV_ULPS
+
+
 def test_error_paths():
     from qwen3mk import Megakernel, weights
     from qwen3mk.kernel import SeqTable
