@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
     __shared__ __align__(8) uint64_t k_full[AT_STAGES], v_full[AT_STAGES], k_empty[AT_STAGES], v_empty[AT_STAGES], q_full, s_full[2], p_full[2], o_full[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_flag;
-    __shared__ float s_max[2][2][128];              // per group: the tile's maximum of a row's two halves
+    __shared__ float s_max[2][2][2][128];           // per group and parity of its tiles: the tile's maximum of a row's two halves
     __shared__ float s_m[2][128], s_l[2][2][128];   // at the end: per group, a row's maximum and the two halves of its sum
 
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
@@ -274,9 +274,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
             const uint32_t ts = trow + (uint32_t)(grp * 128), to = trow + 256u + (uint32_t)(grp * 128 + part * 64);
             float m = -INFINITY, lsum = 0.f;
             bool ok = true;
+            // Two warps share their rows and wait for themselves, so one may give up where the other does not.  They stay together all the same: one that
+            // gives up leaves NaN as its maxima (a maximum is never one) and both leave the loop behind the same barrier.  Maxima of alternate tiles
+            // have places of their own: a warp that gave up on O is at the next barrier while the other still reads.
             for (int t = grp, i = 0; t < n_kt; t += 2, ++i) {
-                ok = at_wait_warp(&s_full[grp], i & 1, &abort_flag, a.status, 44);
-                if (!ok) break;
+                ok = ok && at_wait_warp(&s_full[grp], i & 1, &abort_flag, a.status, 44);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t r[2][32];
                 at_ld32(r[0], ts + (uint32_t)(part * 64));
@@ -293,18 +295,20 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                 float x[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
                 for (int j = 0; j < 32; ++j) { x[j & 1] = fmaxf(x[j & 1], __uint_as_float(r[0][j])); x[2 + (j & 1)] = fmaxf(x[2 + (j & 1)], __uint_as_float(r[1][j])); }
-                const float x0 = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
+                const float x0 = ok ? fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])) : NAN;
                 // the row's other half is a thread of the warp four further; behind the barrier both have read their part of S, too
-                s_max[grp][part][row] = x0;
+                s_max[grp][i & 1][part][row] = x0;
                 asm volatile("bar.sync %0, 64;" ::"r"(1 + grp * 4 + quad) : "memory");
-                const float top = fmaxf(x0, s_max[grp][part ^ 1][row]);   // finite: the first key of a tile is visible to every row
+                const float x1 = s_max[grp][i & 1][part ^ 1][row];
+                if (!ok || x1 != x1) { ok = false; break; }
+                const float top = fmaxf(x0, x1);   // finite: the first key of a tile is visible to every row
                 const bool raise = top > m + AT_LAG;
                 if (__any_sync(0xffffffffu, raise)) {
                     const float mn = raise ? top : m, c = at_ex2(m - mn);
                     m = mn;
                     if (i > 0) {           // O of the tiles so far, once the last of them has been added
                         ok = at_wait_warp(&o_full[grp], (i - 1) & 1, &abort_flag, a.status, 45);
-                        if (!ok) break;
+                        if (!ok) continue;      // (P of this tile is not handed over: its S is the last)
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         lsum *= c;
 #pragma unroll 1
