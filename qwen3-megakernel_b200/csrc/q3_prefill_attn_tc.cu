@@ -28,6 +28,7 @@
 
 #include "q3_engine.h"
 #include "q3_prompt.h"
+#include "q3_tc_ptx.cuh"
 
 namespace q3 {
 
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                                                                         const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                                                                         const PrefillAttnTcArgs a) {
     extern __shared__ __align__(1024) unsigned char at_raw[];
-    __shared__ __align__(8) uint64_t k_full[AT_STAGES], v_full[AT_STAGES], k_empty[AT_STAGES], v_empty[AT_STAGES], q_full, s_full[2], p_full[2], o_full[2];
+    __shared__ __align__(8) uint64_t k_full[AT_STAGES], v_full[AT_STAGES], k_empty[AT_STAGES], v_empty[AT_STAGES], q_full, s_full[2], p_full[2], o_full[2], drain_bar;
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_flag;
     __shared__ float s_max[2][2][2][128];           // per group and parity of its tiles: the tile's maximum of a row's two halves
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(at_smem(&p_full[b])) : "memory");   // the group's warps
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&q_full)) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&drain_bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         abort_flag = 0;
     }
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
 
     const int q0 = ((a.T + AT_QT - 1) / AT_QT - 1 - (int)blockIdx.x / KV_HEADS) * AT_QT;   // the query tiles with the most key tiles come first
     const int n_kt = (q0 + AT_QT - 1) / AT_KT + 1;          // key tiles up to and including the diagonal one
+    int armed_k = 0, armed_v = 0;                           // tiles whose K and V the producer has requested
     {
         if (warp == AT_SOFT / 32) {
             // ------------------------------------------------------------------ TMA producer
@@ -207,12 +210,14 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                     for (int b = 0; b < 2; ++b)        // the two 64-dim halves of the head
                         asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                                      ::"r"(at_smem(sk + b * AT_BOX)), "l"(&tm_k), "r"(g * HEAD_DIM + 64 * b), "r"(t * AT_KT), "r"(a.layer), "r"(at_smem(&k_full[s])) : "memory");
+                    armed_k = t + 1;
                     if (t >= AT_STAGES && !at_wait(&v_empty[s], ((t / AT_STAGES) - 1) & 1, &abort_flag, a.status, 47)) break;
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&v_full[s])), "r"(AT_KV_BYTES) : "memory");
 #pragma unroll
                     for (int b = 0; b < 2; ++b)
                         asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                                      ::"r"(at_smem(sv + b * AT_BOX)), "l"(&tm_v), "r"(g * HEAD_DIM + 64 * b), "r"(t * AT_KT), "r"(a.layer), "r"(at_smem(&v_full[s])) : "memory");
+                    armed_v = t + 1;
                 }
             }
         } else if (warp == AT_SOFT / 32 + 1) {
@@ -373,7 +378,19 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    // After a wait gave up (nobody waits any more, so the flag is what it will be): the loads land and the products end before this block's memory and
+    // columns are somebody else's.
+    if (warp == AT_SOFT / 32 && abort_flag && elect_one()) {
+        tc_drain(&q_full, 0);
+        for (int t = max(0, armed_k - AT_STAGES); t < armed_k; ++t) tc_drain(&k_full[t % AT_STAGES], (t / AT_STAGES) & 1);
+        for (int t = max(0, armed_v - AT_STAGES); t < armed_v; ++t) tc_drain(&v_full[t % AT_STAGES], (t / AT_STAGES) & 1);
+    }
     if (warp == AT_SOFT / 32 + 1) {
+        if (abort_flag && elect_one()) {
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(at_smem(&drain_bar)) : "memory");
+            tc_drain(&drain_bar, 0);
+        }
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }

@@ -228,3 +228,16 @@ def test_a_wait_by_one_lane_orders_memory_for_its_warp():
     for name, helper in (("q3_tc_ptx.cuh", "tc_wait_warp"), ("q3_prefill_attn_tc.cu", "at_wait_warp")):
         body = re.search(rf"bool {helper}\([^{{]*\{{(.*?)\n\}}", (csrc / name).read_text(), re.S).group(1)
         assert "one_lane_waits(" in body and "__shfl_sync" not in body, name
+
+
+def test_what_is_under_way_is_drained_after_the_last_wait():
+    """A kernel may not give its tensor memory back while products run, nor leave while loads are on their way.  After a wait gave up it drains them, and
+    looks whether one did only where none is left that could: behind the block's last barrier."""
+    for name, kernels in (("q3_prefill_attn_tc.cu", 1),):
+        code = re.sub(r"//[^\n]*", "", (ROOT / "qwen3-megakernel_b200" / "csrc" / name).read_text())
+        ends = [m.start() for m in re.finditer(r"tcgen05\.dealloc", code)]
+        assert len(ends) == kernels, name
+        for end in ends:
+            barrier = max(code.rfind("__syncthreads();", 0, end), code.rfind("bar.sync", 0, end))
+            tail = code[barrier:end]
+            assert "abort_flag" in tail and "tc_drain(" in tail, f"{name}:{code.count(chr(10), 0, end) + 1}"
