@@ -102,6 +102,11 @@ __device__ __forceinline__ float at_ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ float at_max_nan(float a, float b) {   // NaN if either is
+    float y;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+    return y;
+}
 __device__ __forceinline__ uint32_t at_pack_bf16(float lo, float hi) {
     uint32_t d;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
@@ -304,11 +309,10 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                 // the row's other half is a thread of the warp four further; behind the barrier both have read their part of S, too
                 s_max[grp][i & 1][part][row] = x0;
                 asm volatile("bar.sync %0, 64;" ::"r"(1 + grp * 4 + quad) : "memory");
-                const float x1 = s_max[grp][i & 1][part ^ 1][row];
-                if (!ok || x1 != x1) { ok = false; break; }
-                const float top = fmaxf(x0, x1);   // finite: the first key of a tile is visible to every row
-                const bool raise = top > m + AT_LAG;
+                const float top = at_max_nan(x0, s_max[grp][i & 1][part ^ 1][row]);   // finite: the first key of a tile is visible to every row
+                const bool raise = !(top <= m + AT_LAG);
                 if (__any_sync(0xffffffffu, raise)) {
+                    if (top != top) { ok = false; break; }      // (here, where few tiles come: looking in every tile cost 0.3 us a launch)
                     const float mn = raise ? top : m, c = at_ex2(m - mn);
                     m = mn;
                     if (i > 0) {           // O of the tiles so far, once the last of them has been added
