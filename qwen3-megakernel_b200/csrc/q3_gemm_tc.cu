@@ -411,8 +411,9 @@ __global__ void __launch_bounds__(LmShape<BN>::THREADS, 1) lm_head_kernel(const 
                                                                           const LmHeadParams p) {
     using S = LmShape<BN>;
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[S::STAGES], empty_bar[S::STAGES], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t full_bar[S::STAGES], empty_bar[S::STAGES], acc_full[2], acc_empty[2], drain_bar;
     __shared__ uint32_t tmem_base_s;
+    __shared__ int armed_s;
     __shared__ volatile int abort_flag;
     __shared__ float s_scale[BN];
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -427,6 +428,7 @@ __global__ void __launch_bounds__(LmShape<BN>::THREADS, 1) lm_head_kernel(const 
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&acc_full[b])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(&acc_empty[b])), "r"(S::EPI_WARPS) : "memory");
         }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&drain_bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         abort_flag = 0;
     }
@@ -464,8 +466,7 @@ __global__ void __launch_bounds__(LmShape<BN>::THREADS, 1) lm_head_kernel(const 
                     }
                     tc_load_planes(st0 + s * S::STAGE + S::A_BYTES, &tm_x, kb * TC_BK, 0, &full_bar[s]);
                 }
-            if (abort_flag)                                  // (what is under way lands before this memory is somebody else's)
-                for (int k = max(0, armed - S::STAGES); k < armed; ++k) tc_drain(&full_bar[k % S::STAGES], (k / S::STAGES) & 1);
+            armed_s = armed;
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -492,9 +493,7 @@ __global__ void __launch_bounds__(LmShape<BN>::THREADS, 1) lm_head_kernel(const 
                                      ::"r"(tmem_base + (uint32_t)acc * S::ACC), "l"(da0 + ds + 2 * k), "l"(db0 + ds + 2 * k), "r"(idesc), "r"((uint32_t)(kb | k)), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&empty_bar[s])) : "memory");
                 }
-                // (also after a wait that gave up: whoever waits for the accumulator sees the flag, and the products end before the columns go)
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&acc_full[acc])) : "memory");
-                if (!ok) tc_drain(&acc_full[acc], (li >> 1) & 1);
+                if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&acc_full[acc])) : "memory");
             }
         }
         __syncwarp();
@@ -529,6 +528,16 @@ __global__ void __launch_bounds__(LmShape<BN>::THREADS, 1) lm_head_kernel(const 
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
     __syncthreads();
+    // After a wait gave up (nobody waits any more, so the flag is what it will be): the loads land and the products end before the columns and this memory go.
+    if (abort_flag && warp < 2 && elect_one()) {
+        if (warp == 0) {
+            for (int k = max(0, armed_s - S::STAGES); k < armed_s; ++k) tc_drain(&full_bar[k % S::STAGES], (k / S::STAGES) & 1);
+        } else {
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&drain_bar)) : "memory");
+            tc_drain(&drain_bar, 0);
+        }
+    }
+    __syncwarp();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * S::ACC) : "memory");

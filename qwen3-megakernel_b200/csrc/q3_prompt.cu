@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(PS_THREADS, 2) prompt_split_kernel(const __gri
 // 256 bytes.
 //
 // A wait that gives up ends the loops of its block; the peer's waits give up too.  The loads of both blocks are counted on the first one's
-// barriers: it drains them, and the products, before the pair's last barrier.
+// barriers: it drains them, and the products, between its own last barrier and the pair's.
 // ------------------------------------------------------------------------------------------------------------------------------
 constexpr int PP_EPI_WARPS = 8;
 constexpr int PP_THREADS = 64 + 32 * PP_EPI_WARPS;   // warp 0: TMA, warp 1: MMA and TMEM, warps 2..9: epilogue (two per TMEM quadrant, half the columns each)
@@ -454,6 +454,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prompt_pair_kernel(const __grid
     extern __shared__ __align__(1024) unsigned char pp_raw[];
     __shared__ __align__(8) uint64_t full_bar[PP_MAX_STAGES], empty_bar[PP_MAX_STAGES], acc_full[2], acc_empty[2], drain_bar;
     __shared__ uint32_t tmem_base_s;
+    __shared__ int armed_s;
     __shared__ volatile int abort_flag;
     unsigned char* const base = pp_raw;
 
@@ -502,7 +503,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prompt_pair_kernel(const __grid
                 if (rank == 0) pr_expect(&full_bar[s], 2 * S::STAGE);                            // both blocks' loads
                 pp_load_box(st + S::A_BYTES, tm_w, kb * TC_BK, r0, bar);
             };
-            int armed = 0;
+            int armed = 0;                                   // k blocks whose loads have been requested
             const int ahead = min(p.kb_total, STAGES);       // the first ring's weights before the wait
             decode(pair);
             for (int kb = 0; kb < ahead; ++kb, bar += 8, st += S::STAGE) weights(kb, kb);
@@ -526,8 +527,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prompt_pair_kernel(const __grid
                     pp_load_box(st, &tm_x, kb * TC_BK, m0, bar);
                 }
             }
-            if (abort_flag && rank == 0)
-                for (int k = max(0, armed - STAGES); k < armed; ++k) tc_drain(&full_bar[k % STAGES], (k / STAGES) & 1);
+            armed_s = armed;
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -557,10 +557,6 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prompt_pair_kernel(const __grid
                     pp_commit(&empty_bar[s]);
                 }
                 if (ok) pp_commit(&acc_full[acc]);
-            }
-            if (abort_flag) {      // the products that were issued end before the columns go
-                asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&drain_bar)) : "memory");
-                tc_drain(&drain_bar, 0);
             }
         }
         __syncwarp();
@@ -704,6 +700,17 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prompt_pair_kernel(const __grid
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    // After a wait gave up (nobody of this block waits any more, so the flag is what it will be): the loads land and the products end before the pair's
+    // columns and memory go.
+    if (rank == 0 && abort_flag && warp < 2 && elect_one()) {
+        if (warp == 0) {
+            for (int k = max(0, armed_s - STAGES); k < armed_s; ++k) tc_drain(&full_bar[k % STAGES], (k / STAGES) & 1);
+        } else {
+            asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&drain_bar)) : "memory");
+            tc_drain(&drain_bar, 0);
+        }
+    }
+    __syncwarp();
     pr_cluster_arrive();
     pr_cluster_wait();            // nothing of the pair is under way to this block any more
     if (warp == 1) {

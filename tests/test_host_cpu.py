@@ -233,10 +233,11 @@ def test_a_wait_by_one_lane_orders_memory_for_its_warp():
 def test_what_is_under_way_is_drained_after_the_last_wait():
     """A kernel may not give its tensor memory back while products run, nor leave while loads are on their way.  After a wait gave up it drains them, and
     looks whether one did only where none is left that could: behind the block's last barrier."""
-    for name, kernels in (("q3_prefill_attn_tc.cu", 1),):
+    for name, kernels in (("q3_prefill_attn_tc.cu", ["prefill_attn_tc_kernel"]), ("q3_prompt.cu", ["prompt_split_kernel", "prompt_pair_kernel"]),
+                          ("q3_gemm_tc.cu", ["lm_head_kernel"])):
         code = re.sub(r"//[^\n]*", "", (ROOT / "qwen3-megakernel_b200" / "csrc" / name).read_text())
-        ends = [m.start() for m in re.finditer(r"tcgen05\.dealloc", code)]
-        assert len(ends) == kernels, name
+        begins = [re.search(rf"__global__ void [^;{{]*\b{k}\(", code).end() for k in kernels]
+        ends = [code.index("tcgen05.dealloc", b) for b in begins]
         for end in ends:
             barrier = max(code.rfind("__syncthreads();", 0, end), code.rfind("bar.sync", 0, end))
             tail = code[barrier:end]
