@@ -99,13 +99,6 @@ __device__ __forceinline__ void ld_row8(uint32_t& a, uint32_t& b, const void* pt
                  : "=&r"(a), "=&r"(b) : "l"(ptr), "r"((int)live));
 }
 
-// Four entries of a RoPE table.  The caller's table needs no more than a float's alignment: one load where it has 16 bytes', four where not
-// (no slower for prompts of 128, 777 and 2048 tokens).  It is nobody's output, so the read-only path may hold it past the stores around it.
-__device__ __forceinline__ float4 ld_rope4(const float* p) {
-    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) return __ldg(reinterpret_cast<const float4*>(p));
-    return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
-}
-
 // One lane of a converged warp.  A branch on elect.sync tells the compiler that exactly one thread follows it; behind
 // `lane == 0` it has to make every tcgen05 and TMA instruction's descriptors warp-uniform at run time.
 __device__ __forceinline__ bool elect_one() {

@@ -58,11 +58,11 @@ __device__ __forceinline__ float pr_scale(const PromptParams& p, int t) {
     return rsqrtf(ss / (float)HIDDEN + EPS);
 }
 
-// RoPE's cosines and sines of dims d .. d + 3 of position t
+// RoPE's cosines and sines of dims d .. d + 3 of position t.  The table is nobody's output: read past the stores around it.
 struct PrRope { float4 c, s; };
 __device__ __forceinline__ PrRope pr_rope(const PromptParams& p, int t, int d) {
     const float* row = p.rope + (size_t)t * HEAD_DIM + d;
-    return PrRope{ld_rope4(row), ld_rope4(row + 64)};
+    return PrRope{__ldg(reinterpret_cast<const float4*>(row)), __ldg(reinterpret_cast<const float4*>(row + 64))};
 }
 // One half-row step of a finished q, k or v head: dims d .. d + 3 (lo) and 64 + d .. 64 + d + 3 (hi) of `col0`'s head (a multiple of 128
 // in q | k | v) of token t.  lo and hi are normalised except for the head's gain (v: final).

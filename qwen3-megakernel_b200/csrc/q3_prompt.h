@@ -26,7 +26,7 @@ struct PromptGemmCall {
     float* qkv;                    // [T][4096] fp32 q, k, v rows (read by the split attention of few tokens)
     bf16_raw *kc, *vc;             // this layer's cache rows [T..][1024]
     const bf16_raw *qn, *kn;       // [128] head gains of this layer
-    const float* rope;             // [positions][128]
+    const float* rope;             // [positions][128], 16-byte aligned
     // PR_RESID
     float* x;                      // [T][1024], updated in place
     bf16_raw* xn;                  // [T][1024] plane of x * gain
