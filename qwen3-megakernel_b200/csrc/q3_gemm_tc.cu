@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(LmShape<BN>::THREADS, 1) lm_head_kernel(const 
     }
     __syncthreads();
     // After a wait gave up (nobody waits any more, so the flag is what it will be): the loads land and the products end before the columns and this memory go.
-    if (abort_flag && warp < 2 && elect_one()) {
+    if (warp < 2 && abort_flag && elect_one()) {
         if (warp == 0) {
             for (int k = max(0, armed_s - S::STAGES); k < armed_s; ++k) tc_drain(&full_bar[k % S::STAGES], (k / S::STAGES) & 1);
         } else {

@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prompt_pair_kernel(const __grid
     __syncthreads();
     // After a wait gave up (nobody of this block waits any more, so the flag is what it will be): the loads land and the products end before the pair's
     // columns and memory go.
-    if (rank == 0 && abort_flag && warp < 2 && elect_one()) {
+    if (warp < 2 && rank == 0 && abort_flag && elect_one()) {
         if (warp == 0) {
             for (int k = max(0, armed_s - STAGES); k < armed_s; ++k) tc_drain(&full_bar[k % STAGES], (k / STAGES) & 1);
         } else {
