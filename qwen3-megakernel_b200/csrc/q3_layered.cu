@@ -493,14 +493,7 @@ cudaError_t launch_argmax_rows(const float* logits, int vocab, long long* next_t
 template <int K, int EPI, int BT>
 static cudaError_t launch_gemv_bt(const GemvArgs& a, int grid_x, cudaStream_t st) {
     constexpr size_t smem = (size_t)BT * K * sizeof(float);
-    if constexpr (smem > 48 * 1024) {
-        static bool attr_done = false;  // > 48 KB needs the opt-in once per function
-        if (!attr_done) {
-            cudaError_t e = cudaFuncSetAttribute(gemv_kernel<K, EPI, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-            attr_done = true;
-        }
-    }
+    static_assert(smem <= 40 * 1024, "with the kernel's own arrays below the 48 KB that a launch may ask for without an opt-in");
     gemv_kernel<K, EPI, BT><<<dim3(grid_x, (a.batch + BT - 1) / BT), 256, smem, st>>>(a);
     return cudaGetLastError();
 }
@@ -511,7 +504,9 @@ static cudaError_t launch_gemv_k(const GemvArgs& a, int grid_x, cudaStream_t st)
     if (a.batch == 1) return launch_gemv_bt<K, EPI, 1>(a, grid_x, st);
     if (a.batch == 2) return launch_gemv_bt<K, EPI, 2>(a, grid_x, st);
     if (a.batch == 3) return launch_gemv_bt<K, EPI, 3>(a, grid_x, st);
-    return launch_gemv_bt<K, EPI, 4>(a, grid_x, st);
+    // (more than three take the tensor cores everywhere but in the LM head of a vocabulary that is no multiple of 128)
+    if constexpr (EPI == EPI_LOGITS) return launch_gemv_bt<K, EPI, 4>(a, grid_x, st);
+    else return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_gemv(int K, int epi, const GemvArgs& a, int grid_x, cudaStream_t st) {
