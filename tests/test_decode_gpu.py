@@ -368,8 +368,8 @@ def test_rebound_launches_are_stable(oracle, small, path):
 
 @pytest.mark.parametrize("T", [5, 37, 64, 200, 700, 1600])
 def test_prefill_matches_oracle(oracle, small, T):
-    """T < 9: matrix-vector kernels; T >= 9: tcgen05 GEMMs; T >= 64: the tiled causal attention kernel; 1600: the persistent
-    GEMM (q/k/v, and gate + up with SiLU in the epilogue) with a last token tile that is partly padding."""
+    """Products cut in K (5, 37: with the split attention; 64, 200: with the tiled causal one), whole tiles beside the pair kernel (700), the pair
+    kernel for q/k/v, too, with a last token tile that is partly padding (1600)."""
     from qwen3mk import prefill
 
     shp, inp, w = small
@@ -393,17 +393,18 @@ def test_prefill_matches_oracle(oracle, small, T):
         print(f"prefill T={T}: arg-max {top} against {want} on a near-tie (margin {margin:.3e})")
 
 
-@pytest.mark.parametrize("T", [4, 63, 65, 128, 129, 256, 257, 385, 512, 513, 1025])
+@pytest.mark.parametrize("T", [4, 63, 65, 128, 129, 256, 257, 385, 512, 513, 640, 769, 897, 1025, 1152, 1153, 1281, 2304, 2305, 2700])
 def test_prompt_products_at_the_edges_of_their_tiles(oracle, small, T):
-    """Prompt lengths around the tiles of the prompt's products (128 tokens a block, 256 a pair, every cut of K and the pair kernel) on an
-    engine with more room than the prompt needs, twice: no atomics, so the same bits."""
+    """Prompt lengths around the tiles of the prompt's products (128 tokens a block, 256 a pair) and around every change of their form on 148 SMs: the cuts
+    of K, whole tiles, the pair kernel (gate/up from 513 tokens on, q/k/v from 1153, Wo and down from 2305).  On an engine with more
+    room than the prompt needs, twice: no atomics, so the same bits."""
     from qwen3mk import Megakernel, prefill
 
     shp, inp, w = small
     g = torch.Generator().manual_seed(T)
     ids = torch.randint(0, 4096, (T,), generator=g).tolist()
     wdev = to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES})
-    mk = Megakernel("cuda", layers=2, vocab=4096, max_tokens=1100, max_positions=1200)
+    mk = Megakernel("cuda", layers=2, vocab=4096, max_tokens=max(1100, T + 75), max_positions=max(1200, T + 80))
     kc, vc, last = prefill.prefill(wdev, ids, "cuda", capacity=T + 3, engine=mk)
     mk.status()
     rk, rv, rlast = oracle.prefill(w, ids)
