@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
                 asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                              ::"r"(tc_smem(st)), "l"(tm_w), "r"((kb_begin + kb) * TC_BK), "r"(m0), "r"(tc_smem(&full_bar[kb])) : "memory");
             }
+            int armed = ahead;                    // k blocks whose loads have been requested
             pdl_wait();
             // (slot and phase are counted along: `stages` is no constant, and a division is longer than the rest of the loop)
             for (int kb = 0, s = 0, turn = 0; kb < nkb; ++kb, ++s) {
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
                 if (turn > 0 && !tc_wait(&empty_bar[s], (turn - 1) & 1, &abort_flag, p.status, 30)) break;
                 unsigned char* st = base + (size_t)s * stage_bytes;
                 if (kb >= ahead) {
+                    armed = kb + 1;
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(&full_bar[s])), "r"(stage_bytes) : "memory");
                     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                                  ::"r"(tc_smem(st)), "l"(tm_w), "r"((kb_begin + kb) * TC_BK), "r"(m0), "r"(tc_smem(&full_bar[s])) : "memory");
@@ -116,6 +118,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
                                  ::"r"(tc_smem(st + a_bytes + sp * b_bytes)), "l"(&tm_x), "r"((kb_begin + kb) * TC_BK), "r"(sp * p.plane_rows + n0),
                                    "r"(tc_smem(&full_bar[s])) : "memory");
             }
+            // Neither this thread nor the issuing one ends before the products have: in the shadow of the epilogue (a look behind the block's last barrier
+            // cost 0.08 us a launch).  If a wait of theirs gave up, some of the last loads have no product: they land before this memory is somebody else's.
+            tc_drain(&acc_bar, 0);
+            if (abort_flag)
+                for (int k = max(0, armed - stages); k < armed; ++k) tc_drain(&full_bar[k % stages], (k / stages) & 1);
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
@@ -145,6 +152,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&empty_bar[s])) : "memory");
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&acc_bar)) : "memory");
+            tc_drain(&acc_bar, 0);
         }
     } else {
         // ------------------------------------------------------------------ epilogue: TMEM -> registers -> global
@@ -238,8 +246,9 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
     constexpr int BN = TP_BN;                       // tokens per item
     constexpr int ACC = BN;                         // TMEM columns of one accumulator buffer
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[8], empty_bar[8], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t full_bar[8], empty_bar[8], acc_full[2], acc_empty[2], drain_bar;
     __shared__ uint32_t tmem_base_s;
+    __shared__ int armed_s;
     __shared__ volatile int abort_flag;
 
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -257,6 +266,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&acc_full[b])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 256;" ::"r"(tc_smem(&acc_empty[b])) : "memory");
         }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&drain_bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         abort_flag = 0;
     }
@@ -279,13 +289,14 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
         // ------------------------------------------------------------------ TMA producer
         if (elect_one()) {
             pdl_wait();
-            int s = 0, turn = 0;
+            int s = 0, turn = 0, armed = 0;      // armed: k blocks whose loads have been requested
             for (int it = blockIdx.x; it < w.n_items && !abort_flag; it += gridDim.x) {
                 const Item r = decode(it);
                 for (int kb = 0; kb < nkb; ++kb, ++s) {
                     if (s == stages) { s = 0; ++turn; }
                     if (turn > 0 && !tc_wait(&empty_bar[s], (turn - 1) & 1, &abort_flag, p.status, 36)) break;
                     unsigned char* st = base + (size_t)s * stage_bytes;
+                    ++armed;
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(&full_bar[s])), "r"(stage_bytes) : "memory");
                     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                                  ::"r"(tc_smem(st)), "l"(&tm_w), "r"(kb * TC_BK), "r"(r.m0), "r"(tc_smem(&full_bar[s])) : "memory");
@@ -295,6 +306,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
                                        "r"(tc_smem(&full_bar[s])) : "memory");
                 }
             }
+            armed_s = armed;
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
@@ -374,6 +386,16 @@ __global__ void __launch_bounds__(TP_THREADS, 1) gemm_tc_persist_kernel(const __
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
     __syncthreads();
+    // After a wait gave up (nobody waits any more, so the flag is what it will be): the loads land and the products end before the columns and this memory go.
+    if (warp < 2 && abort_flag && elect_one()) {
+        if (warp == 0) {
+            for (int k = max(0, armed_s - stages); k < armed_s; ++k) tc_drain(&full_bar[k % stages], (k / stages) & 1);
+        } else {
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&drain_bar)) : "memory");
+            tc_drain(&drain_bar, 0);
+        }
+    }
+    __syncwarp();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * ACC)) : "memory");

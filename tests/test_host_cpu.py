@@ -234,7 +234,7 @@ def test_what_is_under_way_is_drained_after_the_last_wait():
     """A kernel may not give its tensor memory back while products run, nor leave while loads are on their way.  After a wait gave up it drains them, and
     looks whether one did only where none is left that could: behind the block's last barrier."""
     for name, kernels in (("q3_prefill_attn_tc.cu", ["prefill_attn_tc_kernel"]), ("q3_prompt.cu", ["prompt_split_kernel", "prompt_pair_kernel"]),
-                          ("q3_gemm_tc.cu", ["lm_head_kernel"])):
+                          ("q3_gemm_tc.cu", ["gemm_tc_persist_kernel", "lm_head_kernel"])):
         code = re.sub(r"//[^\n]*", "", (ROOT / "qwen3-megakernel_b200" / "csrc" / name).read_text())
         begins = [re.search(rf"__global__ void [^;{{]*\b{k}\(", code).end() for k in kernels]
         ends = [code.index("tcgen05.dealloc", b) for b in begins]
@@ -242,3 +242,10 @@ def test_what_is_under_way_is_drained_after_the_last_wait():
             barrier = max(code.rfind("__syncthreads();", 0, end), code.rfind("bar.sync", 0, end))
             tail = code[barrier:end]
             assert "abort_flag" in tail and "tc_drain(" in tail, f"{name}:{code.count(chr(10), 0, end) + 1}"
+    # the one-tile kernel instead keeps its two threads until the products have ended, which both see at the barrier that the last commit arrives at
+    code = (ROOT / "qwen3-megakernel_b200" / "csrc" / "q3_gemm_tc.cu").read_text()
+    body = code[code.index(" gemm_tc_kernel("):]
+    producer, rest = body[body.index("if (warp == 0) {"):].split("} else if (warp == 1) {", 1)
+    issuer = rest[:rest.index("} else {")]
+    assert re.search(r"tc_drain\(&acc_bar, 0\);\s*if \(abort_flag\)\s*for [^;]*;[^;]*;[^;]*tc_drain\(&full_bar", producer)
+    assert re.search(r"tc_smem\(&acc_bar\)\) : \"memory\"\);\s*tc_drain\(&acc_bar, 0\);", issuer)
