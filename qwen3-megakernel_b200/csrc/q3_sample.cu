@@ -66,7 +66,7 @@ struct SampleShared {
     unsigned hist[SAMPLE_BINS];
     unsigned cand[SAMPLE_CAND];             // keys
     int candi[SAMPLE_CAND];                 // and where they are
-    float weight[SAMPLE_KEYS * SAMPLE_THREADS];   // weights of all blocks' candidates, the lists one after the other (before that, the block's own list unordered)
+    __align__(16) float weight[SAMPLE_KEYS * SAMPLE_THREADS];   // weights of all blocks' candidates, the lists one after the other (before that, the block's own list unordered)
     unsigned sel, need, cand_n, cmin;
 };
 
@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
         };
         if (top_k <= n_thr) {
             unsigned* const raw = reinterpret_cast<unsigned*>(sh.weight);    // the candidates as they come: keys, then indices
+            raw[SAMPLE_CAND + tid] = 0xffffffffu;
             if (any) atomicAdd(&sh.hist[bin(mine)], 1u);
             __syncthreads();
             find_bin(sh, sh.hist[2 * tid], sh.hist[2 * tid + 1], (unsigned)top_k, false);
@@ -221,8 +222,11 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
             if (n <= SAMPLE_CAND && tid < n) {
                 const unsigned at = raw[SAMPLE_CAND + tid];
                 int place = 0;
-#pragma unroll 8
-                for (int j = 0; j < n; ++j) place += raw[SAMPLE_CAND + j] < at;
+#pragma unroll 4
+                for (int j = 0; j < n; j += 4) {
+                    const uint4 o = *reinterpret_cast<const uint4*>(raw + SAMPLE_CAND + j);
+                    place += (o.x < at) + (o.y < at) + (o.z < at) + (o.w < at);
+                }
                 sh.cand[place] = raw[tid]; sh.candi[place] = (int)at;
             }
             n_cand = n <= SAMPLE_CAND ? n : -1;
@@ -262,8 +266,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
         peer->bmax[rank] = bmax; peer->ncand[rank] = n_cand; peer->bsum[rank] = bsum;
     }
     cluster.sync();
-    float vmax = sh.bmax[0];
-    for (int r = 1; r < C; ++r) vmax = fmaxf(vmax, sh.bmax[r]);
+    const float vmax = warp_max(lane < C ? sh.bmax[lane] : -INFINITY);
     // the row's lowest index that holds the maximum (every block of the cluster takes part)
     auto write_argmax = [&]() {
         __syncthreads();
@@ -289,25 +292,37 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     float least = -FLT_MAX, base = 0.f, next = 0.f, total = 0.f, scale = 1.f;      // the block's bracket and the total; what its own sums are scaled by
     if (select) {
         // ---- 2b. threshold: the k-th largest key ----
-        bool fits = true;
-        int count = 0, mine0 = 0, list0 = 0;        // candidates of all blocks, of those before this one, and before the one that this warp sums below
-        float odd = 0.f;
-        for (int r = 0; r < C; ++r) {
-            if (r == rank) mine0 = count;
-            if (r == warp) list0 = count;
-            fits = fits && sh.ncand[r] >= 0; count += max(sh.ncand[r], 0); odd += sh.bsum[r];
+        auto for_blocks = [&](auto&& f) {           // (without a loop where it would be the longest: one row, k = 50, 12.4 us with it, 12.2 without)
+            if (C == SAMPLE_MAX_CLUSTER) {
+#pragma unroll
+                for (int r = 0; r < SAMPLE_MAX_CLUSTER; ++r) f(r);
+            } else {
+                for (int r = 0; r < C; ++r) f(r);
+            }
+        };
+        // a lane per block: how many candidates it has, where its list begins in the union and where that ends
+        const int listed = lane < C ? sh.ncand[lane] : 0;
+        int list_end = listed;
+#pragma unroll
+        for (int o = 1; o < SAMPLE_MAX_CLUSTER; o <<= 1) {
+            const int p = __shfl_up_sync(0xffffffffu, list_end, o);
+            if (lane >= o) list_end += p;
         }
-        fits = fits && count <= SAMPLE_KEYS * SAMPLE_THREADS;
+        const int count = __shfl_sync(0xffffffffu, list_end, SAMPLE_MAX_CLUSTER - 1), mine0 = __shfl_sync(0xffffffffu, list_end - listed, rank);
+        const bool fits = __all_sync(0xffffffffu, listed >= 0) && count <= SAMPLE_KEYS * SAMPLE_THREADS;
+        const float odd = __any_sync(0xffffffffu, lane < C && sh.bsum[lane] != 0.f) ? NAN : 0.f;      // (a block's is 0 or NaN)
         if (fits) {
             // this thread's share of the union: the blocks' lists one after the other (0 is below every key of a number)
             unsigned key[SAMPLE_KEYS];
 #pragma unroll
             for (int q = 0; q < SAMPLE_KEYS; ++q) {
-                int e = q * SAMPLE_THREADS + tid, r = 0;
+                const int e = q * SAMPLE_THREADS + tid;
                 key[q] = 0u;
-                if (e < count) {
-                    while (e >= sh.ncand[r]) e -= sh.ncand[r++];
-                    key[q] = cluster.map_shared_rank(&sh, r)->cand[e];
+                if (q * SAMPLE_THREADS < count) {
+                    int r = 0;
+                    for_blocks([&](int k) { r += e >= __shfl_sync(0xffffffffu, list_end, k); });
+                    const int at = e - __shfl_sync(0xffffffffu, list_end - listed, r & (SAMPLE_MAX_CLUSTER - 1));
+                    if (e < count) key[q] = cluster.map_shared_rank(&sh, r)->cand[at];
                 }
             }
             // Every block has read every list when it may leave; this one's own lists stay until then.
@@ -347,17 +362,19 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
             if (tid == 0) { sh.need = 0xffffffffu; sh.cand_n = 0u; }
             __syncthreads();
             if (warp < C) {
+                const int end = __shfl_sync(0xffffffffu, list_end, warp);
                 float ws = 0.f;
-                for (int j = lane; j < sh.ncand[warp]; j += 32) ws += sh.weight[list0 + j];
+                for (int j = __shfl_sync(0xffffffffu, list_end - listed, warp) + lane; j < end; j += 32) ws += sh.weight[j];
                 ws = warp_sum(ws);
                 if (lane == 0) sh.wf[warp] = ws;
             }
             __syncthreads();
-            for (int r = 0; r < C; ++r) {
+            const float list_sum = lane < C ? sh.wf[lane] : 0.f;
+            for_blocks([&](int r) {
                 if (r == rank) base = total;
-                total += sh.wf[r];
+                total += __shfl_sync(0xffffffffu, list_sum, r);
                 if (r == rank) next = total;
-            }
+            });
             total += odd;
             // Weights that are not numbers (infinite logits, or a NaN in the row), or a u outside [0, 1): no draw, the arg-max.
             if (!(total > 0.f && total < INFINITY && u >= 0.f && u < 1.f)) { cluster.barrier_wait(); write_argmax(); return; }
@@ -366,14 +383,20 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
             if (base <= target && target < next) {
                 // the first of this block's kept words, in the order of their indices, whose inclusive prefix sum exceeds the target.  (next > base:
                 // one of them has a weight)
-                const float* const w = sh.weight + mine0;
-                const float own = tid < n_cand ? w[tid] : 0.f;
+                const float own = tid < n_cand ? sh.weight[mine0 + tid] : 0.f;
+                float p = own;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const float v = __shfl_up_sync(0xffffffffu, p, o);
+                    if (lane >= o) p += v;
+                }
+                if (lane == 31) sh.wg[warp] = p;
+                __syncthreads();
+                if (warp > 0 && 32 * warp < n_cand) p += warp_sum(lane < warp ? sh.wg[lane] : 0.f);
                 if (own > 0.f) {
-                    const int at = sh.candi[tid];
-                    float p = 0.f;
-                    for (int j = 0; j <= tid; ++j) p += w[j];
-                    if (base + p > target) atomicMin(&sh.need, (unsigned)at);
-                    atomicMax(&sh.cand_n, (unsigned)at);
+                    const unsigned at = (unsigned)sh.candi[tid];
+                    if (base + p > target) atomicMin(&sh.need, at);
+                    atomicMax(&sh.cand_n, at);
                 }
                 __syncthreads();
                 // rounding may leave the target a hair beyond the block's own sum: then its last word with a weight
