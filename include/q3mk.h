@@ -179,8 +179,9 @@ int q3_noalloc_status(void* stream, uint32_t* words, int32_t n);
  * [n_tok, n_rows] (resid may be NULL or alias out).  x is split into `nsplit` bf16 planes (1: rounded to
  * bf16, 3: exact to fp32) in the caller's `planes` buffer of at least nsplit * round_up(n_tok, tile) * K * 2
  * bytes, tile = 32 / 64 / 128 for n_tok <= 32 / <= 64 / more.  This is the dense product the reference's
- * prefill writes as `xn @ w.T` (qwen3mk/prefill.py:61-80); the engine uses it for prefill and for decode
- * batches too large for the persistent kernel.  Allocates nothing. */
+ * prefill writes as `xn @ w.T` (qwen3mk/prefill.py:61-80), for callers with products of their own.  The engine uses the same
+ * kernel for decode batches of more than 64 sequences; its prompts run on products that finish a layer's rows
+ * themselves.  One plane and at least 256 tokens take a persistent kernel that nothing else uses.  Allocates nothing. */
 int q3_linear_tc(const void* w, const float* x, float* out, const float* resid, int32_t n_rows, int32_t n_tok, int32_t K,
                  int32_t nsplit, void* planes, int64_t planes_bytes, void* stream);
 

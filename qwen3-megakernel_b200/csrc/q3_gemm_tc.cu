@@ -597,10 +597,10 @@ bool tc_make_map(CUtensorMap* m, const void* ptr, uint64_t planes, uint64_t rows
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Few output tiles (decode batches, short prompts) cannot fill the GPU: slice K so that about `fill` CTAs per SM stream
-// weights, at least two k blocks per slice.  Measured with fill = 1 / 2 / 3: prefill of 2048 tokens 13.9 / 11.2 / 10.9 ms
-// (the Wo and down launches have 128 tiles of long K: one wave of long serial CTAs unless K is cut), batch-8 decode step
-// 1322 / 1250 / 1249 us, batch 64 3017 / 3031 / 3000 us; a prompt of 128 tokens (one 128-token tile) is the exception:
+// Few output tiles cannot fill the GPU: slice K so that about `fill` CTAs per SM stream weights, at least two k blocks per
+// slice.  Measured with fill = 1 / 2 / 3 when prompts and all decode batches ran on this kernel: prompts of 2048 tokens 13.9 / 11.2 / 10.9 ms
+// (Wo and down have 128 tiles of long K: one wave of long serial CTAs unless K is cut), steps of 8 sequences
+// 1322 / 1250 / 1249 us, of 64 3017 / 3031 / 3000 us; 128 tokens (one 128-token tile) are the exception:
 // 1.70 / 1.86 / 1.82 ms.  k blocks per slice at least 2 (batch 64 / batch 8 steps: 2 -> 3077 / 1433 us, 4 -> 3121 / 1477).
 // Capping the slices of a batch-64 launch at two CTAs per SM (what its 256 TMEM columns per CTA allow at once) was slower:
 // 2509 against 2479 us per step.
@@ -679,8 +679,8 @@ static cudaError_t launch_bn(const CUtensorMap* tw, const CUtensorMap& tx, GemmT
     int stages = (int)((200u * 1024u) / stage_bytes);
     if (stages > 8) stages = 8;
     if (stages > p.kb_per_split) stages = p.kb_per_split;
-    // Grids of more than two tiles per SM (prompts): two stages, so that two CTAs share an SM and the epilogue of one
-    // overlaps the MMAs of the other (measured, prefill of 2048 tokens: 14.0 ms against 15.6 ms with four stages).
+    // Grids of more than two tiles per SM: two stages, so that two CTAs share an SM and the epilogue of one
+    // overlaps the MMAs of the other (measured when prompts ran on this kernel, 2048 tokens: 14.0 ms against 15.6 ms with four stages).
     if (tiles * ksplit > 2 * sm_count && stages > 2) stages = 2;
     if (stages < 1) return cudaErrorInvalidValue;
     p.stages = stages;
@@ -768,7 +768,7 @@ cudaError_t launch_lm_head(const LmHeadCall& c, cudaStream_t st) {
 
 cudaError_t launch_gemm_tc(const GemmTcCall& c, cudaStream_t st) {
     if (c.K % TC_BK || c.n_rows % TC_BM || c.nsplit < 1 || c.nsplit > 3 || c.n_tok < 1) return cudaErrorInvalidValue;
-    // token tile: the smallest of 32 / 64 / 128 that covers the batch, 128 for long prompts
+    // token tile: the smallest of 32 / 64 / 128 that covers the tokens, 128 beyond
     const int bn = c.n_tok <= 32 ? 32 : (c.n_tok <= 64 ? 64 : 128);
     if (c.plane_rows % bn) return cudaErrorInvalidValue;
     CUtensorMap tw, tx;

@@ -1,4 +1,4 @@
-// Tensor-core GEMM (tcgen05 + TMEM + TMA) used by prefill and large-batch decode.
+// Tensor-core GEMM (tcgen05 + TMEM + TMA) of decode batches of more than 64 sequences and of q3_linear_tc.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

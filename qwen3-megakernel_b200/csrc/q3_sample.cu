@@ -15,17 +15,19 @@
 //      few elements at or above that bound (about 1.1 k of them) are the block's candidates, in the order of their indices.  The union of all blocks'
 //      candidates contains every word that is kept; every block finds the threshold among them (binary search over the bits of
 //      the keys, held in registers, below the bits they share and until exactly k are above it) and adds up the weights of the kept
-//      ones, in the same order as every other block.  A row whose candidates do not fit (large k, many equal values) goes
+//      ones, list by list, in the same order as every other block.  A row whose candidates do not fit (large k, many equal values) goes
 //      through a radix select instead: three passes of 11, 11 and 10 bits over the order-preserving integer image of the
 //      floats, histograms summed over the cluster, then the weights' sums.  Every logit >= the k-th value is kept, so ties are all kept;
 //   3. the token is the first index whose inclusive prefix sum exceeds u * total, u in [0, 1) supplied per row
 //      by the caller (a seeded generator on the host side keeps runs reproducible); the block whose words
-//      bracket the target finds it among its candidates, a thread each, or walks the run of the warp that brackets it.
+//      bracket the target finds it among its candidates, a thread each, or walks the run of the warp that brackets it.  Only a word with a
+//      weight above zero (in fp32, under the row's maximum) is drawn, and the same numbers draw the same word on every run.
 // T <= 0 or k == 1 degenerate to the arg-max (ties -> lowest index), like the decode kernels.
 //
 // A single row is bound by latency (0.6 MB, but a dozen dependent block-wide steps), a full batch by the row's bytes and the same steps.
-// Measured, us, before the sums under a block's own maximum and the draw from the candidates -> now: 1 row, k = 50: 14.7 -> 12.0; 64 rows, k = 50:
-// 32.8 -> 24.6; 64 rows, whole vocabulary: 24.7 -> 20.5 (the second pass over the row is gone).
+// Measured, us, before the sums under a block's own maximum and the draw from the candidates -> now: 1 row, k = 50: 14.7 -> 12.3; 64 rows, k = 50:
+// 32.8 -> 24.6; 64 rows, whole vocabulary: 24.7 -> 20.5 (the second pass over the row is gone).  Logits that the caches have not seen before gain
+// less: 1.06 and 1.09 in the first and the last of these.
 #include <cooperative_groups.h>
 
 #include <cfloat>
@@ -111,8 +113,9 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     // warp w of block r: elements [i0, i1), `per` of them but for the last runs of the row
     const int per = sample_run(vocab, C);
     const int i0 = (int)min((long long)vocab, (long long)(rank * SAMPLE_WARPS + warp) * per), i1 = min(vocab, i0 + per);
-    // 0: the arg-max, 1: the k largest words take part, 2: all do.  (Opaque to the compiler: nvcc 12.9 mixes up the flags of this kernel when
-    // it can see what they are made of.)
+    // 0: the arg-max, 1: the k largest words take part, 2: all do.  (Opaque to the compiler: built by nvcc 12.9 from flags whose
+    // terms it could see, an earlier form of this kernel failed every top-k test, as if the threshold had been skipped.  Why is not known: neither a
+    // smaller case nor a fault in the source was found.)
     int mode = !(temperature > 0.f) || top_k == 1 ? 0 : top_k > 1 && top_k < vocab ? 1 : 2;
     asm volatile("" : "+r"(mode));
     const bool greedy = mode == 0, select = mode == 1;
@@ -528,7 +531,8 @@ extern "C" int q3_sample(const float* logits, int32_t batch, int32_t vocab, floa
     if (batch < 1 || vocab < 1 || top_k < 0) return q3::engine_fail(nullptr, Q3_ERR_INVALID, "q3_sample: batch=%d vocab=%d top_k=%d out of range", batch, vocab, top_k);
     if (temperature > 0.f && top_k != 1 && !uniform) return q3::engine_fail(nullptr, Q3_ERR_INVALID, "q3_sample: sampling needs one uniform number per row");
     // Blocks per row: as many as keep all rows' clusters resident at once, and at least 1024 words a block.  Measured with the
-    // full vocabulary, us with clusters of 1 / 2 / 4 / 8 / 16 blocks: 1 row, k = 50: 24.4 / 18.5 / 15.8 / 12.3 / 12.1; 8 rows, k = 50:
+    // full vocabulary, us with clusters of 1 / 2 / 4 / 8 / 16 blocks, before lists were put in order (those in use, k = 50, with it: 1 and 8 rows 12.3, 16
+    // rows 16.4, 64 rows 24.6): 1 row, k = 50: 24.4 / 18.5 / 15.8 / 12.3 / 12.1; 8 rows, k = 50:
     // 24.7 / 19.1 / 16.4 / 12.3 / 20.2; 16 rows, k = 50: 25.3 / 19.5 / 16.4 / 20.5 / 29.1; 33 rows, all words: 25.1 / 18.5 / 14.4 / 20.5 / 32.8;
     // 40 rows, all words: 26.7 / 19.2 / 20.7 / 22.6; 64 rows, all words: 27.5 / 20.5 / 21.6 / 35.0; 64 rows, k = 50: 30.7 / 24.6 / 26.6 / 48.1.
     // A thread keeps its elements in registers where it has at most three groups of four, or five.
