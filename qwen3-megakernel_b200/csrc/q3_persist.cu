@@ -58,13 +58,14 @@ constexpr int GROUP_CTAS = 2 * WO_SLICES;     // CTAs sharing one kv head
 constexpr int WO_ROWS_MAX = 116;              // largest slice: 4 * ceil(256 / 9)
 constexpr int PERSIST_MAX_BATCH = 3;          // sequences served by back-to-back launches when the caller asks for this kernel
 constexpr int MIN_GRID = 147;                 // row shares must fit the shared-memory slots
-constexpr int SC_HALF = 128;                  // the score buffer holds 3 * SC_HALF floats
-constexpr int SPLIT_SC = 3 * SC_HALF / 2;     // split attention: scores kept per head = the most positions a CTA takes (192)
-constexpr int PERSIST_MAX_LEN = GROUP_CTAS * SPLIT_SC - GROUP_CTAS;   // 3438 cached positions
+constexpr int SC_HALF = 128;                  // the score buffer of the local attention holds 3 * SC_HALF floats
+// Most cached positions this kernel is picked for: the longest at which it was timed against the launch chain (one sequence, us per step, this
+// kernel / the chain: 5000 positions 542 / 768, 16000 826 / 1268, 29999 1183 / 1881).
+constexpr int PERSIST_MAX_LEN = 30000;
+constexpr int PERSIST_ASKED_LEN = 3438;       // ... and that a caller may ask for who names this kernel: the limit that request has always had
 constexpr int WROW = 1032;                    // elements between weight rows in shared memory: 1024 + 8 of padding, so that
                                               // the eight row addresses of an ldmatrix fall into different banks
 constexpr int WOROW = 136;                    // the same for the 128-column Wo slice rows
-constexpr int ATT_WARPS = 8;                  // split attention: warps that attend positions (32 positions per pass)
 // Local attention (every CTA attends its whole head over all cached positions) serves up to 255 positions; measured,
 // splitting the positions over the 18 CTAs of a kv group wins beyond that.
 #ifndef Q3_N_ACC
@@ -119,6 +120,7 @@ struct PersistParams {
     int* pidx;
     unsigned long long* trace;   // optional [grid][4 + 12 * n_layers] %globaltimer stamps of thread 0, or nullptr
     int n_layers, vocab, append;
+    int max_len;                 // longest cache this launch serves: its variant's, and what the RoPE table and the host's bound allow
 };
 
 struct PersistState {
@@ -355,7 +357,7 @@ __device__ __forceinline__ int local_v_pos(int w, int i) { return w + CW * i; }
 //   1  local attention, up to 191 cached positions (a third K pass and four more V rows in 16 more registers)
 //   2  local attention, up to 255 cached positions (a fourth K pass and another four V rows)
 //   3  split attention, up to PERSIST_MAX_LEN cached positions
-// (measured per step at 192 / 255 / 319 / 383 positions: local 392 / 417 / 475 / 511 us, split 450 us throughout).
+// (measured per step at 192 / 255 / 319 / 383 positions: local 392 / 417 / 475 / 511 us, split 450 us throughout, 415 since).
 // The host picks the variant from its upper bound of the length; a cache longer than the variant serves is reported.
 constexpr int N_MODES = 4;
 __host__ __device__ constexpr int mode_max_len(int mode) { return mode == 0 ? 128 : mode < N_MODES - 1 ? 127 + 64 * mode : PERSIST_MAX_LEN; }
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     const int c = blockIdx.x, G = gridDim.x;
     const int L = p.n_layers;
     const unsigned long long wait_ns = p.wait_ns;
-    if (p.seq_len[0] > mode_max_len(MODE) || p.seq_len[0] < 0) {   // the same for every CTA: nothing has been started yet
+    if (p.seq_len[0] > p.max_len || p.seq_len[0] < 0) {   // the same for every CTA: nothing has been started yet
         if (tid == 0) report(p.status, ST_BAD_LEN, (uint32_t)MODE, (uint32_t)p.seq_len[0]);
         return;
     }
@@ -397,7 +399,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     uint32_t* xsp = reinterpret_cast<uint32_t*>(fbuf);   // Q, GD: activations split in three bf16 parts, [3][512] pairs (6 KB)
     float* part = fbuf + 1536;                           // Q: per-warp partial row sums [16][32] (2 KB)
     float* gpart = fbuf + 1536;                          // GD: per-warp partial sums of the 48 gate/up tile rows [16][48] (3 KB: runs into q_s, idle in GD)
-    float* om = fbuf;                                    // F: [8 warps][2 heads][128] attention partials
+    float* om = fbuf;                                    // F: [16 warps][128] outputs of the local attention
     float* wo_part = fbuf;                               // F: [2 k-halves][128] Wo slice partial sums (after the partials are published)
     float* dout = fbuf;                                  // GD: [1024] down-projection outputs of this CTA (after the gate/up rows)
     float* xs = fbuf;                                    // LM head: [1024] fp32 activations
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     float* red = reinterpret_cast<float*>(hsp + 48);          // [32]
     float* lw = red + 32;        // [16] per-warp probability sums, [w][head]
     float* misc = lw + 16;       // [16]: [0] score of the new row for this CTA's head
-    float* sc = misc + 16;       // split attention: [2][SPLIT_SC] scores of this CTA's positions; local: [3 * SC_HALF] scores of all positions
+    float* sc = misc + 16;       // local attention: [3 * SC_HALF] scores of all positions; split: the partials' maxima and sums
     uint64_t* full = reinterpret_cast<uint64_t*>(sc + 3 * SC_HALF);   // [4] slot filled
     volatile int* abort_flag = reinterpret_cast<volatile int*>(full + 8);
 
@@ -583,8 +585,8 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     // this CTA's share of the cached positions of kv head fg: [cp0, cp1)
     const int chunk = (len + GROUP_CTAS - 1) / GROUP_CTAS;
     const int cp0 = min(len, fj * chunk), cp1 = min(len, cp0 + chunk);
-    const int npass = (cp1 - cp0 + 31) >> 5;                  // 32 positions per pass (warps 0..7, a quarter-warp each)
-    const int att_slot = warp * 4 + quarter;                  // < 32 for the attending warps
+    const int npass = (cp1 - cp0 + 31) >> 5;                  // 32 positions per pass, half a warp each
+    const int att_slot = warp * 4 + quarter;
     // Short caches: every CTA recomputes the attention of its own head over all positions (no exchange between
     // CTAs; the K/V rows come from L2).  Longer caches: the 18 CTAs of a kv group split the positions.
     constexpr bool local_attn = MODE < N_MODES - 1;
@@ -593,6 +595,16 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
 
     // gains of the next GEMV phase, fetched ahead of the barrier wait
     uint32_t gain2 = *reinterpret_cast<const uint32_t*>(p.ln1 + 2 * tid);
+
+    // split attention: the K and V row of this half warp's position of pass `ps` (32 positions), zeros past the CTA's share
+    const int hl = lane & 15, split_slot = warp * 2 + (lane >> 4);
+    auto split_load = [&](uint4 (&kv)[2], int ps, const bf16_raw* kl, const bf16_raw* vl) {
+        const int pos = cp0 + ps * 32 + split_slot;
+        const bool live = pos < cp1;
+        const size_t row = (size_t)(live ? pos : 0) * KV_DIM;
+        ld_row16(kv[0], reinterpret_cast<const uint4*>(kl + row) + hl, live);
+        ld_row16(kv[1], reinterpret_cast<const uint4*>(vl + row) + hl, live);
+    };
 
     uint4 ring[4][2];
     uint4 ring3[XPASS > 0 ? XPASS : 1][2];    // passes 2..: K row of position 64 pass + slot
@@ -609,7 +621,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
         const unsigned tag = tag_base + (unsigned)l + 1u;
         // K and V rows of the cached positions, fetched at the very start of the layer (they depend on nothing of this
         // step), so that they have arrived, and the SM's input path is quiet, when the q/k/v exchange starts polling.
-        // Split attention: [0], [1] = K passes, [2], [3] = V passes of the CTA's positions.  Local attention:
+        // Split attention: [i] = K and V of pass i of the CTA's positions.  Local attention:
         // [0], [1] = K passes 0, 1 (a quarter-warp per position) and [2], [3] = V[warp + 16 i][4 lane .. 4 lane + 3]
         // for i < 8, two positions per uint4.
         const bf16_raw* kl = kcache + (size_t)l * lstride + fg * HEAD_DIM;
@@ -641,23 +653,9 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                         uint4& dst = ring[2 + (i >> 2)][(i >> 1) & 1];
                         if (i & 1) ld_row8(dst.z, dst.w, vp, live); else ld_row8(dst.x, dst.y, vp, live);
                     }
-                } else if (warp < ATT_WARPS) {
+                } else {
 #pragma unroll
-                    for (int ps = 0; ps < 2; ++ps) {   // K: a quarter-warp per position
-                        const int pos = cp0 + ps * 32 + att_slot;
-                        const bool live = pos < cp1;
-                        const uint4* kr = reinterpret_cast<const uint4*>(kl + (size_t)(live ? pos : 0) * KV_DIM);
-                        ld_row16(ring[ps][0], kr + sub, live);
-                        ld_row16(ring[ps][1], kr + 8 + sub, live);
-                    }
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {      // V: a warp per position, four dims per lane
-                        const int pos = cp0 + warp + ATT_WARPS * i;
-                        const bool live = pos < cp1;
-                        const bf16_raw* vp = vl + (size_t)(live ? pos : 0) * KV_DIM + lane * 4;
-                        uint4& dst = ring[2 + (i >> 2)][(i >> 1) & 1];
-                        if (i & 1) ld_row8(dst.z, dst.w, vp, live); else ld_row8(dst.x, dst.y, vp, live);
-                    }
+                    for (int i = 0; i < 4; ++i) split_load(ring[i], i, kl, vl);
                 }
             }
         };
@@ -891,92 +889,101 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                 }
                 cta_sync();
             } else {
-            // ---- scores of this CTA's cached positions, both heads: a quarter-warp per position ----
-                float tmax0 = -INFINITY, tmax1 = -INFINITY;
-                if (warp < ATT_WARPS) {
-                    float qa[2][16];
-#pragma unroll
-                    for (int hh = 0; hh < 2; ++hh)
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) { qa[hh][i] = q_s[hh * 128 + sub * 8 + i]; qa[hh][8 + i] = q_s[hh * 128 + 64 + sub * 8 + i]; }
-                    for (int ps = 0; ps < npass; ++ps) {
-                        const int idx = ps * 32 + att_slot, pos = cp0 + idx;
-                        uint4 k0 = make_uint4(0, 0, 0, 0), k1 = k0;
-                        if (ps == 0) { k0 = ring[0][0]; k1 = ring[0][1]; }
-                        else if (ps == 1) { k0 = ring[1][0]; k1 = ring[1][1]; }
-                        else if (pos < cp1) {
-                            const uint4* kr = reinterpret_cast<const uint4*>(kl + (size_t)pos * KV_DIM);
-                            k0 = ld_stream(kr + sub); k1 = ld_stream(kr + 8 + sub);
-                        }
-                        float kf[16];
-                        unpack8f(k0, kf); unpack8f(k1, kf + 8);
-                        float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) { s0 = fmaf(qa[0][i], kf[i], s0); s1 = fmaf(qa[1][i], kf[i], s1); }
-#pragma unroll
-                        for (int o = 1; o <= 4; o <<= 1) {
-                            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-                            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-                        }
-                        if (pos < cp1) {
-                            tmax0 = fmaxf(tmax0, s0); tmax1 = fmaxf(tmax1, s1);
-                            if (sub == 0) { sc[idx] = s0; sc[SPLIT_SC + idx] = s1; }
-                        }
-                    }
-                    tmax0 = warp_max(tmax0); tmax1 = warp_max(tmax1);
-                    if (lane == 0) { red[warp] = tmax0; red[8 + warp] = tmax1; }
-                } else if (warp == 12) {   // the new row's score for this CTA's own head: q . k_new in fp32, unrounded
+                // ---- this CTA's cached positions, both heads, in one pass over K and V: half a warp per position, eight dims of its two rows
+                //      a lane.  Either half keeps a running maximum and sum of its own, so that nothing crosses them until the end.  All
+                //      sixteen warps attend, the first four passes (128 positions) were requested in Q, and a pass that has been consumed
+                //      makes room for the one four further: 64 KB in flight per SM.  Bound by the rows' bytes beyond about 2300 positions (27 ns
+                //      a position and step, 4.3 TB/s), by the layer's exchanges below.  us per step, with eight warps, scores in shared memory and
+                //      rows beyond the first 64 fetched as they are needed -> now: 1000 positions 455 -> 443, 2200 563 -> 466, 3438 673 -> 498.
+                //      (Rows asked into L2 a layer ahead: 555 instead of 542 at 5000.) ----
+                if (warp == 12) {   // the new row's score for this CTA's own head: q . k_new in fp32, unrounded
                     const float4 a = *reinterpret_cast<const float4*>(q_s + fhh * 128 + lane * 4);
                     const float4 b = *reinterpret_cast<const float4*>(k_s + lane * 4);
                     const float sn_ = warp_sum(a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w);
                     if (lane == 0) misc[0] = sn_;
                 }
-                cta_sync();
-                float M0 = (lane < ATT_WARPS) ? red[lane] : -INFINITY, M1 = (lane < ATT_WARPS) ? red[8 + lane] : -INFINITY;
-                M0 = warp_max(M0); M1 = warp_max(M1);
-
-                // ---- probabilities and P.V against the CTA-wide maxima: the partial sums just add.  A warp per position
-                //      and four dims per lane: every lane forms the same two probabilities, nothing crosses lanes ----
-                if (warp < ATT_WARPS) {
-                    float l0 = 0.f, l1 = 0.f, acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                float qa[2][8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int idx = warp + ATT_WARPS * i;
-                        const bool live = cp0 + idx < cp1;
-                        const float p0 = live ? __expf(sc[idx] - M0) : 0.f, p1 = live ? __expf(sc[SPLIT_SC + idx] - M1) : 0.f;
-                        l0 += p0; l1 += p1;
-                        const uint4& src = ring[2 + (i >> 2)][(i >> 1) & 1];
-                        const uint32_t vx = (i & 1) ? src.z : src.x, vy = (i & 1) ? src.w : src.y;
-                        const float f0 = bf_lo(vx), f1 = bf_hi(vx), f2 = bf_lo(vy), f3 = bf_hi(vy);
-                        acc[0][0] = fmaf(p0, f0, acc[0][0]); acc[0][1] = fmaf(p0, f1, acc[0][1]); acc[0][2] = fmaf(p0, f2, acc[0][2]); acc[0][3] = fmaf(p0, f3, acc[0][3]);
-                        acc[1][0] = fmaf(p1, f0, acc[1][0]); acc[1][1] = fmaf(p1, f1, acc[1][1]); acc[1][2] = fmaf(p1, f2, acc[1][2]); acc[1][3] = fmaf(p1, f3, acc[1][3]);
+                for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) qa[hh][i] = q_s[hh * 128 + hl * 8 + i];
+                float mx[2] = {-INFINITY, -INFINITY}, ls[2] = {0.f, 0.f}, acc[2][8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[0][i] = acc[1][i] = 0.f;
+                auto attend = [&](const uint4 (&kv)[2], int ps) {
+                    float f[8], s2[2];
+                    unpack8f(kv[0], f);
+#pragma unroll
+                    for (int hh = 0; hh < 2; ++hh) {
+                        float s0 = qa[hh][0] * f[0], s1 = qa[hh][1] * f[1];
+#pragma unroll
+                        for (int i = 2; i < 8; i += 2) { s0 = fmaf(qa[hh][i], f[i], s0); s1 = fmaf(qa[hh][i + 1], f[i + 1], s1); }
+                        s2[hh] = s0 + s1;
                     }
-#pragma unroll 2
-                    for (int idx = warp + ATT_WARPS * 8; cp0 + idx < cp1; idx += ATT_WARPS) {
-                        const uint2 v = ld_stream8(vl + (size_t)(cp0 + idx) * KV_DIM + lane * 4);
-                        const float p0 = __expf(sc[idx] - M0), p1 = __expf(sc[SPLIT_SC + idx] - M1);
-                        l0 += p0; l1 += p1;
-                        const float f0 = bf_lo(v.x), f1 = bf_hi(v.x), f2 = bf_lo(v.y), f3 = bf_hi(v.y);
-                        acc[0][0] = fmaf(p0, f0, acc[0][0]); acc[0][1] = fmaf(p0, f1, acc[0][1]); acc[0][2] = fmaf(p0, f2, acc[0][2]); acc[0][3] = fmaf(p0, f3, acc[0][3]);
-                        acc[1][0] = fmaf(p1, f0, acc[1][0]); acc[1][1] = fmaf(p1, f1, acc[1][1]); acc[1][2] = fmaf(p1, f2, acc[1][2]); acc[1][3] = fmaf(p1, f3, acc[1][3]);
+#pragma unroll
+                    for (int o = 1; o <= 8; o <<= 1) {
+                        s2[0] += __shfl_xor_sync(0xffffffffu, s2[0], o);
+                        s2[1] += __shfl_xor_sync(0xffffffffu, s2[1], o);
                     }
-                    *reinterpret_cast<float4*>(om + (warp * 2) * 128 + lane * 4) = make_float4(acc[0][0], acc[0][1], acc[0][2], acc[0][3]);
-                    *reinterpret_cast<float4*>(om + (warp * 2 + 1) * 128 + lane * 4) = make_float4(acc[1][0], acc[1][1], acc[1][2], acc[1][3]);
-                    if (lane == 0) { lw[warp * 2] = l0; lw[warp * 2 + 1] = l1; }
+                    const bool live = cp0 + ps * 32 + split_slot < cp1;
+                    unpack8f(kv[1], f);
+#pragma unroll
+                    for (int hh = 0; hh < 2; ++hh) {
+                        const float mn = live ? fmaxf(mx[hh], s2[hh]) : mx[hh];
+                        const float keep = mx[hh] == mn ? 1.f : __expf(mx[hh] - mn);     // (the first row: exp(-inf) = 0)
+                        const float pr = live ? __expf(s2[hh] - mn) : 0.f;
+                        mx[hh] = mn;
+                        ls[hh] = fmaf(ls[hh], keep, pr);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[hh][i] = fmaf(pr, f[i], acc[hh][i] * keep);
+                    }
+                };
+                for (int ps = 0; ps < npass; ps += 4)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (ps + j < npass) {
+                            attend(ring[j], ps + j);
+                            if (ps + j + 4 < npass) split_load(ring[j], ps + j + 4, kl, vl);
+                        }
+                // the halves under the warp's maximum; the lower one keeps head 0, the upper one head 1
+                float* const oms = reinterpret_cast<float*>(sA);           // [16 warps][2 heads][128], then [2][16] maxima and sums: the q/k/v rows are
+                float* const oml = oms + CW * 256;                         // dead until GD fetches the next layer's
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const float M = fmaxf(mx[hh], __shfl_xor_sync(0xffffffffu, mx[hh], 16));
+                    const float w = mx[hh] == -INFINITY ? 0.f : __expf(mx[hh] - M);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[hh][i] *= w;
+                    float t = ls[hh] * w;
+                    t += __shfl_xor_sync(0xffffffffu, t, 16);
+                    if (lane == 0) { oml[hh * CW + warp] = M; oml[2 * CW + hh * CW + warp] = t; }
+                }
+                {
+                    const bool upper = lane & 16;
+                    float t[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) t[i] = (upper ? acc[1][i] : acc[0][i]) + __shfl_xor_sync(0xffffffffu, upper ? acc[0][i] : acc[1][i], 16);
+                    float* dst = oms + (warp * 2 + (lane >> 4)) * 128 + hl * 8;
+                    *reinterpret_cast<float4*>(dst) = make_float4(t[0], t[1], t[2], t[3]);
+                    *reinterpret_cast<float4*>(dst + 4) = make_float4(t[4], t[5], t[6], t[7]);
                 }
                 cta_sync();
                 // ---- publish the CTA's partial of both heads: (max, sum, unnormalised output), every word tagged ----
                 if (tid < 256) {
                     const int hh = tid >> 7, d = tid & 127;
-                    float o = 0.f, Ls = 0.f;
+                    float o = 0.f;
+                    const float mw = oml[hh * CW + (lane & 15)];                // lanes 0..15 (and again 16..31): a warp's maximum
+                    const float M = warp_max(mw);
+                    const float wgt = mw == -INFINITY ? 0.f : __expf(mw - M);
+                    const float Ls = warp_sum(lane < CW ? oml[2 * CW + hh * CW + lane] * wgt : 0.f);
 #pragma unroll
-                    for (int w = 0; w < ATT_WARPS; ++w) { o += om[(w * 2 + hh) * 128 + d]; Ls += lw[w * 2 + hh]; }
+                    for (int w = 0; w < CW; ++w) o = fmaf(oms[(w * 2 + hh) * 128 + d], __shfl_sync(0xffffffffu, wgt, w), o);
                     const unsigned long long t64 = (unsigned long long)tag << 32;
                     unsigned long long* dst = p.xp + (size_t)((fg * 2 + hh) * GROUP_CTAS + fj) * XP_STRIDE;
                     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(dst + 4 + d), "l"(t64 | __float_as_uint(o)) : "memory");
                     __syncwarp();
                     if (d == 127) {   // the (max, sum) pair goes last: it is what the readers poll
-                        asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(dst), "l"(t64 | __float_as_uint(hh ? M1 : M0)), "l"(t64 | __float_as_uint(Ls)) : "memory");
+                        asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(dst), "l"(t64 | __float_as_uint(M)), "l"(t64 | __float_as_uint(Ls)) : "memory");
                     }
                 }
                 Q3_TRACE(ev + 4);
@@ -1487,7 +1494,8 @@ bool persist_supports(const q3_engine* e, const q3_decode_args* a) {
     if (s == nullptr || a->batch < 1) return false;
     if (reinterpret_cast<uintptr_t>(e->rope) & 15) return false;   // the kernel reads the table 16 bytes at a time (a test of it there: 3 us a step)
     if (s->tp_size > 1) return a->batch == 1 && a->max_len <= mode_max_len(N_MODES - 2);   // one sequence, local attention
-    return a->batch <= PERSIST_MAX_BATCH && a->max_len <= PERSIST_MAX_LEN;
+    const bool asked = (a->flags & Q3_F_PATH_MASK) == Q3_F_PATH_PERSIST;
+    return a->batch <= PERSIST_MAX_BATCH && a->max_len <= (asked ? PERSIST_ASKED_LEN : PERSIST_MAX_LEN);
 }
 
 // (Re)pack the layer matrices when one of the caller's pointers changes.  Runs on the legacy default
@@ -1601,6 +1609,8 @@ int persist_decode(q3_engine* e, const q3_decode_args* a, cudaStream_t st) {
     p.n_layers = e->cfg.n_layers; p.vocab = e->cfg.vocab; p.append = (a->flags & Q3_F_APPEND_KV) ? 1 : 0;
     int mode = 0;
     while (mode + 1 < N_MODES && a->max_len > mode_max_len(mode)) ++mode;
+    p.max_len = mode < N_MODES - 1 ? mode_max_len(mode) : a->max_len > PERSIST_ASKED_LEN ? a->max_len : PERSIST_ASKED_LEN;
+    if (p.max_len > e->rope_n - 1) p.max_len = e->rope_n - 1;
     // A small batch is one launch per sequence, back to back on the stream: the kernel reads entry 0 of every
     // per-sequence array, so the arrays are simply offset (outputs are [batch][...] with the batch axis leading).
     const size_t kv_row = (size_t)e->cfg.n_layers * KV_DIM;

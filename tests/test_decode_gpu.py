@@ -94,6 +94,32 @@ def test_any_position(oracle, path, ctx):
     gate_step(oracle, out, ref, f"{path} ctx {ctx}")
 
 
+@pytest.mark.parametrize("ctx", [575, 576, 577, 2304, 2305, 2900, 3439, 4608, 4610, 8191])
+def test_one_sequence_is_one_launch_at_any_length(oracle, ctx):
+    """The 18 blocks of a kv head take 32 positions a pass and hold four passes in registers: lengths around one pass (576), around four (2304)
+    and beyond what a caller that names the persistent kernel may ask for (3438)."""
+    from qwen3mk.kernel import SeqTable
+
+    shp = oracle.Shape(layers=2, vocab=2048)
+    inp = oracle.synthetic(500 + ctx, shp, context=ctx)
+    dev = to_dev(inp)
+    mk = engine("auto", layers=2, vocab=2048)
+    mk.step(dev)
+    before = mk.launch_count
+    out = mk.step(dev)
+    mk.status()
+    assert mk.launch_count == before + 1
+    ref = oracle.decode_step(oracle.to_fp32(inp), inp["token"], inp["kcache"], inp["vcache"])
+    gate_step(oracle, out, ref, f"ctx {ctx}")
+    if ctx > 4000:   # a cache longer than the host said is reported, not served
+        seqs = SeqTable([dev["kcache"]], [dev["vcache"]], lens=[ctx - 1])
+        mk.bind_sequences({k: dev[k] for k in oracle.WEIGHT_NAMES}, dev["token"].reshape(1), seqs)
+        seqs.len.fill_(ctx)
+        mk.launch()
+        with pytest.raises(RuntimeError, match="code 5"):
+            mk.status()
+
+
 @pytest.mark.parametrize("ctx", [40, 200, 300])
 def test_persist_on_a_grid_one_short_of_the_sm_count(oracle, ctx):
     """147 CTAs is the smallest grid the persistent kernel's shared-memory slots allow; the row shares differ from 148's."""
