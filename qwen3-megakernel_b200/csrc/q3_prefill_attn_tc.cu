@@ -365,18 +365,30 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
             at_ld32(o0, trow + 256u + (uint32_t)dim0);
             at_ld32(o1, trow + 384u + (uint32_t)dim0);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (!abort_flag && qpos < a.T) {   // 32 dims = 64 contiguous bytes
+            // Through shared memory (Q's: all products have completed), so that a warp writes a position's 512 bytes (a thread per row: 1 us more a block).
+            // 16-byte chunks of a position's row are XORed by the position.
+            uint4* const so = reinterpret_cast<uint4*>(sQh);
+            {
                 float o[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     o[j] = __uint_as_float(o0[j]) * w0;
                     if (n_kt > 1) o[j] = fmaf(__uint_as_float(o1[j]), w1, o[j]);   // (TMEM that nothing was added to may hold anything)
                 }
-                bf16_raw* dst = a.plane + (size_t)qpos * Q_DIM + (2 * g + (row >> 6)) * HEAD_DIM + dim0;
+                const int pos = row & 63, chunk = (row >> 6) * 16 + dim0 / 8;
 #pragma unroll
-                for (int j = 0; j < 32; j += 8)
-                    *reinterpret_cast<uint4*>(dst + j) = make_uint4(at_pack_bf16(o[j], o[j + 1]), at_pack_bf16(o[j + 2], o[j + 3]),
-                                                                    at_pack_bf16(o[j + 4], o[j + 5]), at_pack_bf16(o[j + 6], o[j + 7]));
+                for (int j = 0; j < 4; ++j)
+                    so[pos * 32 + ((chunk + j) ^ (pos & 7))] = make_uint4(at_pack_bf16(o[8 * j], o[8 * j + 1]), at_pack_bf16(o[8 * j + 2], o[8 * j + 3]),
+                                                                           at_pack_bf16(o[8 * j + 4], o[8 * j + 5]), at_pack_bf16(o[8 * j + 6], o[8 * j + 7]));
+            }
+            asm volatile("bar.sync 9, %0;" ::"n"(AT_SOFT) : "memory");
+            if (!abort_flag) {
+                bf16_raw* const dst = a.plane + (size_t)q0 * Q_DIM + 2 * g * HEAD_DIM + lane * 8;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int pos = warp + 16 * i;
+                    if (q0 + pos < a.T) *reinterpret_cast<uint4*>(dst + (size_t)pos * Q_DIM) = so[pos * 32 + (lane ^ (pos & 7))];
+                }
             }
         }
     }
