@@ -613,8 +613,10 @@ static int prefill_chain(q3_engine* e, const q3_prefill_args* a, const q3_decode
     bf16_raw *hid = xn + cap * HIDDEN, *attn = hid + cap * INTER;
     bf16_raw *q_hi = reinterpret_cast<bf16_raw*>(e->qkv), *q_lo = q_hi + (size_t)T * Q_DIM;
     float* ssq = e->gate;
+    int parts = PR_SSQ_PARTS;
     CUtensorMap m_xn, m_hid, m_attn, m_qh, m_ql, m_k, m_v;
-    bool ok = tc_make_map(&m_xn, xn, 0, T, HIDDEN, 1, 128) && tc_make_map(&m_hid, hid, 0, T, INTER, 1, 128) && tc_make_map(&m_attn, attn, 0, T, Q_DIM, 1, 128);
+    const uint32_t box = (uint32_t)prompt_box_rows(T);
+    bool ok = tc_make_map(&m_xn, xn, 0, T, HIDDEN, 1, box) && tc_make_map(&m_hid, hid, 0, T, INTER, 1, box) && tc_make_map(&m_attn, attn, 0, T, Q_DIM, 1, box);
     if (tiled)
         ok = ok && tc_make_map(&m_qh, q_hi, 0, T, Q_DIM, 1, 64) && tc_make_map(&m_ql, q_lo, 0, T, Q_DIM, 1, 64) &&
              tc_make_map(&m_k, a->kcache, L, T, KV_DIM, 1, 128, a->cache_capacity) && tc_make_map(&m_v, a->vcache, L, T, KV_DIM, 1, 128, a->cache_capacity);
@@ -636,7 +638,7 @@ static int prefill_chain(q3_engine* e, const q3_prefill_args* a, const q3_decode
     LAUNCH(launch_prompt_embed(reinterpret_cast<const long long*>(a->ids), bf(w.embed), V, e->x, bf(w.ln1), xn, ssq, T, e->status, T, st));
     for (int l = 0; l < L; ++l) {
         PromptGemmCall c{};
-        c.T = T; c.ssq = ssq; c.ssq_ld = T; c.status = e->status;
+        c.T = T; c.ssq = ssq; c.ssq_ld = T; c.parts = &parts; c.status = e->status;
         PromptGemmCall q = c;
         q.kind = PR_QKV; q.K = HIDDEN; q.in = &m_xn;
         q.w[0] = bf(w.wq) + (size_t)l * Q_DIM * HIDDEN; q.w[1] = bf(w.wk) + (size_t)l * KV_DIM * HIDDEN; q.w[2] = bf(w.wv) + (size_t)l * KV_DIM * HIDDEN;

@@ -20,7 +20,7 @@ constexpr int PR_BM = 128;         // tokens of a block
 constexpr float PR_QS = ATTN_SCALE * 1.4426950408889634f;   // scores in units of log2, as the tiled attention wants them
 
 struct PromptParams {
-    int T, kb_total, ssq_ld;
+    int T, kb_total, ssq_ld, ssq_parts;   // ssq_parts: partial sums of squares a row of ssq_in has
     const float* ssq_in;
     float* ssq_out;
     bf16_raw *q_hi, *q_lo;
@@ -34,6 +34,7 @@ struct PromptParams {
     bf16_raw* hid;
     uint32_t* status;
     int n_tiles, n_items, stages;   // pair kernel
+    int a_rows;                     // rows of the activations' box
 };
 
 __device__ __forceinline__ uint32_t pr_pack(float lo, float hi) {
@@ -53,8 +54,9 @@ __device__ __forceinline__ float pr_silu(float g, float u) { return __fdividef(g
 // scale of token t's RMS norm from the partial sums of squares
 __device__ __forceinline__ float pr_scale(const PromptParams& p, int t) {
     float ss = 0.f;
+    for (int i0 = 0; i0 < p.ssq_parts; i0 += 16)
 #pragma unroll
-    for (int i = 0; i < PR_SSQ_PARTS; ++i) ss += p.ssq_in[(size_t)i * p.ssq_ld + t];
+        for (int i = 0; i < 16; ++i) ss += p.ssq_in[(size_t)(i0 + i) * p.ssq_ld + t];
     return rsqrtf(ss / (float)HIDDEN + EPS);
 }
 
@@ -112,84 +114,91 @@ __device__ __forceinline__ void pr_expect(uint64_t* bar, uint32_t bytes) {
 }
 
 // ------------------------------------------------------------------------------------------------------------------------------
-// Short prompts: a block takes 128 tokens x BN weight rows x one of C slices of K; the C slices are the blocks of a cluster.  Every
-// block owns a run of the tile's token rows, sends its partial sums of the others' rows to their owners with bulk copies through distributed
-// shared memory, and finishes its own: no atomics, no cleared buffers, the same result on every run.
+// Short prompts: a block takes 128 tokens x BN weight rows (PR_RESID: x one of C slices of K).  What such a launch takes is a chain of latencies, so BN
+// is chosen for about one block an SM, and the epilogue for the fewest exchanges:
+//   PR_QKV    BN columns of a head, half of them from either half of the head, so that RoPE's pairs stay in a thread; the blocks of a head are a
+//             cluster and exchange the sums of squares of their columns (512 bytes), nothing else
+//   PR_SILU   BN / 2 rows of Wg and the same of Wu, nothing to exchange
+//   PR_RESID  K is long (2048, 3072) and N short (1024): the C slices of K are the blocks of a cluster, each owns a run of the tile's token rows,
+//             sends its partial sums of the others' rows to their owners with bulk copies through distributed shared memory and finishes its
+//             own: no atomics, no cleared buffers, the same result on every run
+// Exchanging partial tiles is what costs (48 KB a block 2 to 4 us, 16 KB about 1): q/k/v of 128 tokens in four slices of K took 9.2 us from its wait
+// to its last exit, without slices 7.4; gate/up in two slices 7.9, without 6.0.
 //
-// Shared memory stays under 113 KB, so that a block of the next launch fits beside one of this launch, sets up and requests its weight
-// tiles while this launch ends.  A partial tile is [row][BN] fp32 with the 16-byte chunks of a row XORed by row & 7, so
-// that a thread per row writes it and half a warp per row reads it without bank conflicts; it overlays the stages.
+// OCC: blocks that fit an SM.  One with a ring of up to 222 KB has nearly all of its loads under way at once; two overlap one another's
+// phases where a launch has more blocks than SMs.  Either way a block of the next launch finds room as this launch's blocks end, sets up and requests its
+// weights before the wait.  A partial tile is [row][BN] fp32 with the 16-byte chunks of a row XORed by row & 7, so
+// that a thread per row writes it and a group of lanes per row reads it without bank conflicts; it overlays the stages.
 //
 // Tensor memory of an SM: a block waits for its cluster while it holds its columns, so the blocks that fit on an SM may not ask for more than 512
-// together (q3_gemm_cl.cu).  Two of these are 256 and leave no room for a decode product's 58 KB; one of them and two decode products are 384.
+// together (q3_gemm_cl.cu).  Two of these are 256 at most and leave no room for a decode product's 58 KB; one of a single-block shape leaves none
+// either, and has no cluster to wait for or 64 columns at most.
 // A block of the pair kernel (512 columns) has more shared memory than any of them leaves.
 //
 // A wait that gives up: as in q3_gemm_cl.cu (a block without its sums sends and stores nothing, everyone meets at every cluster
 // barrier, and what was under way is drained before the block leaves).
 // ------------------------------------------------------------------------------------------------------------------------------
 constexpr int PS_THREADS = 192;    // warp 0: TMA, warp 1: MMA and TMEM, warps 2..5: epilogue
-constexpr int PS_MAX_STAGES = 4;
+constexpr int PS_MAX_STAGES = 12;
 constexpr unsigned long long PS_RED_WAIT_NS = 2 * TC_WAIT_NS;
 
-template <int KIND, int C> struct PsShape {
-    static constexpr int BN = KIND == PR_QKV ? 128 : KIND == PR_RESID ? 64 : 96;     // weight rows of a tile (PR_SILU: 48 of Wg, then 48 of Wu)
-    static constexpr int ROWS = PR_BM / C;                                            // most rows a block owns
+template <int KIND, int BN, int C, int OCC> struct PsShape {
+    static constexpr int CL = KIND == PR_QKV ? HEAD_DIM / BN : C;                     // blocks of a cluster: a head's columns, or the slices of K
+    static constexpr int ROWS = PR_BM / C;                                            // most rows a block finishes
     static constexpr uint32_t A_BYTES = PR_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2, STAGE = A_BYTES + B_BYTES;
     static constexpr uint32_t RED = (C - 1) * ROWS * BN * 4;                          // partial rows from the other blocks
-    static constexpr uint32_t TAIL = 128 + PR_BM * 4;                                 // barriers and flags, the owned rows' scales
-    static constexpr uint32_t ROOM = 113 * 1024 - TAIL - RED;
-    static constexpr int STAGES = ROOM / STAGE < PS_MAX_STAGES ? ROOM / STAGE : PS_MAX_STAGES;
-    static constexpr size_t SMEM = STAGES * STAGE + RED + TAIL;
-    static constexpr uint32_t COLS = BN <= 64 ? 64 : 128;                             // TMEM columns
-    static_assert(STAGES >= 2 && STAGES * STAGE >= PR_BM * BN * 4, "the stages hold the block's partial tile");
+    static constexpr int FIT = ((OCC == 1 ? 222 : KIND == PR_QKV && CL > 1 ? 110 : 112) * 1024 - RED) / STAGE;   // (two blocks an SM: 113 KB each, with the static ones)
+    static constexpr int STAGES = FIT < PS_MAX_STAGES ? FIT : PS_MAX_STAGES;
+    static constexpr size_t SMEM = STAGES * STAGE + RED;
+    static constexpr uint32_t COLS = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;   // TMEM columns
+    static_assert(C == 1 || STAGES * STAGE >= PR_BM * BN * 4, "the stages hold the block's partial tile");
     static_assert(ROWS % 8 == 0, "the chunk swizzle of a row is the same at its owner");
+    static_assert(KIND == PR_RESID || C == 1, "only Wo and down are cut along K");
 };
 
-template <int KIND, int C>
-__global__ void __launch_bounds__(PS_THREADS, 2) prompt_split_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
+template <int KIND, int BN, int C, int OCC>
+__global__ void __launch_bounds__(PS_THREADS, OCC) prompt_split_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
                                                                      const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_x,
                                                                      const PromptParams p) {
-    using S = PsShape<KIND, C>;
-    constexpr int BN = S::BN, STAGES = S::STAGES;
+    using S = PsShape<KIND, BN, C, OCC>;
+    constexpr int STAGES = S::STAGES, CL = S::CL;
     extern __shared__ __align__(1024) unsigned char ps_raw[];
+    __shared__ __align__(8) uint64_t full_bar[PS_MAX_STAGES], empty_bar[PS_MAX_STAGES], acc_bar, red_bar;
+    __shared__ uint32_t tmem_base_s;
+    __shared__ volatile int abort_flag;
+    __shared__ float s_ss[KIND == PR_QKV ? CL : 1][PR_BM];      // q/k/v: the sums of squares of a row's columns in every block of the cluster
     unsigned char* const base = ps_raw;
     float* const red = reinterpret_cast<float*>(base + (size_t)STAGES * S::STAGE);      // [C - 1][R][BN]
-    uint64_t* const full_bar = reinterpret_cast<uint64_t*>(base + (size_t)STAGES * S::STAGE + S::RED);
-    uint64_t* const empty_bar = full_bar + PS_MAX_STAGES;
-    uint64_t* const acc_bar = empty_bar + PS_MAX_STAGES;
-    uint64_t* const red_bar = acc_bar + 1;
-    uint32_t* const tmem_base_s = reinterpret_cast<uint32_t*>(red_bar + 1);
-    volatile int* const abort_flag = reinterpret_cast<volatile int*>(tmem_base_s + 1);
-    float* const s_r = reinterpret_cast<float*>(base + (size_t)STAGES * S::STAGE + S::RED + 128);
 
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
-    const int rank = C > 1 ? (int)blockIdx.x : 0;      // the cluster spans x
+    const int rank = CL > 1 ? (int)blockIdx.x : 0;     // the cluster spans x
     const int tile = blockIdx.y, m0 = blockIdx.z * PR_BM;
+    const int slice = C > 1 ? rank : 0;
     const int base_kb = p.kb_total / C, rem_kb = p.kb_total % C;
-    const int kb0 = rank * base_kb + min(rank, rem_kb), nkb = base_kb + (rank < rem_kb ? 1 : 0);
+    const int kb0 = slice * base_kb + min(slice, rem_kb), nkb = base_kb + (slice < rem_kb ? 1 : 0);
     const int rows = min(PR_BM, p.T - m0);             // tokens of this tile
-    const int R = C > 1 ? (((rows + C - 1) / C + 7) & ~7) : PR_BM;      // rows a block owns: [rank R, rank R + R)
+    const int R = C > 1 ? (((rows + C - 1) / C + 7) & ~7) : PR_BM;      // rows a block owns: [slice R, slice R + R)
     auto rows_of = [&](int owner) { return max(0, min(R, rows - owner * R)); };
-    const int my_rows = rows_of(rank);
+    const int my_rows = rows_of(slice);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { pr_mbar_init(&full_bar[s], 1); pr_mbar_init(&empty_bar[s], 1); }
-        pr_mbar_init(acc_bar, 1);
-        pr_mbar_init(red_bar, 1);
+        pr_mbar_init(&acc_bar, 1);
+        pr_mbar_init(&red_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (C > 1 && my_rows > 0) pr_expect(red_bar, (uint32_t)((C - 1) * my_rows * BN * 4));
-        *abort_flag = 0;
+        if (C > 1 && my_rows > 0) pr_expect(&red_bar, (uint32_t)((C - 1) * my_rows * BN * 4));
+        abort_flag = 0;
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(tmem_base_s)), "r"(S::COLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_base_s)), "r"(S::COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = *tmem_base_s;
+    const uint32_t tmem_base = tmem_base_s;
     pdl_launch();
-    if (C > 1) pr_cluster_arrive();      // (matched before the first remote copy: every block of the cluster has set its barriers up by then)
+    if (CL > 1) pr_cluster_arrive();      // (matched before the first remote write: every block of the cluster has set its barriers up by then)
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
@@ -198,15 +207,18 @@ __global__ void __launch_bounds__(PS_THREADS, 2) prompt_split_kernel(const __gri
         if (one) {
             const CUtensorMap* tm_w = &tm_w0;
             int r0 = tile * BN;
-            if (KIND == PR_QKV) {
-                if (tile >= Q_DIM / BN) { tm_w = &tm_w1; r0 -= Q_DIM; }
-                if (tile >= (Q_DIM + KV_DIM) / BN) { tm_w = &tm_w2; r0 -= KV_DIM; }
+            if (KIND == PR_QKV) {        // dims [rank BN / 2, ..) of head `tile` and those 64 further: RoPE's pairs stay in a block
+                r0 = tile * HEAD_DIM + rank * (BN / 2);
+                if (tile >= Q_HEADS) { tm_w = &tm_w1; r0 -= Q_DIM; }
+                if (tile >= Q_HEADS + KV_HEADS) { tm_w = &tm_w2; r0 -= KV_DIM; }
             }
             if (KIND == PR_SILU) r0 = tile * (BN / 2);
+            const uint32_t bytes = (uint32_t)p.a_rows * TC_BK * 2 + S::B_BYTES;
             auto weights = [&](int kb, int s) {
                 const uint32_t st = tc_smem(base + (size_t)s * S::STAGE) + S::A_BYTES;
-                pr_expect(&full_bar[s], S::STAGE);
+                pr_expect(&full_bar[s], bytes);
                 tc_load_box(st, tm_w, (kb0 + kb) * TC_BK, r0, &full_bar[s]);
+                if (KIND == PR_QKV) tc_load_box(st + S::B_BYTES / 2, tm_w, (kb0 + kb) * TC_BK, r0 + 64, &full_bar[s]);
                 if (KIND == PR_SILU) tc_load_box(st + S::B_BYTES / 2, &tm_w1, (kb0 + kb) * TC_BK, r0, &full_bar[s]);
                 armed = kb + 1;
             };
@@ -217,16 +229,16 @@ __global__ void __launch_bounds__(PS_THREADS, 2) prompt_split_kernel(const __gri
             for (int kb = 0, s = 0, turn = 0; kb < nkb; ++kb, ++s) {
                 if (s == STAGES) { s = 0; ++turn; }
                 if (turn > 0) {
-                    if (!tc_wait(&empty_bar[s], (turn - 1) & 1, abort_flag, p.status, 60)) break;
+                    if (!tc_wait(&empty_bar[s], (turn - 1) & 1, &abort_flag, p.status, 60)) break;
                     weights(kb, s);
                 }
                 tc_load_box(tc_smem(base + (size_t)s * S::STAGE), &tm_x, (kb0 + kb) * TC_BK, m0, &full_bar[s]);
             }
         }
         __syncwarp();
-        if (C > 1) { pr_cluster_wait(); pr_cluster_arrive(); pr_cluster_wait(); }
+        if (CL > 1) { pr_cluster_wait(); pr_cluster_arrive(); pr_cluster_wait(); }
         else asm volatile("bar.sync 3, 192;" ::: "memory");
-        if (one && *abort_flag)          // (the last STAGES of them may still be on their way)
+        if (one && abort_flag)           // (the last STAGES of them may still be on their way)
             for (int kb = max(0, armed - STAGES); kb < armed; ++kb) tc_drain(&full_bar[kb % STAGES], (kb / STAGES) & 1);
         return;
     }
@@ -239,7 +251,7 @@ __global__ void __launch_bounds__(PS_THREADS, 2) prompt_split_kernel(const __gri
             uint64_t ds = 0;
             for (int kb = 0, s = 0, phase = 0; kb < nkb; ++kb, ++s, ds += S::STAGE >> 4) {
                 if (s == STAGES) { s = 0; phase ^= 1; ds = 0; }
-                if (!tc_wait(&full_bar[s], phase, abort_flag, p.status, 61)) break;
+                if (!tc_wait(&full_bar[s], phase, &abort_flag, p.status, 61)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (int k = 0; k < TC_BK / 16; ++k) {
@@ -250,55 +262,195 @@ __global__ void __launch_bounds__(PS_THREADS, 2) prompt_split_kernel(const __gri
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&empty_bar[s])) : "memory");
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(acc_bar)) : "memory");
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&acc_bar)) : "memory");
         }
         __syncwarp();
-        if (C > 1) pr_cluster_wait();
+        if (CL > 1) pr_cluster_wait();
         asm volatile("bar.sync 2, 160;" ::: "memory");              // the epilogue warps have read the accumulator
-        if (*abort_flag) tc_drain(acc_bar, 0);                      // ... or gave it up: the products that were issued end first
+        if (abort_flag) tc_drain(&acc_bar, 0);                      // ... or gave it up: the products that were issued end first
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S::COLS) : "memory");
-        if (C > 1) { pr_cluster_arrive(); pr_cluster_wait(); }
+        if (CL > 1) { pr_cluster_arrive(); pr_cluster_wait(); }
         else asm volatile("bar.sync 3, 192;" ::: "memory");
         return;
     }
 
     // ---------------------------------------------------------------------- epilogue
-    const int te = (int)threadIdx.x - 64, ew = warp - 2, quad = warp & 3;
-    const int sub = lane & 15, hw = lane >> 4;          // half a warp takes a row: 16 chunks of 16 bytes
-    constexpr int PER = S::ROWS / 8;                    // rows a half-warp finishes
-    const int t0 = m0 + rank * R;                       // first owned token
-    float4 xr[KIND == PR_RESID ? PER : 1];
-    constexpr int RB = PER < 4 ? PER : 4;               // rows whose RoPE entries are requested together
-    PrRope rope[KIND == PR_QKV ? RB : 1];
-    auto rope_rows = [&](int i0) {
+    const int te = (int)threadIdx.x - 64, quad = warp & 3;
+    const uint32_t tacc = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const int row = quad * 32 + lane, trow = m0 + row;  // this thread's accumulator row and its token
+    const bool live = row < rows;
+
+    if constexpr (KIND == PR_QKV) {
+        // A thread holds BN / 2 dims of a head's row and the BN / 2 that RoPE pairs them with, for the row's scale and norm; then the warp's 32 rows go
+        // through shared memory (a stage: every MMA has completed), so that SUBS lanes finish a row and global accesses are runs of 8 SUBS to 16 SUBS bytes
+        // (a thread per row all the way: prompts of 128 / 256 / 512 tokens 1002 / 1154 / 1550 us, so 975 / 1079 / 1437).
+        constexpr int HALF = BN / 2, SUBS = BN / 8, STEP = 32 / SUBS, RB = SUBS < 8 ? SUBS : 8, LD = BN + 4;   // RB: rows whose RoPE entries are requested together
+        const int col0 = tile * HEAD_DIM, d0 = rank * HALF, sub = lane % SUBS, lr0 = lane / SUBS, w0 = m0 + quad * 32, wrows = min(32, rows - quad * 32);
+        const bool normed = col0 < Q_DIM + KV_DIM;
+        float* const piece = reinterpret_cast<float*>(base) + (size_t)quad * 32 * LD;
+        static_assert(STAGES * S::STAGE >= 128 * LD * 4, "the stages hold the rows");
+        PrRope rope[RB];
+        auto rope_rows = [&](int i0) {
 #pragma unroll
-        for (int i = 0; i < RB; ++i) rope[KIND == PR_QKV ? i : 0] = pr_rope(p, t0 + max(0, min((i0 + i) * 8 + ew * 2 + hw, my_rows - 1)), sub * 4);
-    };
-    if (KIND == PR_QKV && my_rows > 0) rope_rows(0);
-    pdl_wait();
-    // while the products run: the scales of the owned rows, or the residual they are added to
-    if (KIND != PR_RESID) {
-        if (te < my_rows) s_r[te] = pr_scale(p, t0 + te);
-    } else {
+            for (int i = 0; i < RB; ++i) rope[i] = pr_rope(p, w0 + max(0, min((i0 + i) * STEP + lr0, wrows - 1)), d0 + sub * 4);
+        };
+        if (normed && wrows > 0) rope_rows(0);
+        const bf16_raw* gp = pr_head_gain(p, col0) + d0 + sub * 4;
+        const float4 glo = pr_unpack4(__ldg(reinterpret_cast<const uint2*>(gp))), ghi = pr_unpack4(__ldg(reinterpret_cast<const uint2*>(gp + 64)));
+        pdl_wait();
+        const float r = live ? pr_scale(p, trow) : 0.f;
+        const bool summed = __all_sync(0xffffffffu, tc_wait_warp(&acc_bar, 0, &abort_flag, p.status, 62) && !abort_flag);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // (a whole head's 128 columns are read twice: once for their squares, once to be scaled)
+        constexpr bool TWICE = BN > 64;
+        uint32_t v[TWICE ? 1 : BN / 32][32];
+        float ss4[4] = {0.f, 0.f, 0.f, 0.f};
+        auto squares = [&](const uint32_t (&u)[32]) {
 #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            const int lr = i * 8 + ew * 2 + hw;
-            xr[i] = lr < my_rows ? *reinterpret_cast<const float4*>(p.x + (size_t)(t0 + lr) * HIDDEN + tile * BN + sub * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int j = 0; j < 32; ++j) { const float y = __uint_as_float(u[j]) * r; ss4[j & 3] = fmaf(y, y, ss4[j & 3]); }
+        };
+        auto read_out = [&]() {                          // the accumulator may go
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            asm volatile("bar.arrive 2, 160;" ::: "memory");
+        };
+        if constexpr (TWICE) {
+            if (normed)
+#pragma unroll
+                for (int c = 0; c < BN / 32; ++c) {
+                    tc_ld32(v[0], tacc + (uint32_t)(c * 32));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    squares(v[0]);
+                }
+        } else {
+#pragma unroll
+            for (int c = 0; c < BN / 32; ++c) tc_ld32(v[c], tacc + (uint32_t)(c * 32));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            read_out();
+#pragma unroll
+            for (int c = 0; c < BN / 32; ++c) squares(v[c]);
         }
+        float ss = (ss4[0] + ss4[1]) + (ss4[2] + ss4[3]);
+        if (CL > 1) {
+            // (a block whose sums are not complete sends NaN: no other passes its rows off as whole)
+            if (!summed) ss = __int_as_float(0x7fffffff);
+            pr_cluster_wait();
+            s_ss[rank][row] = ss;
+#pragma unroll
+            for (int o = 1; o < CL; ++o)
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(pr_map(tc_smem(&s_ss[rank][row]), (rank + o) % CL)), "f"(ss) : "memory");
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+            ss = 0.f;
+#pragma unroll
+            for (int o = 0; o < CL; ++o) ss += s_ss[o][row];
+        }
+        const float f = normed ? r * rsqrtf(ss / (float)HEAD_DIM + EPS) : r;
+        auto put = [&](const uint32_t (&u)[32], int c) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+                *reinterpret_cast<float4*>(piece + lane * LD + c * 32 + j) = make_float4(__uint_as_float(u[j]) * f, __uint_as_float(u[j + 1]) * f, __uint_as_float(u[j + 2]) * f, __uint_as_float(u[j + 3]) * f);
+        };
+        if constexpr (TWICE) {
+#pragma unroll
+            for (int c = 0; c < BN / 32; ++c) {
+                tc_ld32(v[0], tacc + (uint32_t)(c * 32));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (summed) put(v[0], c);
+            }
+            read_out();
+        }
+        if (summed && wrows > 0) {
+            if constexpr (!TWICE) {
+#pragma unroll
+                for (int c = 0; c < BN / 32; ++c) put(v[c], c);
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int i0 = 0; i0 * STEP < wrows; i0 += RB) {
+#pragma unroll
+                for (int i = 0; i < RB; ++i) {
+                    const int lr = (i0 + i) * STEP + lr0;
+                    if (lr < wrows)
+                        pr_finish_head(p, col0, w0 + lr, d0 + sub * 4, *reinterpret_cast<const float4*>(piece + lr * LD + sub * 4),
+                                       *reinterpret_cast<const float4*>(piece + lr * LD + HALF + sub * 4), glo, ghi, rope[i]);
+                }
+                if (normed && (i0 + RB) * STEP < wrows) rope_rows(i0 + RB);
+            }
+        }
+        if (CL == 1) asm volatile("bar.sync 3, 192;" ::: "memory");
+        return;
+    }
+    if constexpr (KIND == PR_SILU) {
+        // (through shared memory, for runs of BN bytes in a row: the warp's 32 rows, an odd number of 16-byte units apart)
+        constexpr int HALF = BN / 2, STEP = HALF % 16 ? 8 : 16, UNITS = HALF / 8, LD = UNITS | 1;
+        uint4* const piece = reinterpret_cast<uint4*>(base) + (size_t)quad * 32 * LD;
+        static_assert(STAGES * S::STAGE >= 128 * LD * 16, "the stages hold the rows");
+        pdl_wait();
+        const float r = live ? pr_scale(p, trow) : 0.f;
+        const bool summed = __all_sync(0xffffffffu, tc_wait_warp(&acc_bar, 0, &abort_flag, p.status, 62) && !abort_flag);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int wrows = min(32, rows - quad * 32);
+        if (summed && wrows > 0) {
+#pragma unroll
+            for (int c0 = 0; c0 < HALF; c0 += 3 * STEP) {
+                uint32_t g[3][STEP], u[3][STEP];
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    if (c0 + c * STEP < HALF) {
+                        if constexpr (STEP == 16) { tc_ld16(g[c], tacc + (uint32_t)(c0 + c * STEP)); tc_ld16(u[c], tacc + (uint32_t)(HALF + c0 + c * STEP)); }
+                        else { tc_ld8(g[c], tacc + (uint32_t)(c0 + c * STEP)); tc_ld8(u[c], tacc + (uint32_t)(HALF + c0 + c * STEP)); }
+                    }
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    if (c0 + c * STEP < HALF) {
+                        uint32_t w[STEP / 2];
+#pragma unroll
+                        for (int j = 0; j < STEP / 2; ++j)
+                            w[j] = pr_pack(pr_silu(__uint_as_float(g[c][2 * j]) * r, __uint_as_float(u[c][2 * j]) * r),
+                                           pr_silu(__uint_as_float(g[c][2 * j + 1]) * r, __uint_as_float(u[c][2 * j + 1]) * r));
+#pragma unroll
+                        for (int j = 0; j < STEP / 8; ++j) piece[lane * LD + (c0 + c * STEP) / 8 + j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+                    }
+            }
+            __syncwarp();
+            bf16_raw* const dst = p.hid + (size_t)(m0 + quad * 32) * INTER + tile * HALF;
+#pragma unroll 4
+            for (int i = lane; i < wrows * UNITS; i += 32) {
+                const int lr = i / UNITS, j = i - lr * UNITS;
+                *reinterpret_cast<uint4*>(dst + (size_t)lr * INTER + j * 8) = piece[lr * LD + j];
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        asm volatile("bar.arrive 2, 160;" ::: "memory");
+        asm volatile("bar.sync 3, 192;" ::: "memory");
+        return;
+    }
+    if constexpr (KIND == PR_RESID) {
+    constexpr int SUBS = BN / 4, STEP = 128 / SUBS;     // lanes a row (a chunk of 16 bytes each), rows the four warps take at a time
+    constexpr int PER = (S::ROWS + STEP - 1) / STEP;    // rows a thread has a chunk of
+    const int sub = te % SUBS, lr0 = te / SUBS;
+    const int t0 = m0 + slice * R;                      // first owned token
+    float4 xr[PER];
+    pdl_wait();
+    // while the products run: the residual they are added to
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int lr = i * STEP + lr0;
+        xr[i] = lr < my_rows ? *reinterpret_cast<const float4*>(p.x + (size_t)(t0 + lr) * HIDDEN + tile * BN + sub * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     // (the MMA thread commits to acc_bar after a wait of its own gave up, too, so that its products can be drained: the flag tells)
-    const bool summed = __all_sync(0xffffffffu, tc_wait_warp(acc_bar, 0, abort_flag, p.status, 62) && !*abort_flag);
+    const bool summed = __all_sync(0xffffffffu, tc_wait_warp(&acc_bar, 0, &abort_flag, p.status, 62) && !abort_flag);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // the partial tile, a thread per token row (the stages are free: every MMA has completed)
     if (summed && quad * 32 < rows) {
-        const int row = quad * 32 + lane;
         unsigned char* dst = base + (size_t)row * BN * 4;
 #pragma unroll
         for (int c0 = 0; c0 < BN; c0 += 32) {
             uint32_t r[32];
-            tc_ld32(r, tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0);
+            tc_ld32(r, tacc + (uint32_t)c0);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int j = 0; j < 8; ++j)
@@ -310,17 +462,17 @@ __global__ void __launch_bounds__(PS_THREADS, 2) prompt_split_kernel(const __gri
     asm volatile("bar.arrive 2, 160;" ::: "memory");
     if (C > 1) pr_cluster_wait();                       // every block of the cluster has set its mbarriers up
     asm volatile("bar.sync 1, 128;" ::: "memory");
-    const bool whole = !*abort_flag;                    // no warp of this block gave up on the accumulator
+    const bool whole = !abort_flag;                     // no warp of this block gave up on the accumulator
     bool received = whole;
     if (C > 1) {
-        if (whole && te < C && te != rank && rows_of(te) > 0) {
-            const int slot = rank < te ? rank : rank - 1;
+        if (whole && te < C && te != slice && rows_of(te) > 0) {
+            const int slot = slice < te ? slice : slice - 1;
             const uint32_t src = tc_smem(base) + (uint32_t)(te * R * BN * 4);
             asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(pr_map(tc_smem(red) + (uint32_t)(slot * R * BN * 4), te)), "r"(src), "r"((uint32_t)(rows_of(te) * BN * 4)), "r"(pr_map(tc_smem(red_bar), te)) : "memory");
+                         ::"r"(pr_map(tc_smem(red) + (uint32_t)(slot * R * BN * 4), te)), "r"(src), "r"((uint32_t)(rows_of(te) * BN * 4)), "r"(pr_map(tc_smem(&red_bar), te)) : "memory");
         }
         __syncwarp();
-        received = my_rows > 0 && whole && tc_wait_warp(red_bar, 0, abort_flag, p.status, 63, PS_RED_WAIT_NS);
+        received = my_rows > 0 && whole && tc_wait_warp(&red_bar, 0, &abort_flag, p.status, 63, PS_RED_WAIT_NS);
     }
 
     // 16-byte chunk `j` of owned row `lr`, the slices added in order
@@ -329,81 +481,37 @@ __global__ void __launch_bounds__(PS_THREADS, 2) prompt_split_kernel(const __gri
         float4 v;
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            const unsigned char* src = c == rank ? base + (size_t)rank * R * BN * 4 : reinterpret_cast<unsigned char*>(red) + (size_t)(c < rank ? c : c - 1) * R * BN * 4;
+            const unsigned char* src = c == slice ? base + (size_t)slice * R * BN * 4 : reinterpret_cast<unsigned char*>(red) + (size_t)(c < slice ? c : c - 1) * R * BN * 4;
             const float4 u = *reinterpret_cast<const float4*>(src + off);
             v = c ? pr_add(v, u) : u;
         }
         return v;
     };
     if (received) {
-        if constexpr (KIND == PR_QKV) {
-            const int col0 = tile * BN;
-            const bf16_raw* gp = pr_head_gain(p, col0);
-            const float4 glo = pr_unpack4(*reinterpret_cast<const uint2*>(gp + sub * 4)), ghi = pr_unpack4(*reinterpret_cast<const uint2*>(gp + 64 + sub * 4));
-#pragma unroll 1
-            for (int i0 = 0; i0 < PER && i0 * 8 + ew * 2 < my_rows; i0 += RB) {
-                float4 lo[RB], hi[RB];
+        const float4 g = pr_unpack4(*reinterpret_cast<const uint2*>(p.gain + tile * BN + sub * 4));
 #pragma unroll
-                for (int i = 0; i < RB; ++i) {
-                    const int lc = min((i0 + i) * 8 + ew * 2 + hw, my_rows - 1);
-                    const float r = s_r[lc];
-                    lo[i] = pr_mul(sum(lc, sub), r); hi[i] = pr_mul(sum(lc, 16 + sub), r);
-                }
-                if (col0 < Q_DIM + KV_DIM) {
-                    float ss[RB];
+        for (int i = 0; i < PER; ++i) {
+            if (i * STEP + (te & ~31) / SUBS >= my_rows) break;     // (the same for the whole warp)
+            const int lr = i * STEP + lr0, lc = min(lr, my_rows - 1), t = t0 + lr;
+            const float4 x = pr_add(xr[i], sum(lc, sub));
+            float ss = pr_dot(x, x);
 #pragma unroll
-                    for (int i = 0; i < RB; ++i) ss[i] = pr_dot(lo[i], lo[i]) + pr_dot(hi[i], hi[i]);
-#pragma unroll
-                    for (int o = 8; o > 0; o >>= 1)
-#pragma unroll
-                        for (int i = 0; i < RB; ++i) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], o);
-#pragma unroll
-                    for (int i = 0; i < RB; ++i) {
-                        const float n = rsqrtf(ss[i] / (float)HEAD_DIM + EPS);
-                        lo[i] = pr_mul(lo[i], n); hi[i] = pr_mul(hi[i], n);
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < RB; ++i) {
-                    const int lr = (i0 + i) * 8 + ew * 2 + hw;
-                    if (lr < my_rows) pr_finish_head(p, col0, t0 + lr, sub * 4, lo[i], hi[i], glo, ghi, rope[i]);
-                }
-                if (i0 + RB < PER) rope_rows(i0 + RB);
-            }
-        } else if constexpr (KIND == PR_RESID) {
-            const float4 g = pr_unpack4(*reinterpret_cast<const uint2*>(p.gain + tile * BN + sub * 4));
-#pragma unroll
-            for (int i = 0; i < PER; ++i) {
-                if (i * 8 + ew * 2 >= my_rows) break;
-                const int lr = i * 8 + ew * 2 + hw, lc = min(lr, my_rows - 1), t = t0 + lr;
-                const float4 x = pr_add(xr[i], sum(lc, sub));
-                float ss = pr_dot(x, x);
-#pragma unroll
-                for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                if (lr < my_rows) {
-                    const size_t o = (size_t)t * HIDDEN + tile * BN + sub * 4;
-                    *reinterpret_cast<float4*>(p.x + o) = x;
-                    *reinterpret_cast<uint2*>(p.xn + o) = pr_pack4(pr_mul(x, g));
-                    if (sub == 0) p.ssq_out[(size_t)tile * p.ssq_ld + t] = ss;
-                }
-            }
-        } else {
-            constexpr int CH = BN / 8;                  // 16-byte chunks of a half row
-            for (int i = te; i < my_rows * CH; i += 128) {
-                const int lr = i / CH, j = i - lr * CH;
-                const float r = s_r[lr];
-                const float4 g = pr_mul(sum(lr, j), r), u = pr_mul(sum(lr, CH + j), r);
-                *reinterpret_cast<uint2*>(p.hid + (size_t)(t0 + lr) * INTER + tile * (BN / 2) + j * 4) =
-                    pr_pack4(make_float4(pr_silu(g.x, u.x), pr_silu(g.y, u.y), pr_silu(g.z, u.z), pr_silu(g.w, u.w)));
+            for (int o = SUBS / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (lr < my_rows) {
+                const size_t o = (size_t)t * HIDDEN + tile * BN + sub * 4;
+                *reinterpret_cast<float4*>(p.x + o) = x;
+                *reinterpret_cast<uint2*>(p.xn + o) = pr_pack4(pr_mul(x, g));
+                if (sub == 0) p.ssq_out[(size_t)tile * p.ssq_ld + t] = ss;
             }
         }
     }
     if (C > 1) {
         pr_cluster_arrive();      // (matched before the exit: this block's copies have been counted by their receivers or given up)
         pr_cluster_wait();
-        if (my_rows > 0 && !received && te == 0) tc_drain(red_bar, 0);
+        if (my_rows > 0 && !received && te == 0) tc_drain(&red_bar, 0);
     } else {
         asm volatile("bar.sync 3, 192;" ::: "memory");
+    }
     }
 }
 
@@ -757,16 +865,16 @@ static cudaError_t pr_prepare(K kernel, size_t smem, bool (&done)[64]) {   // (a
     return e;
 }
 
-template <int KIND, int C>
+template <int KIND, int BN, int C, int OCC>
 static cudaError_t launch_split(const CUtensorMap* tw, const CUtensorMap& tx, const PromptParams& p, cudaStream_t st) {
-    using S = PsShape<KIND, C>;
+    using S = PsShape<KIND, BN, C, OCC>;
     static bool done[64] = {};
-    cudaError_t e = pr_prepare(prompt_split_kernel<KIND, C>, S::SMEM, done);
+    cudaError_t e = pr_prepare(prompt_split_kernel<KIND, BN, C, OCC>, S::SMEM, done);
     if (e != cudaSuccess) return e;
-    constexpr int tiles = KIND == PR_QKV ? QKV_DIM / S::BN : KIND == PR_RESID ? HIDDEN / S::BN : 2 * INTER / S::BN;
-    const dim3 grid(C, tiles, (p.T + PR_BM - 1) / PR_BM);
-    if constexpr (C == 1) return launch_chain(prompt_split_kernel<KIND, C>, grid, dim3(PS_THREADS), S::SMEM, st, tw[0], tw[1], tw[2], tx, p);
-    else return launch_chain_cluster(prompt_split_kernel<KIND, C>, grid, dim3(PS_THREADS), S::SMEM, C, st, tw[0], tw[1], tw[2], tx, p);
+    constexpr int tiles = KIND == PR_QKV ? QKV_DIM / HEAD_DIM : KIND == PR_RESID ? HIDDEN / BN : 2 * INTER / BN;
+    const dim3 grid(S::CL, tiles, (p.T + PR_BM - 1) / PR_BM);
+    if constexpr (S::CL == 1) return launch_chain(prompt_split_kernel<KIND, BN, C, OCC>, grid, dim3(PS_THREADS), S::SMEM, st, tw[0], tw[1], tw[2], tx, p);
+    else return launch_chain_cluster(prompt_split_kernel<KIND, BN, C, OCC>, grid, dim3(PS_THREADS), S::SMEM, S::CL, st, tw[0], tw[1], tw[2], tx, p);
 }
 
 template <int KIND, int BN>
@@ -784,48 +892,52 @@ static cudaError_t launch_pair(const CUtensorMap* tw, const CUtensorMap& tx, Pro
 cudaError_t launch_prompt_gemm(const PromptGemmCall& c, cudaStream_t st) {
     if (c.T < 1 || c.K % TC_BK || c.K < 8 * TC_BK || c.ssq_ld < c.T) return cudaErrorInvalidValue;
     PromptParams p{};
+    p.a_rows = prompt_box_rows(c.T);
     p.T = c.T; p.kb_total = c.K / TC_BK; p.ssq_ld = c.ssq_ld; p.ssq_in = c.ssq; p.ssq_out = c.ssq;
     p.q_hi = c.q_hi; p.q_lo = c.q_lo; p.qkv = c.qkv; p.kc = c.kc; p.vc = c.vc; p.qn = c.qn; p.kn = c.kn; p.rope = c.rope;
     p.x = c.x; p.xn = c.xn; p.gain = c.gain; p.hid = c.hid; p.status = c.status;
     const int sm = tc_sm_count();
     if (sm < 2) return cudaErrorInvalidDevice;
     const int mt = (c.T + PR_BM - 1) / PR_BM;
-    // The deepest cut of K whose blocks still fit the GPU at once (two on an SM), the pair kernel when not even whole tiles do.  Measured,
-    // us a launch in a stream of its own kind, pair / uncut / 2 / 4 / 8 slices:
-    //   q/k/v    128 tokens 14.2 / 11.8 / 11.7 / 10.6;  512: 14.5 / 13.1 / 11.7 / 20.5;  1024: 14.2 / 13.6;  1280: 19.7 / 22.5
-    //   Wo       128 tokens 14.1 / 13.2 / 9.0 / 8.1 / 7.0;  512: 14.5 / 13.2 / 9.6 / 8.8 / 14.0;  777: 14.6 / 13.2 / 10.0 / 14.9;  2048: 14.8 / 14.4
-    //   down     128 tokens 17.9 / 17.6 / 11.2 / 9.5 / 7.5;  512: 18.4 / 17.2 / 11.6 / 10.1 / 15.6;  777: 18.6 / 17.0 / 12.4 / 17.4;  2048: 18.7 / 19.5
-    //   gate/up  64 tokens 10.6 / 8.6 / 7.3 / 6.6;  128: 11.0 / 9.7 / 8.6 / 9.2;  512: 11.4 / 9.8 / 16.1;  640: 11.2 / 17.1;  2048: 22.1 / 36.5
-    // (four slices of gate/up exchange three quarters of a tile: up to 64 tokens that is less than the two waits for its ring that it saves)
-    const int blocks = (c.kind == PR_QKV ? 32 : c.kind == PR_RESID ? 16 : 64) * mt, most = c.kind == PR_QKV ? 4 : c.kind == PR_RESID ? 8 : c.T <= 64 ? 4 : 2;
-    const bool pair = blocks > 2 * sm;
-    int cut = 1;
-    while (cut < most && 2 * cut * blocks <= 2 * sm) cut *= 2;
+    // The shape by the number of 128-token tiles: about one block an SM while tiles are narrow enough for that, then two an SM, then pairs.
+    // Measured, us a prompt with every product as below but for one (128-row columns / slices / blocks an SM; 0: the pair kernel):
+    //   q/k/v    128 tokens 32//1 970, 32//2 1010, 64//1 1007;  256: 64//1 1099, 32//2 1099, 64//2 1108;  300: 64//2 1292, 128//1 1316;  512: 64//2 1388, 128//1
+    //            1411;  640: 128//2 1750, 0 1807, 64//2 1865;  1000: 2030, 0 2080;  1150: 2092, 0 2333;  1290: 0 2456, 128//2 2502
+    //   gate/up  64 tokens 48//2 917, 48//1 933;  128: 970, 977, 96//1 1007;  256: 96//1 1101, 48//2 1098;  300: 128//1 1292, 192//1 1346;  512: 192//1 1388, 96//2
+    //            1393, 0 1437;  520: 128//2 1733, 0 1742;  777: 0 1952, 192//1 1967;  1290: 0 2454, 128//2 2571
+    //   Wo, down 64 tokens 32/8/2 917, 32/4/1 938;  128: 970, 972, 64/4/1 1032;  256: 64/4/1 1099, 32/4/2 1169;  300: 64/4/2 1292, 64/2/1 1306;  512: 1388, 1416;
+    //            640: 64/2/2 1772, 0 1964;  1150: 64/2/2 2096, 0 2201;  1290: 0 2455, 64/1/2 2588
+    const bool pair = mt > (c.kind == PR_SILU ? 4 : 9);
+    const int bn = c.kind == PR_QKV ? (mt == 1 ? 32 : mt <= 4 ? 64 : 128) : c.kind == PR_RESID ? (mt == 1 ? 32 : 64) : mt == 1 ? 48 : mt == 2 ? 96 : mt == 3 ? 128 : 192;
     const int rows[3] = {c.kind == PR_QKV ? Q_DIM : c.kind == PR_RESID ? HIDDEN : INTER, c.kind == PR_QKV ? KV_DIM : INTER, KV_DIM};
     const int n_w = c.kind == PR_QKV ? 3 : c.kind == PR_RESID ? 1 : 2;
-    const uint32_t box = c.kind == PR_QKV ? 128u : c.kind == PR_RESID ? 64u : pair ? 128u : 48u;
+    const uint32_t box = pair ? (c.kind == PR_RESID ? 64u : 128u) : c.kind == PR_RESID ? (uint32_t)bn : (uint32_t)bn / 2;
     CUtensorMap tw[3];
     for (int i = 0; i < 3; ++i) {
         if (i >= n_w) tw[i] = tw[0];
         else if (!tc_cached_map(c.w[i], (uint64_t)rows[i], (uint64_t)c.K, box, &tw[i])) return cudaErrorUnknown;
     }
+    p.ssq_parts = *c.parts;
+    if (c.kind == PR_RESID) *c.parts = pair ? HIDDEN / 64 : HIDDEN / bn;
     switch (c.kind) {
         case PR_QKV:
             if (pair) return launch_pair<PR_QKV, 256>(tw, *c.in, p, sm, st);
-            if (cut == 4) return launch_split<PR_QKV, 4>(tw, *c.in, p, st);
-            if (cut == 2) return launch_split<PR_QKV, 2>(tw, *c.in, p, st);
-            return launch_split<PR_QKV, 1>(tw, *c.in, p, st);
+            if (mt == 1) return launch_split<PR_QKV, 32, 1, 1>(tw, *c.in, p, st);
+            if (mt == 2) return launch_split<PR_QKV, 64, 1, 1>(tw, *c.in, p, st);
+            if (mt <= 4) return launch_split<PR_QKV, 64, 1, 2>(tw, *c.in, p, st);
+            return launch_split<PR_QKV, 128, 1, 2>(tw, *c.in, p, st);
         case PR_RESID:
             if (pair) return launch_pair<PR_RESID, 128>(tw, *c.in, p, sm, st);
-            if (cut == 8) return launch_split<PR_RESID, 8>(tw, *c.in, p, st);
-            if (cut == 4) return launch_split<PR_RESID, 4>(tw, *c.in, p, st);
-            if (cut == 2) return launch_split<PR_RESID, 2>(tw, *c.in, p, st);
-            return launch_split<PR_RESID, 1>(tw, *c.in, p, st);
+            if (mt == 1) return launch_split<PR_RESID, 32, 8, 2>(tw, *c.in, p, st);
+            if (mt == 2) return launch_split<PR_RESID, 64, 4, 1>(tw, *c.in, p, st);
+            if (mt <= 4) return launch_split<PR_RESID, 64, 4, 2>(tw, *c.in, p, st);
+            return launch_split<PR_RESID, 64, 2, 2>(tw, *c.in, p, st);
         case PR_SILU:
             if (pair) return launch_pair<PR_SILU, 256>(tw, *c.in, p, sm, st);
-            if (cut == 4) return launch_split<PR_SILU, 4>(tw, *c.in, p, st);
-            if (cut == 2) return launch_split<PR_SILU, 2>(tw, *c.in, p, st);
-            return launch_split<PR_SILU, 1>(tw, *c.in, p, st);
+            if (mt == 1) return launch_split<PR_SILU, 48, 1, 2>(tw, *c.in, p, st);
+            if (mt == 2) return launch_split<PR_SILU, 96, 1, 1>(tw, *c.in, p, st);
+            if (mt == 3) return launch_split<PR_SILU, 128, 1, 1>(tw, *c.in, p, st);
+            return launch_split<PR_SILU, 192, 1, 1>(tw, *c.in, p, st);
     }
     return cudaErrorInvalidValue;
 }

@@ -9,7 +9,8 @@ struct CUtensorMap_st;   // <cuda.h>'s tensor map
 
 namespace q3 {
 
-constexpr int PR_SSQ_PARTS = 16;   // partial sums of squares of a residual row: one per 64 elements
+constexpr int PR_SSQ_PARTS = 16;   // partial sums of squares of a residual row that the embedding gather leaves: one per 64 elements
+constexpr int PR_SSQ_MOST = 32;    // ... that a launch may leave: one per tile of weight rows
 
 enum { PR_QKV = 0, PR_RESID = 1, PR_SILU = 2 };
 
@@ -18,9 +19,10 @@ enum { PR_QKV = 0, PR_RESID = 1, PR_SILU = 2 };
 struct PromptGemmCall {
     int kind, T, K;
     const void* w[3];              // PR_QKV: Wq, Wk, Wv; PR_RESID: Wo or Wd; PR_SILU: Wg, Wu
-    const ::CUtensorMap_st* in;    // boxes of 128 rows x 64 columns over [T][K]
-    float* ssq;                    // [PR_SSQ_PARTS][ssq_ld]: written by PR_RESID, read by the other two
+    const ::CUtensorMap_st* in;    // boxes of prompt_box_rows(T) rows x 64 columns over [T][K]
+    float* ssq;                    // [PR_SSQ_MOST][ssq_ld]: written by PR_RESID, read by the other two
     int ssq_ld;
+    int* parts;                    // how many of them a row has: set by PR_RESID, read by the other two
     // PR_QKV: head norm, RoPE, then
     bf16_raw *q_hi, *q_lo;         // [T][2048] q times the softmax scale as two planes (read by the tiled attention), or
     float* qkv;                    // [T][4096] fp32 q, k, v rows (read by the split attention of few tokens)
@@ -35,6 +37,8 @@ struct PromptGemmCall {
     bf16_raw* hid;                 // [T][3072]
     uint32_t* status;
 };
+// rows of the boxes over the activations: no more than the prompt has (rows past it would be filled with zeros at a row's price: 16 tokens 1045 -> 837 us)
+inline int prompt_box_rows(int T) { return T < 128 ? (T + 15) / 16 * 16 : 128; }
 cudaError_t launch_prompt_gemm(const PromptGemmCall& c, cudaStream_t st);
 
 // x[t] = embed[ids[t]], its plane times `gain`, its partial sums of squares; a bad id is reported and read as 0

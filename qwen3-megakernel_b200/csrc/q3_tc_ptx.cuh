@@ -79,6 +79,11 @@ __device__ __forceinline__ void tc_ld16(uint32_t* r, uint32_t taddr) {   // 16 c
                  : "r"(taddr) : "memory");
 }
 
+__device__ __forceinline__ void tc_ld8(uint32_t* r, uint32_t taddr) {   // 8 columns of this warp's 32 TMEM lanes; no wait
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+
 __device__ __forceinline__ void tc_ld4(uint32_t (&r)[4], uint32_t taddr) {   // 4 columns of this warp's 32 TMEM lanes; no wait
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
 }

@@ -442,6 +442,13 @@ def test_prompt_products_at_the_edges_of_their_tiles(oracle, small, T):
     assert torch.equal(again[0], kc) and torch.equal(again[1], vc) and torch.equal(again[2], last)
 
 
+@pytest.mark.parametrize("T", [15, 16, 17, 33, 100, 112, 127, 255, 300, 384])
+def test_prompts_of_narrow_tiles(oracle, small, T):
+    """Prompts that fill no 128-token tile load boxes of their own length, in steps of 16 rows; up to four tiles the products take narrow
+    tiles of weight rows (a quarter or half of a head, 24 to 96 columns of gate and up) and no or few slices of K."""
+    test_prompt_products_at_the_edges_of_their_tiles(oracle, small, T)
+
+
 @pytest.mark.parametrize("floats", [1, 2, 3])
 def test_rope_table_at_any_address(oracle, small, floats):
     """A RoPE table that is not 16-byte aligned gives the results of one that is: prompts (matrix-vector kernels, k slices with either
