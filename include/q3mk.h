@@ -35,7 +35,7 @@ extern "C" {
 
 /* q3_decode_args.flags */
 #define Q3_F_APPEND_KV    0x1u  /* write the new K/V rows into cache slot seq_len[b], then seq_len[b] += 1 */
-#define Q3_F_PATH_AUTO    0x0u  /* engine picks: persistent kernel for one sequence it serves, layered otherwise */
+#define Q3_F_PATH_AUTO    0x0u  /* engine picks: persistent kernel for up to three sequences it serves, layered otherwise */
 #define Q3_F_PATH_LAYERED 0x10u /* a chain of launches: five per layer up to 64 sequences, one per phase beyond */
 #define Q3_F_PATH_FUSED   0x30u /* layered, but batches of 4..64 run two launches per layer: split attention + one persistent
                                    kernel for Wo, norm, gate/up, SiLU, down, norm and the next layer's q/k/v (opt-in: measured
@@ -144,7 +144,7 @@ int q3_tp_attach(q3_engine* e, int32_t rank, int32_t size, const void* handles);
 /* RoPE table: device fp32 [n_positions][128], row p = cos(p * f_0..f_63) then sin(p * f_0..f_63),
  * f_i = 1e6^(-2i/128).  Generalises the reference's single-position table
  * (qwen3mk/kernel.py:102-106).  Any address a float may have serves; the persistent kernel
- * only takes a 16-byte aligned table, one sequence takes the launch chain otherwise.  Borrowed. */
+ * only takes a 16-byte aligned table, its sequences take the launch chain otherwise.  Borrowed. */
 int q3_set_rope(q3_engine* e, const float* table, int32_t n_positions);
 
 /* Enqueue one decode step on `stream` (a cudaStream_t; NULL = default stream).  No host sync.

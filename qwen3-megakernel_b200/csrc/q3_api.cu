@@ -45,10 +45,11 @@ int q3::engine_fail(q3_engine* e, int code, const char* fmt, ...) {
 // ------------------------------------------------------------------------------------------------
 // The key holds the addresses of one bind, so every bind captures anew.  A capture costs the host 450 to 850 us, beside 360 for the
 // plain launches of a step; after three steps that are launched without waiting the GPU is far enough behind to hide it (8 x 1024, a fresh
-// bind of 8 steps, capture on the 2nd / 4th: 6070 / 5910 us; of 2 steps 1680 / 1540).  Two sequences pay it back more slowly,
-// for the persistent kernel serves them almost as fast: from eight steps on even a caller who waits for every step has gained it (at 16
-// positions 4 steps: persistent 2880, captured on the 4th 3110; a plain step 669 against 728).
-static int plain_uses(int batch) { return batch == 2 ? 8 : 3; }
+// bind of 8 steps, capture on the 2nd / 4th: 6070 / 5910 us; of 2 steps 1680 / 1540).  Where
+// the steps before the capture are not plain launches of the chain but launches of the persistent kernel (three sequences: a replay saves 5 to 25 us
+// on those), and for two sequences of a caller who names the chain (at 16 positions 4 steps: a persistent launch a sequence 2880, captured on
+// the 4th 3110), the capture waits until the ninth.
+static int plain_uses(int batch, bool persist) { return batch == 2 || persist ? 8 : 3; }
 struct GraphEntry {
     q3_decode_args key;
     int n_splits;
@@ -539,12 +540,14 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
     CU(e, cudaSetDevice(e->device));
     cudaStream_t st = (cudaStream_t)stream;
     uint32_t path = a->flags & Q3_F_PATH_MASK;
-    // The persistent kernel decodes one sequence per launch: from two on, one chain over all of them is faster and as close to fp64 (one
-    // after the other against the chain: two sequences at 16 / 250 / 3400 positions 702 / 755 / 1341 and 593 / 622 / 766 us, three at 900
-    // 1331 and 651 us; in plain launches, before a graph replays them, two at 16 positions 703 and 650 us; one sequence at 16 / 250 /
-    // 1000 347 / 384 / 456 us against 567 and more).
-    if (path == Q3_F_PATH_AUTO)
-        path = a->batch == 1 && persist_supports(e, a) ? Q3_F_PATH_PERSIST : Q3_F_PATH_LAYERED;
+    // One launch of the persistent kernel for one or two sequences, a chain of launches for more; three take the kernel as long as the chain would
+    // be plain launches (the times stand at q3_persist.cu's limits).
+    bool until_captured = false;
+    if (path == Q3_F_PATH_AUTO) {
+        path = persist_supports(e, a) ? Q3_F_PATH_PERSIST : Q3_F_PATH_LAYERED;
+        until_captured = path == Q3_F_PATH_PERSIST && a->batch == 3 && (a->flags & Q3_F_GRAPH);
+        if (until_captured) path = Q3_F_PATH_LAYERED;
+    }
     if (path == Q3_F_PATH_PERSIST) {
         if (!persist_supports(e, a))
             return fail(e, Q3_ERR_UNSUPPORTED, "q3_decode: the persistent kernel does not serve batch %d at length %d with a RoPE table at %p", a->batch, a->max_len, (const void*)e->rope);
@@ -575,7 +578,7 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
         e->launches += hit->launches;
         return Q3_OK;
     }
-    if (hit->seen++ < plain_uses(a->batch)) return decode_layered(e, a, st, false, layer_kernel);
+    if (hit->seen++ < plain_uses(a->batch, until_captured)) return until_captured ? persist_decode(e, a, st) : decode_layered(e, a, st, false, layer_kernel);
     const int64_t before = e->launches;
     // capture on the engine's own stream (the legacy default stream cannot be captured); nothing runs during capture
     cudaStream_t cs = static_cast<cudaStream_t>(e->capture_stream);

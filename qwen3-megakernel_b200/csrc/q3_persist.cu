@@ -1,4 +1,4 @@
-// Persistent cooperative decode kernel: one launch runs a whole batch-1 decode step.
+// Persistent cooperative decode kernel: one launch runs a whole decode step of one, two or three sequences.
 //
 // One CTA of 16 warps per SM.  The schedule is static (every CTA owns fixed weight rows, all of them resident
 // in its 227 KB of shared memory for the layer at hand) and a layer has ONE grid barrier; the other two exchanges
@@ -56,22 +56,30 @@ constexpr int WO_SLICES = 9;                  // row slices of Wo; CTA c < 144 o
 constexpr int F_CTAS = Q_HEADS * WO_SLICES;   // 144
 constexpr int GROUP_CTAS = 2 * WO_SLICES;     // CTAs sharing one kv head
 constexpr int WO_ROWS_MAX = 116;              // largest slice: 4 * ceil(256 / 9)
-constexpr int PERSIST_MAX_BATCH = 3;          // sequences served by back-to-back launches when the caller asks for this kernel
+constexpr int PERSIST_MAX_BATCH = 3;          // sequences a launch decodes; one after the other where the caller asks for this kernel by name
 constexpr int MIN_GRID = 147;                 // row shares must fit the shared-memory slots
-constexpr int SC_HALF = 128;                  // the score buffer of the local attention holds 3 * SC_HALF floats
+constexpr int SC_FLOATS = 360;                // the score buffer of the local attention, which serves up to 255 positions
 // Most cached positions this kernel is picked for: the longest at which it was timed against the launch chain (one sequence, us per step, this
-// kernel / the chain: 5000 positions 542 / 768, 16000 826 / 1268, 29999 1183 / 1881).
+// kernel / the chain: 5000 positions 513 / 768, 16000 826 / 1268, 29999 1183 / 1881).
 constexpr int PERSIST_MAX_LEN = 30000;
+// Two sequences at 16 / 1500 / 8000 / 29000 positions 502 / 577 / 903 / 1930 us against 573 / 657 / 987 / 2029.  Three at 16 / 600 / 1300 / 2000
+// 599 / 632 / 679 / 733 (24 columns are three MMAs a tile, and the registers of a pass do not all fit: 164 bytes of spills) against 624 / 668 /
+// 697 / 729 in plain launches and 576 / 626 / 654 / 685 from a graph: in place of plain launches, up to
+constexpr int PERSIST_THREE_LEN = 1500;
 constexpr int PERSIST_ASKED_LEN = 3438;       // ... and that a caller may ask for who names this kernel: the limit that request has always had
 constexpr int WROW = 1032;                    // elements between weight rows in shared memory: 1024 + 8 of padding, so that
                                               // the eight row addresses of an ldmatrix fall into different banks
+// Words between the three parts of an activation vector in shared memory: a lane of the products reads word `kp` of the part of its column, so
+// parts a multiple of 32 words apart would meet in the same banks (three columns 13 us of 338 a step at 128 positions).
+constexpr int XLD = 516, OLD = 68, HLD = 20, LLD = 528;   // x (512 words), a head's output (64), hid (16), the LM head's input (512, read 16 bytes a lane)
 constexpr int WOROW = 136;                    // the same for the 128-column Wo slice rows
 // Local attention (every CTA attends its whole head over all cached positions) serves up to 255 positions; measured,
 // splitting the positions over the 18 CTAs of a kv group wins beyond that.
-#ifndef Q3_N_ACC
-#define Q3_N_ACC 2
-#endif
-constexpr int N_ACC = Q3_N_ACC;               // accumulators for the FFN delta (fewer same-address atomics each)
+// Accumulators of the FFN delta, for launches of nb sequences.  Every block adds to one of them, so fewer adds meet on an address and fewer roundings
+// follow one another.  One sequence: two.  Several: four, which keeps their logits as close to fp64 as the launch chain's (rel-L2, two sequences
+// of 16 / 250 / 1000 / 4000 positions, chain 1.00 / 1.69 / 1.65 / 1.81e-6; two accumulators 1.12 / 1.82 / 1.80 / 1.86; four 1.02 / 1.68 / 1.63 /
+// 1.84) for 7 us of 500 a step; eight cost 40.
+__host__ __device__ constexpr int n_acc(int nb) { return nb > 1 ? 4 : 2; }
 constexpr int EV_PER_LAYER = 12;              // trace stamps per layer
 constexpr unsigned long long WAIT_NS = 200ull * 1000 * 1000;   // default patience of every device-side wait: 200 ms
 constexpr int MAX_TP = 8;                     // tensor-parallel ranks: 1, 2, 4 or 8 (at least one kv head each)
@@ -82,8 +90,8 @@ constexpr float ACC_SCALE = 4294967296.f;     // 2^32: resolution 2.3e-10, finer
 constexpr float ACC_CLAMP = 50000.f;
 constexpr int MAX_GRID = 160;                 // 160 * ACC_CLAMP < 2^23
 constexpr unsigned long long ACC_ONE = 1ull << 56, ACC_HALF = 1ull << 55;
-// fp32 tail of shared memory: 8 KB union | q_s[2][128] k_s v_s | o split [3][128] bf16 | hid split [3][32] bf16 | red lw misc | scores
-constexpr int FBUF_FLOATS = 2048 + 4 * 128 + 192 + 48 + 32 + 16 + 16 + 3 * SC_HALF;
+// fp32 tail of shared memory: 8 KB union | q_s[2][128] k_s v_s | o split [3][OLD] | hid split [3][HLD] | red lw misc | scores
+constexpr int FBUF_FLOATS = 2048 + 4 * 128 + 3 * OLD + 3 * HLD + 32 + 16 + 16 + SC_FLOATS;
 constexpr int TAIL_BYTES = FBUF_FLOATS * 4 + 8 * 8 + 16;
 
 struct PersistParams {
@@ -98,9 +106,10 @@ struct PersistParams {
     long long* next_token;
     bf16_raw* k_write;
     bf16_raw* v_write;
-    unsigned long long* dA;   // [2][1024] counted accumulators: attention delta of layer l in buffer l & 1 (16 contributions an element)
-    float* dB;        // [3][N_ACC][1024] FFN delta of layer l in buffer l % 3 (fp32 accumulators, one contribution per CTA and element)
-    unsigned long long* xq;   // [4096] q | k | v rows of the current layer, each a (tag << 32 | fp32 bits) word
+    // (NB: sequences of the launch)
+    unsigned long long* dA;   // [2][NB][1024] counted accumulators: attention delta of layer l in buffer l & 1 (16 contributions an element)
+    float* dB;        // [3][n_acc(NB)][NB][1024] FFN delta of layer l in buffer l % 3 (fp32 accumulators, one contribution per CTA and element)
+    unsigned long long* xq;   // [NB][4096] q | k | v rows of the current layer, each a (tag << 32 | fp32 bits) word
     const unsigned* epoch;    // launches completed on this state; gives every (launch, layer) its own tag
     unsigned long long* xp;   // [8 groups][2 heads][18 CTAs][XP_STRIDE] split-attention partials (max, sum, -, -, o[128]), tagged like xq
     const float* rope;
@@ -128,7 +137,7 @@ struct PersistState {
     const void* src[7];     // the seven pointers `packed` was built from
     int tp_rank, tp_size;   // tensor-parallel position (0, 1 when off)
     float* peer_X[MAX_TP];  // the state allocations of all ranks as mapped here (own at tp_rank)
-    float* X;               // dA[2] (64-bit words) | dB[3][N_ACC] (fp32) | xq[4096] (64-bit words) | epoch | xp
+    float* X;               // dA[2] (64-bit words) | dB[3][n_acc] (fp32) | xq[4096] (64-bit words) | epoch | xp
     int grid, smem;
 };
 
@@ -136,8 +145,10 @@ struct PersistState {
 // one layer takes.  Used by the decode kernel and by the kernel that packs the weights.
 constexpr int XP_STRIDE = 132;                // 64-bit words per published partial
 constexpr size_t XP_WORDS = (size_t)KV_HEADS * 2 * GROUP_CTAS * XP_STRIDE;
-constexpr size_t ACC_FLOATS = (size_t)(4 + 3 * N_ACC) * HIDDEN;   // two vectors of 64-bit words, 3 * N_ACC of floats
-constexpr size_t TP_OFFSET = ACC_FLOATS + 2 * QKV_DIM + 64 + 2 * XP_WORDS;   // [0] barrier counter of the tensor-parallel mode; mailbox at + 64 floats
+// the delta accumulators of a launch: a sequence's two vectors of 64-bit words, then its three times n_acc() of floats
+__host__ __device__ constexpr size_t acc_floats(int nb) { return (size_t)nb * (4 + 3 * n_acc(nb)) * HIDDEN; }
+constexpr size_t XQ_OFFSET = acc_floats(PERSIST_MAX_BATCH), EPOCH_OFFSET = XQ_OFFSET + (size_t)PERSIST_MAX_BATCH * 2 * QKV_DIM;
+constexpr size_t TP_OFFSET = EPOCH_OFFSET + 64 + 2 * XP_WORDS;   // [0] barrier counter of the tensor-parallel mode; mailbox at + 64 floats
 constexpr size_t X_FLOATS = TP_OFFSET + 128;
 struct Share {
     int q0, nq, qmax;       // rows [q0, q0 + nq) of this rank's [wq; wk; wv] rows, slot rows qmax
@@ -292,6 +303,11 @@ __device__ __forceinline__ float sum16(const float* red) {
     return ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w)) + (((c.x + c.y) + (c.z + c.w)) + ((d.x + d.y) + (d.z + d.w)));
 }
 
+__device__ __forceinline__ float exp2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 __device__ __forceinline__ void unpack8f(const uint4& u, float* f) {
     f[0] = bf_lo(u.x); f[1] = bf_hi(u.x); f[2] = bf_lo(u.y); f[3] = bf_hi(u.y);
     f[4] = bf_lo(u.z); f[5] = bf_hi(u.z); f[6] = bf_lo(u.w); f[7] = bf_hi(u.w);
@@ -330,6 +346,16 @@ __device__ __forceinline__ void fold_cols(const float (&c)[4], float& row_lo, fl
 }
 
 
+// Two sequences in the eight columns (0..2: the three parts of the first, 3..5: of the second): lanes with (lane & 3) == 0 get
+// the first one's two row sums, those with (lane & 3) == 2 the second one's.
+__device__ __forceinline__ void fold_cols2(const float (&c)[4], float& row_lo, float& row_hi) {
+    const bool second = threadIdx.x & 2;
+    const float a0 = __shfl_down_sync(0xffffffffu, c[0], 1), a1 = __shfl_down_sync(0xffffffffu, c[2], 1);
+    const float b0 = __shfl_up_sync(0xffffffffu, c[1], 1), b1 = __shfl_up_sync(0xffffffffu, c[3], 1);
+    row_lo = second ? b0 + (c[0] + c[1]) : (c[0] + c[1]) + a0;
+    row_hi = second ? b1 + (c[2] + c[3]) : (c[2] + c[3]) + a1;
+}
+
 // Local attention keeps its K rows in a ring of four register buffers (a quarter-warp per position,
 // 64 positions per pass): pass i lives in buffer i & 3 and the load of pass i + 4 is issued the moment
 // pass i has been consumed.  The V rows are read dim-major instead (one warp per position, four dims
@@ -363,17 +389,30 @@ constexpr int N_MODES = 4;
 __host__ __device__ constexpr int mode_max_len(int mode) { return mode == 0 ? 128 : mode < N_MODES - 1 ? 127 + 64 * mode : PERSIST_MAX_LEN; }
 // TP: tensor-parallel build of the same kernel (system-scope atomics on the deltas, every rank's CTAs arrive at every
 // rank's barrier, the arg-max is settled through the mailboxes); local attention only.
-template <int MODE, bool TP>
+// NB: sequences decoded together, 1..PERSIST_MAX_BATCH (split attention only beyond one).  Their activations are further columns of the same
+// products (two sequences an MMA), every exchange carries all of them, and the 18 blocks of a kv head share out the sequences by their lengths.
+// What does not fit beside the weights is staged in slots that are idle: the gate/up slot in Q, the Wo slot in GD (its next rows are fetched at
+// the start of Q instead), the q/k/v slot in F.
+template <int MODE, bool TP, int NB>
 __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p) {
+    static_assert(NB == 1 || (!TP && MODE == N_MODES - 1), "several sequences: split attention on one GPU");
+    constexpr int NT = (NB + 1) / 2;              // column tiles of the products
+    constexpr bool MANY = NB > 1;
+    constexpr int NACC = n_acc(NB);
+    // passes of K and V rows held in registers by the split attention.  (A spilled register costs a trip to L2 wherever it is used: every acquire
+    // drops L1.  Three sequences with four passes: 0.5 to 1.3 us more in every phase.)
+    constexpr int PASSES = MANY ? 3 : 4;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int c = blockIdx.x, G = gridDim.x;
     const int L = p.n_layers;
     const unsigned long long wait_ns = p.wait_ns;
-    if (p.seq_len[0] > p.max_len || p.seq_len[0] < 0) {   // the same for every CTA: nothing has been started yet
-        if (tid == 0) report(p.status, ST_BAD_LEN, (uint32_t)MODE, (uint32_t)p.seq_len[0]);
-        return;
-    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+        if (p.seq_len[b] > p.max_len || p.seq_len[b] < 0) {   // the same for every CTA: nothing has been started yet
+            if (tid == 0) report(p.status, ST_BAD_LEN, (uint32_t)MODE, (uint32_t)p.seq_len[b]);
+            return;
+        }
 
     // ---- static ownership ----
     static_assert(!TP || MODE < N_MODES - 1, "tensor parallelism serves the local-attention variants only");
@@ -387,7 +426,33 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     const int fj = fhh * sh.slices + fs;                          // index inside the kv-head group, 0..17 (without tensor parallelism)
     const int fr0 = sh.fr0, fn = sh.fn;
     (void)i0;
-    const bool kv_writer = has_f && fj == 0;                      // one CTA per kv head stores the new K/V rows
+    // The sequence this CTA attends: the group's 18 CTAs are dealt out by the lengths, each sequence at least one; CTA fj is number sj of the sn of
+    // sequence sb.
+    int sb = 0, sj = fj, sn = GROUP_CTAS, ends[NB];
+    if constexpr (MANY) {
+        int n[NB], cnt[NB], left = GROUP_CTAS;
+        long long total = 0;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) { n[b] = p.seq_len[b] + 1; total += n[b]; }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) { cnt[b] = 1 + (int)((long long)(GROUP_CTAS - NB) * n[b] / total); left -= cnt[b]; }
+        for (; left > 0; --left) {                // (fewer than NB: what the divisions dropped, to whoever has most positions a CTA)
+            int most = 0;
+#pragma unroll
+            for (int b = 1; b < NB; ++b)
+                if ((long long)n[b] * (most == 0 ? cnt[0] : most == 1 ? cnt[1] : cnt[NB - 1]) > (long long)(most == 0 ? n[0] : most == 1 ? n[1] : n[NB - 1]) * cnt[b]) most = b;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) cnt[b] += b == most;
+        }
+        int first = 0;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            if (fj >= first) { sb = b; sj = fj - first; sn = cnt[b]; }
+            first += cnt[b];
+            ends[b] = first;
+        }
+    }
+    const bool kv_writer = has_f && sj == 0;                      // one CTA per kv head and sequence stores the new K/V rows
 
     // ---- shared memory carve-up ----
     bf16_raw* sA = reinterpret_cast<bf16_raw*>(smem);                       // qkv rows        [qmax][WROW]
@@ -396,29 +461,41 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     bf16_raw* sD = sC + (size_t)2 * imax * WROW;                            // down^T rows     [imax][WROW]
     float* fbuf = reinterpret_cast<float*>(sD + (size_t)imax * WROW);
     // one 8 KB region with a different tenant per phase
-    uint32_t* xsp = reinterpret_cast<uint32_t*>(fbuf);   // Q, GD: activations split in three bf16 parts, [3][512] pairs (6 KB)
-    float* part = fbuf + 1536;                           // Q: per-warp partial row sums [16][32] (2 KB)
-    float* gpart = fbuf + 1536;                          // GD: per-warp partial sums of the 48 gate/up tile rows [16][48] (3 KB: runs into q_s, idle in GD)
+    uint32_t* const fw = reinterpret_cast<uint32_t*>(fbuf);
+    uint32_t* xsq = MANY ? reinterpret_cast<uint32_t*>(sC) : fw;   // Q: activations split in three bf16 parts, [NB][3][XLD] pairs (6 KB a sequence)
+    uint32_t* xsg = MANY ? reinterpret_cast<uint32_t*>(sB) : fw;   // GD: the same
+    float* part = MANY ? fbuf : fbuf + 3 * XLD;          // Q: per-warp partial row sums [NB][16][32] (2 KB: one sequence's run into q_s, idle in Q)
+    float* gpart = MANY ? reinterpret_cast<float*>(sB) + NB * 3 * XLD : fbuf + 3 * XLD;   // GD: per-warp partial sums of the 48 gate/up tile rows [NB][16][48] (3 KB: one sequence's run into q_s and k_s, idle in GD)
+    static_assert(NB * (3 * XLD + 768 + CW) * 4 <= WO_ROWS_MAX * WOROW * 2 && NB * (512 + CW) <= 2048, "the Wo slot holds GD's staging, the union Q's sums");
     float* om = fbuf;                                    // F: [16 warps][128] outputs of the local attention
-    float* wo_part = fbuf;                               // F: [2 k-halves][128] Wo slice partial sums (after the partials are published)
-    float* dout = fbuf;                                  // GD: [1024] down-projection outputs of this CTA (after the gate/up rows)
-    float* xs = fbuf;                                    // LM head: [1024] fp32 activations
+    float* wo_part = fbuf;                               // F: [NB][2 k-halves][128] Wo slice partial sums (after the partials are published)
+    float* dout = MANY ? reinterpret_cast<float*>(sB) : fbuf;   // GD: [NB][1024] down-projection outputs of this CTA (after the gate/up rows)
+    float* xs = MANY ? reinterpret_cast<float*>(sA) : fbuf;     // LM head: [1024] fp32 activations; several sequences: [NB][3][LLD] pairs, split in three bf16 parts
     float* q_s = fbuf + 2048;    // [2][128] both query heads of the group, scaled by 1/sqrt(128)
     float* k_s = q_s + 256;      // [128] the new K row (after norm + RoPE), fp32
     float* v_s = k_s + 128;      // [128] the new V row, fp32
-    uint32_t* osp = reinterpret_cast<uint32_t*>(v_s + 128);   // [3][64] pairs: attention output of this CTA's head, split
-    uint32_t* hsp = osp + 192;   // [3][16] pairs: this CTA's hid values, split
-    float* red = reinterpret_cast<float*>(hsp + 48);          // [32]
+    uint32_t* const osp1 = reinterpret_cast<uint32_t*>(v_s + 128);
+    uint32_t* osp = MANY ? reinterpret_cast<uint32_t*>(sA) + CW * 256 + 128 : osp1;   // F: [NB][3][OLD] pairs: attention output of this CTA's head, split
+    uint32_t* hsp = MANY ? fw : osp1 + 3 * OLD;               // GD: [NB][3][HLD] pairs: this CTA's hid values, split
+    float* red = reinterpret_cast<float*>(osp1 + 3 * OLD + 3 * HLD);   // [32]
+    float* redq = MANY ? fbuf + NB * 512 : red;               // Q: [NB][16] sums of squares of the warps' elements
+    float* redg = MANY ? gpart + NB * 768 : red;              // GD: the same
     float* lw = red + 32;        // [16] per-warp probability sums, [w][head]
-    float* misc = lw + 16;       // [16]: [0] score of the new row for this CTA's head
-    float* sc = misc + 16;       // local attention: [3 * SC_HALF] scores of all positions; split: the partials' maxima and sums
-    uint64_t* full = reinterpret_cast<uint64_t*>(sc + 3 * SC_HALF);   // [4] slot filled
+    float* misc = lw + 16;       // [16]: [0] score of the new row for this CTA's head (several sequences: [0], [1] of both heads, [8..] s_first)
+    float* sc = misc + 16;       // local attention: scores of all positions; split: the partials' weights
+    uint64_t* full = reinterpret_cast<uint64_t*>(sc + SC_FLOATS);   // [4] slot filled
     volatile int* abort_flag = reinterpret_cast<volatile int*>(full + 8);
 
     const int n_ev = 4 + EV_PER_LAYER * L;
 #define Q3_TRACE(ev) do { if (p.trace != nullptr && tid == 0) p.trace[(size_t)c * n_ev + (ev)] = global_ns(); } while (0)
+    int* const s_first = reinterpret_cast<int*>(misc + 8);    // [NB + 1] first CTA of every sequence
     Q3_TRACE(0);
     if (tid == 0) {
+        if constexpr (MANY) {
+            s_first[0] = 0;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) s_first[b + 1] = ends[b];
+        }
         for (int i = 0; i < 4; ++i) mbar_init(&full[i], 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -469,8 +546,87 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
             }
         }
     };
-    float* const lm_bv = q_s;                               // [CW + NPW] per-warp best values
-    int* const lm_bi = reinterpret_cast<int*>(k_s);         // [CW + NPW] and their rows
+    // The same for several sequences, on the tensor cores: eight rows a warp, straight from memory.  The order of the k's inside a block of 64 is
+    // free, so an instruction takes whole lines: eight lanes 128 bytes of a row, lane l unit l & 7 of row l >> 3.  As rows of the m16n8k16
+    // steps these are labels 2 r (the block's first 32 k's) and 2 r + 1 (the last 32), for which a sequence's tile holds x in columns of their own:
+    // 0..2 its three parts over the first 32, 4..6 over the last.  What a label does not belong to is not read.  (With FMAs the LM head took 91 us for two
+    // sequences and 121 for three, 47 for one; four lanes, 64 bytes, a row 80 to 99: the SM's requests are counted in lines.)
+    auto lm_mma = [&](float& bestv, int& besti) {            // of sequence lane & 7
+        const int v0 = (int)((long long)c * p.vocab / G), v1 = (int)((long long)(c + 1) * p.vocab / G);
+        const int vkeep = v0 + (int)((long long)(v1 - v0) * LM_KEEP_PCT / 100);
+        const int ft = lane & 3, col = lane >> 2, r8 = lane >> 3;
+        const uint32_t* const xw = reinterpret_cast<const uint32_t*>(xs) + (col & 3) * LLD + (col >> 2) * 16 + ft * 4;      // [NB][3][LLD] pairs
+        const bool part = (col & 3) < 3;
+        constexpr int AHEAD = 8;                             // blocks of 64 k's under way: a ring that runs on from group to group
+        const uint4 *ra, *rb;
+        auto rows = [&](int base) {
+            ra = reinterpret_cast<const uint4*>(p.embed + (size_t)min(base + r8, v1 - 1) * HIDDEN) + (lane & 7);
+            rb = reinterpret_cast<const uint4*>(p.embed + (size_t)min(base + 4 + r8, v1 - 1) * HIDDEN) + (lane & 7);
+        };
+        uint4 a[AHEAD], b[AHEAD];
+        auto load = [&](int k, int at, uint64_t pol) {
+            asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;" : "=r"(a[k].x), "=r"(a[k].y), "=r"(a[k].z), "=r"(a[k].w) : "l"(ra + at * 8), "l"(pol));
+            asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;" : "=r"(b[k].x), "=r"(b[k].y), "=r"(b[k].z), "=r"(b[k].w) : "l"(rb + at * 8), "l"(pol));
+        };
+        rows(v0 + warp * 8);
+        if (v0 + warp * 8 < v1)
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k) load(k, k, pol_keep);
+        for (int base = v0 + warp * 8; base < v1; base += CW * 8) {
+            const int after = base + CW * 8;
+            const uint64_t pol = after < vkeep ? pol_keep : pol_stream;
+            float acc[NB][2][4], sum[NB][4];
+#pragma unroll
+            for (int q = 0; q < NB; ++q)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[q][i >> 2][i & 3] = sum[q][i & 3] = 0.f;
+#pragma unroll 1
+            for (int k0 = 0; k0 < HIDDEN / 64; k0 += AHEAD) {
+                const bool turn = k0 + AHEAD == HIDDEN / 64;              // the ring goes on with the next group
+                if (turn) rows(after);
+                const int at = turn ? 0 : k0 + AHEAD;
+                const bool more = !turn || after < v1;
+#pragma unroll
+                for (int k = 0; k < AHEAD; ++k) {
+                    const uint32_t f0[4] = {a[k].x, b[k].x, a[k].y, b[k].y}, f1[4] = {a[k].z, b[k].z, a[k].w, b[k].w};
+#pragma unroll
+                    for (int q = 0; q < NB; ++q) {
+                        uint4 x = make_uint4(0, 0, 0, 0);
+                        if (part) x = *reinterpret_cast<const uint4*>(xw + q * 3 * LLD + (k0 + k) * 32);
+                        mma_bf16(acc[q][0], f0, x.x, x.y);
+                        mma_bf16(acc[q][1], f1, x.z, x.w);
+                    }
+                    if (more) load(k, at + k, pol);
+                }
+                // (the tensor cores truncate where they add: eight products in a row, then a rounded sum)
+#pragma unroll
+                for (int q = 0; q < NB; ++q)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) { sum[q][i] += acc[q][0][i] + acc[q][1][i]; acc[q][0][i] = acc[q][1][i] = 0.f; }
+            }
+            const bool own = ((lane & 4) != 0) == (ft >= 2);             // the columns of this label's half
+#pragma unroll
+            for (int q = 0; q < NB; ++q) {
+                const float (&s4)[4] = sum[q];
+                float va = own ? ((ft & 1) ? s4[0] : s4[0] + s4[1]) : 0.f, vb = own ? ((ft & 1) ? s4[2] : s4[2] + s4[3]) : 0.f;
+#pragma unroll
+                for (int o = 1; o <= 4; o <<= 1) { va += __shfl_xor_sync(0xffffffffu, va, o); vb += __shfl_xor_sync(0xffffffffu, vb, o); }
+                if ((lane & 7) == q) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int row = base + 4 * h + r8;
+                        const float v = h ? vb : va;
+                        if (row < v1) {
+                            if (p.logits) p.logits[(size_t)q * p.vocab + row] = v;
+                            if (v > bestv) { bestv = v; besti = row; }
+                        }
+                    }
+                }
+            }
+        }
+    };
+    float* const lm_bv = q_s;                               // [NB][CW] per-warp best values
+    int* const lm_bi = reinterpret_cast<int*>(k_s);         // [NB][CW] and their rows
 
     // ================================================================================ weight delivery
     // There are no producer warps.  One thread (lane 0 of warp 1) moves the CTA's packed rows into the four slots
@@ -503,21 +659,23 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     fetch_slot(1, 0);
 
     // ================================================================================ the step
-    long long tok = p.token[0];
-    if (tok < 0 || tok >= p.vocab) {
-        if (tid == 0) report(p.status, ST_BAD_TOKEN, 0, (uint32_t)tok);
-        tok = 0;
-    }
-    const int len = p.seq_len[0];
-    const bf16_raw* kcache = reinterpret_cast<const bf16_raw*>(p.seq_k[0]);
-    const bf16_raw* vcache = reinterpret_cast<const bf16_raw*>(p.seq_v[0]);
-    const long long lstride = p.seq_layer_stride[0];
+    const int len = p.seq_len[sb];                // of the sequence this CTA attends
+    // this CTA's kv head in the layer at hand (one layer on at the end of every layer)
+    const bf16_raw* kl = reinterpret_cast<const bf16_raw*>(p.seq_k[sb]) + fg * HEAD_DIM;
+    const bf16_raw* vl = reinterpret_cast<const bf16_raw*>(p.seq_v[sb]) + fg * HEAD_DIM;
+    const long long lstride = p.seq_layer_stride[sb];
     const float* rope_row = p.rope + (size_t)len * HEAD_DIM;
     // The residual stream: elements 2 tid and 2 tid + 1 of x, the same values in every CTA.
-    float x0, x1;
-    {
+    float x0[NB], x1[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        long long tok = p.token[b];
+        if (tok < 0 || tok >= p.vocab) {
+            if (tid == 0) report(p.status, ST_BAD_TOKEN, 0, (uint32_t)tok);
+            tok = 0;
+        }
         const uint32_t e = *reinterpret_cast<const uint32_t*>(p.embed + (size_t)tok * HIDDEN + 2 * tid);
-        x0 = bf_lo(e); x1 = bf_hi(e);
+        x0[b] = bf_lo(e); x1[b] = bf_hi(e);
     }
     // x += the attention delta, once all 16 contributions to this thread's two words have arrived (bounded).  The wait IS
     // the load: no counter, no fence; a word that is complete cannot change any more until the buffer is cleared.
@@ -529,8 +687,8 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
             unsigned it = 0;
             unsigned long long t0 = 0;
             for (;;) {
-                if (TP) asm volatile("ld.relaxed.sys.global.b64 %0, [%1];" : "=l"(ws) : "l"(vec + HIDDEN - 1) : "memory");
-                else asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(ws) : "l"(vec + HIDDEN - 1) : "memory");
+                if (TP) asm volatile("ld.relaxed.sys.global.b64 %0, [%1];" : "=l"(ws) : "l"(vec + NB * HIDDEN - 1) : "memory");
+                else asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(ws) : "l"(vec + NB * HIDDEN - 1) : "memory");
                 if (acc_count(ws) + 2u >= expect) break;
                 if ((++it & 63u) == 0) {
                     const unsigned long long t = global_ns();
@@ -540,38 +698,70 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
             }
         }
         cta_sync();
-        unsigned long long w0 = 0, w1 = 0;
+        unsigned long long w0[NB], w1[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) w0[b] = w1[b] = 0;
         if (!*abort_flag) {
             const unsigned long long* src = vec + 2 * tid;
             unsigned it = 0;
             unsigned long long t0 = 0;
             for (;;) {
-                acc_load2<TP>(src, w0, w1);
-                if (acc_count(w0) == expect && acc_count(w1) == expect) break;
+                bool whole = true;
+#pragma unroll
+                for (int b = 0; b < NB; ++b) acc_load2<TP>(src + b * HIDDEN, w0[b], w1[b]);
+#pragma unroll
+                for (int b = 0; b < NB; ++b) whole = whole && acc_count(w0[b]) == expect && acc_count(w1[b]) == expect;
+                if (whole) break;
                 if ((++it & 63u) == 0) {
                     if (*abort_flag) break;
                     const unsigned long long t = global_ns();
                     if (t0 == 0) t0 = t;
                     else if (t - t0 > wait_ns) {
-                        report(p.status, ST_BARRIER_TIMEOUT, site, acc_count(w0));
+                        report(p.status, ST_BARRIER_TIMEOUT, site, acc_count(w0[0]));
                         *abort_flag = 1;
                         break;
                     }
                 }
             }
-            if (*abort_flag) { w0 = 0; w1 = 0; }
+            if (*abort_flag) {
+#pragma unroll
+                for (int b = 0; b < NB; ++b) w0[b] = w1[b] = 0;
+            }
         }
-        x0 += acc_value(w0); x1 += acc_value(w1);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) { x0[b] += acc_value(w0[b]); x1[b] += acc_value(w1[b]); }
     };
     // x += the FFN delta: the sum of its fp32 accumulators (after the layer's grid barrier)
     auto add_ffn_delta = [&](const float* dBl) {
-        float2 d[N_ACC];
+        float2 d[NB][NACC];
 #pragma unroll
-        for (int i = 0; i < N_ACC; ++i) d[i] = ldcg2(dBl + (size_t)i * HIDDEN + 2 * tid);
-        float s0 = d[0].x, s1 = d[0].y;
+        for (int b = 0; b < NB; ++b)
 #pragma unroll
-        for (int i = 1; i < N_ACC; ++i) { s0 += d[i].x; s1 += d[i].y; }
-        x0 += s0; x1 += s1;
+            for (int i = 0; i < NACC; ++i) d[b][i] = ldcg2(dBl + (size_t)(i * NB + b) * HIDDEN + 2 * tid);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            float s0 = d[b][0].x, s1 = d[b][0].y;
+#pragma unroll
+            for (int i = 1; i < NACC; ++i) { s0 += d[b][i].x; s1 += d[b][i].y; }
+            x0[b] += s0; x1[b] += s1;
+        }
+    };
+    // stage x * gain split in three bf16 parts (the 1/rms factor is applied to the row sums), and the sums of squares
+    auto stage_x = [&](uint32_t* xsp, float* ssum, uint32_t gain) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            bf16_raw h0, m0, l0, h1, m1, l1;
+            split3(x0[b] * bf_lo(gain), h0, m0, l0);
+            split3(x1[b] * bf_hi(gain), h1, m1, l1);
+            xsp[b * 3 * XLD + tid] = (uint32_t)h0 | ((uint32_t)h1 << 16);
+            xsp[(b * 3 + 1) * XLD + tid] = (uint32_t)m0 | ((uint32_t)m1 << 16);
+            xsp[(b * 3 + 2) * XLD + tid] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const float ss = warp_sum(x0[b] * x0[b] + x1[b] * x1[b]);
+            if (lane == 0) ssum[b * CW + warp] = ss;
+        }
     };
     unsigned* bar = TP ? p.tp_bar[rank] : p.sync;
     unsigned target = 0;
@@ -581,10 +771,26 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     // ldmatrix.x4 row addresses of a 16 x 16 A tile: lanes 0-7 rows 0-7, 8-15 rows 8-15 (k 0-7); 16-31 the same rows at k 8-15
     const int lm_row = (lane & 7) + ((lane >> 3) & 1) * 8, lm_k = (lane >> 4) * 8;
     const int fr_n = lane >> 2, fr_k = (lane & 3) * 2;   // B fragment: column n, k pair; C fragment: rows fr_n, fr_n + 8
+    // column n of tile t: part n % 3 of sequence 2 t + n / 3
+    auto b_col = [&](const uint32_t* src, int t, int stride, int kp) -> uint32_t {   // its word `kp`, where a part takes `stride` words
+        if (!MANY) return fr_n < 3 ? src[fr_n * stride + kp] : 0u;
+        return fr_n < (2 * t + 1 < NB ? 6 : 3) ? src[(6 * t + fr_n) * stride + kp] : 0u;
+    };
+    // f(b, row sum of fr_n, of fr_n + 8) in the lanes that hold them
+    auto fold = [&](const float (&c)[4], int t, auto&& f) {
+        float r0, r1;
+        if (!MANY) {
+            fold_cols(c, r0, r1);
+            if ((lane & 3) == 0) f(0, r0, r1);
+        } else {
+            fold_cols2(c, r0, r1);
+            if ((lane & 1) == 0 && 2 * t + ((lane & 3) >> 1) < NB) f(2 * t + ((lane & 3) >> 1), r0, r1);
+        }
+    };
 
     // this CTA's share of the cached positions of kv head fg: [cp0, cp1)
-    const int chunk = (len + GROUP_CTAS - 1) / GROUP_CTAS;
-    const int cp0 = min(len, fj * chunk), cp1 = min(len, cp0 + chunk);
+    const int chunk = (len + sn - 1) / sn;
+    const int cp0 = min(len, sj * chunk), cp1 = min(len, cp0 + chunk);
     const int npass = (cp1 - cp0 + 31) >> 5;                  // 32 positions per pass, half a warp each
     const int att_slot = warp * 4 + quarter;
     // Short caches: every CTA recomputes the attention of its own head over all positions (no exchange between
@@ -616,20 +822,15 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
         // of layer l - 2 (next written in GD of layer l + 1): it has passed the grid barrier of layer l - 1, which every CTA
         // reaches after its last read of both, and its arrival at the barrier of layer l releases the stores to every
         // later writer.
-        unsigned long long* dAl = p.dA + (size_t)(l & 1) * HIDDEN;
-        float* dBl = p.dB + (size_t)(l % 3) * N_ACC * HIDDEN;
+        unsigned long long* dAl = p.dA + (size_t)(l & 1) * NB * HIDDEN;
         const unsigned tag = tag_base + (unsigned)l + 1u;
         // K and V rows of the cached positions, fetched at the very start of the layer (they depend on nothing of this
         // step), so that they have arrived, and the SM's input path is quiet, when the q/k/v exchange starts polling.
         // Split attention: [i] = K and V of pass i of the CTA's positions.  Local attention:
         // [0], [1] = K passes 0, 1 (a quarter-warp per position) and [2], [3] = V[warp + 16 i][4 lane .. 4 lane + 3]
         // for i < 8, two positions per uint4.
-        const bf16_raw* kl = kcache + (size_t)l * lstride + fg * HEAD_DIM;
-        const bf16_raw* vl = vcache + (size_t)l * lstride + fg * HEAD_DIM;
-        auto kv_prefetch = [&](int ll) {
-            const bf16_raw* kl = kcache + (size_t)ll * lstride + fg * HEAD_DIM;
-            const bf16_raw* vl = vcache + (size_t)ll * lstride + fg * HEAD_DIM;
-            if (has_f && ll < L) {
+        auto kv_prefetch = [&]() {
+            if (has_f) {
                 if (local_attn) {
 #pragma unroll
                     for (int i = 0; i < 2; ++i) ring_load(ring[i], i, npl, len, att_slot, sub, kl);
@@ -655,80 +856,84 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                     }
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) split_load(ring[i], i, kl, vl);
+                    for (int i = 0; i < PASSES; ++i) split_load(ring[i], i, kl, vl);
                 }
             }
         };
         // ==================================================================== Q
         {
-            if (l > 0) add_ffn_delta(p.dB + (size_t)((l - 1) % 3) * N_ACC * HIDDEN);
+            if (l > 0) add_ffn_delta(p.dB + (size_t)((l - 1) % 3) * NACC * NB * HIDDEN);
             fetch_slot(3, l);   // down rows of this layer: landed before the q/k/v exchange starts polling
-            {   // stage x * gain split in three bf16 parts (the 1/rms factor is applied to the row sums)
-                bf16_raw h0, m0, l0, h1, m1, l1;
-                split3(x0 * bf_lo(gain2), h0, m0, l0);
-                split3(x1 * bf_hi(gain2), h1, m1, l1);
-                xsp[tid] = (uint32_t)h0 | ((uint32_t)h1 << 16);
-                xsp[512 + tid] = (uint32_t)m0 | ((uint32_t)m1 << 16);
-                xsp[1024 + tid] = (uint32_t)l0 | ((uint32_t)l1 << 16);
-            }
-            const float ss = warp_sum(x0 * x0 + x1 * x1);
-            if (lane == 0) red[warp] = ss;
+            if (MANY && l > 0) fetch_slot(1, l);   // (GD had its slot)
+            stage_x(xsq, redq, gain2);
             // the warps that will poll the q/k/v exchange request their K/V rows now (x is staged: nothing queues behind
             // these loads), the others while they wait for the exchange
-            if (warp >= 8 && warp < 12) kv_prefetch(l);
+            if (warp >= 8 && warp < 12) kv_prefetch();
             cta_sync();
             Q3_TRACE(ev + 0);
             // warp w: k range [64 w, 64 w + 64) of both 16-row tiles of this CTA's rows
-            uint32_t bq[4][2];
+            uint32_t bq[NT][4][2];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const int kp = (64 * warp + 16 * t + fr_k) >> 1;
-                bq[t][0] = (fr_n < 3) ? xsp[fr_n * 512 + kp] : 0u;
-                bq[t][1] = (fr_n < 3) ? xsp[fr_n * 512 + kp + 4] : 0u;
-            }
+            for (int ct = 0; ct < NT; ++ct)
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const int kp = (64 * warp + 16 * t + fr_k) >> 1;
+                    bq[ct][t][0] = b_col(xsq, ct, XLD, kp);
+                    bq[ct][t][1] = b_col(xsq, ct, XLD, kp + 4);
+                }
             slot_wait(&full[0], l & 1, abort_flag, p.status, 10, wait_ns);
             {
-                uint32_t af[2][4][4];
+                constexpr int RG = MANY ? 1 : 2;          // row tiles at a time (registers)
 #pragma unroll
-                for (int rt = 0; rt < 2; ++rt) {
-                    const uint32_t abase = smem_u32(sA + (size_t)(16 * rt + lm_row) * WROW + 64 * warp + lm_k);
+                for (int r0t = 0; r0t < 2; r0t += RG) {
+                    uint32_t af[RG][4][4];
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) ldsm_x4(af[rt][t], abase + 32 * t);
-                }
-                float cc[2][2][4];
+                    for (int rt = 0; rt < RG; ++rt) {
+                        const uint32_t abase = smem_u32(sA + (size_t)(16 * (r0t + rt) + lm_row) * WROW + 64 * warp + lm_k);
 #pragma unroll
-                for (int rt = 0; rt < 2; ++rt)
+                        for (int t = 0; t < 4; ++t) ldsm_x4(af[rt][t], abase + 32 * t);
+                    }
+                    float cc[NT][RG][2][4];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
+                    for (int ct = 0; ct < NT; ++ct)
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) cc[rt][h][i] = 0.f;
+                        for (int rt = 0; rt < RG; ++rt)
 #pragma unroll
-                for (int t = 0; t < 4; ++t)
+                            for (int i = 0; i < 8; ++i) cc[ct][rt][i >> 2][i & 3] = 0.f;
 #pragma unroll
-                    for (int rt = 0; rt < 2; ++rt) mma_bf16(cc[rt][t & 1], af[rt][t], bq[t][0], bq[t][1]);
+                    for (int t = 0; t < 4; ++t)
 #pragma unroll
-                for (int rt = 0; rt < 2; ++rt) {
+                        for (int ct = 0; ct < NT; ++ct)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) cc[rt][0][i] += cc[rt][1][i];
-                    float r0, r1;
-                    fold_cols(cc[rt][0], r0, r1);
-                    if ((lane & 3) == 0) { part[warp * 32 + 16 * rt + fr_n] = r0; part[warp * 32 + 16 * rt + fr_n + 8] = r1; }
+                            for (int rt = 0; rt < RG; ++rt) mma_bf16(cc[ct][rt][t & 1], af[rt][t], bq[ct][t][0], bq[ct][t][1]);
+#pragma unroll
+                    for (int ct = 0; ct < NT; ++ct)
+#pragma unroll
+                        for (int rt = 0; rt < RG; ++rt) {
+                            float (&c0)[4] = cc[ct][rt][0];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) c0[i] += cc[ct][rt][1][i];
+                            fold(c0, ct, [&](int b, float r0, float r1) {
+                                float* dst = part + b * 512 + warp * 32 + 16 * (r0t + rt) + fr_n;
+                                dst[0] = r0; dst[8] = r1;
+                            });
+                        }
                 }
             }
             cta_sync();
-            if (warp == 0) {   // nq <= 28: the row sums and the 1/rms factor sit in warp 0
-                if (tid < nq) {
-                    const float r = rsqrtf(sum16(red) / (float)HIDDEN + EPS);
+            if (warp < NB) {   // nq <= 28: warp b has the row sums and the 1/rms factor of sequence b
+                if (lane < nq) {
+                    const float r = rsqrtf(sum16(redq + warp * CW) / (float)HIDDEN + EPS);
                     float v0 = 0.f, v1 = 0.f;
 #pragma unroll
-                    for (int w = 0; w < CW; w += 2) { v0 += part[w * 32 + tid]; v1 += part[w * 32 + 32 + tid]; }
+                    for (int w = 0; w < CW; w += 2) { v0 += part[warp * 512 + w * 32 + lane]; v1 += part[warp * 512 + w * 32 + 32 + lane]; }
                     // value and tag travel in one 64-bit word: no barrier between Q and F, the readers poll the tags
                     const unsigned long long word = ((unsigned long long)tag << 32) | (unsigned long long)__float_as_uint((v0 + v1) * r);
-                    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p.xq + q0 + tid), "l"(word) : "memory");
+                    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p.xq + (size_t)warp * QKV_DIM + q0 + lane), "l"(word) : "memory");
                 }
                 Q3_TRACE(ev + 1);
             }
-            if (warp < 8 || warp >= 12) kv_prefetch(l);   // after the rows are published: nothing waits for these warps now
+            if (warp < 8 || warp >= 12) kv_prefetch();   // after the rows are published: nothing waits for these warps now
         }
 
         // ---- what the F phase needs that no other CTA produces: norm gains and the RoPE row ----
@@ -752,7 +957,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
             // ---- q (both heads of the group), k, v of the new position: warps 8..11 ----
             if (warp >= 8 && warp < 12) {
                 const int role = warp - 8;   // 0, 1: q heads 2g, 2g+1;  2: k;  3: v
-                const unsigned long long* src = p.xq + (role < 2 ? (2 * fgl + role) * HEAD_DIM : (role == 2 ? qrows + fgl * HEAD_DIM : qrows + kvrows + fgl * HEAD_DIM)) + lane * 4;
+                const unsigned long long* src = p.xq + (size_t)sb * QKV_DIM + (role < 2 ? (2 * fgl + role) * HEAD_DIM : (role == 2 ? qrows + fgl * HEAD_DIM : qrows + kvrows + fgl * HEAD_DIM)) + lane * 4;
                 unsigned long long w0, w1, w2, w3;
                 {   // bounded poll: the four words of this lane must all carry this layer's tag
                     unsigned it = 0;
@@ -779,7 +984,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                 if (role < 3) {
                     const float ss = warp_sum(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
                     const float r = rsqrtf(ss / (float)HEAD_DIM + EPS);
-                    const float post = (role < 2) ? ATTN_SCALE : 1.f;
+                    const float post = (role < 2) ? (local_attn ? ATTN_SCALE : ATTN_SCALE * 1.4426950408889634f) : 1.f;   // (split attention: scores in units of log2, one rounding less in every weight)
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float n = (v[i] * r) * gq[i];
@@ -796,10 +1001,10 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                     pk.x = (uint32_t)f_to_bf(v[0]) | ((uint32_t)f_to_bf(v[1]) << 16);
                     pk.y = (uint32_t)f_to_bf(v[2]) | ((uint32_t)f_to_bf(v[3]) << 16);
                     bf16_raw* wr = (role == 2) ? p.k_write : p.v_write;
-                    if (wr) *reinterpret_cast<uint2*>(wr + ((size_t)l * KV_HEADS + fg) * HEAD_DIM + lane * 4) = pk;
+                    if (wr) *reinterpret_cast<uint2*>(wr + (((size_t)sb * L + l) * KV_HEADS + fg) * HEAD_DIM + lane * 4) = pk;
                     if (p.append) {
-                        bf16_raw* cb = const_cast<bf16_raw*>(role == 2 ? kcache : vcache);
-                        *reinterpret_cast<uint2*>(cb + (size_t)l * lstride + (size_t)len * KV_DIM + fg * HEAD_DIM + lane * 4) = pk;
+                        bf16_raw* cb = const_cast<bf16_raw*>(role == 2 ? kl : vl);
+                        *reinterpret_cast<uint2*>(cb + (size_t)len * KV_DIM + lane * 4) = pk;
                     }
                 }
             }
@@ -851,7 +1056,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
 #pragma unroll
                 for (int i = 0; i < LOCAL_V_PRE; ++i) {
                     const int pos = warp + CW * i;
-                    const float pr = (pos < len) ? __expf(sc[min(pos, 3 * SC_HALF - 1)] - M) : 0.f;   // the rows past the cache were fetched as zeros
+                    const float pr = (pos < len) ? __expf(sc[min(pos, SC_FLOATS - 1)] - M) : 0.f;   // the rows past the cache were fetched as zeros
                     lsum += pr;
                     const uint4& src = ring[2 + (i >> 2)][(i >> 1) & 1];
                     const uint32_t vx = (i & 1) ? src.z : src.x, vy = (i & 1) ? src.w : src.y;
@@ -862,7 +1067,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
 #pragma unroll
                     for (int i = 0; i < 4 * XPASS; ++i) {
                         const int pos = warp + CW * (LOCAL_V_PRE + i);
-                        const float pr = (pos < len) ? __expf(sc[min(pos, 3 * SC_HALF - 1)] - M) : 0.f;
+                        const float pr = (pos < len) ? __expf(sc[min(pos, SC_FLOATS - 1)] - M) : 0.f;
                         lsum += pr;
                         const uint4& src = vext[i >> 1];
                         const uint32_t vx = (i & 1) ? src.z : src.x, vy = (i & 1) ? src.w : src.y;
@@ -884,8 +1089,8 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                     bf16_raw h, m, lo_;
                     split3(o / Ls, h, m, lo_);
                     reinterpret_cast<bf16_raw*>(osp)[tid] = h;
-                    reinterpret_cast<bf16_raw*>(osp + 64)[tid] = m;
-                    reinterpret_cast<bf16_raw*>(osp + 128)[tid] = lo_;
+                    reinterpret_cast<bf16_raw*>(osp + OLD)[tid] = m;
+                    reinterpret_cast<bf16_raw*>(osp + 2 * OLD)[tid] = lo_;
                 }
                 cta_sync();
             } else {
@@ -896,11 +1101,11 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                 //      a position and step, 4.3 TB/s), by the layer's exchanges below.  us per step, with eight warps, scores in shared memory and
                 //      rows beyond the first 64 fetched as they are needed -> now: 1000 positions 455 -> 443, 2200 563 -> 466, 3438 673 -> 498.
                 //      (Rows asked into L2 a layer ahead: 555 instead of 542 at 5000.) ----
-                if (warp == 12) {   // the new row's score for this CTA's own head: q . k_new in fp32, unrounded
-                    const float4 a = *reinterpret_cast<const float4*>(q_s + fhh * 128 + lane * 4);
+                if (warp == 12 || (MANY && warp == 13)) {   // the new row's score for this CTA's own head (several sequences: for both), q . k_new in fp32, unrounded
+                    const float4 a = *reinterpret_cast<const float4*>(q_s + (MANY ? warp - 12 : fhh) * 128 + lane * 4);
                     const float4 b = *reinterpret_cast<const float4*>(k_s + lane * 4);
                     const float sn_ = warp_sum(a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w);
-                    if (lane == 0) misc[0] = sn_;
+                    if (lane == 0) misc[warp - 12] = sn_;
                 }
                 float qa[2][8];
 #pragma unroll
@@ -930,20 +1135,20 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
 #pragma unroll
                     for (int hh = 0; hh < 2; ++hh) {
                         const float mn = live ? fmaxf(mx[hh], s2[hh]) : mx[hh];
-                        const float keep = mx[hh] == mn ? 1.f : __expf(mx[hh] - mn);     // (the first row: exp(-inf) = 0)
-                        const float pr = live ? __expf(s2[hh] - mn) : 0.f;
+                        const float keep = mx[hh] == mn ? 1.f : exp2_approx(mx[hh] - mn);     // (the first row: exp(-inf) = 0)
+                        const float pr = live ? exp2_approx(s2[hh] - mn) : 0.f;
                         mx[hh] = mn;
                         ls[hh] = fmaf(ls[hh], keep, pr);
 #pragma unroll
                         for (int i = 0; i < 8; ++i) acc[hh][i] = fmaf(pr, f[i], acc[hh][i] * keep);
                     }
                 };
-                for (int ps = 0; ps < npass; ps += 4)
+                for (int ps = 0; ps < npass; ps += PASSES)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < PASSES; ++j)
                         if (ps + j < npass) {
                             attend(ring[j], ps + j);
-                            if (ps + j + 4 < npass) split_load(ring[j], ps + j + 4, kl, vl);
+                            if (ps + j + PASSES < npass) split_load(ring[j], ps + j + PASSES, kl, vl);
                         }
                 // the halves under the warp's maximum; the lower one keeps head 0, the upper one head 1
                 float* const oms = reinterpret_cast<float*>(sA);           // [16 warps][2 heads][128], then [2][16] maxima and sums: the q/k/v rows are
@@ -951,7 +1156,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
                     const float M = fmaxf(mx[hh], __shfl_xor_sync(0xffffffffu, mx[hh], 16));
-                    const float w = mx[hh] == -INFINITY ? 0.f : __expf(mx[hh] - M);
+                    const float w = mx[hh] == -INFINITY ? 0.f : exp2_approx(mx[hh] - M);
 #pragma unroll
                     for (int i = 0; i < 8; ++i) acc[hh][i] *= w;
                     float t = ls[hh] * w;
@@ -973,9 +1178,16 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                     const int hh = tid >> 7, d = tid & 127;
                     float o = 0.f;
                     const float mw = oml[hh * CW + (lane & 15)];                // lanes 0..15 (and again 16..31): a warp's maximum
-                    const float M = warp_max(mw);
-                    const float wgt = mw == -INFINITY ? 0.f : __expf(mw - M);
-                    const float Ls = warp_sum(lane < CW ? oml[2 * CW + hh * CW + lane] * wgt : 0.f);
+                    // (several sequences: the first CTA of a sequence counts the new row among its positions, one: the readers add it)
+                    const bool with_new = MANY && sj == 0;
+                    const float M = fmaxf(warp_max(mw), with_new ? misc[hh] : -INFINITY);
+                    const float wgt = mw == -INFINITY ? 0.f : exp2_approx(mw - M);
+                    float Ls = warp_sum(lane < CW ? oml[2 * CW + hh * CW + lane] * wgt : 0.f);
+                    if (with_new) {
+                        const float wn = exp2_approx(misc[hh] - M);
+                        Ls += wn;
+                        o = wn * v_s[d];
+                    }
 #pragma unroll
                     for (int w = 0; w < CW; ++w) o = fmaf(oms[(w * 2 + hh) * 128 + d], __shfl_sync(0xffffffffu, wgt, w), o);
                     const unsigned long long t64 = (unsigned long long)tag << 32;
@@ -992,20 +1204,26 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                 //      (max, sum) pairs, which their writers store last, so that the polling stays light; step 2:
                 //      eight warps read the outputs, half h = tid / 128 merging partials [9 h, 9 h + 9) for dim
                 //      tid % 128, and go round again in the rare case that a word does not carry the tag yet.
-                constexpr int HALF = GROUP_CTAS / 2;
                 const unsigned long long* xsrc = p.xp + (size_t)((fg * 2 + fhh) * GROUP_CTAS) * XP_STRIDE;
-                float* pm_s = misc + 8;          // [18] maxima   (misc[8..25] runs into sc, which is dead by now)
-                float* pl_s = sc + 32;           // [18] sums
-                unsigned long long wc[HALF];   // warps 0..7: this thread's nine output words
-                const int mhalf = tid >> 7, md = tid & 127;
-                const unsigned long long* msrc = xsrc + (size_t)(mhalf * HALF) * XP_STRIDE + 4 + md;
+                float* const pm_s = sc + 32;     // [18] maxima
+                float* const pl_s = sc + 64;     // [18] sums
+                // One sequence: half h = tid / 128 of eight warps merges partials [9 h, 9 h + 9).  Several: four warps a sequence.
+                constexpr int PARTS = MANY ? GROUP_CTAS - NB + 1 : GROUP_CTAS / 2, MERGERS = MANY ? NB : 2;
+                unsigned long long wc[PARTS];    // this thread's output words
+                const int mg = tid >> 7, md = tid & 127;
+                int s0 = 0, sc_n = GROUP_CTAS, mfirst = mg * PARTS, mcount = PARTS;   // the sequence's partials, and this thread's among them
+                if constexpr (MANY) {
+                    s0 = s_first[min(mg, NB - 1)];
+                    mfirst = s0; sc_n = mcount = s_first[min(mg, NB - 1) + 1] - s0;
+                }
+                const unsigned long long* msrc = xsrc + (size_t)mfirst * XP_STRIDE + 4 + md;
                 auto load_outputs = [&]() {
 #pragma unroll
-                    for (int j = 0; j < HALF; ++j)
-                        asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(wc[j]) : "l"(msrc + (size_t)j * XP_STRIDE) : "memory");
+                    for (int j = 0; j < PARTS; ++j)
+                        if (!MANY || j < mcount) asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(wc[j]) : "l"(msrc + (size_t)j * XP_STRIDE) : "memory");
                 };
-                if (warp < 8) load_outputs();   // speculative: usually fresh by the time the pairs are, which saves a round trip
-                if (warp == 8) {
+                if (warp < 4 * MERGERS) load_outputs();   // speculative: usually fresh by the time the pairs are, which saves a round trip
+                if (warp == CW - 1) {
                     unsigned long long wa = (unsigned long long)tag << 32, wb = wa;
                     unsigned it = 0;
                     unsigned long long t0 = 0;
@@ -1027,24 +1245,25 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                     if (lane < GROUP_CTAS) { pm_s[lane] = __uint_as_float((unsigned)wa); pl_s[lane] = __uint_as_float((unsigned)wb); }
                 }
                 cta_sync();
-                if (tid < 2 * HEAD_DIM) {
-                    const int half = mhalf, d = md;
-                    float M, Ls, o;
+                if (tid < MERGERS * HEAD_DIM) {
+                    // a lane per partial of the sequence: its weight under the sequence's maximum, over the sequence's sum (one sequence: with the new row)
+                    const bool mine = lane < sc_n;
+                    const float pm = mine ? pm_s[s0 + lane] : -INFINITY, pl = mine ? pl_s[s0 + lane] : 0.f, s_new = MANY ? -INFINITY : misc[0];
+                    const float M = fmaxf(warp_max(pm), s_new);
+                    const float e = pm == -INFINITY ? 0.f : exp2_approx(pm - M), en = MANY ? 0.f : exp2_approx(s_new - M);
+                    const float inv = 1.f / (warp_sum(e * pl) + en), wgt = e * inv;
+                    float o;
                     unsigned it = 0;
                     unsigned long long t0 = 0;
                     for (;;) {
                         bool fresh = true;
-                        M = -INFINITY; Ls = 0.f; o = 0.f;
+                        o = 0.f;
 #pragma unroll
-                        for (int j = 0; j < HALF; ++j) {
-                            fresh = fresh && (unsigned)(wc[j] >> 32) == tag;
-                            const float mj = pm_s[half * HALF + j];   // -inf for a CTA that had no positions
-                            const float Mn = fmaxf(M, mj);
-                            const float keep = (M == -INFINITY) ? 0.f : __expf(M - Mn), wgt = (mj == -INFINITY) ? 0.f : __expf(mj - Mn);
-                            Ls = fmaf(pl_s[half * HALF + j], wgt, Ls * keep);
-                            o = fmaf(__uint_as_float((unsigned)wc[j]), wgt, o * keep);
-                            M = Mn;
-                        }
+                        for (int j = 0; j < PARTS; ++j)
+                            if (!MANY || j < mcount) {
+                                fresh = fresh && (unsigned)(wc[j] >> 32) == tag;
+                                o = fmaf(__uint_as_float((unsigned)wc[j]), __shfl_sync(0xffffffffu, wgt, mfirst - s0 + j), o);
+                            }
                         if (__all_sync(0xffffffffu, fresh)) break;
                         if (*abort_flag) break;
                         if ((++it & 63u) == 0) {
@@ -1057,22 +1276,24 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                         }
                         load_outputs();
                     }
-                    q_s[half * 128 + d] = o;                       // the queries are dead by now
-                    if (d == 0) { misc[4 + 2 * half] = M; misc[5 + 2 * half] = Ls; }
+                    if constexpr (MANY) {              // the new row is among the partials: this is the head's output
+                        bf16_raw h, m, lo_;
+                        split3(o, h, m, lo_);
+                        bf16_raw* dst = reinterpret_cast<bf16_raw*>(osp + mg * 3 * OLD);
+                        dst[md] = h; dst[2 * OLD + md] = m; dst[4 * OLD + md] = lo_;
+                    } else {
+                        q_s[mg * 128 + md] = mg == 0 ? fmaf(en * inv, v_s[md], o) : o;      // the queries are dead by now
+                    }
                 }
-                cta_sync();
-                if (tid < HEAD_DIM) {
-                    const float s_new = misc[0], m0 = misc[4], m1 = misc[6];
-                    const float M = fmaxf(s_new, fmaxf(m0, m1));
-                    const float pn = __expf(s_new - M);
-                    const float w0 = (m0 == -INFINITY) ? 0.f : __expf(m0 - M), w1 = (m1 == -INFINITY) ? 0.f : __expf(m1 - M);
-                    const float Ls = pn + misc[5] * w0 + misc[7] * w1;
-                    const float o = pn * v_s[tid] + q_s[tid] * w0 + q_s[128 + tid] * w1;
-                    bf16_raw h, m, lo_;
-                    split3(o / Ls, h, m, lo_);
-                    reinterpret_cast<bf16_raw*>(osp)[tid] = h;
-                    reinterpret_cast<bf16_raw*>(osp + 64)[tid] = m;
-                    reinterpret_cast<bf16_raw*>(osp + 128)[tid] = lo_;
+                if constexpr (!MANY) {
+                    cta_sync();
+                    if (tid < HEAD_DIM) {
+                        bf16_raw h, m, lo_;
+                        split3(q_s[tid] + q_s[128 + tid], h, m, lo_);
+                        reinterpret_cast<bf16_raw*>(osp)[tid] = h;
+                        reinterpret_cast<bf16_raw*>(osp + OLD)[tid] = m;
+                        reinterpret_cast<bf16_raw*>(osp + 2 * OLD)[tid] = lo_;
+                    }
                 }
                 Q3_TRACE(ev + 5);
                 cta_sync();
@@ -1083,26 +1304,33 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
             slot_wait(&full[1], l & 1, abort_flag, p.status, 11, wait_ns);
             {
                 const int rt = warp >> 1, kh = warp & 1;
-                float cc[4] = {0.f, 0.f, 0.f, 0.f};
+                float cc[NT][4];
+#pragma unroll
+                for (int ct = 0; ct < NT; ++ct)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) cc[ct][i] = 0.f;
                 const uint32_t abase = smem_u32(sB + (size_t)(16 * rt + lm_row) * WOROW + 64 * kh + lm_k);
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
                     const int kp = (64 * kh + 16 * t + fr_k) >> 1;
-                    const uint32_t b0 = (fr_n < 3) ? osp[fr_n * 64 + kp] : 0u;
-                    const uint32_t b1 = (fr_n < 3) ? osp[fr_n * 64 + kp + 4] : 0u;
                     uint32_t af[4];
                     ldsm_x4(af, abase + 32 * t);
-                    mma_bf16(cc, af, b0, b1);
+#pragma unroll
+                    for (int ct = 0; ct < NT; ++ct) mma_bf16(cc[ct], af, b_col(osp, ct, OLD, kp), b_col(osp, ct, OLD, kp + 4));
                 }
-                float r0, r1;
-                fold_cols(cc, r0, r1);
-                if ((lane & 3) == 0) { wo_part[kh * 128 + 16 * rt + fr_n] = r0; wo_part[kh * 128 + 16 * rt + fr_n + 8] = r1; }
+#pragma unroll
+                for (int ct = 0; ct < NT; ++ct)
+                    fold(cc[ct], ct, [&](int b, float r0, float r1) {
+                        wo_part[b * 256 + kh * 128 + 16 * rt + fr_n] = r0; wo_part[b * 256 + kh * 128 + 16 * rt + fr_n + 8] = r1;
+                    });
             }
             cta_sync();
-            if (tid < fn) {   // fn <= 116: the slice joins the attention delta (of every rank)
-                const unsigned long long w = acc_word(wo_part[tid] + wo_part[128 + tid]);
-                if (TP) { for (int r = 0; r < T; ++r) acc_add<true>(p.tp_dA[r] + (size_t)(l & 1) * HIDDEN + fr0 + tid, w); }
-                else acc_add<false>(dAl + fr0 + tid, w);
+            // fn <= 116: the slice joins the attention delta (of every rank); four warps a sequence
+            if ((tid & 127) < fn && (tid >> 7) < NB) {
+                const int b = tid >> 7, r = tid & 127;
+                const unsigned long long w = acc_word(wo_part[b * 256 + r] + wo_part[b * 256 + 128 + r]);
+                if (TP) { for (int t = 0; t < T; ++t) acc_add<true>(p.tp_dA[t] + (size_t)(l & 1) * HIDDEN + fr0 + r, w); }
+                else acc_add<false>(dAl + b * HIDDEN + fr0 + r, w);
             }
         }   // (wo_part is the next phase's staging area: the wait below passes a CTA barrier before anything is staged)
         Q3_TRACE(ev + 6);
@@ -1113,78 +1341,83 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
             acc_wait(dAl, (unsigned)Q_HEADS, 200 + l);   // every row of the attention delta receives one slice per query head
             Q3_TRACE(ev + 7);
             fetch_slot(0, l + 1);   // q/k/v rows and Wo slice of the next layer: landed before this phase's barrier is polled
-            fetch_slot(1, l + 1);
-            if (c == G - 1) {   // recycle the delta buffers (see the top of the loop): 8 KB each, 16 bytes a thread
-                static_assert(N_ACC == 2, "both buffers are cleared as 8 KB");
-                __stcg(reinterpret_cast<float4*>(p.dA + (size_t)((l + 1) & 1) * HIDDEN) + tid, make_float4(0.f, 0.f, 0.f, 0.f));
-                __stcg(reinterpret_cast<float4*>(p.dB + (size_t)((l + 1) % 3) * N_ACC * HIDDEN) + tid, make_float4(0.f, 0.f, 0.f, 0.f));
+            if (!MANY) fetch_slot(1, l + 1);
+            if (c == G - 1) {   // recycle the delta buffers (see the top of the loop): 16 bytes a thread
+                #pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    __stcg(reinterpret_cast<float4*>(p.dA + (size_t)((l + 1) & 1) * NB * HIDDEN) + b * CT + tid, make_float4(0.f, 0.f, 0.f, 0.f));
+#pragma unroll
+                    for (int i = 0; i < NACC / 2; ++i) __stcg(reinterpret_cast<float4*>(p.dB + (size_t)((l + 1) % 3) * NACC * NB * HIDDEN) + (b * (NACC / 2) + i) * CT + tid, make_float4(0.f, 0.f, 0.f, 0.f));
+                }
             }
-            {
-                bf16_raw h0, m0, l0, h1, m1, l1;
-                split3(x0 * bf_lo(gain2), h0, m0, l0);
-                split3(x1 * bf_hi(gain2), h1, m1, l1);
-                xsp[tid] = (uint32_t)h0 | ((uint32_t)h1 << 16);
-                xsp[512 + tid] = (uint32_t)m0 | ((uint32_t)m1 << 16);
-                xsp[1024 + tid] = (uint32_t)l0 | ((uint32_t)l1 << 16);
-            }
-            const float ss = warp_sum(x0 * x0 + x1 * x1);
-            if (lane == 0) red[warp] = ss;
+            stage_x(xsg, redg, gain2);
             cta_sync();
             Q3_TRACE(ev + 8);
             {
                 // The slot holds one matrix of 2 * imax = 42 rows (gate rows, then up rows): three 16-row tiles cover it
                 // (the last six rows of the third tile belong to the next slot and are never used).  Warp w takes
                 // the k range [64 w, 64 w + 64) of all three tiles.
-                uint32_t bx[4][2];
+                uint32_t bx[NT][4][2];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const int kp = (64 * warp + 16 * t + fr_k) >> 1;
-                    bx[t][0] = (fr_n < 3) ? xsp[fr_n * 512 + kp] : 0u;
-                    bx[t][1] = (fr_n < 3) ? xsp[fr_n * 512 + kp + 4] : 0u;
-                }
+                for (int ct = 0; ct < NT; ++ct)
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        const int kp = (64 * warp + 16 * t + fr_k) >> 1;
+                        bx[ct][t][0] = b_col(xsg, ct, XLD, kp);
+                        bx[ct][t][1] = b_col(xsg, ct, XLD, kp + 4);
+                    }
                 slot_wait(&full[2], l & 1, abort_flag, p.status, 12, wait_ns);
-                uint32_t af[3][4][4];
+                constexpr int RG = MANY ? 1 : 3;
 #pragma unroll
-                for (int rt = 0; rt < 3; ++rt) {
-                    const uint32_t abase = smem_u32(sC + (size_t)(16 * rt + lm_row) * WROW + 64 * warp + lm_k);
+                for (int r0t = 0; r0t < 3; r0t += RG) {
+                    uint32_t af[RG][4][4];
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) ldsm_x4(af[rt][t], abase + 32 * t);
-                }
-                float cg[3][2][4];
+                    for (int rt = 0; rt < RG; ++rt) {
+                        const uint32_t abase = smem_u32(sC + (size_t)(16 * (r0t + rt) + lm_row) * WROW + 64 * warp + lm_k);
 #pragma unroll
-                for (int rt = 0; rt < 3; ++rt)
+                        for (int t = 0; t < 4; ++t) ldsm_x4(af[rt][t], abase + 32 * t);
+                    }
+                    float cg[NT][RG][2][4];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
+                    for (int ct = 0; ct < NT; ++ct)
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) cg[rt][h][i] = 0.f;
+                        for (int rt = 0; rt < RG; ++rt)
 #pragma unroll
-                for (int t = 0; t < 4; ++t)
+                            for (int i = 0; i < 8; ++i) cg[ct][rt][i >> 2][i & 3] = 0.f;
 #pragma unroll
-                    for (int rt = 0; rt < 3; ++rt) mma_bf16(cg[rt][t & 1], af[rt][t], bx[t][0], bx[t][1]);
+                    for (int t = 0; t < 4; ++t)
 #pragma unroll
-                for (int rt = 0; rt < 3; ++rt) {
+                        for (int ct = 0; ct < NT; ++ct)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) cg[rt][0][i] += cg[rt][1][i];
-                    float r0, r1;
-                    fold_cols(cg[rt][0], r0, r1);
-                    if ((lane & 3) == 0) { gpart[warp * 48 + 16 * rt + fr_n] = r0; gpart[warp * 48 + 16 * rt + fr_n + 8] = r1; }
+                            for (int rt = 0; rt < RG; ++rt) mma_bf16(cg[ct][rt][t & 1], af[rt][t], bx[ct][t][0], bx[ct][t][1]);
+#pragma unroll
+                    for (int ct = 0; ct < NT; ++ct)
+#pragma unroll
+                        for (int rt = 0; rt < RG; ++rt) {
+                            float (&c0)[4] = cg[ct][rt][0];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) c0[i] += cg[ct][rt][1][i];
+                            fold(c0, ct, [&](int b, float r0, float r1) {
+                                float* dst = gpart + b * 768 + warp * 48 + 16 * (r0t + rt) + fr_n;
+                                dst[0] = r0; dst[8] = r1;
+                            });
+                        }
                 }
                 cta_sync();
-                if (tid < 32) {   // hid of this CTA's rows, split for the down projection; rows past the share are zero
+                if (warp < NB) {   // hid of this CTA's rows, a warp a sequence, split for the down projection; rows past the share are zero
                     float hv = 0.f;
-                    if (tid < ni) {
-                        const float r = rsqrtf(sum16(red) / (float)HIDDEN + EPS);
+                    if (lane < ni) {
+                        const float r = rsqrtf(sum16(redg + warp * CW) / (float)HIDDEN + EPS);
                         float g = 0.f, u = 0.f;
 #pragma unroll
-                        for (int w = 0; w < CW; ++w) { g += gpart[w * 48 + tid]; u += gpart[w * 48 + imax + tid]; }
+                        for (int w = 0; w < CW; ++w) { g += gpart[warp * 768 + w * 48 + lane]; u += gpart[warp * 768 + w * 48 + imax + lane]; }
                         g *= r; u *= r;
                         hv = (g / (1.f + expf(-g))) * u;
                     }
                     bf16_raw h, m, lo_;
                     split3(hv, h, m, lo_);
-                    reinterpret_cast<bf16_raw*>(hsp)[tid] = h;
-                    reinterpret_cast<bf16_raw*>(hsp + 16)[tid] = m;
-                    reinterpret_cast<bf16_raw*>(hsp + 32)[tid] = lo_;
+                    bf16_raw* dst = reinterpret_cast<bf16_raw*>(hsp + warp * 3 * HLD);
+                    dst[lane] = h; dst[2 * HLD + lane] = m; dst[4 * HLD + lane] = lo_;
                 }
             }
             cta_sync();   // hid ready; the activations and the gate/up slot are no longer needed
@@ -1192,13 +1425,15 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
 
             slot_wait(&full[3], l & 1, abort_flag, p.status, 13, wait_ns);
             {   // out[n] = sum_i wdT[i][n] * hid[i]: A = transposed tiles of the slot, k = this CTA's (<= 32) rows
-                uint32_t bh[2][2];
+                uint32_t bh[NT][2][2];
 #pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    const int kp = (16 * t + fr_k) >> 1;
-                    bh[t][0] = (fr_n < 3) ? hsp[fr_n * 16 + kp] : 0u;
-                    bh[t][1] = (fr_n < 3) ? hsp[fr_n * 16 + kp + 4] : 0u;
-                }
+                for (int ct = 0; ct < NT; ++ct)
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        const int kp = (16 * t + fr_k) >> 1;
+                        bh[ct][t][0] = b_col(hsp, ct, HLD, kp);
+                        bh[ct][t][1] = b_col(hsp, ct, HLD, kp + 4);
+                    }
                 // transposed ldmatrix: lanes 0-7 / 8-15 / 16-23 / 24-31 address rows i of the blocks (n 0-7, i 0-7), (n 8-15, i 0-7), (n 0-7, i 8-15), (n 8-15, i 8-15)
                 const int ti = (lane & 7) + ((lane >> 4) & 1) * 8, tn = ((lane >> 3) & 1) * 8;
                 uint32_t af[4][2][4];
@@ -1210,27 +1445,29 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                         if (i >= ni) i = 0;   // hid is zero there; any finite row will do
                         ldsm_x4_trans(af[nt][t], smem_u32(sD + (size_t)i * WROW + 64 * warp + 16 * nt + tn));
                     }
-                float cc[4][4];
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt)
+                for (int ct = 0; ct < NT; ++ct) {
+                    float cc[4][4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) cc[nt][i] = 0.f;
+                    for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-                for (int t = 0; t < 2; ++t)
+                        for (int i = 0; i < 4; ++i) cc[nt][i] = 0.f;
 #pragma unroll
-                    for (int nt = 0; nt < 4; ++nt) mma_bf16(cc[nt], af[nt][t], bh[t][0], bh[t][1]);
+                    for (int t = 0; t < 2; ++t)
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt) {
-                    const int n0 = 64 * warp + 16 * nt;
-                    float r0, r1;
-                    fold_cols(cc[nt], r0, r1);
-                    if ((lane & 3) == 0) { dout[n0 + fr_n] = r0; dout[n0 + fr_n + 8] = r1; }
+                        for (int nt = 0; nt < 4; ++nt) mma_bf16(cc[nt], af[nt][t], bh[ct][t][0], bh[ct][t][1]);
+#pragma unroll
+                    for (int nt = 0; nt < 4; ++nt)
+                        fold(cc[nt], ct, [&](int b, float r0, float r1) {
+                            dout[b * HIDDEN + 64 * warp + 16 * nt + fr_n] = r0; dout[b * HIDDEN + 64 * warp + 16 * nt + fr_n + 8] = r1;
+                        });
                 }
             }
             cta_sync();
-            if (tid < 256) {
-                const float4 t = *reinterpret_cast<const float4*>(dout + tid * 4);
-                const size_t off = (size_t)(l % 3) * N_ACC * HIDDEN + (size_t)(c & (N_ACC - 1)) * HIDDEN + tid * 4;
+            for (int q = tid; q < 256 * NB; q += CT) {
+                const int b = q >> 8, e = (q & 255) * 4;
+                const float4 t = *reinterpret_cast<const float4*>(dout + q * 4);
+                const size_t off = (size_t)(l % 3) * NACC * NB * HIDDEN + (size_t)((c & (NACC - 1)) * NB + b) * HIDDEN + e;
                 if (TP) { for (int r = 0; r < T; ++r) red_add_v4<true>(p.tp_dB[r] + off, t.x, t.y, t.z, t.w); }
                 else red_add_v4<false>(p.dB + off, t.x, t.y, t.z, t.w);
             }
@@ -1244,40 +1481,76 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
         target += (unsigned)(T * G);
         gain2 = (l + 1 < L) ? *reinterpret_cast<const uint32_t*>(p.ln1 + (size_t)(l + 1) * HIDDEN + 2 * tid)
                             : *reinterpret_cast<const uint32_t*>(p.fnorm + 2 * tid);
+        kl += lstride;
+        vl += lstride;
         counter_wait<TP>(bar, target, abort_flag, p.status, 300 + l, wait_ns);
         Q3_TRACE(ev + 11);
     }
 
     // ======================================================================== LM head + argmax
     {
-        add_ffn_delta(p.dB + (size_t)((L - 1) % 3) * N_ACC * HIDDEN);
-        const float ss = warp_sum(x0 * x0 + x1 * x1);
-        if (lane == 0) red[warp] = ss;
+        add_ffn_delta(p.dB + (size_t)((L - 1) % 3) * NACC * NB * HIDDEN);
+        float* const reds = MANY ? fbuf : red;     // [NB][16]
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const float ss = warp_sum(x0[b] * x0[b] + x1[b] * x1[b]);
+            if (lane == 0) reds[b * CW + warp] = ss;
+        }
         cta_sync();
-        float tot = (lane < CW) ? red[lane] : 0.f;
-        tot = warp_sum(tot);
-        const float r = rsqrtf(tot / (float)HIDDEN + EPS);
-        xs[act_slot(2 * tid)] = (x0 * r) * bf_lo(gain2);
-        xs[act_slot(2 * tid + 1)] = (x1 * r) * bf_hi(gain2);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            float tot = (lane < CW) ? reds[b * CW + lane] : 0.f;
+            tot = warp_sum(tot);
+            const float r = rsqrtf(tot / (float)HIDDEN + EPS);
+            const float y0 = (x0[b] * r) * bf_lo(gain2), y1 = (x1[b] * r) * bf_hi(gain2);
+            if constexpr (!MANY) {
+                xs[act_slot(2 * tid)] = y0;
+                xs[act_slot(2 * tid + 1)] = y1;
+            } else {
+                uint32_t* xw = reinterpret_cast<uint32_t*>(xs) + b * 3 * LLD + tid;
+                bf16_raw h0, m0, l0, h1, m1, l1;
+                split3(y0, h0, m0, l0);
+                split3(y1, h1, m1, l1);
+                xw[0] = (uint32_t)h0 | ((uint32_t)h1 << 16);
+                xw[LLD] = (uint32_t)m0 | ((uint32_t)m1 << 16);
+                xw[2 * LLD] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+            }
+        }
         cta_sync();
 
-        float bestv = -INFINITY;
+        float bestv = -INFINITY;      // one sequence: the warp's, in lane 0; several: of sequence lane & 7, in the lanes that hold its rows
         int besti = 0x7fffffff;
-        lm_stream(warp, CW, bestv, besti);
+        if constexpr (!MANY) lm_stream(warp, CW, bestv, besti);
+        else {
+            lm_mma(bestv, besti);
+#pragma unroll
+            for (int o = 8; o <= 16; o <<= 1) {
+                const float ov = __shfl_xor_sync(0xffffffffu, bestv, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, besti, o);
+                if (ov > bestv || (ov == bestv && oi < besti)) { bestv = ov; besti = oi; }
+            }
+        }
         Q3_TRACE(1 + EV_PER_LAYER * L);
         // CTA argmax (ties -> lowest index), then the last CTA to finish reduces over CTAs
         float* bv_s = lm_bv;
         int* bi_s = lm_bi;
-        if (lane == 0) { bv_s[warp] = bestv; bi_s[warp] = besti; }
+        if (lane < NB) { bv_s[lane * CW + warp] = bestv; bi_s[lane * CW + warp] = besti; }
         cta_sync();
         int* last_flag = reinterpret_cast<int*>(v_s);
-        if (tid == 0) {
-            float bv = bv_s[0];
-            int bi = bi_s[0];
+        auto best_of_warps = [&](int b, float& bv, int& bi) {
+            bv = bv_s[b * CW]; bi = bi_s[b * CW];
             for (int w = 1; w < CW; ++w)
-                if (bv_s[w] > bv || (bv_s[w] == bv && bi_s[w] < bi)) { bv = bv_s[w]; bi = bi_s[w]; }
-            __stcg(p.pval + c, bv);
-            __stcg(p.pidx + c, bi);
+                if (bv_s[b * CW + w] > bv || (bv_s[b * CW + w] == bv && bi_s[b * CW + w] < bi)) { bv = bv_s[b * CW + w]; bi = bi_s[b * CW + w]; }
+        };
+        if (tid == 0) {
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                float bv;
+                int bi;
+                best_of_warps(b, bv, bi);
+                __stcg(p.pval + b * G + c, bv);
+                __stcg(p.pidx + b * G + c, bi);
+            }
             __threadfence();
             const unsigned prev = atomicAdd(p.sync + 2, 1u);
             *last_flag = (prev == (unsigned)G - 1u);
@@ -1285,28 +1558,32 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
         }
         cta_sync();
         if (*last_flag) {
-            float bv = -INFINITY;
-            int bi = 0x7fffffff;
-            for (int i = tid; i < G; i += CT) {
-                const float v = __ldcg(p.pval + i);
-                const int ix = __ldcg(p.pidx + i);
-                if (v > bv || (v == bv && ix < bi)) { bv = v; bi = ix; }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-            }
             cta_sync();
-            if (lane == 0) { bv_s[warp] = bv; bi_s[warp] = bi; }
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                float bv = -INFINITY;
+                int bi = 0x7fffffff;
+                for (int i = tid; i < G; i += CT) {
+                    const float v = __ldcg(p.pval + b * G + i);
+                    const int ix = __ldcg(p.pidx + b * G + i);
+                    if (v > bv || (v == bv && ix < bi)) { bv = v; bi = ix; }
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                    if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+                }
+                if (lane == 0) { bv_s[b * CW + warp] = bv; bi_s[b * CW + warp] = bi; }
+            }
             cta_sync();
             // every CTA has read its last delta: the next launch starts from clean accumulators (dA and dB are adjacent)
-            for (int i = tid; i < (int)(ACC_FLOATS / 4); i += CT) __stcg(reinterpret_cast<float4*>(p.dA) + i, make_float4(0.f, 0.f, 0.f, 0.f));
+            for (int i = tid; i < (int)(acc_floats(NB) / 4); i += CT) __stcg(reinterpret_cast<float4*>(p.dA) + i, make_float4(0.f, 0.f, 0.f, 0.f));
             cta_sync();
             if (tid == 0) {
-                for (int w = 1; w < CW; ++w)
-                    if (bv_s[w] > bv || (bv_s[w] == bv && bi_s[w] < bi)) { bv = bv_s[w]; bi = bi_s[w]; }
+                float bv;
+                int bi;
+                best_of_warps(0, bv, bi);
                 if (TP) {
                     // This rank's best word goes to every rank's mailbox; the best of all ranks is the token.  The mail is
                     // also the hand-over to the next launch: a peer that holds it may start adding to this rank's deltas
@@ -1339,7 +1616,11 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                     p.sync[0] = 0;   // every CTA has passed every barrier: rearm the counter for the next launch
                 }
                 p.next_token[0] = bi;
-                if (p.append) p.seq_len[0] = len + 1;
+#pragma unroll
+                for (int b = 1; b < NB; ++b) { best_of_warps(b, bv, bi); p.next_token[b] = bi; }
+                if (p.append)
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) p.seq_len[b] += 1;
                 p.sync[2] = 0;
                 *const_cast<unsigned*>(p.epoch) = tag_base / 64u + 1u;
             }
@@ -1422,19 +1703,21 @@ static int smem_bytes_for(int grid) {
     return (qmax + 3 * imax) * WROW * 2 + WO_ROWS_MAX * WOROW * 2 + TAIL_BYTES;
 }
 
-static const void* persist_kernel(int mode, bool tp = false) {
+static const void* persist_kernel(int mode, bool tp = false, int together = 1) {
+    if (together == 2) return reinterpret_cast<const void*>(q3_persist_decode<N_MODES - 1, false, 2>);
+    if (together == 3) return reinterpret_cast<const void*>(q3_persist_decode<N_MODES - 1, false, 3>);
     if (tp) {
         switch (mode) {
-            case 0: return reinterpret_cast<const void*>(q3_persist_decode<0, true>);
-            case 1: return reinterpret_cast<const void*>(q3_persist_decode<1, true>);
-            default: return reinterpret_cast<const void*>(q3_persist_decode<2, true>);
+            case 0: return reinterpret_cast<const void*>(q3_persist_decode<0, true, 1>);
+            case 1: return reinterpret_cast<const void*>(q3_persist_decode<1, true, 1>);
+            default: return reinterpret_cast<const void*>(q3_persist_decode<2, true, 1>);
         }
     }
     switch (mode) {
-        case 0: return reinterpret_cast<const void*>(q3_persist_decode<0, false>);
-        case 1: return reinterpret_cast<const void*>(q3_persist_decode<1, false>);
-        case 2: return reinterpret_cast<const void*>(q3_persist_decode<2, false>);
-        default: return reinterpret_cast<const void*>(q3_persist_decode<3, false>);
+        case 0: return reinterpret_cast<const void*>(q3_persist_decode<0, false, 1>);
+        case 1: return reinterpret_cast<const void*>(q3_persist_decode<1, false, 1>);
+        case 2: return reinterpret_cast<const void*>(q3_persist_decode<2, false, 1>);
+        default: return reinterpret_cast<const void*>(q3_persist_decode<3, false, 1>);
     }
 }
 
@@ -1450,8 +1733,10 @@ int persist_setup(q3_engine* e) {
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, e->device) != cudaSuccess) return engine_fail(e, Q3_ERR_CUDA, "cudaGetDeviceProperties failed");
     if ((size_t)smem > prop.sharedMemPerBlockOptin) return Q3_OK;
-    for (int variant = 0; variant < 2 * N_MODES - 1; ++variant) {   // the four attention variants, then the three tensor-parallel ones
-        const void* fn = variant < N_MODES ? persist_kernel(variant) : persist_kernel(variant - N_MODES, true);
+    // the four attention variants, the three tensor-parallel ones, then those of several sequences
+    for (int variant = 0; variant < 2 * N_MODES - 1 + PERSIST_MAX_BATCH - 1; ++variant) {
+        const void* fn = variant < N_MODES ? persist_kernel(variant) : variant < 2 * N_MODES - 1 ? persist_kernel(variant - N_MODES, true)
+                                                                                                : persist_kernel(N_MODES - 1, false, variant - (2 * N_MODES - 1) + 2);
         cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (err != cudaSuccess) return engine_fail(e, Q3_ERR_CUDA, "persist: set smem attribute (%d B): %s", smem, cudaGetErrorString(err));
         int per_sm = 0;
@@ -1488,14 +1773,14 @@ void persist_teardown(q3_engine* e) {
     e->p_state = nullptr;
 }
 
-// Batches of up to PERSIST_MAX_BATCH sequences are served as one launch per sequence (q3_decode picks it for one sequence only).
+// Batches of up to PERSIST_MAX_BATCH sequences: one launch for all of them, or one after the other for a caller that names this kernel.
 bool persist_supports(const q3_engine* e, const q3_decode_args* a) {
     const PersistState* s = static_cast<const PersistState*>(e->p_state);
     if (s == nullptr || a->batch < 1) return false;
     if (reinterpret_cast<uintptr_t>(e->rope) & 15) return false;   // the kernel reads the table 16 bytes at a time (a test of it there: 3 us a step)
     if (s->tp_size > 1) return a->batch == 1 && a->max_len <= mode_max_len(N_MODES - 2);   // one sequence, local attention
     const bool asked = (a->flags & Q3_F_PATH_MASK) == Q3_F_PATH_PERSIST;
-    return a->batch <= PERSIST_MAX_BATCH && a->max_len <= (asked ? PERSIST_ASKED_LEN : PERSIST_MAX_LEN);
+    return a->batch <= PERSIST_MAX_BATCH && a->max_len <= (asked ? PERSIST_ASKED_LEN : a->batch == 3 ? PERSIST_THREE_LEN : PERSIST_MAX_LEN);
 }
 
 // (Re)pack the layer matrices when one of the caller's pointers changes.  Runs on the legacy default
@@ -1530,7 +1815,7 @@ int persist_recover(q3_engine* e) {
 void* persist_accumulators(const q3_engine* e, int64_t* bytes) {
     PersistState* s = static_cast<PersistState*>(e->p_state);
     if (!s) return nullptr;
-    *bytes = (int64_t)(ACC_FLOATS * sizeof(float));
+    *bytes = (int64_t)(acc_floats(1) * sizeof(float));
     return s->X;
 }
 
@@ -1590,10 +1875,12 @@ int persist_decode(q3_engine* e, const q3_decode_args* a, cudaStream_t st) {
     p.seq_k = a->seq_k; p.seq_v = a->seq_v; p.seq_layer_stride = reinterpret_cast<const long long*>(a->seq_layer_stride);
     p.seq_len = a->seq_len; p.logits = a->logits; p.next_token = reinterpret_cast<long long*>(a->next_token);
     p.k_write = reinterpret_cast<bf16_raw*>(a->k_write); p.v_write = reinterpret_cast<bf16_raw*>(a->v_write);
-    p.dA = reinterpret_cast<unsigned long long*>(s->X); p.dB = s->X + 4 * HIDDEN;
-    p.xq = reinterpret_cast<unsigned long long*>(s->X + ACC_FLOATS);
-    p.epoch = reinterpret_cast<const unsigned*>(s->X + ACC_FLOATS + 2 * QKV_DIM);
-    p.xp = reinterpret_cast<unsigned long long*>(s->X + ACC_FLOATS + 2 * QKV_DIM + 64);
+    const bool asked = (a->flags & Q3_F_PATH_MASK) == Q3_F_PATH_PERSIST;
+    const int together = asked ? 1 : a->batch;             // sequences of a launch
+    p.dA = reinterpret_cast<unsigned long long*>(s->X); p.dB = s->X + 4 * HIDDEN * together;
+    p.xq = reinterpret_cast<unsigned long long*>(s->X + XQ_OFFSET);
+    p.epoch = reinterpret_cast<const unsigned*>(s->X + EPOCH_OFFSET);
+    p.xp = reinterpret_cast<unsigned long long*>(s->X + EPOCH_OFFSET + 64);
     p.wait_ns = e->cfg.wait_limit_us > 0 ? (unsigned long long)e->cfg.wait_limit_us * 1000ull : WAIT_NS;
     const bool tp = s->tp_size > 1;
     p.tp_rank = s->tp_rank; p.tp_size = s->tp_size;
@@ -1609,12 +1896,13 @@ int persist_decode(q3_engine* e, const q3_decode_args* a, cudaStream_t st) {
     p.n_layers = e->cfg.n_layers; p.vocab = e->cfg.vocab; p.append = (a->flags & Q3_F_APPEND_KV) ? 1 : 0;
     int mode = 0;
     while (mode + 1 < N_MODES && a->max_len > mode_max_len(mode)) ++mode;
-    p.max_len = mode < N_MODES - 1 ? mode_max_len(mode) : a->max_len > PERSIST_ASKED_LEN ? a->max_len : PERSIST_ASKED_LEN;
+    if (together > 1) mode = N_MODES - 1;
+    p.max_len = together > 1 ? a->max_len : mode < N_MODES - 1 ? mode_max_len(mode) : a->max_len > PERSIST_ASKED_LEN ? a->max_len : PERSIST_ASKED_LEN;
     if (p.max_len > e->rope_n - 1) p.max_len = e->rope_n - 1;
-    // A small batch is one launch per sequence, back to back on the stream: the kernel reads entry 0 of every
-    // per-sequence array, so the arrays are simply offset (outputs are [batch][...] with the batch axis leading).
+    // A batch of a caller that names this kernel is one launch per sequence, back to back on the stream: the per-sequence
+    // arrays are simply offset (outputs are [batch][...] with the batch axis leading).
     const size_t kv_row = (size_t)e->cfg.n_layers * KV_DIM;
-    for (int b = 0; b < a->batch; ++b) {
+    for (int b = 0; b < a->batch; b += together) {
         PersistParams q = p;
         q.token = p.token + b; q.seq_k = p.seq_k + b; q.seq_v = p.seq_v + b; q.seq_layer_stride = p.seq_layer_stride + b;
         q.seq_len = p.seq_len + b; q.next_token = p.next_token + b;
@@ -1622,7 +1910,7 @@ int persist_decode(q3_engine* e, const q3_decode_args* a, cudaStream_t st) {
         q.k_write = p.k_write ? p.k_write + b * kv_row : nullptr;
         q.v_write = p.v_write ? p.v_write + b * kv_row : nullptr;
         void* args[] = {&q};
-        cudaError_t err = cudaLaunchCooperativeKernel(persist_kernel(mode, tp), dim3(s->grid), dim3(PT), args, (size_t)s->smem, st);
+        cudaError_t err = cudaLaunchCooperativeKernel(persist_kernel(mode, tp, together), dim3(s->grid), dim3(PT), args, (size_t)s->smem, st);
         ++e->launches;
         if (err != cudaSuccess) return engine_fail(e, Q3_ERR_CUDA, "persist: cooperative launch failed: %s", cudaGetErrorString(err));
     }

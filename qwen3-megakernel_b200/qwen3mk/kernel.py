@@ -130,7 +130,7 @@ class Megakernel:
     path: fixed inputs, outputs overwritten by every launch, no synchronisation.
     `bind_sequences` is the batched / growing-cache form of `bind`.
 
-    path: "auto" (persistent kernel for one sequence it serves, else layered), "layered" (a chain of launches), "fused" (layered, with
+    path: "auto" (persistent kernel for up to three sequences it serves, else layered), "layered" (a chain of launches), "fused" (layered, with
     one persistent kernel for everything between two attentions for batches of 4..64; opt-in) or "persist".
     """
 

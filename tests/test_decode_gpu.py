@@ -120,6 +120,56 @@ def test_one_sequence_is_one_launch_at_any_length(oracle, ctx):
             mk.status()
 
 
+@pytest.mark.parametrize("grid", [0, 147])
+def test_two_and_three_sequences_are_one_launch(oracle, grid):
+    """One engine, batches of one to three in turn on the same scratch.  The 18 blocks of a kv head are dealt out by the lengths: empty caches, one
+    that takes all blocks but one, shares around a pass of 32 positions a block, the longest three
+    (1500); one position more is the chain's, and so is a ninth step of three sequences."""
+    from qwen3mk.kernel import SeqTable
+
+    shp = oracle.Shape(layers=2, vocab=2052)       # (the last rows of the LM head are no whole tile)
+    inp = oracle.synthetic(77, shp, context=1)
+    w = oracle.to_fp32(inp)
+    dev = to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES})
+    mk = engine("auto", layers=2, vocab=2052, max_batch=3, grid_limit=grid)
+    g = torch.Generator().manual_seed(5)
+    for lens in [(0, 0), (300,), (0, 5, 1), (1, 3400), (577, 31, 33), (288, 289), (1499, 1, 600), (40,), (1152, 1153), (1501, 9, 40), (33, 20, 2)]:
+        toks = torch.randint(0, 2052, (len(lens),), generator=g)
+        kcs = [torch.randn(2, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens]
+        vcs = [torch.randn(2, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens]
+        room = [[torch.cat([t, torch.zeros(2, 10, 8, 128, dtype=t.dtype)], 1).cuda() for t in side] for side in (kcs, vcs)]
+        seqs = SeqTable(room[0], room[1], lens=list(lens))
+        out = mk.bind_sequences(dev, toks.cuda(), seqs, append=True)
+        before = mk.launch_count
+        mk.launch()
+        mk.status()
+        assert (mk.launch_count == before + 1) == (lens[0] != 1501), lens
+        refs = oracle.decode_batch(w, toks.tolist(), kcs, vcs)
+        for b, ref in enumerate(refs):
+            gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{lens} seq {b}")
+            assert torch.equal(room[0][b][:, lens[b]], out["k_write"][b]) and torch.equal(room[1][b][:, lens[b]], out["v_write"][b])
+        assert seqs.len.tolist() == [n + 1 for n in lens]
+        steps = 9 if lens[0] == 33 else 2
+        for i in range(2, steps + 1):              # the appended rows are read
+            one = mk.launch_count
+            mk.launch()
+            assert (mk.launch_count == one + 1) == (lens[0] != 1501 and i < 9), (lens, i)
+        mk.status()
+        n1 = [n + steps - 1 for n in lens]
+        refs = oracle.decode_batch(w, toks.tolist(), [k[:, :n].cpu() for k, n in zip(room[0], n1)], [v[:, :n].cpu() for v, n in zip(room[1], n1)])
+        for b, ref in enumerate(refs):
+            gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{lens} seq {b}, step {steps}")
+    seqs = SeqTable(room[0][:1] * 2, room[1][:1] * 2, lens=[30, 20])
+    mk.bind_sequences(dev, toks[:2].cuda(), seqs)
+    seqs.len.copy_(torch.tensor([30, 31]))       # longer than the host said: reported
+    mk.launch()
+    with pytest.raises(RuntimeError, match="code 5"):
+        mk.status()
+    seqs.len.copy_(torch.tensor([30, 20]))
+    mk.launch()
+    mk.status()
+
+
 @pytest.mark.parametrize("ctx", [40, 200, 300])
 def test_persist_on_a_grid_one_short_of_the_sm_count(oracle, ctx):
     """147 CTAs is the smallest grid the persistent kernel's shared-memory slots allow; the row shares differ from 148's."""
