@@ -25,9 +25,9 @@
 // T <= 0 or k == 1 degenerate to the arg-max (ties -> lowest index), like the decode kernels.
 //
 // A single row is bound by latency (0.6 MB, but a dozen dependent block-wide steps), a full batch by the row's bytes and the same steps.
-// Measured, us, before the sums under a block's own maximum and the draw from the candidates -> now: 1 row, k = 50: 14.7 -> 12.3; 64 rows, k = 50:
-// 32.8 -> 24.6; 64 rows, whole vocabulary: 24.7 -> 20.5 (the second pass over the row is gone).  Logits that the caches have not seen before gain
-// less: 1.06 and 1.09 in the first and the last of these.
+// Measured, us: 1 row, k = 50: 10.9 (12.3 before a warp took its largest value in one instruction); 15 / 36 / 64 rows, whole vocabulary: 12.6 / 18.9 / 18.6 (before a run's last loads left together, four words a thread
+// in the walk, and up to 64 rows the next loads under way behind the ones at work: 13.8 / 20.7 / 20.7); 15 / 36 / 64 rows, k = 50: 15.1 / 18.7 / 18.7 (before
+// lanes shared the second look at the row: 16.6 / 22.8 / 24.8).
 #include <cooperative_groups.h>
 
 #include <cfloat>
@@ -51,6 +51,13 @@ __device__ __forceinline__ unsigned ordered_key(float f) {   // monotonic in the
 }
 
 __device__ __forceinline__ float key_value(unsigned k) { return __uint_as_float((k >> 31) ? k ^ 0x80000000u : ~k); }   // the inverse
+
+// the largest of a warp's values (one instruction; a NaN loses to any number, as in fmaxf)
+__device__ __forceinline__ float row_max(float v) {
+    float m;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(v));
+    return m;
+}
 
 // elements of a warp's run when a row of `vocab` words goes to `cluster` blocks
 __host__ __device__ inline int sample_run(int vocab, int cluster) {
@@ -100,10 +107,12 @@ __device__ __forceinline__ void find_bin(SampleShared& sh, unsigned c0, unsigned
 }
 
 // Elements are dealt out in groups of 128 per warp, four neighbours a lane: element 4 lane + q of group j.  NQ > 0: a thread's
-// elements of the row (at most NQ groups) stay in registers; NQ == 0: every pass reads the row again (from L2).
-template <int NQ>
-__global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(const float* __restrict__ logits, int vocab, float temperature, int top_k,
+// elements of the row (at most NQ groups) stay in registers; NQ == 0: every pass reads the row again (from L2).  TWO: two blocks an SM (32 registers a
+// thread).  SHARE: the threads with candidates read again with the help of their warp.
+template <int NQ, bool TWO, bool SHARE>
+__global__ void __launch_bounds__(SAMPLE_THREADS, TWO ? 2 : 1) sample_kernel(const float* __restrict__ logits, int vocab, float temperature, int top_k,
                                                                              const float* __restrict__ uniform, long long* __restrict__ out) {
+    constexpr int WALK = NQ > 0 || (TWO && !SHARE) ? 1 : 4;     // words a thread takes of the run that is walked (a run of up to 640, and where registers are short: one)
     __shared__ SampleShared sh;
     cg::cluster_group cluster = cg::this_cluster();
     const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
@@ -122,8 +131,8 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     const bool vec = ((vocab & 3) | (int)(reinterpret_cast<uintptr_t>(logits) & 15)) == 0;
     cluster.barrier_arrive();   // (a peer's shared memory may be written once the peer runs: waited for before the first exchange)
 
-    auto fetch = [&](int j) -> float4 {  // group j; elements past the run are -inf, which no pass below counts
-        const int i = i0 + 128 * j + 4 * lane;
+    auto fetch = [&](int j, int of) -> float4 {  // group j of lane `of`; elements past the run are -inf, which no pass below counts
+        const int i = i0 + 128 * j + 4 * of;
         if (vec && i + 3 < i1) return *reinterpret_cast<const float4*>(row + i);
         float4 v;
         v.x = i < i1 ? row[i] : -INFINITY; v.y = i + 1 < i1 ? row[i + 1] : -INFINITY;
@@ -133,9 +142,30 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     float4 x[NQ > 0 ? NQ : 1];
     if constexpr (NQ > 0) {
 #pragma unroll
-        for (int j = 0; j < NQ; ++j) x[j] = fetch(j);
+        for (int j = 0; j < NQ; ++j) x[j] = fetch(j, lane);
     }
     const int groups = (i1 - i0 + 127) / 128, whole = vec ? (i1 - i0) / 128 : 0;
+    // NQ == 0: f(first group, four groups' elements) over the run.  The loads of the next four groups are under way while these are at work where the
+    // registers allow it (a block an SM), and the last ones leave together.
+    auto batches = [&](auto&& f) {
+        auto load = [&](int j, float4 (&v)[4]) {
+            if (j + 4 <= whole) {                  // (no guards)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = *reinterpret_cast<const float4*>(row + i0 + 128 * (j + q) + 4 * lane);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = fetch(j + q, lane);
+            }
+        };
+        float4 v[2][4];
+        if (groups > 0) load(0, v[0]);
+        for (int j = 0; j < groups; j += 8) {
+            if (j + 4 < groups) load(j + 4, v[1]);
+            f(j, v[0]);
+            if (j + 8 < groups) load(j + 8, v[0]);
+            if (j + 4 < groups) f(j + 4, v[1]);
+        }
+    };
     auto each = [&](auto&& f) {          // f(index, value) over this thread's elements, in ascending order
         auto four = [&](int j, const float4& v) {
             const int i = i0 + 128 * j + 4 * lane;
@@ -145,15 +175,22 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
 #pragma unroll
             for (int j = 0; j < NQ; ++j) four(j, x[j]);
         } else {
-            int j = 0;
-            for (; j + 4 <= whole; j += 4) {       // (no guards: the four loads leave together)
-                float4 v[4];
+            if constexpr (TWO) {
+                int j = 0;
+                for (; j + 4 <= whole; j += 4) {   // (no guards: the four loads leave together)
+                    float4 v[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) v[q] = *reinterpret_cast<const float4*>(row + i0 + 128 * (j + q) + 4 * lane);
+                    for (int q = 0; q < 4; ++q) v[q] = *reinterpret_cast<const float4*>(row + i0 + 128 * (j + q) + 4 * lane);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) four(j + q, v[q]);
+                    for (int q = 0; q < 4; ++q) four(j + q, v[q]);
+                }
+                for (; j < groups; ++j) four(j, fetch(j, lane));
+            } else {
+                batches([&](int j, const float4 (&v)[4]) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) four(j + q, v[q]);
+                });
             }
-            for (; j < groups; ++j) four(j, fetch(j));
         }
     };
 
@@ -173,28 +210,35 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
         };
         auto top4 = [&](const float4& v) { return fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); };
         auto add4 = [&](const float4& v) { wsum += (weight(v.x, mine) + weight(v.y, mine)) + (weight(v.z, mine) + weight(v.w, mine)); };
-        int j = 0;
-        for (; j + 4 <= whole; j += 4) {
-            float4 v[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) v[q] = *reinterpret_cast<const float4*>(row + i0 + 128 * (j + q) + 4 * lane);
+        auto sixteen = [&](const float4 (&v)[4]) {
             raise(fmaxf(fmaxf(top4(v[0]), top4(v[1])), fmaxf(top4(v[2]), top4(v[3]))));
 #pragma unroll
             for (int q = 0; q < 4; ++q) add4(v[q]);
+        };
+        if constexpr (TWO) {
+            int j = 0;
+            for (; j + 4 <= whole; j += 4) {
+                float4 v[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = *reinterpret_cast<const float4*>(row + i0 + 128 * (j + q) + 4 * lane);
+                sixteen(v);
+            }
+            for (; j < groups; ++j) { const float4 v = fetch(j, lane); raise(top4(v)); add4(v); }
+        } else {
+            batches([&](int, const float4 (&v)[4]) { sixteen(v); });
         }
-        for (; j < groups; ++j) { const float4 v = fetch(j); raise(top4(v)); add4(v); }
     } else {
         each([&](int, float v) { mine = fmaxf(mine, v); nan = nan || v != v; });
     }
     {
-        const float bv = warp_max(mine), lo = -warp_max(any ? -mine : -INFINITY);
+        const float bv = row_max(mine), lo = -row_max(any ? -mine : -INFINITY);
         if (lane == 0) { sh.wf[warp] = bv; sh.wg[warp] = lo; }
     }
     if (select)
         for (int b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) sh.hist[b] = 0u;
     if (tid == 0) { sh.cand_n = 0u; sh.need = 0x7fffffffu; sh.cmin = 0xffffffffu; }
     const int n_thr = __syncthreads_count(any);     // threads that have an element
-    const float bmax = warp_max(sh.wf[lane]), blo = -warp_max(-sh.wg[lane]);
+    const float bmax = row_max(sh.wf[lane]), blo = -row_max(-sh.wg[lane]);
 
     // ---- 2a. the block's candidates for the k largest ----
     int n_cand = -1;
@@ -211,14 +255,36 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
             __syncthreads();
             find_bin(sh, sh.hist[2 * tid], sh.hist[2 * tid + 1], (unsigned)top_k, false);
             const int last = (int)sh.sel;
-            if (any && bin(mine) <= last)           // (a thread whose maximum is below the bound has no candidate)
-                each([&](int i, float v) {
-                    if (bin(v) <= last && i < i1) {
-                        const unsigned n = atomicAdd(&sh.cand_n, 1u), key = ordered_key(v);
-                        if (n < SAMPLE_CAND) { raw[n] = key; raw[SAMPLE_CAND + n] = (unsigned)i; }
-                        atomicMin(&sh.cmin, key);
+            auto take = [&](int i, float v) {
+                if (bin(v) <= last && i < i1) {
+                    const unsigned n = atomicAdd(&sh.cand_n, 1u), key = ordered_key(v);
+                    if (n < SAMPLE_CAND) { raw[n] = key; raw[SAMPLE_CAND + n] = (unsigned)i; }
+                    atomicMin(&sh.cmin, key);
+                }
+            };
+            const bool has = any && bin(mine) <= last;          // (a thread whose maximum is below the bound has no candidate)
+            if constexpr (!SHARE) {
+                if (has) each(take);
+            } else {
+                // The few threads that have some read their elements again, all of a thread's groups at once: a lane a group, four threads' loads
+                // under way.
+                for (unsigned m = __ballot_sync(0xffffffffu, has); m; ) {
+                    int of[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) { of[q] = m ? __ffs(m) - 1 : -1; m &= m - 1; }
+                    for (int j = lane; j < groups; j += 32) {
+                        float4 v[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (of[q] >= 0) v[q] = fetch(j, of[q]);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const int i = i0 + 128 * j + 4 * of[q];
+                            if (of[q] >= 0) { take(i, v[q].x); take(i + 1, v[q].y); take(i + 2, v[q].z); take(i + 3, v[q].w); }
+                        }
                     }
-                });
+                }
+            }
             __syncthreads();
             // In the order of their indices: sums of weights must not depend on which thread came first.  (A list is about 1.1 k words long.)
             const int n = (int)sh.cand_n;
@@ -269,7 +335,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
         peer->bmax[rank] = bmax; peer->ncand[rank] = n_cand; peer->bsum[rank] = bsum;
     }
     cluster.sync();
-    const float vmax = warp_max(lane < C ? sh.bmax[lane] : -INFINITY);
+    const float vmax = row_max(lane < C ? sh.bmax[lane] : -INFINITY);
     // the row's lowest index that holds the maximum (every block of the cluster takes part)
     auto write_argmax = [&]() {
         __syncthreads();
@@ -460,7 +526,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     if (!(target < total)) target = __uint_as_float(__float_as_uint(total) - 1u);   // u * total rounded up to the total: the last word with a weight
     if (!(base <= target && target < next)) return;
     // Inside the block: `from` of the first warp is base, `to` of the last one is next (the same roundings), and both are the same sums for
-    // the neighbouring warps, so exactly one warp's run takes it.  The whole block walks that run, 1024 elements a round.
+    // the neighbouring warps, so exactly one warp's run takes it.  The whole block walks that run, WALK words a thread.
     const float from = __fadd_rn(base, __fmul_rn(scale, lo)), to = __fadd_rn(base, __fmul_rn(scale, hi));
     if (lane == 0 && from <= target && target < to) { sh.sel = (unsigned)warp; sh.wg[0] = from; }
     if (tid == 0) { sh.need = 0xffffffffu; sh.cand_n = 0u; }
@@ -472,31 +538,44 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     float run = sh.wg[0];
     int first = r0, end = r1, span = 0;             // 0: the run, 1: what follows it, 2: what is before it
     for (;;) {
-        const int i = first + tid;
-        const float v = i < end ? row[i] : -INFINITY;
+        const int i = first + WALK * tid;
+        float own[WALK], incl[WALK];
+#pragma unroll
+        for (int q = 0; q < WALK; ++q) own[q] = i + q < end ? row[i + q] : -INFINITY;
         // (the scan adds the same weights in another order for every lane, so a word without weight may see a larger prefix than the
         // word before it: only one with a weight is a candidate)
-        const float own = v >= least ? __expf((v - vmax) * inv_t) : 0.f;
-        const bool kept = own > 0.f;
-        float incl = own;
+#pragma unroll
+        for (int q = 0; q < WALK; ++q) {
+            own[q] = own[q] >= least ? __expf((own[q] - vmax) * inv_t) : 0.f;
+            incl[q] = q ? incl[q - 1] + own[q] : own[q];
+        }
+        float sum = incl[WALK - 1];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const float p = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += p;
+            const float p = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += p;
         }
-        if (lane == 31) sh.wf[warp] = incl;
+        if (lane == 31) sh.wf[warp] = sum;
+        float lower = __shfl_up_sync(0xffffffffu, sum, 1);     // of the lanes before this one
+        if (lane == 0) lower = 0.f;
         __syncthreads();
         float before = run;
         for (int w = 0; w < SAMPLE_WARPS; ++w) {
             if (w == warp) before = run;
             run += sh.wf[w];
         }
-        const unsigned hit = __ballot_sync(0xffffffffu, kept && (span > 0 || before + incl > target)), all = __ballot_sync(0xffffffffu, kept);
-        if (lane == 0 && hit) atomicMin(&sh.need, (unsigned)(first + 32 * warp + __ffs(hit) - 1));
-        if (lane == 0 && all) atomicMax(&sh.cand_n, (unsigned)(first + 32 * warp + 32 - __clz(all)));   // (0: none so far)
+        unsigned hit = 0xffffffffu, last = 0u;
+#pragma unroll
+        for (int q = WALK - 1; q >= 0; --q) {
+            if (own[q] > 0.f && (span > 0 || before + (lower + incl[q]) > target)) hit = (unsigned)(i + q);
+            if (own[q] > 0.f && last == 0u) last = (unsigned)(i + q + 1);
+        }
+        hit = __reduce_min_sync(0xffffffffu, hit); last = __reduce_max_sync(0xffffffffu, last);
+        if (lane == 0 && hit != 0xffffffffu) atomicMin(&sh.need, hit);
+        if (lane == 0 && last) atomicMax(&sh.cand_n, last);    // (0: none so far)
         __syncthreads();
         if (sh.need != 0xffffffffu) break;
-        first += SAMPLE_THREADS;
+        first += WALK * SAMPLE_THREADS;
         if (first >= end) {
             if (sh.cand_n > 0u || span == 2) break;
             ++span;
@@ -507,11 +586,11 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, NQ > 0 ? 1 : 2) sample_kernel(
     if (tid == 0) out[row_id] = sh.need != 0xffffffffu ? (long long)sh.need : (long long)sh.cand_n - 1;
 }
 
-template <int NQ>
+template <int NQ, bool TWO, bool SHARE>
 static cudaError_t launch_sample(int cluster, const float* logits, int batch, int vocab, float temperature, int top_k, const float* uniform,
                                  long long* out, cudaStream_t st) {
     if (cluster > 8) {   // sizes above 8 are opt-in, per device and function (setting it again changes nothing)
-        const cudaError_t e = cudaFuncSetAttribute(sample_kernel<NQ>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        const cudaError_t e = cudaFuncSetAttribute(sample_kernel<NQ, TWO, SHARE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg{};
@@ -520,7 +599,7 @@ static cudaError_t launch_sample(int cluster, const float* logits, int batch, in
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, sample_kernel<NQ>, logits, vocab, temperature, top_k, uniform, out);
+    return cudaLaunchKernelEx(&cfg, sample_kernel<NQ, TWO, SHARE>, logits, vocab, temperature, top_k, uniform, out);
 }
 
 }  // namespace q3
@@ -536,15 +615,20 @@ extern "C" int q3_sample(const float* logits, int32_t batch, int32_t vocab, floa
     // 24.7 / 19.1 / 16.4 / 12.3 / 20.2; 16 rows, k = 50: 25.3 / 19.5 / 16.4 / 20.5 / 29.1; 33 rows, all words: 25.1 / 18.5 / 14.4 / 20.5 / 32.8;
     // 40 rows, all words: 26.7 / 19.2 / 20.7 / 22.6; 64 rows, all words: 27.5 / 20.5 / 21.6 / 35.0; 64 rows, k = 50: 30.7 / 24.6 / 26.6 / 48.1.
     // A thread keeps its elements in registers where it has at most three groups of four, or five.
+    // One block an SM, with registers for eight loads, where that is room for every cluster: pairs of blocks for up to 64 rows (64 rows 18.6 us, with two
+    // blocks an SM 20.4; clusters of four do not fit 148 SMs one by one: 36 rows, k = 50, 31.0 and 22.8).
+    // The candidates' threads are read by a lane a group, four threads at a time, while a warp (k / 32 such threads) has few of them for its groups: k =
+    // 50, 15 / 64 rows 15.1 / 18.7 us, each thread by itself 16.6 / 22.8; k = 200, 64 rows 23.0 / 26.8, but 36 rows 28.9 / 26.9 and 15 rows 21.0 / 18.9.
     int cluster = batch <= 4 ? 16 : batch <= 14 ? 8 : batch <= 36 ? 4 : batch <= 148 ? 2 : 1;
     while (cluster > 1 && vocab < cluster * q3::SAMPLE_THREADS) cluster /= 2;
     const int groups = q3::sample_run(vocab, cluster) / 128;
     cudaStream_t st = (cudaStream_t)stream;
     long long* out = reinterpret_cast<long long*>(out_tokens);
-    cudaError_t err;
-    if (groups <= 3) err = q3::launch_sample<3>(cluster, logits, batch, vocab, temperature, top_k, uniform, out, st);
-    else if (groups <= 5) err = q3::launch_sample<5>(cluster, logits, batch, vocab, temperature, top_k, uniform, out, st);
-    else err = q3::launch_sample<0>(cluster, logits, batch, vocab, temperature, top_k, uniform, out, st);
+    const bool share = top_k <= 12 * groups || top_k >= vocab, deep = cluster == 2 && batch <= 64;
+    auto* const launch = groups <= 3 ? q3::launch_sample<3, false, false> : groups <= 5 ? q3::launch_sample<5, false, false>
+                         : deep ? (share ? q3::launch_sample<0, false, true> : q3::launch_sample<0, false, false>)
+                                : (share ? q3::launch_sample<0, true, true> : q3::launch_sample<0, true, false>);
+    const cudaError_t err = launch(cluster, logits, batch, vocab, temperature, top_k, uniform, out, st);
     if (err != cudaSuccess) return q3::engine_fail(nullptr, Q3_ERR_CUDA, "q3_sample: %s", cudaGetErrorString(err));
     return Q3_OK;
 }

@@ -242,6 +242,34 @@ def test_draws_over_every_number_of_blocks_a_row(batch, vocab, top_k, temperatur
         assert lo - CDF_TOL <= float(u[b]) <= float(cdf[b, j]) + CDF_TOL, (b, j, float(u[b]), lo, float(cdf[b, j]))
 
 
+@pytest.mark.parametrize("batch,top_k", [(15, 120), (36, 120), (36, 121), (37, 228), (64, 228), (64, 229), (65, 228), (65, 229), (37, 0), (64, 0), (65, 0)])
+@pytest.mark.parametrize("vocab", [151936, 151933])
+def test_rows_that_are_read_twice(batch, top_k, vocab):
+    """Clusters of two and four blocks whose threads re-read the row, on both sides of the rules (blocks an SM: 64 rows; a lane a group: twelve times the
+    10 or 19 groups of a run), the largest words of some rows side by side in one warp's run or at the very end.  fp64 rule, as above."""
+    from qwen3mk import sampling
+
+    g = torch.Generator(device="cuda").manual_seed(batch + top_k)
+    logits = torch.randn(batch, vocab, generator=g, device="cuda") * 3.0
+    logits[1, 5000:5000 + 4 * max(top_k, 30):4] += 30.0       # every lane of a warp has candidates
+    logits[2, -top_k - 5:] += 30.0
+    logits[3, 7000] = float("nan")
+    u = torch.rand(batch, generator=g, device="cuda")
+    got = sampling.sample(logits, 0.9, top_k, u=u).tolist()
+    assert got == sampling.sample(logits, 0.9, top_k, u=u).tolist()
+    logits[3] = torch.where(logits[3].isnan(), float("-inf"), logits[3])
+    assert got[3] == int(logits[3].argmax())                    # (a row with a NaN is not drawn from)
+    keep = logits.double() > float("-inf")
+    if top_k:
+        keep &= logits >= logits.topk(top_k, dim=-1).values[:, -1:]
+    w = torch.where(keep, torch.exp((logits.double() - logits.double().max(dim=-1, keepdim=True).values) / 0.9), 0.0)
+    cdf = (w / w.sum(dim=-1, keepdim=True)).cumsum(dim=-1).cpu()
+    for b in range(batch):
+        j = got[b]
+        lo = float(cdf[b, j - 1]) if j else 0.0
+        assert bool(keep[b, j]) and (b == 3 or lo - CDF_TOL <= float(u[b]) <= float(cdf[b, j]) + CDF_TOL), (b, j)
+
+
 def block_ends(vocab, blocks):
     """Where the kernel's blocks end that share a row: 32 warps a block, a run of whole groups of 128 words a warp."""
     run = (-(-vocab // (blocks * 32)) + 127) // 128 * 128
