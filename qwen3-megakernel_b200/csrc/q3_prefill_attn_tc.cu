@@ -16,7 +16,8 @@
 // O are combined under one maximum and written as the bf16 plane the Wo GEMM reads.
 // The MMA thread issues S of tile t + 2 right behind the product of tile t, whose P it overwrites (the pipe works in order).
 // One block per (query tile, kv group) in order of work (a query tile has 1..n key tiles), so that the SMs that finish early pick up the
-// light tiles.  Every mbarrier wait is bounded.
+// light tiles.  Where SMs would stay idle, two blocks of a cluster share a long query tile, half of the key tiles each, and finish half of its positions
+// each (O, maxima and sums travel through distributed shared memory).  Every mbarrier wait is bounded.
 //
 // What bounds it: a key tile is 24 products of 128 x 128 x 16 (0.8 us at the measured bf16 rate) and 16 K exponentials and 8 K conversions on
 // the XU pipe (0.8 us).  A tile takes 1.2 us: the products wait
@@ -40,6 +41,8 @@ constexpr int AT_STAGES = 2;
 constexpr uint32_t AT_BOX = 128 * 128;    // bytes of one [128 rows x 64 columns] bf16 box, 128-byte swizzle
 constexpr uint32_t AT_Q_BYTES = 2 * AT_BOX, AT_KV_BYTES = 2 * AT_BOX;   // 128 x 128 bf16 = two boxes
 constexpr size_t AT_SMEM = 2 * AT_Q_BYTES + AT_STAGES * 2 * AT_KV_BYTES;   // Q hi, Q lo, stages x (K, V) = 192 KB
+constexpr int AT_SPLIT_MIN = 3;           // key tiles of a query tile that two blocks share, at least
+constexpr int AT_ONE_WAVE = 18;           // blocks of a kv group that are resident at once (148 SMs, a block each)
 constexpr float AT_LAG = 8.f;             // how far (in log2) scores may exceed the maximum that P is taken under
 constexpr unsigned long long AT_WAIT_NS = 200ull * 1000 * 1000;
 
@@ -136,12 +139,25 @@ __device__ __forceinline__ void at_st16(uint32_t taddr, const uint32_t* r) {
                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
 }
 
+// both blocks of a cluster, all threads; writes to the other's shared memory before it are seen behind it
+__device__ __forceinline__ void at_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t at_map(uint32_t smem_addr, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+
 struct PrefillAttnTcArgs {
     bf16_raw* plane;      // [T][2048] bf16: the output, as the Wo GEMM reads it
     int T, layer;
+    int shared;           // PAIR: query tiles (of a kv group, the longest) that two blocks share
     uint32_t* status;
 };
 
+template <bool PAIR>
 __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_constant__ CUtensorMap tm_ql,
                                                                         const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                                                                         const PrefillAttnTcArgs a) {
@@ -153,7 +169,16 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
     __shared__ float s_m[2][128], s_l[2][2][128];   // at the end: per group, a row's maximum and the two halves of its sum
 
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
-    const int g = (int)blockIdx.x % KV_HEADS;       // kv head; query heads 2g and 2g + 1
+    // The query tiles with the most key tiles come first.  PAIR: a cluster of two blocks shares one of the `shared` longest, its key tiles cut in two, or
+    // takes two tiles, a block each.
+    const int tiles = (a.T + AT_QT - 1) / AT_QT, unit = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, place = unit / KV_HEADS, rank = PAIR ? (int)blockIdx.x & 1 : 0;
+    const int g = unit % KV_HEADS;                  // kv head; query heads 2g and 2g + 1
+    const bool both = PAIR && place < a.shared;
+    const int nth = !PAIR || both ? place : a.shared + 2 * (place - a.shared) + rank;
+    if (PAIR && nth >= tiles) return;               // (an odd tile's other block)
+    const int q0 = (tiles - 1 - nth) * AT_QT;
+    const int all_kt = (q0 + AT_QT - 1) / AT_KT + 1;        // key tiles up to and including the diagonal one
+    const int kt0 = both && rank ? (all_kt + 1) / 2 : 0, n_kt = both ? (rank ? all_kt / 2 : (all_kt + 1) / 2) : all_kt;     // this block's
     unsigned char* sQh = at_raw;
     unsigned char* sQl = sQh + AT_Q_BYTES;
     unsigned char* sKV = sQl + AT_Q_BYTES;          // stage s: K at s * 2 * AT_KV_BYTES, V right after it
@@ -186,8 +211,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
 
     pdl_launch();
 
-    const int q0 = ((a.T + AT_QT - 1) / AT_QT - 1 - (int)blockIdx.x / KV_HEADS) * AT_QT;   // the query tiles with the most key tiles come first
-    const int n_kt = (q0 + AT_QT - 1) / AT_KT + 1;          // key tiles up to and including the diagonal one
     int armed_k = 0, armed_v = 0;                           // tiles whose K and V the producer has requested
     {
         if (warp == AT_SOFT / 32) {
@@ -214,14 +237,14 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
 #pragma unroll
                     for (int b = 0; b < 2; ++b)        // the two 64-dim halves of the head
                         asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                                     ::"r"(at_smem(sk + b * AT_BOX)), "l"(&tm_k), "r"(g * HEAD_DIM + 64 * b), "r"(t * AT_KT), "r"(a.layer), "r"(at_smem(&k_full[s])) : "memory");
+                                     ::"r"(at_smem(sk + b * AT_BOX)), "l"(&tm_k), "r"(g * HEAD_DIM + 64 * b), "r"((kt0 + t) * AT_KT), "r"(a.layer), "r"(at_smem(&k_full[s])) : "memory");
                     armed_k = t + 1;
                     if (t >= AT_STAGES && !at_wait(&v_empty[s], ((t / AT_STAGES) - 1) & 1, &abort_flag, a.status, 47)) break;
                     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&v_full[s])), "r"(AT_KV_BYTES) : "memory");
 #pragma unroll
                     for (int b = 0; b < 2; ++b)
                         asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                                     ::"r"(at_smem(sv + b * AT_BOX)), "l"(&tm_v), "r"(g * HEAD_DIM + 64 * b), "r"(t * AT_KT), "r"(a.layer), "r"(at_smem(&v_full[s])) : "memory");
+                                     ::"r"(at_smem(sv + b * AT_BOX)), "l"(&tm_v), "r"(g * HEAD_DIM + 64 * b), "r"((kt0 + t) * AT_KT), "r"(a.layer), "r"(at_smem(&v_full[s])) : "memory");
                     armed_v = t + 1;
                 }
             }
@@ -294,8 +317,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
                 at_ld32(r[0], ts + (uint32_t)(part * 64));
                 at_ld32(r[1], ts + (uint32_t)(part * 64 + 32));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (t == n_kt - 1) {   // the diagonal tile: causal mask (it also hides keys past the prompt)
-                    const int key0 = t * AT_KT + part * 64;
+                if (kt0 + t == all_kt - 1) {   // the diagonal tile: causal mask (it also hides keys past the prompt)
+                    const int key0 = (kt0 + t) * AT_KT + part * 64;
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
                         if (key0 + j > qpos) r[0][j] = 0xff800000u;            // -inf
@@ -358,39 +381,69 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_attn_tc_kernel(const __
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const float m0 = s_m[0][row], m1 = s_m[1][row], mx = fmaxf(m0, m1);      // (a block of one tile has no second group: m1 is -inf)
             const float f0 = at_ex2(m0 - mx), f1 = at_ex2(m1 - mx);
-            const float inv = 1.f / ((s_l[0][0][row] + s_l[0][1][row]) * f0 + (s_l[1][0][row] + s_l[1][1][row]) * f1);
-            const float w0 = f0 * inv, w1 = f1 * inv;
+            const float sum = (s_l[0][0][row] + s_l[0][1][row]) * f0 + (s_l[1][0][row] + s_l[1][1][row]) * f1;
+            const float inv = both ? 1.f : 1.f / sum, w0 = f0 * inv, w1 = f1 * inv;
             const int dim0 = (warp >> 2) * 32;          // a quarter of the row's dims
             uint32_t o0[32], o1[32];
             at_ld32(o0, trow + 256u + (uint32_t)dim0);
             at_ld32(o1, trow + 384u + (uint32_t)dim0);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float o[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                o[j] = __uint_as_float(o0[j]) * w0;
+                if (n_kt > 1) o[j] = fmaf(__uint_as_float(o1[j]), w1, o[j]);   // (TMEM that nothing was added to may hold anything)
+            }
+            const int pos = row & 63;
+            const bool own = !both || (pos >> 5) == rank;
+            if (both) {
+                // Each block finishes 32 of the positions: the other's sums, and O under its maximum, come through distributed shared memory into the place
+                // of Q hi (every product of both blocks has completed), the two numbers of a row into that of Q lo.
+                const int slot = (row >> 6) * 4 + (warp >> 2);
+                at_cluster_sync();
+                if (!own) {
+                    const uint32_t to_o = at_map(at_smem(sQh) + (uint32_t)(slot * 8 * 32 + lane) * 16u, rank ^ 1), to_n = at_map(at_smem(sQl) + (uint32_t)((row >> 6) * 32 + lane) * 8u, rank ^ 1);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to_o + (uint32_t)j * 512u), "f"(o[4 * j]), "f"(o[4 * j + 1]), "f"(o[4 * j + 2]), "f"(o[4 * j + 3]) : "memory");
+                    // (a block that gave up sends NaN: the other does not pass its rows off as whole)
+                    if (warp < 4) asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(to_n), "f"(mx), "f"(abort_flag ? NAN : sum) : "memory");
+                }
+                at_cluster_sync();
+                if (own) {
+                    const float2 n2 = reinterpret_cast<const float2*>(sQl)[(row >> 6) * 32 + lane];
+                    const float top = fmaxf(mx, n2.x), a0 = at_ex2(mx - top), a1 = at_ex2(n2.x - top), r = 1.f / (sum * a0 + n2.y * a1), u0 = a0 * r, u1 = a1 * r;
+                    const float4* in = reinterpret_cast<const float4*>(sQh) + slot * 8 * 32 + lane;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float4 v = in[j * 32];
+                        o[4 * j] = fmaf(v.x, u1, o[4 * j] * u0); o[4 * j + 1] = fmaf(v.y, u1, o[4 * j + 1] * u0);
+                        o[4 * j + 2] = fmaf(v.z, u1, o[4 * j + 2] * u0); o[4 * j + 3] = fmaf(v.w, u1, o[4 * j + 3] * u0);
+                    }
+                }
+            }
             // Through shared memory (Q's: all products have completed), so that a warp writes a position's 512 bytes (a thread per row: 1 us more a block).
             // 16-byte chunks of a position's row are XORed by the position.
-            uint4* const so = reinterpret_cast<uint4*>(sQh);
-            {
-                float o[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    o[j] = __uint_as_float(o0[j]) * w0;
-                    if (n_kt > 1) o[j] = fmaf(__uint_as_float(o1[j]), w1, o[j]);   // (TMEM that nothing was added to may hold anything)
-                }
-                const int pos = row & 63, chunk = (row >> 6) * 16 + dim0 / 8;
+            uint4* const so = reinterpret_cast<uint4*>(both ? sQl + 1024 : sQh);
+            if (own) {
+                const int at = both ? pos & 31 : pos, chunk = (row >> 6) * 16 + dim0 / 8;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    so[pos * 32 + ((chunk + j) ^ (pos & 7))] = make_uint4(at_pack_bf16(o[8 * j], o[8 * j + 1]), at_pack_bf16(o[8 * j + 2], o[8 * j + 3]),
-                                                                           at_pack_bf16(o[8 * j + 4], o[8 * j + 5]), at_pack_bf16(o[8 * j + 6], o[8 * j + 7]));
+                    so[at * 32 + ((chunk + j) ^ (pos & 7))] = make_uint4(at_pack_bf16(o[8 * j], o[8 * j + 1]), at_pack_bf16(o[8 * j + 2], o[8 * j + 3]),
+                                                                          at_pack_bf16(o[8 * j + 4], o[8 * j + 5]), at_pack_bf16(o[8 * j + 6], o[8 * j + 7]));
             }
             asm volatile("bar.sync 9, %0;" ::"n"(AT_SOFT) : "memory");
             if (!abort_flag) {
-                bf16_raw* const dst = a.plane + (size_t)q0 * Q_DIM + 2 * g * HEAD_DIM + lane * 8;
+                const int p0 = both ? q0 + 32 * rank : q0, count = both ? 2 : 4;
+                bf16_raw* const dst = a.plane + (size_t)p0 * Q_DIM + 2 * g * HEAD_DIM + lane * 8;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const int pos = warp + 16 * i;
-                    if (q0 + pos < a.T) *reinterpret_cast<uint4*>(dst + (size_t)pos * Q_DIM) = so[pos * 32 + (lane ^ (pos & 7))];
+                    const int at = warp + 16 * i;
+                    if (i < count && p0 + at < a.T) *reinterpret_cast<uint4*>(dst + (size_t)at * Q_DIM) = so[at * 32 + (lane ^ (at & 7))];
                 }
             }
         }
+        if (both && warp >= AT_SOFT / 32) { __syncwarp(); at_cluster_sync(); at_cluster_sync(); }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -420,15 +473,26 @@ cudaError_t launch_prefill_attn_tc(const CUtensorMap& q_hi, const CUtensorMap& q
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
         if (!attr_set[dev]) {   // (a benign race between host threads: the attribute is set to the same value)
-            e = cudaFuncSetAttribute(prefill_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM);
+            e = cudaFuncSetAttribute(prefill_attn_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_attn_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM);
             if (e != cudaSuccess) return e;
             attr_set[dev] = true;
         }
     }
+    // A launch takes as long as its longest query tile.  While there are SMs without a block, pairs of blocks share the longest ones, as many as still leave
+    // every block resident at once (us a prompt, shared / not: 512 tokens 1379 / 1413, 777 1817 / 1874, 1088 1985 / 2013; tiles of two key tiles as well: 256
+    // tokens 1099 / 1080; in two waves 1090 tokens 2105 / 2019, 1400 2606 / 2506).
+    const int tiles = (T + AT_QT - 1) / AT_QT;
+    const int long_ones = tiles - 2 * (AT_SPLIT_MIN - 1);        // query tiles of at least AT_SPLIT_MIN key tiles (every key tile is the last of two)
+    const int shared = min(AT_ONE_WAVE - tiles, long_ones);
+    if (shared > 0) {
+        PrefillAttnTcArgs a{reinterpret_cast<bf16_raw*>(plane), T, layer, shared, status};
+        return launch_chain_cluster(prefill_attn_tc_kernel<true>, dim3(2 * (shared + (tiles - shared + 1) / 2) * KV_HEADS), dim3(AT_THREADS), AT_SMEM, 2, st, q_hi, q_lo, k, v, a);
+    }
     // one block per (query tile, kv group), dispatched in the order of their work (a query tile has 1..n key tiles), so that the
     // SMs that finish early pick up the light tiles: greedy longest-first over all SMs
-    PrefillAttnTcArgs a{reinterpret_cast<bf16_raw*>(plane), T, layer, status};
-    return launch_chain(prefill_attn_tc_kernel, dim3((T + AT_QT - 1) / AT_QT * KV_HEADS), dim3(AT_THREADS), AT_SMEM, st, q_hi, q_lo, k, v, a);
+    PrefillAttnTcArgs a{reinterpret_cast<bf16_raw*>(plane), T, layer, 0, status};
+    return launch_chain(prefill_attn_tc_kernel<false>, dim3(tiles * KV_HEADS), dim3(AT_THREADS), AT_SMEM, st, q_hi, q_lo, k, v, a);
 }
 
 }  // namespace q3

@@ -499,6 +499,13 @@ def test_prompts_of_narrow_tiles(oracle, small, T):
     test_prompt_products_at_the_edges_of_their_tiles(oracle, small, T)
 
 
+@pytest.mark.parametrize("T", [256, 257, 320, 321, 449, 576, 577, 641, 1087, 1088, 1089])
+def test_prompts_whose_longest_query_tiles_are_shared(oracle, small, T):
+    """Two blocks share the query tiles (64 positions) of three key tiles (128) and more while all blocks fit the SMs: none up to 256 tokens, an odd number of
+    tiles and one block without any (449), all of the long ones up to 576, then fewer, one at 1088, none beyond."""
+    test_prefill_matches_oracle(oracle, small, T)
+
+
 @pytest.mark.parametrize("floats", [1, 2, 3])
 def test_rope_table_at_any_address(oracle, small, floats):
     """A RoPE table that is not 16-byte aligned gives the results of one that is: prompts (matrix-vector kernels, k slices with either
