@@ -11,14 +11,20 @@ __device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__
 __device__ __forceinline__ unsigned long long tc_ns() { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
 
 // bounded mbarrier wait; on timeout sets *abort_flag and returns false
+// PARK: the thread may sleep up to 20 us between two looks (it wakes when the phase completes).
+template <bool PARK = false>
 [[nodiscard]] __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t site,
                                                       unsigned long long limit = TC_WAIT_NS) {
     unsigned it = 0;
     unsigned long long t0 = 0;
     for (;;) {
         uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(tc_smem(bar)), "r"(parity) : "memory");
+        if constexpr (PARK)
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(ok) : "r"(tc_smem(bar)), "r"(parity), "r"(20000u) : "memory");
+        else
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(ok) : "r"(tc_smem(bar)), "r"(parity) : "memory");
         if (ok) return true;
         if (*abort_flag) return false;
         if ((++it & 63u) == 0) {
@@ -34,10 +40,11 @@ __device__ __forceinline__ unsigned long long tc_ns() { unsigned long long t; as
 }
 
 // The same for a whole converged warp: one lane polls.  32 polling lanes are 32 requests to the barrier unit, and those of the
-// epilogue warps stand in front of the MMA thread's own (a wait that was already over took it 190 ns instead of 30).
+// epilogue warps stand in front of the MMA thread's own (a wait that was already over took it 190 ns instead of 30).  It is
+// parked: looks in quick succession cost 40 / 64 sequences 1330 / 2031 us a step, parked 1318 / 2022, a prompt of 512 tokens 1380 and 1370.
 [[nodiscard]] __device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t site,
                                                            unsigned long long limit = TC_WAIT_NS) {
-    return one_lane_waits([&] { return tc_wait(bar, parity, abort_flag, status, site, limit); });
+    return one_lane_waits([&] { return tc_wait<true>(bar, parity, abort_flag, status, site, limit); });
 }
 
 // After a wait has given up: let what is still under way to this block land before its memory is somebody else's.  Bounded, reports nothing.
