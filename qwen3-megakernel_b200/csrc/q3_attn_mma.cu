@@ -126,10 +126,29 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
     };
 #pragma unroll
     for (int i = 0; i < AM_STAGES - 1; ++i) issue(i);
+    // ... and this warp's gains and RoPE entries (a warp per vector below: q head 2g, q head 2g + 1, k, v; four dims a lane).  Loaded behind the wait, an
+    // element at a time, they cost 8 x 1024 / 27 ragged / 64 x 128 / 64 x 1024 710 / 1355 / 1114 / 2024 us a step; so 699 / 1340 / 1102 / 2015.
+    static_assert(AM_WARPS >= 4, "a warp per vector");
+    const int role = warp;
+    uint2 gain;                  // (nothing is done with them before the wait: that would be a wait for them)
+    float cs[4], sn[4];
+    if (a.fused_prep && role < 3) {
+        const bf16_raw* gp = (role < 2 ? a.qn : a.kn) + (size_t)a.layer * HEAD_DIM + lane * 4;
+        const float* tab = a.rope + (size_t)len * HEAD_DIM + ((lane * 4) & 63);
+        gain = *reinterpret_cast<const uint2*>(gp);
+        if ((reinterpret_cast<uintptr_t>(a.rope) & 15) == 0) {       // (a table may begin at any float)
+            const float4 c4 = *reinterpret_cast<const float4*>(tab), s4 = *reinterpret_cast<const float4*>(tab + 64);
+            cs[0] = c4.x; cs[1] = c4.y; cs[2] = c4.z; cs[3] = c4.w;
+            sn[0] = s4.x; sn[1] = s4.y; sn[2] = s4.z; sn[3] = s4.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { cs[i] = tab[i]; sn[i] = tab[64 + i]; }
+        }
+    }
     if (a.early) pdl_wait();     // lengths and cached rows were complete before this launch could start: only `qkv` is the predecessor's
 
     // ---- the two q heads, the k row and the v row of the new token: as prepared by head_prep_kernel, or prepared here ----
-    for (int role = warp; role < 4; role += AM_WARPS) {   // a warp per vector: q head 2g, q head 2g + 1, k, v; four dims a lane
+    if (role < 4) {
     if (a.fused_prep) {
         const float* src = role == 0 ? qkv + (2 * g) * HEAD_DIM : role == 1 ? qkv + (2 * g + 1) * HEAD_DIM
                          : role == 2 ? qkv + Q_DIM + g * HEAD_DIM : qkv + Q_DIM + KV_DIM + g * HEAD_DIM;
@@ -141,15 +160,12 @@ __global__ void __launch_bounds__(AM_WARPS * 32, AM_WARPS == 4 ? 2 : 1) attn_mma
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
             const float r = rsqrtf(ss / (float)HEAD_DIM + EPS);
-            const bf16_raw* gain = (role < 2 ? a.qn : a.kn) + (size_t)a.layer * HEAD_DIM + lane * 4;
-            const float* tab = a.rope + (size_t)len * HEAD_DIM;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float nrm = (v[i] * r) * bf_to_f(gain[i]);
+                const float nrm = (v[i] * r) * (i == 0 ? bf_lo(gain.x) : i == 1 ? bf_hi(gain.x) : i == 2 ? bf_lo(gain.y) : bf_hi(gain.y));
                 const float partner = __shfl_xor_sync(0xffffffffu, nrm, 16);   // dim d +- 64 sits 16 lanes away
                 const float rot = (lane < 16) ? -partner : partner;
-                const int d = (lane * 4 + i) & 63;
-                v[i] = nrm * tab[d] + rot * tab[64 + d];
+                v[i] = nrm * cs[i] + rot * sn[i];
             }
         }
         *reinterpret_cast<float4*>(&s_new[role][lane * 4]) = make_float4(v[0], v[1], v[2], v[3]);
