@@ -542,6 +542,7 @@ template <int BN> struct PpShape {
     static constexpr uint32_t PIECES = PP_EPI_WARPS * PP_PIECE;
     static constexpr int STAGES = (225 * 1024 - PIECES) / STAGE < PP_MAX_STAGES ? (225 * 1024 - PIECES) / STAGE : PP_MAX_STAGES;
     static constexpr size_t SMEM = STAGES * STAGE + PIECES;
+    static constexpr uint32_t COLS = BN <= 128 ? 256 : 512;      // TMEM columns: two accumulators, a power of two
 };
 
 __device__ __forceinline__ void pp_load_box(uint32_t dst, const void* map, int k, int row, uint32_t leader_bar) {
@@ -577,7 +578,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prompt_pair_kernel(const __grid
         abort_flag = 0;
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_base_s)), "r"((uint32_t)(2 * BN)) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_base_s)), "r"(S::COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -771,8 +772,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prompt_pair_kernel(const __grid
                             if (sub == 0) p.ssq_out[(size_t)(tile * 2 + half) * p.ssq_ld + m0 + lr] = ss;
                         }
                     }
-                } else {
-                    static_assert(KIND != PR_SILU || BN == 256, "64 gate and 64 up columns a warp");
+                } else if constexpr (BN == 256) {
                     uint32_t g[2][32], u[2][32], out[32];   // 64 columns of this lane's row, under one wait
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {
@@ -796,6 +796,32 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prompt_pair_kernel(const __grid
                         const int lr = lr0 + STEP * i;
                         if (lr < rows)
                             *reinterpret_cast<uint4*>(p.hid + (size_t)(m0 + lr) * INTER + tile * (BN / 2) + half * 64 + sub * 8) = *reinterpret_cast<const uint4*>(piece + lr * PP_LD + sub * 4);
+                    }
+                } else {
+                    static_assert(BN == 192, "a warp reads 64 gate and 64 up columns, or 48");
+                    constexpr int HC = BN / 4, UNITS = HC / 8;   // gate and up columns a warp, 16-byte units of a row's output
+                    uint32_t g[2][32], u[2][32], out[32];        // of this lane's row, under one wait
+                    const uint32_t tg = tacc + (uint32_t)(half * HC), tu = tg + (uint32_t)(BN / 2);
+                    tc_ld32(g[0], tg);
+                    tc_ld32(u[0], tu);
+                    tc_ld16(g[1], tg + 32u);
+                    tc_ld16(u[1], tu + 32u);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < HC / 2; ++j) {
+                        const int c = j >> 4, k = 2 * (j & 15);
+                        out[j] = pr_pack(pr_silu(__uint_as_float(g[c][k]) * r, __uint_as_float(u[c][k]) * r), pr_silu(__uint_as_float(g[c][k + 1]) * r, __uint_as_float(u[c][k + 1]) * r));
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < UNITS; ++j)
+                        *reinterpret_cast<uint4*>(piece + lane * PP_LD + 4 * j) = make_uint4(out[4 * j], out[4 * j + 1], out[4 * j + 2], out[4 * j + 3]);
+                    __syncwarp();
+                    bf16_raw* const dst = p.hid + (size_t)m0 * INTER + tile * (BN / 2) + half * HC;
+#pragma unroll
+                    for (int i = 0; i < UNITS; ++i) {   // six lanes a row of 96 bytes
+                        const int at = i * 32 + lane, lr = at / UNITS, j = at - lr * UNITS;
+                        if (lr < rows) *reinterpret_cast<uint4*>(dst + (size_t)lr * INTER + j * 8) = *reinterpret_cast<const uint4*>(piece + lr * PP_LD + j * 4);
                     }
                 }
             }
@@ -823,7 +849,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prompt_pair_kernel(const __grid
     pr_cluster_wait();            // nothing of the pair is under way to this block any more
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * BN)) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S::COLS) : "memory");
     }
 }
 
@@ -911,7 +937,11 @@ cudaError_t launch_prompt_gemm(const PromptGemmCall& c, cudaStream_t st) {
     const int bn = c.kind == PR_QKV ? (mt == 1 ? 32 : mt <= 4 ? 64 : 128) : c.kind == PR_RESID ? (mt == 1 ? 32 : 64) : mt == 1 ? 48 : mt == 2 ? 96 : mt == 3 ? 128 : 192;
     const int rows[3] = {c.kind == PR_QKV ? Q_DIM : c.kind == PR_RESID ? HIDDEN : INTER, c.kind == PR_QKV ? KV_DIM : INTER, KV_DIM};
     const int n_w = c.kind == PR_QKV ? 3 : c.kind == PR_RESID ? 1 : 2;
-    const uint32_t box = pair ? (c.kind == PR_RESID ? 64u : 128u) : c.kind == PR_RESID ? (uint32_t)bn : (uint32_t)bn / 2;
+    // gate/up on pairs of SMs: items of 192 columns where their rounds are shorter than those of 256 (us a prompt, 192 / 256: 640 tokens, one round of
+    // 256, 1770 / 1656; 777, two rounds either way, 1806 / 1828; 1024 1899 / 1949; 1100 2068 / 2020; 1400 2561 / 2520; 2048, four and three, the same)
+    const int pairs = sm / 2, mt2 = (mt + 1) / 2, rounds256 = (mt2 * (2 * INTER / 256) + pairs - 1) / pairs, rounds192 = (mt2 * (2 * INTER / 192) + pairs - 1) / pairs;
+    const bool finer = c.kind == PR_SILU && rounds192 * 192 < rounds256 * 256;
+    const uint32_t box = pair ? (c.kind == PR_RESID ? 64u : finer ? 96u : 128u) : c.kind == PR_RESID ? (uint32_t)bn : (uint32_t)bn / 2;
     CUtensorMap tw[3];
     for (int i = 0; i < 3; ++i) {
         if (i >= n_w) tw[i] = tw[0];
@@ -933,7 +963,7 @@ cudaError_t launch_prompt_gemm(const PromptGemmCall& c, cudaStream_t st) {
             if (mt <= 4) return launch_split<PR_RESID, 64, 4, 2>(tw, *c.in, p, st);
             return launch_split<PR_RESID, 64, 2, 2>(tw, *c.in, p, st);
         case PR_SILU:
-            if (pair) return launch_pair<PR_SILU, 256>(tw, *c.in, p, sm, st);
+            if (pair) return finer ? launch_pair<PR_SILU, 192>(tw, *c.in, p, sm, st) : launch_pair<PR_SILU, 256>(tw, *c.in, p, sm, st);
             if (mt == 1) return launch_split<PR_SILU, 48, 1, 2>(tw, *c.in, p, st);
             if (mt == 2) return launch_split<PR_SILU, 96, 1, 1>(tw, *c.in, p, st);
             if (mt == 3) return launch_split<PR_SILU, 128, 1, 1>(tw, *c.in, p, st);

@@ -499,6 +499,13 @@ def test_prompts_of_narrow_tiles(oracle, small, T):
     test_prompt_products_at_the_edges_of_their_tiles(oracle, small, T)
 
 
+@pytest.mark.parametrize("T", [768, 770, 800, 1023, 1024])
+def test_prompts_of_finer_gate_and_up_items(oracle, small, T):
+    """From 769 to 1024 tokens (four tiles of 256) gate and up go in items of 192 columns: a warp's rows of 48, first and last token of a tile, a pair whose
+    second block has few rows or none."""
+    test_prompt_products_at_the_edges_of_their_tiles(oracle, small, T)
+
+
 @pytest.mark.parametrize("T", [256, 257, 320, 321, 449, 576, 577, 641, 1087, 1088, 1089])
 def test_prompts_whose_longest_query_tiles_are_shared(oracle, small, T):
     """Two blocks share the query tiles (64 positions) of three key tiles (128) and more while all blocks fit the SMs: none up to 256 tokens, an odd number of
