@@ -949,7 +949,13 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                 sn[0] = sv.x; sn[1] = sv.y; sn[2] = sv.z; sn[3] = sv.w;
             }
         }
-        fetch_slot(2, l);       // gate/up rows of this layer: in flight during F, landed before its barrier is polled
+        // Gate/up rows of this layer, in flight during F.  They leave behind the q/k/v exchange, which they slow, where F has no cached rows to fetch
+        // then: us per step at 16 / 64 / 128 / 191 / 300 / 1000 / 2200 positions 348 / 351 / 330 / 353 / 407 / 428 / 447 asked for here, 321 / 323 / 330 / 348 /
+        // 395 / 401 / 430 behind the exchange; two sequences at 16 / 600 / 1000 500 / 534 / 549 and 488 / 508 / 549.  But 255 / 3400 / 5000 375 / 473 / 513 and 380 / 481 / 529,
+        // two at 1500 580 and 585, three at 16 564 and 567.
+        // (two sequences: by the host's bound, for a flag of the block's own is a register too many)
+        auto rows_late = [&]() { return has_f && (local_attn ? MODE < 2 : NB == 1 ? npass <= PASSES : NB == 2 && p.max_len <= 1000); };
+        if (!rows_late()) fetch_slot(2, l);
         Q3_TRACE(ev + 2);
 
         // ==================================================================== F
@@ -1009,6 +1015,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                 }
             }
             cta_sync();
+            if (rows_late()) fetch_slot(2, l);
             Q3_TRACE(ev + 3);
 
             if (local_attn) {
