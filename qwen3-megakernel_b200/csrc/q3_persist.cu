@@ -62,7 +62,7 @@ constexpr int SC_FLOATS = 360;                // the score buffer of the local a
 // Most cached positions this kernel is picked for: the longest at which it was timed against the launch chain (one sequence, us per step, this
 // kernel / the chain: 5000 positions 513 / 768, 16000 826 / 1268, 29999 1183 / 1881).
 constexpr int PERSIST_MAX_LEN = 30000;
-// Two sequences at 16 / 1500 / 8000 / 29000 positions 502 / 577 / 903 / 1930 us against 573 / 657 / 987 / 2029.  Three at 16 / 600 / 1300 / 2000
+// Two sequences at 16 / 1500 / 8000 / 29000 positions 488 / 575 / 895 / 1930 us against 573 / 657 / 987 / 2029.  Three at 16 / 600 / 1300 / 2000
 // 599 / 632 / 679 / 733 (24 columns are three MMAs a tile, and the registers of a pass do not all fit: 164 bytes of spills) against 624 / 668 /
 // 697 / 729 in plain launches and 576 / 626 / 654 / 685 from a graph: in place of plain launches, up to
 constexpr int PERSIST_THREE_LEN = 1500;
