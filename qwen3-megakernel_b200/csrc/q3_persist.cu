@@ -58,7 +58,7 @@ constexpr int GROUP_CTAS = 2 * WO_SLICES;     // CTAs sharing one kv head
 constexpr int WO_ROWS_MAX = 116;              // largest slice: 4 * ceil(256 / 9)
 constexpr int PERSIST_MAX_BATCH = 3;          // sequences a launch decodes; one after the other where the caller asks for this kernel by name
 constexpr int MIN_GRID = 147;                 // row shares must fit the shared-memory slots
-constexpr int SC_FLOATS = 360;                // the score buffer of the local attention, which serves up to 255 positions
+constexpr int SC_FLOATS = 344;                // the score buffer of the local attention, which serves up to 255 positions
 // Most cached positions this kernel is picked for: the longest at which it was timed against the launch chain (one sequence, us per step, this
 // kernel / the chain: 5000 positions 513 / 768, 16000 826 / 1268, 29999 1183 / 1881).
 constexpr int PERSIST_MAX_LEN = 30000;
@@ -90,8 +90,12 @@ constexpr float ACC_SCALE = 4294967296.f;     // 2^32: resolution 2.3e-10, finer
 constexpr float ACC_CLAMP = 50000.f;
 constexpr int MAX_GRID = 160;                 // 160 * ACC_CLAMP < 2^23
 constexpr unsigned long long ACC_ONE = 1ull << 56, ACC_HALF = 1ull << 55;
-// fp32 tail of shared memory: 8 KB union | q_s[2][128] k_s v_s | o split [3][OLD] | hid split [3][HLD] | red lw misc | scores
-constexpr int FBUF_FLOATS = 2048 + 4 * 128 + 3 * OLD + 3 * HLD + 32 + 16 + 16 + SC_FLOATS;
+// The union holds Q's row sums [16][32] behind its staged activations, whole: warp 0 still adds them while other warps, which pass no barrier of the block
+// between, poll the q/k/v exchange and write q_s, the next thing in memory.
+constexpr int UNION_FLOATS = 2064;
+static_assert(3 * XLD + CW * 32 <= UNION_FLOATS, "Q's row sums end before q_s");
+// fp32 tail of shared memory: union | q_s[2][128] k_s v_s | o split [3][OLD] | hid split [3][HLD] | red lw misc | scores
+constexpr int FBUF_FLOATS = UNION_FLOATS + 4 * 128 + 3 * OLD + 3 * HLD + 32 + 16 + 16 + SC_FLOATS;
 constexpr int TAIL_BYTES = FBUF_FLOATS * 4 + 8 * 8 + 16;
 
 struct PersistParams {
@@ -460,18 +464,18 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     bf16_raw* sC = sB + WO_ROWS_MAX * WOROW;                                // gate | up rows  [2][imax][WROW]
     bf16_raw* sD = sC + (size_t)2 * imax * WROW;                            // down^T rows     [imax][WROW]
     float* fbuf = reinterpret_cast<float*>(sD + (size_t)imax * WROW);
-    // one 8 KB region with a different tenant per phase
+    // one region with a different tenant per phase
     uint32_t* const fw = reinterpret_cast<uint32_t*>(fbuf);
     uint32_t* xsq = MANY ? reinterpret_cast<uint32_t*>(sC) : fw;   // Q: activations split in three bf16 parts, [NB][3][XLD] pairs (6 KB a sequence)
     uint32_t* xsg = MANY ? reinterpret_cast<uint32_t*>(sB) : fw;   // GD: the same
-    float* part = MANY ? fbuf : fbuf + 3 * XLD;          // Q: per-warp partial row sums [NB][16][32] (2 KB: one sequence's run into q_s, idle in Q)
-    float* gpart = MANY ? reinterpret_cast<float*>(sB) + NB * 3 * XLD : fbuf + 3 * XLD;   // GD: per-warp partial sums of the 48 gate/up tile rows [NB][16][48] (3 KB: one sequence's run into q_s and k_s, idle in GD)
-    static_assert(NB * (3 * XLD + 768 + CW) * 4 <= WO_ROWS_MAX * WOROW * 2 && NB * (512 + CW) <= 2048, "the Wo slot holds GD's staging, the union Q's sums");
+    float* part = MANY ? fbuf : fbuf + 3 * XLD;          // Q: per-warp partial row sums [NB][16][32]
+    float* gpart = MANY ? reinterpret_cast<float*>(sB) + NB * 3 * XLD : fbuf + 3 * XLD;   // GD: per-warp partial sums of the 48 gate/up tile rows [NB][16][48] (3 KB: one sequence's run into q_s, idle in GD)
+    static_assert(NB * (3 * XLD + 768 + CW) * 4 <= WO_ROWS_MAX * WOROW * 2 && NB * (512 + CW) <= UNION_FLOATS, "the Wo slot holds GD's staging, the union Q's sums");
     float* om = fbuf;                                    // F: [16 warps][128] outputs of the local attention
     float* wo_part = fbuf;                               // F: [NB][2 k-halves][128] Wo slice partial sums (after the partials are published)
     float* dout = MANY ? reinterpret_cast<float*>(sB) : fbuf;   // GD: [NB][1024] down-projection outputs of this CTA (after the gate/up rows)
     float* xs = MANY ? reinterpret_cast<float*>(sA) : fbuf;     // LM head: [1024] fp32 activations; several sequences: [NB][3][LLD] pairs, split in three bf16 parts
-    float* q_s = fbuf + 2048;    // [2][128] both query heads of the group, scaled by 1/sqrt(128)
+    float* q_s = fbuf + UNION_FLOATS;   // [2][128] both query heads of the group, scaled by 1/sqrt(128)
     float* k_s = q_s + 256;      // [128] the new K row (after norm + RoPE), fp32
     float* v_s = k_s + 128;      // [128] the new V row, fp32
     uint32_t* const osp1 = reinterpret_cast<uint32_t*>(v_s + 128);

@@ -249,3 +249,18 @@ def test_what_is_under_way_is_drained_after_the_last_wait():
     issuer = rest[:rest.index("} else {")]
     assert re.search(r"tc_drain\(&acc_bar, 0\);\s*if \(abort_flag\)\s*for [^;]*;[^;]*;[^;]*tc_drain\(&full_bar", producer)
     assert re.search(r"tc_smem\(&acc_bar\)\) : \"memory\"\);\s*tc_drain\(&acc_bar, 0\);", issuer)
+
+
+@pytest.mark.parametrize("many", [0, 1, 2, 3])
+def test_row_sums_of_the_persistent_kernel_end_before_the_query_heads(many):
+    """Behind Q's last barrier warp 0 adds the block's row sums while warps 8 to 11 write the heads they have polled: the two regions of shared memory may
+    not meet, for one sequence (0: as it stands alone) or several."""
+    code = (ROOT / "qwen3-megakernel_b200" / "csrc" / "q3_persist.cu").read_text()
+    names = {"fbuf": 0, "NB": max(many, 1)}
+    for line in re.findall(r"^constexpr int (.*?);", code, re.M):
+        for name, value in re.findall(r"(\w+) = (\d+)", line):
+            names[name] = int(value)
+    sums = re.search(r"float\* part = MANY \? ([^:;]+) : ([^;]+);", code)
+    heads = re.search(r"float\* q_s = ([^;]+);", code)
+    begin, words = eval(sums.group(1 if many else 2), names), 512 * names["NB"]
+    assert begin + words <= eval(heads.group(1), names), (begin, words)
