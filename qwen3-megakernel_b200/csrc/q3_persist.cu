@@ -84,12 +84,14 @@ constexpr int EV_PER_LAYER = 12;              // trace stamps per layer
 constexpr unsigned long long WAIT_NS = 200ull * 1000 * 1000;   // default patience of every device-side wait: 200 ms
 constexpr int MAX_TP = 8;                     // tensor-parallel ranks: 1, 2, 4 or 8 (at least one kv head each)
 constexpr int MAX_LAYERS = 63;                // the q/k/v tags of a launch are epoch * 64 + layer + 1
-// Counted accumulators: word = (contributions << 56) + sum of round(v * 2^32) as a 56-bit two's complement number.
-// A contribution is clamped to +-ACC_CLAMP so that MAX_GRID of them cannot reach the count field (2^55 / 2^32 = 8.4e6).
+// Counted accumulators: word = (contributions << 56) + (those kept apart << 51) + sum of round(v * 2^32) of the others as a 51-bit two's complement
+// number.  A contribution that is larger than ACC_LIMIT, infinite or a NaN is kept apart: as a tagged float in a place of its own (one per query head and
+// word), which the readers of a word that counts any add to the sum.
 constexpr float ACC_SCALE = 4294967296.f;     // 2^32: resolution 2.3e-10, finer than fp32 for every |x| above 4e-3
-constexpr float ACC_CLAMP = 50000.f;
-constexpr int MAX_GRID = 160;                 // 160 * ACC_CLAMP < 2^23
-constexpr unsigned long long ACC_ONE = 1ull << 56, ACC_HALF = 1ull << 55;
+constexpr float ACC_LIMIT = 16000.f;
+constexpr int MAX_GRID = 160;
+constexpr unsigned long long ACC_ONE = 1ull << 56, ACC_APART = 1ull << 51, ACC_HALF = 1ull << 50;
+static_assert(Q_HEADS * (unsigned long long)ACC_LIMIT << 32 < ACC_HALF && Q_HEADS < 32, "a contribution per query head: neither their sum nor their numbers leave their fields");
 // The union holds Q's row sums [16][32] behind its staged activations, whole: warp 0 still adds them while other warps, which pass no barrier of the block
 // between, poll the q/k/v exchange and write q_s, the next thing in memory.
 constexpr int UNION_FLOATS = 2064;
@@ -141,7 +143,7 @@ struct PersistState {
     const void* src[7];     // the seven pointers `packed` was built from
     int tp_rank, tp_size;   // tensor-parallel position (0, 1 when off)
     float* peer_X[MAX_TP];  // the state allocations of all ranks as mapped here (own at tp_rank)
-    float* X;               // dA[2] (64-bit words) | dB[3][n_acc] (fp32) | xq[4096] (64-bit words) | epoch | xp
+    float* X;               // dA[2] (64-bit words) | dB[3][n_acc] (fp32) | xq[4096] (64-bit words) | epoch | xp | contributions kept apart
     int grid, smem;
 };
 
@@ -153,7 +155,8 @@ constexpr size_t XP_WORDS = (size_t)KV_HEADS * 2 * GROUP_CTAS * XP_STRIDE;
 __host__ __device__ constexpr size_t acc_floats(int nb) { return (size_t)nb * (4 + 3 * n_acc(nb)) * HIDDEN; }
 constexpr size_t XQ_OFFSET = acc_floats(PERSIST_MAX_BATCH), EPOCH_OFFSET = XQ_OFFSET + (size_t)PERSIST_MAX_BATCH * 2 * QKV_DIM;
 constexpr size_t TP_OFFSET = EPOCH_OFFSET + 64 + 2 * XP_WORDS;   // [0] barrier counter of the tensor-parallel mode; mailbox at + 64 floats
-constexpr size_t X_FLOATS = TP_OFFSET + 128;
+constexpr size_t APART_OFFSET = TP_OFFSET + 128;                 // [16 heads][2][NB][1024] attention contributions kept apart, (tag << 32 | fp32 bits)
+constexpr size_t X_FLOATS = APART_OFFSET + (size_t)Q_HEADS * 2 * PERSIST_MAX_BATCH * HIDDEN * 2;
 struct Share {
     int q0, nq, qmax;       // rows [q0, q0 + nq) of this rank's [wq; wk; wv] rows, slot rows qmax
     int i0, ni, imax;       // FFN rows [i0, i0 + ni) of gate, up and down^T (global row numbers), slot rows imax
@@ -212,9 +215,11 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
 }
 __device__ __forceinline__ float2 ldcg2(const float* p) { return __ldcg(reinterpret_cast<const float2*>(p)); }
 // ---- counted accumulators ----------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long acc_word(float v) {
-    v = fminf(fmaxf(v, -ACC_CLAMP), ACC_CLAMP);
-    return ACC_ONE + (unsigned long long)__float2ll_rn(v * ACC_SCALE);
+__device__ __forceinline__ unsigned long long acc_word(float v) { return ACC_ONE + (unsigned long long)__float2ll_rn(v * ACC_SCALE); }   // |v| <= ACC_LIMIT
+// Where a head's contribution to the word at `acc` is kept apart: a copy of the accumulators' layout (two times `nb` vectors) for each head.  (By the address
+// of the word, which is at hand either way: indexed by sequence, head and element, it cost two sequences 44 bytes of spills.)
+__device__ __forceinline__ unsigned long long* acc_apart(const unsigned long long* acc, int head, int nb) {
+    return const_cast<unsigned long long*>(acc) + APART_OFFSET / 2 + (size_t)head * 2 * nb * HIDDEN;
 }
 template <bool SYS>
 __device__ __forceinline__ void acc_add(unsigned long long* addr, unsigned long long w) {
@@ -227,9 +232,31 @@ __device__ __forceinline__ void acc_load2(const unsigned long long* src, unsigne
     else asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(src) : "memory");
 }
 __device__ __forceinline__ unsigned acc_count(unsigned long long w) { return (unsigned)((w + ACC_HALF) >> 56); }
+__device__ __forceinline__ unsigned acc_counts(unsigned long long w) { return (unsigned)((w + ACC_HALF) >> 51); }   // (contributions << 5) + those kept apart
 __device__ __forceinline__ float acc_value(unsigned long long w) {
-    const long long s = (long long)((w + ACC_HALF) & (ACC_ONE - 1)) - (long long)ACC_HALF;
+    const long long s = (long long)((w + ACC_HALF) & (ACC_APART - 1)) - (long long)ACC_HALF;
     return __ll2float_rn(s) * (1.f / ACC_SCALE);
+}
+template <bool SYS>
+__device__ __forceinline__ void acc_keep_apart(unsigned long long* dst, unsigned tag, float v) {
+    const unsigned long long word = (unsigned long long)tag << 32 | __float_as_uint(v);
+    if (SYS) asm volatile("st.relaxed.sys.global.b64 [%0], %1;\n\tfence.acq_rel.sys;" ::"l"(dst), "l"(word) : "memory");
+    else asm volatile("st.relaxed.gpu.global.b64 [%0], %1;\n\tfence.acq_rel.gpu;" ::"l"(dst), "l"(word) : "memory");
+}
+// the sum of what was kept apart for the two words at `src` under this tag
+template <bool SYS, int NB>
+__device__ __forceinline__ float2 acc_sum_apart(const unsigned long long* src, unsigned tag) {
+    if (SYS) asm volatile("fence.acq_rel.sys;" ::: "memory");
+    else asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int h = 0; h < Q_HEADS; ++h) {
+        unsigned long long w0, w1;
+        acc_load2<SYS>(acc_apart(src, h, NB), w0, w1);
+        if ((unsigned)(w0 >> 32) == tag) s.x += __uint_as_float((unsigned)w0);
+        if ((unsigned)(w1 >> 32) == tag) s.y += __uint_as_float((unsigned)w1);
+    }
+    return s;
 }
 // barrier of the whole CTA (512 threads)
 __device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
@@ -685,7 +712,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     // the load: no counter, no fence; a word that is complete cannot change any more until the buffer is cleared.
     // Thread 0 first polls one sentinel word until it is nearly complete, so that the grid does not hammer lines that
     // are still being added to (measured: 0.5 us faster per wait than every thread polling from the start).
-    auto acc_wait = [&](const unsigned long long* vec, unsigned expect, uint32_t site) {
+    auto acc_wait = [&](const unsigned long long* vec, unsigned expect, uint32_t site, unsigned tag) {
         if (tid == 0 && !*abort_flag) {
             unsigned long long ws;
             unsigned it = 0;
@@ -714,8 +741,19 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
 #pragma unroll
                 for (int b = 0; b < NB; ++b) acc_load2<TP>(src + b * HIDDEN, w0[b], w1[b]);
 #pragma unroll
-                for (int b = 0; b < NB; ++b) whole = whole && acc_count(w0[b]) == expect && acc_count(w1[b]) == expect;
+                for (int b = 0; b < NB; ++b) whole = whole && acc_counts(w0[b]) == expect << 5 && acc_counts(w1[b]) == expect << 5;
                 if (whole) break;
+                whole = true;
+#pragma unroll
+                for (int b = 0; b < NB; ++b) whole = whole && acc_count(w0[b]) == expect && acc_count(w1[b]) == expect;
+                if (whole) {              // complete, but for what is kept apart
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        const float2 a = acc_sum_apart<TP, NB>(src + b * HIDDEN, tag);
+                        x0[b] += a.x; x1[b] += a.y;
+                    }
+                    break;
+                }
                 if ((++it & 63u) == 0) {
                     if (*abort_flag) break;
                     const unsigned long long t = global_ns();
@@ -1339,9 +1377,16 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
             // fn <= 116: the slice joins the attention delta (of every rank); four warps a sequence
             if ((tid & 127) < fn && (tid >> 7) < NB) {
                 const int b = tid >> 7, r = tid & 127;
-                const unsigned long long w = acc_word(wo_part[b * 256 + r] + wo_part[b * 256 + 128 + r]);
-                if (TP) { for (int t = 0; t < T; ++t) acc_add<true>(p.tp_dA[t] + (size_t)(l & 1) * HIDDEN + fr0 + r, w); }
-                else acc_add<false>(dAl + b * HIDDEN + fr0 + r, w);
+                const float v = wo_part[b * 256 + r] + wo_part[b * 256 + 128 + r];
+                auto add = [&](unsigned long long w) {
+                    if (TP) { for (int t = 0; t < T; ++t) acc_add<true>(p.tp_dA[t] + (size_t)(l & 1) * HIDDEN + fr0 + r, w); }
+                    else acc_add<false>(dAl + b * HIDDEN + fr0 + r, w);
+                };
+                if (fabsf(v) <= ACC_LIMIT) add(acc_word(v));     // (two adds, and the readers' test behind the one that fails, cost nothing; one behind the test 1 to 5 us a step)
+                else {
+                    for (int t = 0; t < T; ++t) acc_keep_apart<TP>(acc_apart((TP ? p.tp_dA[t] + (size_t)(l & 1) * HIDDEN : dAl + b * HIDDEN) + fr0 + r, TP ? fh : blockIdx.x % Q_HEADS, NB), tag, v);
+                    add(ACC_ONE + ACC_APART);
+                }
             }
         }   // (wo_part is the next phase's staging area: the wait below passes a CTA barrier before anything is staged)
         Q3_TRACE(ev + 6);
@@ -1349,7 +1394,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
 
         // ==================================================================== GD
         {
-            acc_wait(dAl, (unsigned)Q_HEADS, 200 + l);   // every row of the attention delta receives one slice per query head
+            acc_wait(dAl, (unsigned)Q_HEADS, 200 + l, tag);   // every row of the attention delta receives one slice per query head
             Q3_TRACE(ev + 7);
             fetch_slot(0, l + 1);   // q/k/v rows and Wo slice of the next layer: landed before this phase's barrier is polled
             if (!MANY) fetch_slot(1, l + 1);

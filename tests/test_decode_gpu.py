@@ -170,6 +170,39 @@ def test_two_and_three_sequences_are_one_launch(oracle, grid):
     mk.status()
 
 
+@pytest.mark.parametrize("lens", [(40,), (150,), (250,), (300,), (3500,), (30, 50), (16, 700, 90)])
+def test_what_is_not_finite_or_huge_reaches_the_logits(oracle, lens):
+    """The attention's sums over the heads are fixed-point numbers up to 16000 a contribution.  A NaN, an infinity or a larger value in a sequence's cache gives
+    it what fp32 sums give, and leaves the other sequences alone; so does the launch after."""
+    from qwen3mk.kernel import SeqTable
+
+    shp = oracle.Shape(layers=2, vocab=2048)
+    inp = oracle.synthetic(91, shp, context=1)
+    w = oracle.to_fp32(inp)
+    dev = to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES})
+    g = torch.Generator().manual_seed(sum(lens))
+    toks = torch.randint(0, 2048, (len(lens),), generator=g)
+    kcs, vcs = ([torch.randn(2, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens] for _ in range(2))
+    mk = engine("auto", layers=2, vocab=2048, max_batch=len(lens))
+    refs = oracle.decode_batch(w, toks.tolist(), kcs, vcs)
+    for victim in range(len(lens)):
+        for value in (float("nan"), float("inf"), -float("inf"), 3e6, None):
+            v = [t.clone() for t in vcs]
+            if value is not None:
+                v[victim][0, lens[victim] // 2, 3, 5:9] = value
+            out = mk.bind_sequences(dev, toks.cuda(), SeqTable([k.cuda() for k in kcs], [t.cuda() for t in v]))
+            before = mk.launch_count
+            mk.launch()
+            mk.status()
+            assert mk.launch_count == before + 1
+            want = oracle.decode_batch(w, toks.tolist(), kcs, v) if value == 3e6 else refs
+            for b, ref in enumerate(want):
+                if b == victim and value not in (3e6, None):
+                    assert bool(out["logits"][b].isnan().all()), (victim, value)
+                else:
+                    gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{lens} seq {b}, {value} in {victim}")
+
+
 @pytest.mark.parametrize("ctx", [40, 200, 300])
 def test_persist_on_a_grid_one_short_of_the_sm_count(oracle, ctx):
     """147 CTAs is the smallest grid the persistent kernel's shared-memory slots allow; the row shares differ from 148's."""
