@@ -1183,9 +1183,10 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                     unpack8f(kv[1], f);
 #pragma unroll
                     for (int hh = 0; hh < 2; ++hh) {
-                        const float mn = live ? fmaxf(mx[hh], s2[hh]) : mx[hh];
+                        if (!live) s2[hh] = -INFINITY;
+                        const float mn = fmaxf(mx[hh], s2[hh]);
                         const float keep = mx[hh] == mn ? 1.f : exp2_approx(mx[hh] - mn);     // (the first row: exp(-inf) = 0)
-                        const float pr = live ? exp2_approx(s2[hh] - mn) : 0.f;
+                        const float pr = s2[hh] == -INFINITY ? 0.f : exp2_approx(s2[hh] - mn);     // (the maximum may be -inf, too)
                         mx[hh] = mn;
                         ls[hh] = fmaf(ls[hh], keep, pr);
 #pragma unroll
@@ -1233,7 +1234,7 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
                     const float wgt = mw == -INFINITY ? 0.f : exp2_approx(mw - M);
                     float Ls = warp_sum(lane < CW ? oml[2 * CW + hh * CW + lane] * wgt : 0.f);
                     if (with_new) {
-                        const float wn = exp2_approx(misc[hh] - M);
+                        const float wn = misc[hh] == -INFINITY ? 0.f : exp2_approx(misc[hh] - M);
                         Ls += wn;
                         o = wn * v_s[d];
                     }

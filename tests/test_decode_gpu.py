@@ -203,6 +203,41 @@ def test_what_is_not_finite_or_huge_reaches_the_logits(oracle, lens):
                     gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{lens} seq {b}, {value} in {victim}")
 
 
+@pytest.mark.parametrize("lens", [(40,), (250,), (300,), (3500,), (30, 50), (16, 700, 90)])
+def test_scores_of_minus_infinity_weigh_nothing(oracle, lens):
+    """Cached rows whose score is -inf, as a caller masks positions: the first one of a block, all of a block's, all but the last of a sequence."""
+    from qwen3mk.kernel import SeqTable
+
+    shp = oracle.Shape(layers=2, vocab=2048)
+    inp = oracle.synthetic(92, shp, context=1)
+    w = oracle.to_fp32(inp)
+    dev = to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES})
+    g = torch.Generator().manual_seed(sum(lens))
+    toks = torch.randint(0, 2048, (len(lens),), generator=g)
+    kcs, vcs = ([torch.randn(2, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens] for _ in range(2))
+    mk = engine("auto", layers=2, vocab=2048, max_batch=len(lens))
+    for share in (0.04, 0.5, 1.0):
+        ks = [t.clone() for t in kcs]
+        for b, n in enumerate(lens):
+            x = w["embed"][toks[b]]
+            q = (w["wq"][0] @ (x * torch.rsqrt((x * x).mean() + 1e-6) * w["ln1"][0])).view(16, 128)
+            q = q * torch.rsqrt((q * q).mean(-1, keepdim=True) + 1e-6) * w["qn"][0]
+            cos, sin = oracle.rope_cos_sin(torch.tensor([n]))
+            q = (q * cos + torch.cat([-q[:, 64:], q[:, :64]], dim=1) * sin).view(8, 2, 128)
+            for kv in (0, 5):        # a dim in which both heads of the group point the same way, by a margin
+                same = q[kv].min(0).values.clamp(min=0) - q[kv].max(0).values.clamp(max=0)
+                d = int(same.argmax())
+                ks[b][0, :max(1, int(share * n) - 1), kv, d] = -float("inf") if q[kv, 0, d] > 0 else float("inf")
+        out = mk.bind_sequences(dev, toks.cuda(), SeqTable([k.cuda() for k in ks], [v.cuda() for v in vcs]))
+        before = mk.launch_count
+        mk.launch()
+        mk.status()
+        assert mk.launch_count == before + 1
+        for b, ref in enumerate(oracle.decode_batch(w, toks.tolist(), ks, vcs)):
+            assert bool(ref["logits"].isfinite().all())
+            gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{lens} seq {b}, {share} of the rows")
+
+
 @pytest.mark.parametrize("ctx", [40, 200, 300])
 def test_persist_on_a_grid_one_short_of_the_sm_count(oracle, ctx):
     """147 CTAs is the smallest grid the persistent kernel's shared-memory slots allow; the row shares differ from 148's."""
