@@ -35,7 +35,8 @@ extern "C" {
 
 /* q3_decode_args.flags */
 #define Q3_F_APPEND_KV    0x1u  /* write the new K/V rows into cache slot seq_len[b], then seq_len[b] += 1 */
-#define Q3_F_PATH_AUTO    0x0u  /* engine picks: persistent kernel for up to three sequences it serves, layered otherwise */
+#define Q3_F_PATH_AUTO    0x0u  /* engine picks: persistent kernel for up to three sequences it serves (sums in the order of arrival: logits
+                                   differ from run to run by about 1e-6), layered otherwise (a fixed order up to 64 sequences) */
 #define Q3_F_PATH_LAYERED 0x10u /* a chain of launches: five per layer up to 64 sequences, one per phase beyond */
 #define Q3_F_PATH_FUSED   0x30u /* layered, but batches of 4..64 run two launches per layer: split attention + one persistent
                                    kernel for Wo, norm, gate/up, SiLU, down, norm and the next layer's q/k/v (opt-in: measured

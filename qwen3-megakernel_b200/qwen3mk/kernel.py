@@ -131,7 +131,8 @@ class Megakernel:
     `bind_sequences` is the batched / growing-cache form of `bind`.
 
     path: "auto" (persistent kernel for up to three sequences it serves, else layered), "layered" (a chain of launches), "fused" (layered, with
-    one persistent kernel for everything between two attentions for batches of 4..64; opt-in) or "persist".
+    one persistent kernel for everything between two attentions for batches of 4..64; opt-in) or "persist".  The persistent kernel adds
+    the FFN's partial sums as its blocks arrive, so its logits differ from run to run by about 1e-6; "layered" repeats them bit by bit up to 64 sequences.
     """
 
     def __init__(self, device=None, *, max_batch: int = 1, layers: int = LAYERS, vocab: int = VOCAB,

@@ -322,8 +322,27 @@ def test_batches_at_the_edges_of_the_token_tiles(oracle, batch):
         gate_step(oracle, {k: out[k][b] for k in out}, ref, f"seq {b} len {lens[b]}")
     mk.launch()
     mk.status()
-    # (the logits of so small a vocabulary are K-slices added with atomics; the rows have been through every cluster GEMM)
     assert all(torch.equal(first[k], out[k]) for k in ("k_write", "v_write"))
+
+
+@pytest.mark.parametrize("lens", [(3500,), (40, 700), (16, 900, 300), (50, 60, 70, 80, 90)])
+def test_the_launch_chain_repeats_itself_bit_by_bit(oracle, lens):
+    """Plain launches, then a graph's replays: one result, whatever the order in which blocks finish.  (The persistent kernel adds in the order of arrival.)"""
+    from qwen3mk.kernel import SeqTable
+
+    inp = oracle.synthetic(54, oracle.Shape(layers=2, vocab=2048), context=1)
+    g = torch.Generator().manual_seed(len(lens))
+    kvs = [[torch.randn(2, n, 8, 128, generator=g).to(torch.bfloat16).cuda() for n in lens] for _ in range(2)]
+    mk = engine("layered", layers=2, vocab=2048, max_batch=len(lens))
+    out = mk.bind_sequences(to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}), torch.arange(len(lens)).cuda(), SeqTable(*kvs))
+    first = None
+    for _ in range(14):
+        for t in out.values():
+            t.zero_()
+        mk.launch()
+        mk.status()
+        first = first or {k: t.clone() for k, t in out.items()}
+        assert all(torch.equal(first[k], out[k]) for k in out)
 
 
 def decode_fp64(inp, tokens, kcs, vcs, rope):
