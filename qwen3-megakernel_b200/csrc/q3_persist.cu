@@ -56,7 +56,7 @@ constexpr int WO_SLICES = 9;                  // row slices of Wo; CTA c < 144 o
 constexpr int F_CTAS = Q_HEADS * WO_SLICES;   // 144
 constexpr int GROUP_CTAS = 2 * WO_SLICES;     // CTAs sharing one kv head
 constexpr int WO_ROWS_MAX = 116;              // largest slice: 4 * ceil(256 / 9)
-constexpr int PERSIST_MAX_BATCH = 3;          // sequences a launch decodes; one after the other where the caller asks for this kernel by name
+constexpr int PERSIST_MAX_BATCH = 3;          // sequences a launch decodes
 constexpr int MIN_GRID = 147;                 // row shares must fit the shared-memory slots
 constexpr int SC_FLOATS = 344;                // the score buffer of the local attention, which serves up to 255 positions
 // Most cached positions this kernel is picked for: the longest at which it was timed against the launch chain (one sequence, us per step, this
@@ -66,7 +66,9 @@ constexpr int PERSIST_MAX_LEN = 30000;
 // 599 / 632 / 679 / 733 (24 columns are three MMAs a tile, and the registers of a pass do not all fit: 164 bytes of spills) against 624 / 668 /
 // 697 / 729 in plain launches and 576 / 626 / 654 / 685 from a graph: in place of plain launches, up to
 constexpr int PERSIST_THREE_LEN = 1500;
-constexpr int PERSIST_ASKED_LEN = 3438;       // ... and that a caller may ask for who names this kernel: the limit that request has always had
+// ... and that a caller may ask for who names this kernel.  Such a request is answered by this kernel or refused, and a caller may go by the refusal: what
+// was refused stays refused.
+constexpr int PERSIST_ASKED_LEN = 3438;
 constexpr int WROW = 1032;                    // elements between weight rows in shared memory: 1024 + 8 of padding, so that
                                               // the eight row addresses of an ldmatrix fall into different banks
 // Words between the three parts of an activation vector in shared memory: a lane of the products reads word `kp` of the part of its column, so
@@ -1760,9 +1762,9 @@ static int smem_bytes_for(int grid) {
     return (qmax + 3 * imax) * WROW * 2 + WO_ROWS_MAX * WOROW * 2 + TAIL_BYTES;
 }
 
-static const void* persist_kernel(int mode, bool tp = false, int together = 1) {
-    if (together == 2) return reinterpret_cast<const void*>(q3_persist_decode<N_MODES - 1, false, 2>);
-    if (together == 3) return reinterpret_cast<const void*>(q3_persist_decode<N_MODES - 1, false, 3>);
+static const void* persist_kernel(int mode, bool tp = false, int nb = 1) {
+    if (nb == 2) return reinterpret_cast<const void*>(q3_persist_decode<N_MODES - 1, false, 2>);
+    if (nb == 3) return reinterpret_cast<const void*>(q3_persist_decode<N_MODES - 1, false, 3>);
     if (tp) {
         switch (mode) {
             case 0: return reinterpret_cast<const void*>(q3_persist_decode<0, true, 1>);
@@ -1830,7 +1832,7 @@ void persist_teardown(q3_engine* e) {
     e->p_state = nullptr;
 }
 
-// Batches of up to PERSIST_MAX_BATCH sequences: one launch for all of them, or one after the other for a caller that names this kernel.
+// Batches of up to PERSIST_MAX_BATCH sequences, one launch for all of them.
 bool persist_supports(const q3_engine* e, const q3_decode_args* a) {
     const PersistState* s = static_cast<const PersistState*>(e->p_state);
     if (s == nullptr || a->batch < 1) return false;
@@ -1932,9 +1934,8 @@ int persist_decode(q3_engine* e, const q3_decode_args* a, cudaStream_t st) {
     p.seq_k = a->seq_k; p.seq_v = a->seq_v; p.seq_layer_stride = reinterpret_cast<const long long*>(a->seq_layer_stride);
     p.seq_len = a->seq_len; p.logits = a->logits; p.next_token = reinterpret_cast<long long*>(a->next_token);
     p.k_write = reinterpret_cast<bf16_raw*>(a->k_write); p.v_write = reinterpret_cast<bf16_raw*>(a->v_write);
-    const bool asked = (a->flags & Q3_F_PATH_MASK) == Q3_F_PATH_PERSIST;
-    const int together = asked ? 1 : a->batch;             // sequences of a launch
-    p.dA = reinterpret_cast<unsigned long long*>(s->X); p.dB = s->X + 4 * HIDDEN * together;
+    const int nb = a->batch;                               // sequences of the launch
+    p.dA = reinterpret_cast<unsigned long long*>(s->X); p.dB = s->X + 4 * HIDDEN * nb;
     p.xq = reinterpret_cast<unsigned long long*>(s->X + XQ_OFFSET);
     p.epoch = reinterpret_cast<const unsigned*>(s->X + EPOCH_OFFSET);
     p.xp = reinterpret_cast<unsigned long long*>(s->X + EPOCH_OFFSET + 64);
@@ -1953,24 +1954,13 @@ int persist_decode(q3_engine* e, const q3_decode_args* a, cudaStream_t st) {
     p.n_layers = e->cfg.n_layers; p.vocab = e->cfg.vocab; p.append = (a->flags & Q3_F_APPEND_KV) ? 1 : 0;
     int mode = 0;
     while (mode + 1 < N_MODES && a->max_len > mode_max_len(mode)) ++mode;
-    if (together > 1) mode = N_MODES - 1;
-    p.max_len = together > 1 ? a->max_len : mode < N_MODES - 1 ? mode_max_len(mode) : a->max_len > PERSIST_ASKED_LEN ? a->max_len : PERSIST_ASKED_LEN;
+    if (nb > 1) mode = N_MODES - 1;
+    p.max_len = nb > 1 ? a->max_len : mode < N_MODES - 1 ? mode_max_len(mode) : a->max_len > PERSIST_ASKED_LEN ? a->max_len : PERSIST_ASKED_LEN;
     if (p.max_len > e->rope_n - 1) p.max_len = e->rope_n - 1;
-    // A batch of a caller that names this kernel is one launch per sequence, back to back on the stream: the per-sequence
-    // arrays are simply offset (outputs are [batch][...] with the batch axis leading).
-    const size_t kv_row = (size_t)e->cfg.n_layers * KV_DIM;
-    for (int b = 0; b < a->batch; b += together) {
-        PersistParams q = p;
-        q.token = p.token + b; q.seq_k = p.seq_k + b; q.seq_v = p.seq_v + b; q.seq_layer_stride = p.seq_layer_stride + b;
-        q.seq_len = p.seq_len + b; q.next_token = p.next_token + b;
-        q.logits = p.logits ? p.logits + (size_t)b * e->cfg.vocab : nullptr;
-        q.k_write = p.k_write ? p.k_write + b * kv_row : nullptr;
-        q.v_write = p.v_write ? p.v_write + b * kv_row : nullptr;
-        void* args[] = {&q};
-        cudaError_t err = cudaLaunchCooperativeKernel(persist_kernel(mode, tp, together), dim3(s->grid), dim3(PT), args, (size_t)s->smem, st);
-        ++e->launches;
-        if (err != cudaSuccess) return engine_fail(e, Q3_ERR_CUDA, "persist: cooperative launch failed: %s", cudaGetErrorString(err));
-    }
+    void* args[] = {&p};
+    const cudaError_t err = cudaLaunchCooperativeKernel(persist_kernel(mode, tp, nb), dim3(s->grid), dim3(PT), args, (size_t)s->smem, st);
+    ++e->launches;
+    if (err != cudaSuccess) return engine_fail(e, Q3_ERR_CUDA, "persist: cooperative launch failed: %s", cudaGetErrorString(err));
     return Q3_OK;
 }
 

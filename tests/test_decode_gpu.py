@@ -170,6 +170,30 @@ def test_two_and_three_sequences_are_one_launch(oracle, grid):
     mk.status()
 
 
+@pytest.mark.parametrize("lens", [(60, 3438), (3438, 1700, 1), (5, 3439)])
+def test_a_caller_who_names_the_persistent_kernel_gets_one_launch(oracle, lens):
+    """For all sequences together, as "auto" does, three beyond 1500 positions as well; refused beyond 3438."""
+    from qwen3mk.kernel import SeqTable
+
+    inp = oracle.synthetic(78, oracle.Shape(layers=2, vocab=2048), context=1)
+    g = torch.Generator().manual_seed(7)
+    toks = torch.randint(0, 2048, (len(lens),), generator=g)
+    kcs, vcs = ([torch.randn(2, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens] for _ in range(2))
+    mk = engine("persist", layers=2, vocab=2048, max_batch=3)
+    out = mk.bind_sequences(to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}), toks.cuda(), SeqTable([k.cuda() for k in kcs], [v.cuda() for v in vcs]))
+    before = mk.launch_count
+    if max(lens) > 3438:
+        with pytest.raises(RuntimeError, match="persistent kernel"):
+            mk.launch()
+        return
+    for _ in range(10):
+        mk.launch()
+    mk.status()
+    assert mk.launch_count == before + 10
+    for b, ref in enumerate(oracle.decode_batch(oracle.to_fp32(inp), toks.tolist(), kcs, vcs)):
+        gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{lens} seq {b}")
+
+
 @pytest.mark.parametrize("lens", [(40,), (150,), (250,), (300,), (3500,), (30, 50), (16, 700, 90)])
 def test_what_is_not_finite_or_huge_reaches_the_logits(oracle, lens):
     """The attention's sums over the heads are fixed-point numbers up to 16000 a contribution.  A NaN, an infinity or a larger value in a sequence's cache gives
