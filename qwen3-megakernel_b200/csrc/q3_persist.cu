@@ -673,7 +673,9 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     // The first chunk of a slot arms the slot's mbarrier with the slot's byte count; every warp waits on it before it reads the slot.
     const int bytesA = qmax * WROW * 2, bytesB = WO_ROWS_MAX * WOROW * 2, bytesC = 2 * imax * WROW * 2, bytesD = imax * WROW * 2;
     const bool pumper = tid == 32;
-    int pump_armed = 0, pump_parity = 0;                // per slot: armed at all, and the parity of its last armed phase
+    constexpr int FEW_ROWS = 16;                        // (kept among them: a flag of its own is a register too many)
+    int pump_armed = NB == 2 && p.seq_len[0] + p.seq_len[NB - 1] <= 4 * 32 * GROUP_CTAS ? FEW_ROWS : 0;   // per slot: armed at all; two sequences: at most four passes a block
+    int pump_parity = 0;                                // ... and the parity of its last armed phase
     auto fetch_slot = [&](int slot, int layer) {
         if (!pumper || layer >= L || (slot == 1 && !has_f)) return;
         const int bytes = slot == 0 ? bytesA : slot == 1 ? bytesB : slot == 2 ? bytesC : bytesD;
@@ -995,10 +997,10 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
         }
         // Gate/up rows of this layer, in flight during F.  They leave behind the q/k/v exchange, which they slow, where F has no cached rows to fetch
         // then: us per step at 16 / 64 / 128 / 191 / 300 / 1000 / 2200 positions 348 / 351 / 330 / 353 / 407 / 428 / 447 asked for here, 321 / 323 / 330 / 348 /
-        // 395 / 401 / 430 behind the exchange; two sequences at 16 / 600 / 1000 500 / 534 / 549 and 488 / 508 / 549.  But 255 / 3400 / 5000 375 / 473 / 513 and 380 / 481 / 529,
-        // two at 1500 580 and 585, three at 16 564 and 567.
-        // (two sequences: by the host's bound, for a flag of the block's own is a register too many)
-        auto rows_late = [&]() { return has_f && (local_attn ? MODE < 2 : NB == 1 ? npass <= PASSES : NB == 2 && p.max_len <= 1000); };
+        // 395 / 401 / 430 behind the exchange.  But 255 / 3400 / 5000 375 / 473 / 513 and 380 / 481 / 529; three sequences at 16 564 and 567.  Two sequences: by the
+        // sum of their lengths, which is what a block's passes follow from: 16 and 16 / 1000 and 16 / 1500 and 16 / 1700 and 16 / 1000 and 1000 / 2000 and 16 500 / 541 /
+        // 543 / 561 / 551 / 561 here, 486 / 509 / 522 / 548 / 545 / 557 behind; 1500 and 1500 570 and 581, 4000 and 16 607 and 617.
+        auto rows_late = [&]() { return has_f && (local_attn ? MODE < 2 : NB == 1 ? npass <= PASSES : NB == 2 && (pump_armed & FEW_ROWS) != 0); };
         if (!rows_late()) fetch_slot(2, l);
         Q3_TRACE(ev + 2);
 
