@@ -937,10 +937,11 @@ cudaError_t launch_prompt_gemm(const PromptGemmCall& c, cudaStream_t st) {
     const int bn = c.kind == PR_QKV ? (mt == 1 ? 32 : mt <= 4 ? 64 : 128) : c.kind == PR_RESID ? (mt == 1 ? 32 : 64) : mt == 1 ? 48 : mt == 2 ? 96 : mt == 3 ? 128 : 192;
     const int rows[3] = {c.kind == PR_QKV ? Q_DIM : c.kind == PR_RESID ? HIDDEN : INTER, c.kind == PR_QKV ? KV_DIM : INTER, KV_DIM};
     const int n_w = c.kind == PR_QKV ? 3 : c.kind == PR_RESID ? 1 : 2;
-    // gate/up on pairs of SMs: items of 192 columns where their rounds are shorter than those of 256 (us a prompt, 192 / 256: 640 tokens, one round of
-    // 256, 1770 / 1656; 777, two rounds either way, 1806 / 1828; 1024 1899 / 1949; 1100 2068 / 2020; 1400 2561 / 2520; 2048, four and three, the same)
+    // gate/up on pairs of SMs: items of 192 columns where their rounds are shorter than those of 256 by more than an eighth, which the products show: 769 to
+    // 1024 tokens on 148 SMs (us a prompt, 256 / 192: 800 tokens 1868 / 1845, 1000 1995 / 1944; one round of 256, 640, 1656 / 1770; 1100 2020 / 2068; 1400 2520 / 2561).
+    // Where the rounds are shorter by less, both take the same: 2320 3995 / 3954, 2400 4238 / 4190, 2560 4401 / 4413, 2700 4690 / 4717, 4000 6994 / 6957 (runs of one side 80 apart).
     const int pairs = sm / 2, mt2 = (mt + 1) / 2, rounds256 = (mt2 * (2 * INTER / 256) + pairs - 1) / pairs, rounds192 = (mt2 * (2 * INTER / 192) + pairs - 1) / pairs;
-    const bool finer = c.kind == PR_SILU && rounds192 * 192 < rounds256 * 256;
+    const bool finer = c.kind == PR_SILU && rounds192 * 192 * 8 < rounds256 * 256 * 7;
     const uint32_t box = pair ? (c.kind == PR_RESID ? 64u : finer ? 96u : 128u) : c.kind == PR_RESID ? (uint32_t)bn : (uint32_t)bn / 2;
     CUtensorMap tw[3];
     for (int i = 0; i < 3; ++i) {
