@@ -45,10 +45,13 @@ int q3::engine_fail(q3_engine* e, int code, const char* fmt, ...) {
 // ------------------------------------------------------------------------------------------------
 // The key holds the addresses of one bind, so every bind captures anew.  A capture costs the host 450 to 850 us, beside 360 for the
 // plain launches of a step; after three steps that are launched without waiting the GPU is far enough behind to hide it (8 x 1024, a fresh
-// bind of 8 steps, capture on the 2nd / 4th: 6070 / 5910 us; of 2 steps 1680 / 1540).  Where
-// the steps before the capture are not plain launches of the chain but launches of the persistent kernel (three sequences: a replay saves 5 to 25 us
-// on those), and for two sequences of a caller who names the chain (at 16 positions 4 steps: a persistent launch a sequence 2880, captured on
-// the 4th 3110), the capture waits until the ninth.
+// bind of 8 steps, capture on the 2nd / 4th: 6070 / 5910 us; of 2 steps 1680 / 1540).  Three sequences, whose steps before the capture are launches of the
+// persistent kernel, and two of a caller who names the chain wait until the ninth: a replay saves them only 10 to 25 us a step, and a caller who waits for every
+// step pays for the whole capture.  us of a fresh bind of 8 / 16 / 40 steps, capture on the 4th / the 9th / never: three at 16 positions, waiting for every
+// step, 5370 / 10800 / 24610, 5080 / 11000 / 25700, 4990 / 9890 / 24630, without waiting 4730 / 9290 / 23060, 4880 / 9480 / 23420, 4900 / 9670 / 24080; three ragged
+// up to 900 5690 / 10830 / 25890, 5230 / 10830 / 25940, 5210 / 10380 / 25960 and 5050 / 9990 / 24810, 5140 / 10060 / 24880, 5100 / 10150 / 25420; the chain at two
+// of 16 5390 / 10040 / 24960, 5110 / 10610 / 25380, 5130 / 10290 / 25500 and 4760 / 9320 / 23160, 5010 / 9560 / 23640, 5000 / 9960 / 24630.  So the ninth costs 1 to 5
+// per cent where nobody waits, and is worth 5 to 9 per cent of a short turn where somebody does.
 static int plain_uses(int batch, bool persist) { return batch == 2 || persist ? 8 : 3; }
 struct GraphEntry {
     q3_decode_args key;
