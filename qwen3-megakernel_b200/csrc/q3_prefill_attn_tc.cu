@@ -28,6 +28,7 @@
 #include <cuda.h>
 
 #include "q3_engine.h"
+#include "q3_gemm_tc.h"
 #include "q3_prompt.h"
 #include "q3_tc_ptx.cuh"
 
@@ -42,7 +43,6 @@ constexpr uint32_t AT_BOX = 128 * 128;    // bytes of one [128 rows x 64 columns
 constexpr uint32_t AT_Q_BYTES = 2 * AT_BOX, AT_KV_BYTES = 2 * AT_BOX;   // 128 x 128 bf16 = two boxes
 constexpr size_t AT_SMEM = 2 * AT_Q_BYTES + AT_STAGES * 2 * AT_KV_BYTES;   // Q hi, Q lo, stages x (K, V) = 192 KB
 constexpr int AT_SPLIT_MIN = 3;           // key tiles of a query tile that two blocks share, at least
-constexpr int AT_ONE_WAVE = 18;           // blocks of a kv group that are resident at once (148 SMs, a block each)
 constexpr float AT_LAG = 8.f;             // how far (in log2) scores may exceed the maximum that P is taken under
 constexpr unsigned long long AT_WAIT_NS = 200ull * 1000 * 1000;
 
@@ -484,7 +484,8 @@ cudaError_t launch_prefill_attn_tc(const CUtensorMap& q_hi, const CUtensorMap& q
     // tokens 1099 / 1080; in two waves 1090 tokens 2105 / 2019, 1400 2606 / 2506).
     const int tiles = (T + AT_QT - 1) / AT_QT;
     const int long_ones = tiles - 2 * (AT_SPLIT_MIN - 1);        // query tiles of at least AT_SPLIT_MIN key tiles (every key tile is the last of two)
-    const int shared = min(AT_ONE_WAVE - tiles, long_ones);
+    const int one_wave = tc_sm_count() / KV_HEADS;               // blocks of a kv group that are resident at once, one on an SM: 18 of 148
+    const int shared = min(one_wave - tiles, long_ones);
     if (shared > 0) {
         PrefillAttnTcArgs a{reinterpret_cast<bf16_raw*>(plane), T, layer, shared, status};
         return launch_chain_cluster(prefill_attn_tc_kernel<true>, dim3(2 * (shared + (tiles - shared + 1) / 2) * KV_HEADS), dim3(AT_THREADS), AT_SMEM, 2, st, q_hi, q_lo, k, v, a);
