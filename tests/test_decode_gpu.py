@@ -97,7 +97,7 @@ def test_any_position(oracle, path, ctx):
 @pytest.mark.parametrize("ctx", [575, 576, 577, 2304, 2305, 2900, 3439, 4608, 4610, 8191])
 def test_one_sequence_is_one_launch_at_any_length(oracle, ctx):
     """The 18 blocks of a kv head take 32 positions a pass and hold four passes in registers: lengths around one pass (576), around four (2304)
-    and beyond what a caller that names the persistent kernel may ask for (3438)."""
+    and beyond what a caller who names the persistent kernel may ask for (3438)."""
     from qwen3mk.kernel import SeqTable
 
     shp = oracle.Shape(layers=2, vocab=2048)
@@ -168,6 +168,36 @@ def test_two_and_three_sequences_are_one_launch(oracle, grid):
     seqs.len.copy_(torch.tensor([30, 20]))
     mk.launch()
     mk.status()
+
+
+@pytest.mark.parametrize("vocab", [40003, 18944, 9473])
+@pytest.mark.parametrize("batch", [1, 2, 3])
+def test_lm_head_of_many_words_a_block(oracle, batch, vocab):
+    """Several sequences take eight words a warp from a ring of loads that runs on into the warp's next group.  Two or three groups with a ragged end, one whole
+    group a warp, no more than one and some blocks without the last warps'; the best word twice, in another block: the lower index wins."""
+    from qwen3mk.kernel import SeqTable
+
+    inp = oracle.synthetic(79, oracle.Shape(layers=1, vocab=vocab), context=1)
+    g = torch.Generator().manual_seed(vocab)
+    toks = torch.randint(0, vocab, (batch,), generator=g)
+    kcs, vcs = ([torch.randn(1, 20 + b, 8, 128, generator=g).to(torch.bfloat16) for b in range(batch)] for _ in range(2))
+    best = [int(r["next_token"]) for r in oracle.decode_batch(oracle.to_fp32(inp), toks.tolist(), kcs, vcs)]
+    for b, word in enumerate(best):
+        twin = (word + vocab // 2 + 11 * b) % vocab
+        if twin not in toks.tolist() and twin not in best:
+            inp["embed"][twin] = inp["embed"][word]
+    refs = oracle.decode_batch(oracle.to_fp32(inp), toks.tolist(), kcs, vcs)
+    mk = engine("auto", layers=1, vocab=vocab, max_batch=batch)
+    out = mk.bind_sequences(to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}), toks.cuda(), SeqTable([k.cuda() for k in kcs], [v.cuda() for v in vcs]))
+    before = mk.launch_count
+    mk.launch()
+    mk.status()
+    assert mk.launch_count == before + 1
+    for b, ref in enumerate(refs):
+        gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{vocab} words, seq {b}")
+        assert oracle.rel_l2(out["logits"][b], ref["logits"]) <= 1e-5
+        top = out["logits"][b].max()
+        assert int(out["next_token"][b]) == int((out["logits"][b] == top).nonzero()[0])
 
 
 @pytest.mark.parametrize("lens", [(60, 3438), (3438, 1700, 1), (5, 3439)])
@@ -399,35 +429,41 @@ def decode_fp64(inp, tokens, kcs, vcs, rope):
 
 
 def test_few_sequences_are_as_close_to_fp64_as_one(oracle):
-    """Two and three sequences run as a batch, one runs in the persistent kernel, whose products and sums are fp32 or
-    better: a batch must not be further from fp64.  Over nine batches the two differ by the luck of the roundings, a few
-    percent of 2e-6; two bf16 planes of q and the probabilities would be eight times as far."""
+    """One sequence runs in the persistent kernel, whose products and sums are fp32 or better.  Two and three together in it ("auto"), and the launch chain's
+    form for them, which graphs replay and which serves what the kernel does not ("layered"), must not be further from fp64.  Over nine batches they
+    differ by the luck of the roundings, a few percent of 2e-6; two bf16 planes of q and the probabilities would be eight times as far."""
     from qwen3mk.kernel import SeqTable
 
     shp = oracle.Shape(layers=6, vocab=2048)
-    far = {"auto": 0.0, "persist": 0.0}
+    far = {"layered": 0.0, "auto": 0.0, "one": 0.0}
     for seed, lens in enumerate([(16, 30), (250, 250), (1000, 700), (3000, 1500), (900, 600, 300), (3400, 20, 5), (60, 61), (2000, 1), (500, 400, 450)]):
         inp = oracle.synthetic(60 + seed, shp, context=1)
+        dev = to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES})
         g = torch.Generator().manual_seed(seed)
         toks = torch.randint(0, 2048, (len(lens),), generator=g)
         kcs = [torch.randn(6, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens]
         vcs = [torch.randn(6, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens]
+        ref = None
         for path in far:
-            mk = engine(path, layers=6, vocab=2048, max_batch=len(lens))
-            out = mk.bind_sequences(to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}), toks.cuda(), SeqTable([k.cuda() for k in kcs], [v.cuda() for v in vcs]))
-            mk.launch()
-            mk.status()
-            if path == "auto":
-                ref = decode_fp64(inp, toks, kcs, vcs, mk.rope.cpu())
-            far[path] += oracle.rel_l2(out["logits"], ref) / 9
-    print(f"mean logits rel-L2 against fp64: batch {far['auto']:.2e}, one at a time {far['persist']:.2e}")
-    assert far["auto"] <= 1.15 * far["persist"]
+            mk = engine("persist" if path == "one" else path, layers=6, vocab=2048, max_batch=len(lens))
+            ref = decode_fp64(inp, toks, kcs, vcs, mk.rope.cpu()) if ref is None else ref
+            rows = []
+            for some in ([slice(b, b + 1) for b in range(len(lens))] if path == "one" else [slice(None)]):
+                out = mk.bind_sequences(dev, toks[some].cuda(), SeqTable([k.cuda() for k in kcs[some]], [v.cuda() for v in vcs[some]]))
+                before = mk.launch_count
+                mk.launch()
+                mk.status()
+                assert (mk.launch_count > before + 1) == (path == "layered" or (path == "auto" and lens == (3400, 20, 5)))
+                rows.append(out["logits"])
+            far[path] += oracle.rel_l2(torch.cat(rows), ref) / 9
+    print("mean logits rel-L2 against fp64: " + ", ".join(f"{k} {v:.2e}" for k, v in far.items()))
+    assert max(far["layered"], far["auto"]) <= 1.15 * far["one"]
 
 
 def test_a_short_bind_of_two_sequences_is_no_slower_than_one_after_the_other(oracle):
-    """Two steps on tables and outputs at new addresses: a graph captured for them would cost more than it saves (1.3 times the
-    persistent kernel's time at these sizes; plain launches take 0.92 of it).  The best of nine binds, so that a busy
-    host does not decide."""
+    """Two steps on tables and outputs at new addresses.  On the launch chain a graph captured for them would cost more than it saves (1.3 times the
+    time of a persistent launch a sequence at these sizes; plain launches take about as long); "auto" makes one launch a step of it.  The best of nine
+    binds, so that a busy host does not decide."""
     import time
 
     from qwen3mk import weights
@@ -438,19 +474,23 @@ def test_a_short_bind_of_two_sequences_is_no_slower_than_one_after_the_other(ora
     caches = [torch.zeros(28, 20, 8, 128, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
     toks = torch.zeros(2, dtype=torch.int64, device="cuda")
     best, kept = {}, []                       # (kept: a freed table's addresses would come back)
-    for path in ("auto", "persist"):
-        mk = engine(path, max_batch=2)
+    for path in ("auto", "layered", "one"):
+        mk = engine("persist" if path == "one" else path, max_batch=2)
         for _ in range(9):
-            seqs = SeqTable(caches[:2], caches[2:], [16, 16])
-            kept.append((seqs, mk.bind_sequences(w, toks, seqs, append=True)))
+            tables = [SeqTable([caches[b]], [caches[2 + b]], [16]) for b in range(2)] if path == "one" else [SeqTable(caches[:2], caches[2:], [16, 16])]
             torch.cuda.synchronize()
-            t0 = time.perf_counter()
-            mk.launch()
-            mk.launch()
-            torch.cuda.synchronize()
-            best[path] = min(best.get(path, 1.0), time.perf_counter() - t0)
+            spent = 0.0
+            for seqs in tables:
+                kept.append((seqs, mk.bind_sequences(w, toks[:seqs.batch], seqs, append=True)))
+                torch.cuda.synchronize()
+                t0 = time.perf_counter()
+                mk.launch()
+                mk.launch()
+                torch.cuda.synchronize()
+                spent += time.perf_counter() - t0
+            best[path] = min(best.get(path, 1.0), spent)
         mk.status()
-    assert best["auto"] <= 1.2 * best["persist"], best
+    assert best["layered"] <= 1.2 * best["one"] and best["auto"] <= 0.9 * best["one"], best
 
 
 def test_prompt_capacity_pays_for_prompts_only():
@@ -555,8 +595,8 @@ def test_rebound_launches_are_stable(oracle, small, path):
 
 @pytest.mark.parametrize("T", [5, 37, 64, 200, 700, 1600])
 def test_prefill_matches_oracle(oracle, small, T):
-    """Products cut in K (5, 37: with the split attention; 64, 200: with the tiled causal one), whole tiles beside the pair kernel (700), the pair
-    kernel for q/k/v, too, with a last token tile that is partly padding (1600)."""
+    """Narrow tiles and slices of K (5, 37: with the split attention; 64, 200: with the tiled causal one), tiles of 128 rows beside the pair kernel (700), the pair
+    kernel for everything, with a last token tile that is partly padding (1600)."""
     from qwen3mk import prefill
 
     shp, inp, w = small
@@ -583,7 +623,7 @@ def test_prefill_matches_oracle(oracle, small, T):
 @pytest.mark.parametrize("T", [4, 63, 65, 128, 129, 256, 257, 385, 512, 513, 640, 769, 897, 1025, 1152, 1153, 1281, 2304, 2305, 2700])
 def test_prompt_products_at_the_edges_of_their_tiles(oracle, small, T):
     """Prompt lengths around the tiles of the prompt's products (128 tokens a block, 256 a pair) and around every change of their form on 148 SMs: the cuts
-    of K, whole tiles, the pair kernel (gate/up from 513 tokens on, q/k/v from 1153, Wo and down from 2305).  On an engine with more
+    of K, narrow and whole tiles, the pair kernel (gate/up from 513 tokens on, q/k/v, Wo and down from 1153).  On an engine with more
     room than the prompt needs, twice: no atomics, so the same bits."""
     from qwen3mk import Megakernel, prefill
 
@@ -725,12 +765,13 @@ def _gate_batch_stream(oracle, w, toks0, kcs, vcs, got, outs, what):
 
 
 @pytest.mark.parametrize("path,batch,ctx,steps", [("layered", 8, 245, 24), ("layered", 1, 1270, 40), ("layered", 5, 24, 60),
-                                                  ("auto", 2, 500, 30), ("auto", 2, 56, 80), ("auto", 3, 250, 30)])
+                                                  ("layered", 2, 500, 30), ("layered", 2, 56, 80), ("auto", 3, 250, 30), ("auto", 2, 500, 30)])
 def test_layered_graph_replay_follows_a_growing_cache(oracle, path, batch, ctx, steps):
     """Chained launches with append and graph replay, across cache lengths where the attention split changes: the padded chunk
     length, which is part of the captured launch arguments, at a fixed split count above one (batch 8 at 256 positions,
     batch 1 at 1280, batch 2 at 512, batch 3 at 256), and the split count itself (batch 2 at 65, 96 and 128, batch 5 at 65).
-    Graphs are captured before and after each.  A replayed graph must not keep the shorter chunk."""
+    Graphs are captured before and after each.  A replayed graph must not keep the shorter chunk.  ("auto": three sequences run in the persistent kernel before a
+    graph is captured, after every change of the split again; two always do.)"""
     from qwen3mk.kernel import SeqTable
 
     shp = oracle.Shape(layers=2, vocab=2048)
@@ -777,10 +818,10 @@ def test_a_vocabulary_that_is_no_multiple_of_the_tile(oracle, batch):
         gate_step(oracle, {k: out[k][b] for k in out}, ref, f"seq {b} len {lens[b]}")
 
 
-@pytest.mark.parametrize("lens", [[32767], [32768], [33001, 40], [32900, 5, 700, 1, 64]])
+@pytest.mark.parametrize("lens", [[30000], [30001], [29999, 3], [20000, 19000], [30001, 7], [32767], [32768], [33001, 40], [32900, 5, 700, 1, 64]])
 def test_caches_longer_than_a_cluster_of_splits(oracle, lens):
-    """A split takes at most 4096 positions and a cluster eight splits: from 32768 cached positions on, partials in memory and a
-    merge launch."""
+    """One and two sequences of up to 30000 positions are one launch of the persistent kernel, beyond it the chain.  A split takes at most 4096
+    positions and a cluster eight splits: from 32768 cached positions on, partials in memory and a merge launch."""
     from qwen3mk.kernel import SeqTable
 
     shp = oracle.Shape(layers=1, vocab=512)
@@ -795,7 +836,7 @@ def test_caches_longer_than_a_cluster_of_splits(oracle, lens):
     mk.launch()
     mk.status()
     # one layer: embedding, four products, the attention (and its merge), LM head, arg-max
-    assert mk.launch_count - before == (9 if max(lens) >= 32768 else 8)
+    assert mk.launch_count - before == (9 if max(lens) >= 32768 else 8 if max(lens) > 30000 else 1)
     for b, ref in enumerate(oracle.decode_batch(oracle.to_fp32(inp), toks.tolist(), kcs, vcs)):
         gate_step(oracle, {k: out[k][b] for k in out}, ref, f"seq {b} len {lens[b]}")
 
