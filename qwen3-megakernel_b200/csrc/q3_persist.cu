@@ -1380,18 +1380,20 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
             }
             cta_sync();
             // fn <= 116: the slice joins the attention delta (of every rank); four warps a sequence
+            float wo_v = 0.f;
+            auto wo_add = [&](int b, int r, unsigned long long w) {
+                if (TP) { for (int t = 0; t < T; ++t) acc_add<true>(p.tp_dA[t] + (size_t)(l & 1) * HIDDEN + fr0 + r, w); }
+                else acc_add<false>(dAl + b * HIDDEN + fr0 + r, w);
+            };
             if ((tid & 127) < fn && (tid >> 7) < NB) {
                 const int b = tid >> 7, r = tid & 127;
-                const float v = wo_part[b * 256 + r] + wo_part[b * 256 + 128 + r];
-                auto add = [&](unsigned long long w) {
-                    if (TP) { for (int t = 0; t < T; ++t) acc_add<true>(p.tp_dA[t] + (size_t)(l & 1) * HIDDEN + fr0 + r, w); }
-                    else acc_add<false>(dAl + b * HIDDEN + fr0 + r, w);
-                };
-                if (fabsf(v) <= ACC_LIMIT) add(acc_word(v));     // (two adds, and the readers' test behind the one that fails, cost nothing; one behind the test 1 to 5 us a step)
-                else {
-                    for (int t = 0; t < T; ++t) acc_keep_apart<TP>(acc_apart((TP ? p.tp_dA[t] + (size_t)(l & 1) * HIDDEN : dAl + b * HIDDEN) + fr0 + r, TP ? fh : blockIdx.x % Q_HEADS, NB), tag, v);
-                    add(ACC_ONE + ACC_APART);
-                }
+                wo_v = wo_part[b * 256 + r] + wo_part[b * 256 + 128 + r];
+                if (fabsf(wo_v) <= ACC_LIMIT) wo_add(b, r, acc_word(wo_v));
+            }
+            if (!(fabsf(wo_v) <= ACC_LIMIT)) {       // (behind the add that everyone waits for; in its other branch 255 positions 380 us a step instead of 372)
+                const int b = tid >> 7, r = tid & 127;
+                for (int t = 0; t < T; ++t) acc_keep_apart<TP>(acc_apart((TP ? p.tp_dA[t] + (size_t)(l & 1) * HIDDEN : dAl + b * HIDDEN) + fr0 + r, TP ? fh : blockIdx.x % Q_HEADS, NB), tag, wo_v);
+                wo_add(b, r, ACC_ONE + ACC_APART);
             }
         }   // (wo_part is the next phase's staging area: the wait below passes a CTA barrier before anything is staged)
         Q3_TRACE(ev + 6);
