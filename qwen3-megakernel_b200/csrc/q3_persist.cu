@@ -25,8 +25,8 @@
 //
 // Weights never wait for a barrier, and a barrier never waits behind weights.  Each CTA's rows of the seven
 // matrices of a layer are packed once (pack_weights_kernel) in the order and with the row padding of four
-// shared-memory slots; one thread fetches a whole slot with TMA bulk copies at the START of the phase before the
-// one that reads it, so that the copies have landed when the phase's barrier is polled.  The matrix-vector
+// shared-memory slots; one thread fetches a whole slot with TMA bulk copies a phase or so before it is read (the schedule
+// stands at the copies below), so that they have landed when the phase's barrier is polled.  The matrix-vector
 // products run on the tensor cores (mma.sync m16n8k16) with the fp32 activation vector split into three bf16
 // columns, which is exact to fp32 and needs no warp-shuffle reductions.
 //
@@ -60,11 +60,11 @@ constexpr int PERSIST_MAX_BATCH = 3;          // sequences a launch decodes
 constexpr int MIN_GRID = 147;                 // row shares must fit the shared-memory slots
 constexpr int SC_FLOATS = 344;                // the score buffer of the local attention, which serves up to 255 positions
 // Most cached positions this kernel is picked for: the longest at which it was timed against the launch chain (one sequence, us per step, this
-// kernel / the chain: 5000 positions 513 / 768, 16000 826 / 1268, 29999 1183 / 1881).
+// kernel / the chain replayed: 5000 positions 512 / 751, 16000 771 / 1254, 29999 1096 / 1872).
 constexpr int PERSIST_MAX_LEN = 30000;
-// Two sequences at 16 / 1500 / 8000 / 29000 positions 488 / 575 / 895 / 1930 us against 573 / 657 / 987 / 2029.  Three at 16 / 600 / 1300 / 2000
-// 599 / 632 / 679 / 733 (24 columns are three MMAs a tile, and the registers of a pass do not all fit: 164 bytes of spills) against 624 / 668 /
-// 697 / 729 in plain launches and 576 / 626 / 654 / 685 from a graph: in place of plain launches, up to
+// Two sequences at 16 / 1500 / 8000 / 29000 positions each, 29000 and 16: 487 / 572 / 889 / 1909 / 1247 us against 564 / 630 / 963 / 1989 / 1783.  Three at 16 / 600 /
+// 1300 / 1500 / 2000 596 / 629 / 678 / 690 / 731 (nine columns are two MMA tiles, the second half empty, and the registers of a pass do not all fit: 164 bytes
+// of spills) against 612 / 662 / 684 / 689 / 715 in plain launches and 567 / 618 / 645 / 650 / 676 from a graph: in place of plain launches, up to
 constexpr int PERSIST_THREE_LEN = 1500;
 // ... and that a caller may ask for who names this kernel.  Such a request is answered by this kernel or refused, and a caller may go by the refusal: what
 // was refused stays refused.
@@ -416,7 +416,7 @@ __device__ __forceinline__ int local_v_pos(int w, int i) { return w + CW * i; }
 //   1  local attention, up to 191 cached positions (a third K pass and four more V rows in 16 more registers)
 //   2  local attention, up to 255 cached positions (a fourth K pass and another four V rows)
 //   3  split attention, up to PERSIST_MAX_LEN cached positions
-// (measured per step at 192 / 255 / 319 / 383 positions: local 392 / 417 / 475 / 511 us, split 450 us throughout, 415 since).
+// (measured per step at 192 / 255 / 319 / 383 positions: local 392 / 417 / 475 / 511 us, split 450 us throughout; now 370 / 372 local and 398 split).
 // The host picks the variant from its upper bound of the length; a cache longer than the variant serves is reported.
 constexpr int N_MODES = 4;
 __host__ __device__ constexpr int mode_max_len(int mode) { return mode == 0 ? 128 : mode < N_MODES - 1 ? 127 + 64 * mode : PERSIST_MAX_LEN; }
@@ -667,10 +667,13 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
     // the phase ends and nothing is in flight while a grid barrier is polled: measured on B200, a barrier polled
     // while 64 KB per SM of bulk copies are in flight takes 2.1 to 2.6 us instead of 1.55 us (the poll's answer
     // queues behind the copies), and cp.async (LDGSTS) copies in flight slow the other warps' own accesses.
-    //   start of Q  (layer l): down rows of layer l         (43 KB, read in GD)
-    //   start of F  (layer l): gate/up rows of layer l      (87 KB, read in GD)
-    //   start of GD (layer l): q/k/v rows and Wo slice of layer l + 1   (58 + 31 KB)
-    // The first chunk of a slot arms the slot's mbarrier with the slot's byte count; every warp waits on it before it reads the slot.
+    //   slot  rows of layer l          fetched at                                                     staged in it meanwhile
+    //   0     q/k/v (58 KB, Q)         the start of GD of layer l - 1                                 F: split attention's outputs, maxima, sums; several sequences: the
+    //                                                                                                 heads' outputs as well, and the LM head's input
+    //   1     Wo slice (31 KB, F)      the start of GD of layer l - 1; several: of Q of layer l       several sequences, GD: activations, row sums, down outputs
+    //   2     gate/up (87 KB, GD)      behind Q's products, or behind the q/k/v exchange (rows_late)  several sequences, Q: activations
+    //   3     down (43 KB, GD)         the start of Q                                                 -
+    // What is staged in a slot is dead, behind a CTA barrier, before the slot is fetched again.  The first chunk of a slot arms the slot's mbarrier with the slot's byte count; every warp waits on it before it reads the slot.
     const int bytesA = qmax * WROW * 2, bytesB = WO_ROWS_MAX * WOROW * 2, bytesC = 2 * imax * WROW * 2, bytesD = imax * WROW * 2;
     const bool pumper = tid == 32;
     constexpr int FEW_ROWS = 16;                        // (kept among them: a flag of its own is a register too many)
@@ -1149,10 +1152,10 @@ __global__ void __launch_bounds__(PT, 1) q3_persist_decode(const PersistParams p
             } else {
                 // ---- this CTA's cached positions, both heads, in one pass over K and V: half a warp per position, eight dims of its two rows
                 //      a lane.  Either half keeps a running maximum and sum of its own, so that nothing crosses them until the end.  All
-                //      sixteen warps attend, the first four passes (128 positions) were requested in Q, and a pass that has been consumed
-                //      makes room for the one four further: 64 KB in flight per SM.  Bound by the rows' bytes beyond about 2300 positions (27 ns
-                //      a position and step, 4.3 TB/s), by the layer's exchanges below.  us per step, with eight warps, scores in shared memory and
-                //      rows beyond the first 64 fetched as they are needed -> now: 1000 positions 455 -> 443, 2200 563 -> 466, 3438 673 -> 498.
+                //      sixteen warps attend, the first PASSES passes (128 positions; 96 of several sequences) were requested in Q, and a pass that has been
+                //      consumed makes room for the one PASSES further: 64 or 48 KB in flight per SM.  Bound by the rows' bytes beyond about 2300 positions (23 ns
+                //      a position and step, 5.0 TB/s), by the layer's exchanges below.  us per step, with eight warps, scores in shared memory and rows beyond the
+                //      first 64 fetched as they are needed -> so: 1000 positions 455 -> 443, 2200 563 -> 466, 3438 673 -> 498 (with what came later, 403, 432 and 477).
                 //      (Rows asked into L2 a layer ahead: 555 instead of 542 at 5000.) ----
                 if (warp == 12 || (MANY && warp == 13)) {   // the new row's score for this CTA's own head (several sequences: for both), q . k_new in fp32, unrounded
                     const float4 a = *reinterpret_cast<const float4*>(q_s + (MANY ? warp - 12 : fhh) * 128 + lane * 4);
