@@ -1850,7 +1850,8 @@ bool persist_supports(const q3_engine* e, const q3_decode_args* a) {
 }
 
 // (Re)pack the layer matrices when one of the caller's pointers changes.  Runs on the legacy default
-// stream and synchronises: weights change rarely, and later launches may use any stream.  The pack
+// stream and waits for the device before (the weights may still be written, the old copy still read, on any stream)
+// and after (later launches may use any stream): weights change rarely.  The pack
 // is keyed on the pointers: a caller that rewrites weights in place must call q3_set_weights with
 // `Q3_W_REPACK` semantics, i.e. after q3_invalidate_weights.
 int persist_weights_changed(q3_engine* e) {
@@ -1861,10 +1862,12 @@ int persist_weights_changed(q3_engine* e) {
     for (int i = 0; i < 7; ++i) same = same && (s->src[i] == now[i]);
     if (same) return Q3_OK;
     auto bf = [](const void* p) { return reinterpret_cast<const bf16_raw*>(p); };
+    cudaError_t err = cudaDeviceSynchronize();
+    if (err != cudaSuccess) return engine_fail(e, Q3_ERR_CUDA, "persist: waiting for the device before packing the weights failed: %s", cudaGetErrorString(err));
     PackArgs a{bf(now[0]), bf(now[1]), bf(now[2]), bf(now[3]), bf(now[4]), bf(now[5]), bf(now[6]), s->packed, s->tp_size, s->tp_rank};
     pack_weights_kernel<<<dim3(s->grid, e->cfg.n_layers), 256>>>(a);
     ++e->launches;
-    cudaError_t err = cudaDeviceSynchronize();
+    err = cudaDeviceSynchronize();
     if (err != cudaSuccess) return engine_fail(e, Q3_ERR_CUDA, "persist: packing the weights failed: %s", cudaGetErrorString(err));
     for (int i = 0; i < 7; ++i) s->src[i] = now[i];
     return Q3_OK;

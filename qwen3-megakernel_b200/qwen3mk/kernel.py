@@ -17,6 +17,7 @@ it is given and never writes to an input (the caches are written only when `appe
 from __future__ import annotations
 
 import ctypes
+from operator import attrgetter
 
 import torch
 
@@ -25,6 +26,8 @@ from . import _cabi
 INPUT_ORDER = ("token", "ln1", "wq", "wk", "wv", "qn", "kn", "wo", "ln2",
                "wg", "wu", "wd", "fnorm", "embed", "kcache", "vcache")
 WEIGHT_ORDER = _cabi.WEIGHT_FIELDS
+_VERSION = attrgetter("_version")      # PyTorch counts every in-place write
+_PACKED_PATHS = (_cabi.F_PATH_AUTO, _cabi.F_PATH_PERSIST)
 
 LAYERS, HIDDEN, Q_HEADS, KV_HEADS, HEAD_DIM, INTER, VOCAB, CONTEXT = 28, 1024, 16, 8, 128, 3072, 151936, 128
 ROPE_THETA = 1e6
@@ -212,6 +215,7 @@ class Megakernel:
         _cabi.check(self.lib, self.handle, self.lib.q3_set_weights(self.handle, ctypes.byref(w)), "q3_set_weights")
         self._weights_key = key
         self._weights_ref = tensors
+        self._weights_versions = tuple(map(_VERSION, tensors))
 
     def refresh_weights(self) -> None:
         """Forget the engine's packed copy of the layer matrices.  Only needed after a write that PyTorch's version
@@ -355,10 +359,14 @@ class Megakernel:
         return t[0] if t.numel() == 1 else t
 
     def launch(self, stream=None) -> None:
-        """Enqueue one decode step on the bound inputs.  No host sync.  `stream` is a CUDA stream handle (int)."""
+        """Enqueue one decode step on the bound inputs.  No host sync, unless up to three sequences' weights were written in place since the last launch
+        (the engine then packs them anew, which waits for the device).  `stream` is a CUDA stream handle (int)."""
         if self._bound is None:
             raise RuntimeError("call bind(inputs) before launch()")
         a = self._args
+        # the persistent kernel reads a packed copy: weights that were written in place since have to reach it (about 1 us; the chain reads the caller's)
+        if a.batch <= 3 and self._path_flag in _PACKED_PATHS and (self._weights_key is None or tuple(map(_VERSION, self._weights_ref)) != self._weights_versions):
+            self._set_weights(self._bound[0])
         if self._append:
             if self._n_launch >= self._max_launches:
                 raise RuntimeError("launch(): the bound caches are full")

@@ -909,3 +909,36 @@ def test_in_place_weight_update_is_noticed(oracle, small):
     w2 = dict(w, wq=dev["wq"].float().cpu())
     ref = oracle.decode_step(w2, inp["token"], inp["kcache"], inp["vcache"])
     gate_step(oracle, out, ref, "after wq.mul_(0.5)")
+
+
+@pytest.mark.parametrize("path,lens", [("auto", (40,)), ("auto", (3600,)), ("auto", (40, 9)), ("auto", (40, 9, 300)), ("layered", (40, 9)), ("auto", (5, 6, 7, 8))])
+def test_in_place_weight_update_between_launches_is_noticed(oracle, small, path, lens):
+    """A bound engine decodes with the weights as they are when a launch is enqueued, also where it streams a packed copy: after a write on the launch's own
+    stream, behind work that is still running there, and after one that only refresh_weights() tells of."""
+    from qwen3mk.kernel import SeqTable
+
+    shp, inp, w = small
+    dev = {k: v.clone() for k, v in to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}).items()}
+    g = torch.Generator().manual_seed(len(lens))
+    toks = torch.randint(0, 4096, (len(lens),), generator=g)
+    kcs, vcs = ([torch.randn(2, n, 8, 128, generator=g).to(torch.bfloat16) for n in lens] for _ in range(2))
+    mk = engine(path, layers=2, vocab=4096, max_batch=len(lens))
+    out = mk.bind_sequences(dev, toks.cuda(), SeqTable([k.cuda() for k in kcs], [v.cuda() for v in vcs]))
+    for _ in range(2 if len(lens) == 3 else 12):  # (past the capture of a graph; three sequences: before it)
+        mk.launch()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)
+        dev["wq"].mul_(0.5)
+        dev["wd"].mul_(0.5)
+    mk.launch(side.cuda_stream)
+    mk.status(side.cuda_stream)
+    for _ in range(2):
+        w2 = dict(w, wq=dev["wq"].float().cpu(), wd=dev["wd"].float().cpu())
+        for b, ref in enumerate(oracle.decode_batch(w2, toks.tolist(), kcs, vcs)):
+            gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{path} {lens} seq {b}")
+        dev["wd"].data.mul_(2)                    # (.data: the counter does not move)
+        mk.refresh_weights()
+        mk.launch()
+        mk.status()
