@@ -25,7 +25,7 @@
 // T <= 0 or k == 1 degenerate to the arg-max (ties -> lowest index), like the decode kernels.
 //
 // A single row is bound by latency (0.6 MB, but a dozen dependent block-wide steps), a full batch by the row's bytes and the same steps.
-// Measured, us: 1 row, k = 50: 11.6 on logits that no cache has seen (12.1 before a warp took its largest value in one instruction; the same logits again 10.3 and 12.3); 15 / 36 / 64 rows, whole vocabulary: 12.6 / 18.9 / 18.6 (before a run's last loads left together, four words a thread
+// Measured, us: 1 row, k = 50: 10.8 to 11.6 from box to box on changing logits (11.4 to 12.2 before a warp took its largest value in one instruction); 15 / 36 / 64 rows, whole vocabulary: 12.6 / 18.9 / 18.6 (before a run's last loads left together, four words a thread
 // in the walk, and up to 64 rows the next loads under way behind the ones at work: 13.8 / 20.7 / 20.7); 15 / 36 / 64 rows, k = 50: 15.1 / 18.7 / 18.7 (before
 // lanes shared the second look at the row: 16.6 / 22.8 / 24.8).
 #include <cooperative_groups.h>
