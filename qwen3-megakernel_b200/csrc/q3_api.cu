@@ -544,10 +544,17 @@ extern "C" int q3_decode(q3_engine* e, const q3_decode_args* a, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     uint32_t path = a->flags & Q3_F_PATH_MASK;
     // One launch of the persistent kernel for one or two sequences, a chain of launches for more; three take the kernel as long as the chain would
-    // be plain launches (the times stand at q3_persist.cu's limits).
+    // be plain launches (the times stand at q3_persist.cu's limits).  What a caller captures is replayed without this code: only the chain sees weights that are
+    // written in place between two replays, and serves lengths that grow within its split, so it has the captured launches but for those of one sequence up
+    // to the length that always was the kernel's.
     bool until_captured = false;
     if (path == Q3_F_PATH_AUTO) {
         path = persist_supports(e, a) ? Q3_F_PATH_PERSIST : Q3_F_PATH_LAYERED;
+        if (path == Q3_F_PATH_PERSIST && !persist_serves_replays(a)) {
+            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+            CU(e, cudaStreamIsCapturing(st, &capture));
+            if (capture != cudaStreamCaptureStatusNone) path = Q3_F_PATH_LAYERED;
+        }
         until_captured = path == Q3_F_PATH_PERSIST && a->batch == 3 && (a->flags & Q3_F_GRAPH);
         if (until_captured) path = Q3_F_PATH_LAYERED;
     }

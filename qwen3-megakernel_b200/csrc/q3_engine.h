@@ -61,6 +61,7 @@ namespace q3 {
 int persist_setup(q3_engine* e);
 void persist_teardown(q3_engine* e);
 bool persist_supports(const q3_engine* e, const q3_decode_args* a);
+bool persist_serves_replays(const q3_decode_args* a);
 int persist_decode(q3_engine* e, const q3_decode_args* a, cudaStream_t st);
 int persist_weights_changed(q3_engine* e);
 void persist_invalidate_weights(q3_engine* e);

@@ -1849,6 +1849,9 @@ bool persist_supports(const q3_engine* e, const q3_decode_args* a) {
     return a->batch <= PERSIST_MAX_BATCH && a->max_len <= (asked ? PERSIST_ASKED_LEN : a->batch == 3 ? PERSIST_THREE_LEN : PERSIST_MAX_LEN);
 }
 
+// Whether a launch that a caller captures is this kernel's (q3_decode says why the others are not).
+bool persist_serves_replays(const q3_decode_args* a) { return a->batch == 1 && a->max_len <= PERSIST_ASKED_LEN; }
+
 // (Re)pack the layer matrices when one of the caller's pointers changes.  Runs on the legacy default
 // stream and waits for the device before (the weights may still be written, the old copy still read, on any stream)
 // and after (later launches may use any stream): weights change rarely.  The pack

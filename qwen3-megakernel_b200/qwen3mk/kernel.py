@@ -366,7 +366,8 @@ class Megakernel:
         a = self._args
         # the persistent kernel reads a packed copy: weights that were written in place since have to reach it (about 1 us; the chain reads the caller's)
         if a.batch <= 3 and self._path_flag in _PACKED_PATHS and (self._weights_key is None or tuple(map(_VERSION, self._weights_ref)) != self._weights_versions):
-            self._set_weights(self._bound[0])
+            if not torch.cuda.is_current_stream_capturing():     # (packing waits for the device, which a capture does not allow)
+                self._set_weights(self._bound[0])
         if self._append:
             if self._n_launch >= self._max_launches:
                 raise RuntimeError("launch(): the bound caches are full")

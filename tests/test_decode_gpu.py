@@ -904,11 +904,12 @@ def test_in_place_weight_update_is_noticed(oracle, small):
     dev = to_dev(inp)
     mk.step(dev)
     dev["wq"].mul_(0.5)
+    dev["wd"].mul_(0.5)                # (the head norm hides a factor on wq)
     out = mk.step(dev)
     mk.status()
-    w2 = dict(w, wq=dev["wq"].float().cpu())
+    w2 = dict(w, wq=dev["wq"].float().cpu(), wd=dev["wd"].float().cpu())
     ref = oracle.decode_step(w2, inp["token"], inp["kcache"], inp["vcache"])
-    gate_step(oracle, out, ref, "after wq.mul_(0.5)")
+    gate_step(oracle, out, ref, "after wq.mul_(0.5) and wd.mul_(0.5)")
 
 
 @pytest.mark.parametrize("path,lens", [("auto", (40,)), ("auto", (3600,)), ("auto", (40, 9)), ("auto", (40, 9, 300)), ("layered", (40, 9)), ("auto", (5, 6, 7, 8))])
@@ -942,3 +943,43 @@ def test_in_place_weight_update_between_launches_is_noticed(oracle, small, path,
         mk.refresh_weights()
         mk.launch()
         mk.status()
+
+
+@pytest.mark.parametrize("lens", [(3600,), (40, 9), (16, 70, 90)])
+@pytest.mark.parametrize("inside", [True, False])
+def test_a_captured_step_follows_weights_and_lengths(oracle, small, lens, inside):
+    """A caller's graph of an appending step, replayed while weights are written in place, by the graph itself or between its replays, and the caches grow by
+    less than the split the step was captured with reaches: the launch chain's, which reads the caller's tensors."""
+    from qwen3mk.kernel import SeqTable
+
+    shp, inp, w = small
+    dev = {k: v.clone() for k, v in to_dev({k: inp[k] for k in oracle.WEIGHT_NAMES}).items()}
+    g = torch.Generator().manual_seed(len(lens))
+    toks = torch.randint(0, 4096, (len(lens),), generator=g)
+    kcs, vcs = ([torch.randn(2, n + 6, 8, 128, generator=g).to(torch.bfloat16).cuda() for n in lens] for _ in range(2))
+    mk = engine("auto", layers=2, vocab=4096, max_batch=len(lens))
+    out = mk.bind_sequences(dev, toks.cuda(), SeqTable(kcs, vcs, list(lens)), append=True, graph=False)
+    mk.launch()
+    mk.status()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        if inside:
+            dev["wd"].mul_(0.5)
+        mk.launch()
+    for i in range(1, 4):
+        if not inside:
+            dev["wd"].mul_(0.5)
+        graph.replay()
+        mk.status()
+        refs = oracle.decode_batch(dict(w, wd=dev["wd"].float().cpu()), toks.tolist(), [k[:, :n + i].cpu() for k, n in zip(kcs, lens)], [v[:, :n + i].cpu() for v, n in zip(vcs, lens)])
+        for b, ref in enumerate(refs):
+            gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{lens} seq {b}, replay {i}")
+    mk.refresh_weights()                          # (what a graph writes moves no counter)
+    out = mk.bind_sequences(dev, toks.cuda(), SeqTable(kcs, vcs, [n + 4 for n in lens]), graph=False)
+    before = mk.launch_count
+    mk.launch()
+    mk.status()
+    assert mk.launch_count == before + 1
+    refs = oracle.decode_batch(dict(w, wd=dev["wd"].float().cpu()), toks.tolist(), [k[:, :n + 4].cpu() for k, n in zip(kcs, lens)], [v[:, :n + 4].cpu() for v, n in zip(vcs, lens)])
+    for b, ref in enumerate(refs):
+        gate_step(oracle, {k: out[k][b] for k in out}, ref, f"{lens} seq {b}, after the graph")
